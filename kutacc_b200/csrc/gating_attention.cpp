@@ -255,7 +255,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
             wait_for_pair_bias();
             if (ok && v_key_major)
                 ok = dev::tcgen05_attn_core_bf16(stream, q_c, k_c, v_km, s_pad8, g_c, bias_c, bias_s0, nb_dev, nb_sh,
-                                                 nb_sq, a_c, (int)nbr, (int)S, (int)H, (int)D, scale, /*gate_is_sigmoid=*/true);
+                                                 nb_sq, a_c, (int)nbr, (int)S, (int)H, (int)D, scale);
             else
                 ok = ok && dev::launch_attn_core_bf16(stream, q_c, k_c, v_c, g_c, bias_c, bias_s0, nb_dev, nb_sh, nb_sq,
                                                       a_c, (int)nbr, (int)S, (int)H, (int)D, scale);

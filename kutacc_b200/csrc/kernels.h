@@ -23,7 +23,7 @@ bool launch_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, c
 bool launch_linear_bias_bf16(cudaStream_t stream, const void *a, int64_t lda, const void *w, const float *bias,
                              void *out, int64_t ldo, int64_t M, int N, int K);
 
-// tcgen05/TMEM/TMA versions of the two GEMMs above (C % 128 == 0, D in {32, 64}; N % 128 == 0,
+// tcgen05/TMEM/TMA versions of the two GEMMs above (C % 128 == 0 or C == 64, D in {8, 16, 32, 64}; N % 128 == 0 or N == 64,
 // K % 64 == 0, out row stride % 8 == 0). q is written unscaled. With v_transposed, v is written as
 // [B, H, D, S] with row pitch v_pitch (what the tcgen05 attention core consumes) instead of [B, H, S, D].
 // Return false when the shape is not covered.
@@ -87,14 +87,13 @@ bool launch_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, co
                            const void *bias, int64_t bias_stride0, const void *nb, int64_t nb_stride_h,
                            int64_t nb_stride_q, void *avg, int B, int S, int H, int D, float scale);
 
-// The same operator with both products on tcgen05 and the accumulators in tensor memory (head size 32).
-// vt is v transposed, [B, H, D, S] with row pitch vt_pitch, as tcgen05_proj_qkvg_bf16 writes it. With
-// gate_is_sigmoid, `gate` already holds bf16(sigmoid(bf16(x.Wg + bg))) (the projection kernel's gate_sigmoid
-// option) and the kernel only multiplies.
+// The same operator with both products on tcgen05 and the accumulators in tensor memory (head sizes 8, 16, 32).
+// vt is v transposed, [B, H, D, S] with row pitch vt_pitch, as tcgen05_proj_qkvg_bf16 writes it; `gate` already holds
+// bf16(sigmoid(bf16(x.Wg + bg))) (the projection kernel's gate_sigmoid option): the kernel only multiplies.
 bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch,
                             const void *gate, const void *bias, int64_t bias_stride0, const void *nb,
                             int64_t nb_stride_h, int64_t nb_stride_q, void *avg, int B, int S, int H, int D,
-                            float scale, bool gate_is_sigmoid);
+                            float scale);
 
 // ---- generic (any shape, bf16 or fp32 storage, fp32 math) ------------------------------------------
 // c[m, n] = sum_k a[m, k] * w[n, k] (+ bias[n]) (+ beta * c[m, n]); a row stride lda, w row stride

@@ -9,6 +9,21 @@ namespace dev {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// one lane of the (converged) warp. Operands of the tcgen05 and TMA instructions behind this predicate can stay in uniform
+// registers; behind `lane == 0` each of them is moved there lane by lane.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(r));
+    return r != 0;
+}
+
 // 16-byte asynchronous global->shared copy; src_bytes < 16 zero-fills the tail (0 = all zeros).
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int src_bytes)
 {

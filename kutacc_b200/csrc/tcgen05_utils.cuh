@@ -38,6 +38,19 @@ __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, ui
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// the same with A in tensor memory: row r of A in lane r, two consecutive bf16 k per 32-bit column
+__device__ __forceinline__ void tc_mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // this warp's 32 lanes x 32 consecutive fp32 columns
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
 {
@@ -53,6 +66,31 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+// 32 lanes x 16 consecutive columns
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// wait for the loads in flight; the registers pass through, so that no use of them can move ahead of the wait
+__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
+}
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 
 // 32 lanes x 64 consecutive fp32 columns
 __device__ __forceinline__ void tmem_ld_32x64(uint32_t taddr, uint32_t (&r)[64])
@@ -98,7 +136,7 @@ __device__ __forceinline__ void tmem_st_32x1(uint32_t taddr, uint32_t v)
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-// Shared-memory matrix descriptor of a K-major operand whose rows are `swizzle_bytes` wide (64 or 128) and
+// Shared-memory matrix descriptor of a K-major operand whose rows are `swizzle_bytes` wide (32, 64 or 128) and
 // stored with the matching TMA swizzle: 8-row groups are 8*swizzle_bytes apart. `addr` is the byte address
 // of the (1024-aligned) tile plus the K offset inside the swizzle atom.
 __device__ __forceinline__ uint64_t make_smem_desc_kmajor(uint32_t addr, int swizzle_bytes)
@@ -108,7 +146,7 @@ __device__ __forceinline__ uint64_t make_smem_desc_kmajor(uint32_t addr, int swi
     d |= (uint64_t)1 << 16;                                        // leading byte offset (unused here)
     d |= (uint64_t)((8 * swizzle_bytes) >> 4) << 32;               // stride byte offset between 8-row groups
     d |= (uint64_t)1 << 46;                                        // descriptor version of sm_100
-    d |= (uint64_t)(swizzle_bytes == 128 ? 2 : 4) << 61;           // 2 = 128-byte swizzle, 4 = 64-byte swizzle
+    d |= (uint64_t)(swizzle_bytes == 128 ? 2 : swizzle_bytes == 64 ? 4 : 6) << 61;   // 128-, 64-, 32-byte swizzle
     return d;
 }
 // instruction descriptor: D fp32, A and B bf16, both K-major

@@ -16,6 +16,11 @@ bool make_tensor_map_bf16_3d(CUtensorMap *map, const void *base, uint64_t d0, ui
                              uint64_t stride1, uint64_t stride2, uint32_t box0, uint32_t box1, int swizzle_bytes,
                              uint32_t box2 = 1);
 
+// rank-4 bf16 tensor [d3][d2][d1][d0], strides in ELEMENTS for d1..d3, box [box3][1][box1][box0]
+bool make_tensor_map_bf16_4d(CUtensorMap *map, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
+                             uint64_t stride1, uint64_t stride2, uint64_t stride3, uint32_t box0, uint32_t box1, uint32_t box3,
+                             int swizzle_bytes);
+
 // rank-2 tensor [d1][d0] of 2-byte (bf16) or 4-byte (fp32, raw bits) elements, row stride in ELEMENTS, box [box1][box0]
 bool make_tensor_map_2d(CUtensorMap *map, const void *base, int elem_bytes, uint64_t d0, uint64_t d1, uint64_t stride1,
                         uint32_t box0, uint32_t box1, int swizzle_bytes);
@@ -94,9 +99,23 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, i
     }
     return true;
 }
+// The plain test lets the hardware hold the warp until the phase completes or a short time is up. (With the suspend-time
+// hint the compiler adds a sleep of its own and re-tests, which woke late and cost the attention kernel, whose waiting warps
+// share schedulers with working ones, about ten issue slots per test; the clock is read once per 64 tests for the
+// same reason.)
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int *err, int code)
 {
-    return mbar_wait_limit(bar, parity, err, code, 4000000000LL);  // ~2 s at 1.9 GHz
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 64; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
+        if (clock64() - t0 > 4000000000LL) {       // ~2 s at 1.9 GHz
+            if (err) atomicCAS(err, 0, code);
+            return false;
+        }
+    }
 }
 
 // The same wait for a whole warp. Lanes can leave the polling loop at different iterations; the vote at
@@ -184,6 +203,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1)

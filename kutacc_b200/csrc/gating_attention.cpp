@@ -158,7 +158,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
 
     const float scale = (float)(1 / std::sqrt((double)head_size));  // gating_attention.cpp:68
 
-    const bool fast = dt == kBF16 && (C % 64 == 0) && (D == 16 || D == 32 || D == 64) && B <= 65535 && H <= 65535 &&
+    const bool fast = dt == kBF16 && (C % 64 == 0) && ((D == 8 && (C % 128 == 0 || C == 64)) || D == 16 || D == 32 || D == 64) && B <= 65535 && H <= 65535 &&
                       aligned16(d_x.dev) && aligned16(d_wq.dev) && aligned16(d_wk.dev) && aligned16(d_wv.dev) &&
                       aligned16(d_wg.dev) && aligned16(d_wo.dev) && (out_rs % 2 == 0) &&
                       (((uintptr_t)d_out.dev & 3u) == 0);
@@ -190,9 +190,9 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         nb_sh = S * s_pad8;
     }
 
-    // LayerNorm in front: folded into the tcgen05 projection where that kernel runs (head size 32), otherwise the
+    // LayerNorm in front: folded into the tcgen05 projection where that kernel runs (head sizes up to 32), otherwise the
     // rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy
-    const bool ln_folded = ln && fast && D == 32 && C % 128 == 0;
+    const bool ln_folded = ln && fast && D <= 32 && (C % 128 == 0 || C == 64);
     if (ln_folded) {
         const void *w_in[4] = {d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev};
         const float *b_in[4] = {nullptr, nullptr, nullptr, (const float *)d_bg.dev};
@@ -226,7 +226,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         const int64_t Mc = nbr * S;
         bool ok;
         if (fast) {
-            // Tensor-memory kernels where the shape allows it (head size 32: projection with v stored
+            // Tensor-memory kernels where the shape allows it (head sizes 8 to 32: projection with v stored
             // key-major plus the tcgen05 attention core), warp-level MMA kernels otherwise.
             char *v_km = wv_ + (size_t)b0 * C * s_pad8 * es;                   // key-major v: [B, H, D, s_pad8]
             char *v_c = wv_ + b0 * row_bytes;                                  // [B, H, S, D]
@@ -239,7 +239,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
                                                  ln_s, ln_t);
                 if (!ok) return false;
                 v_key_major = true;
-            } else if (D == 32) {
+            } else if (D <= 32) {
                 ok = dev::tcgen05_proj_qkvg_bf16(stream, x_c, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
                                                  (const float *)d_bg.dev, q_c, k_c, v_km, g_c, (int)nbr, (int)S, (int)H,
                                                  (int)D, true, s_pad8, /*gate_sigmoid=*/true);
@@ -417,7 +417,7 @@ extern "C" void kutacc_af2_gating_attention(kutacc_tensor_h input, kutacc_af2_at
 }
 
 // kutacc_af2_gating_attention applied to LayerNorm(input): same arguments plus the LayerNorm's fp32 gamma and beta
-// (nchannels elements each, host or device) and eps. For head size 32 the normalisation is folded into the
+// (nchannels elements each, host or device) and eps. For head sizes up to 32 the normalisation is folded into the
 // projection kernel: the normalised activations are never written to memory.
 extern "C" void kutacc_b200_gating_attention_ln(kutacc_tensor_h input, kutacc_af2_attention_inputs_t *q_based_ptr,
                                                 kutacc_tensor_h bias, kutacc_tensor_h nonbatched_bias,

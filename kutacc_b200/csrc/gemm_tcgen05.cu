@@ -38,7 +38,7 @@ namespace dev {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 64;
+constexpr int BM = 128, BNMAX = 128, BK = 64;
 constexpr int NSTAGE = 2;
 constexpr int ACC_STAGES = 2;
 constexpr int SLAB_BYTES = BM * BK * 2;                 // 16 KB, A and W slabs alike
@@ -46,30 +46,30 @@ constexpr int STAGE_BYTES = 2 * SLAB_BYTES;
 constexpr int EPI_WARPS = 8;                            // two per TMEM lane quarter, 64 columns each
 constexpr int STG_BYTES = 32 * 32 * 2;                  // one 32 x 32 bf16 staging tile
 constexpr int STG_PER_WARP = 2;
-static_assert(STG_PER_WARP == 2, "the epilogue writes its two 32-column halves into staging tiles 0 and 1 of its warp");
+static_assert(STG_PER_WARP == 2, "the epilogue alternates between staging tiles 0 and 1 of its warp");
 constexpr int STG_OFF = NSTAGE * STAGE_BYTES;
 constexpr int BAR_OFF = STG_OFF + EPI_WARPS * STG_PER_WARP * STG_BYTES;
 constexpr int NBARS = 2 * NSTAGE + 2 * ACC_STAGES;
 constexpr int SMEM_BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
-constexpr int TMEM_COLS = ACC_STAGES * BN;              // 256: half of the SM's tensor memory (two CTAs per SM)
+constexpr int TMEM_COLS = ACC_STAGES * BNMAX;              // 256: half of the SM's tensor memory (two CTAs per SM)
 
 struct alignas(64) GemmMaps {
     CUtensorMap a;        // X  [B][S][K], box [64, 128, 1], 128-byte swizzle
-    CUtensorMap w[4];     // W  [1][N_seg][K], box [64, 128, 1], 128-byte swizzle
-    CUtensorMap out[4];   // destination per segment, box [32, 32, 1], 64-byte swizzle
+    CUtensorMap w[4];     // W  [1][N_seg][K], box [64, 128 (segments of 64 channels and 64-wide tiles: 64), 1], 128-byte swizzle
+    CUtensorMap out[4];   // destination per segment, box [32, 32, 1], 64-byte swizzle; head sizes below 32: box [D, 32, 32 / D]
 };
 
 struct GemmParams {
     const float *bias[4];   // per segment, may be null
     int seg_n;              // output channels per segment (multiple of 128)
     int nseg;
+    int pair64;             // segments of 64 channels: a column tile holds two of them
     int head_dim;           // > 0: segment output is [B*H][S][D] (coords d, s, b*H + h); 0: [B][S][N_seg]
     int head_layout_mask;   // bit i set: segment i uses the head layout
-    int transposed_mask;    // bit i set: segment i is stored transposed, [B*H][D][S] (coords s, d, b*H + h)
+    int transposed_mask;    // bit i set: segment i is stored transposed, [B * N_seg][S] (coords s, b * N_seg + n)
     int chanmajor_mask;     // bit i set: segment i is stored transposed and channel-major, [N_seg][B][S] (coords s, b, n)
     int w_batched;          // non-zero: W is [B][N_seg][K], one matrix per batch row (coords k, n, b)
-    int heads;
     int K;
     int S, B;
     int relu;               // non-zero: max(0, .) after the bias, before the bf16 rounding
@@ -94,9 +94,6 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr)
     d |= (uint64_t)2 << 61;                          // 128-byte swizzle
     return d;
 }
-// instruction descriptor: D fp32, A and B bf16, both K-major, N = 128, M = 128
-constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-
 // 1 / (1 + exp(-g)) of the bf16-rounded g as 0.5 * tanh(g / 2) + 0.5: one MUFU operation (relative error about
 // 2^-11, below the bf16 step of the stored result) instead of an exponential and a division
 __device__ __forceinline__ float sigmoid_of_bf16(float y)
@@ -107,9 +104,11 @@ __device__ __forceinline__ float sigmoid_of_bf16(float y)
 
 // Compile-time feature sets, so that each use of the kernel carries only the epilogue code it needs
 // (the sigmoid and the transposed staging cost registers that the plain linear layer would spill).
-constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16;
+// F_HEADS64: head sizes of 8 or 16 and segments of 64 channels, two of them in a column tile.
+constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16, F_HEADS64 = 32;
 
-template <int FEAT>
+// BN: width of a column tile, 128, or 64 for a product with 64 output channels
+template <int FEAT, int BN>
 __global__ void __launch_bounds__(THREADS, 2)
 gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
 {
@@ -122,10 +121,13 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     auto acc_empty = [&](int a) { return bar_base + 8u * (uint32_t)(2 * NSTAGE + ACC_STAGES + a); };
     const uint32_t tmem_slot = bar_base + 8u * NBARS;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int COLS = BN / 2;                        // columns of an epilogue warp
+    constexpr uint32_t instr_desc = make_instr_desc_bf16(BM, BN);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int s_tiles = (p.S + BM - 1) / BM;
     const int n_tiles_seg = (p.seg_n + BN - 1) / BN;    // a ragged last tile is zero-filled on load and clipped on store
-    const int n_tiles = n_tiles_seg * p.nseg;
+    const bool pair64 = (FEAT & F_HEADS64) && p.pair64;
+    const int n_tiles = pair64 ? p.nseg / 2 : n_tiles_seg * p.nseg;
     const int num_tiles = p.B * s_tiles * n_tiles;
     const int nk = (p.K + BK - 1) / BK;                 // columns past K are zero-filled by TMA
     // Tile t covers row tile t / n_tiles and column tile t % n_tiles. A CTA walks t = blockIdx.x + k * gridDim.x, so
@@ -159,10 +161,11 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);          // warp-uniform
 
     if (warp == 0) {
         // ================= producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&maps.a);
             int it = 0;
             bool ok = true;
@@ -170,7 +173,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 int m_tile, n_tile;
                 tile_of(tile, m_tile, n_tile);
                 const int b = m_tile / s_tiles, s0 = (m_tile % s_tiles) * BM;
-                const int seg = n_tile / n_tiles_seg, n0 = (n_tile % n_tiles_seg) * BN;
+                const int seg = pair64 ? 2 * n_tile : n_tile / n_tiles_seg, n0 = pair64 ? 0 : (n_tile % n_tiles_seg) * BN;
                 const CUtensorMap *wmap = &maps.w[seg];
                 for (int kc = 0; kc < nk; ++kc, ++it) {
                     const int s = it % NSTAGE;
@@ -179,9 +182,10 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                         break;
                     }
                     const uint32_t st = smem + (uint32_t)s * STAGE_BYTES;
-                    mbar_arrive_expect_tx(full_bar(s), STAGE_BYTES);
+                    mbar_arrive_expect_tx(full_bar(s), SLAB_BYTES + BN * BK * 2);
                     tma_load_3d(st, &maps.a, full_bar(s), kc * BK, s0, b);
                     tma_load_3d(st + SLAB_BYTES, wmap, full_bar(s), kc * BK, n0, (FEAT & F_WBATCH) ? b : 0);
+                    if (pair64) tma_load_3d(st + SLAB_BYTES + 64 * BK * 2, wmap + 1, full_bar(s), kc * BK, 0, 0);
                 }
             }
         }
@@ -196,7 +200,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 break;
             }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + (uint32_t)(a * BN);
+            const uint32_t d_tmem = tmem_base + (uint32_t)(a * BNMAX);
             for (int kc = 0; kc < nk; ++kc, ++it) {
                 const int s = it % NSTAGE;
                 if (!mbar_wait_warp(full_bar(s), (uint32_t)((it / NSTAGE) & 1), p.err, 13)) {
@@ -204,13 +208,13 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                     break;
                 }
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t st = smem + (uint32_t)s * STAGE_BYTES;
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
                         const uint64_t adesc = make_smem_desc(st + k * 32);
                         const uint64_t bdesc = make_smem_desc(st + SLAB_BYTES + k * 32);
-                        tc_mma_bf16(d_tmem, adesc, bdesc, kInstrDesc, (kc > 0 || k > 0) ? 1u : 0u);
+                        tc_mma_bf16(d_tmem, adesc, bdesc, instr_desc, (kc > 0 || k > 0) ? 1u : 0u);
                     }
                     tc_commit(empty_bar(s));                 // slab may be overwritten once these MMAs retire
                     if (kc == nk - 1) tc_commit(acc_full(a));
@@ -222,7 +226,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
         // ================= epilogue =================
         const int quad = warp & 3;                            // TMEM lanes 32*quad .. 32*quad+31
         const int ew = warp - 2;
-        const int half = ew >> 2;                             // which 64 columns of the 128-column tile
+        const int half = ew >> 2;                             // which half of the tile's columns
         const uint32_t stg0 = smem + STG_OFF + (uint32_t)(ew * STG_PER_WARP) * STG_BYTES;
         int tcount = 0, nstore = 0;
         bool ok = true;
@@ -230,7 +234,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
             int m_tile, n_tile;
             tile_of(tile, m_tile, n_tile);
             const int b = m_tile / s_tiles, s0 = (m_tile % s_tiles) * BM;
-            const int seg = n_tile / n_tiles_seg, n0 = (n_tile % n_tiles_seg) * BN;
+            const int seg = pair64 ? 2 * n_tile + half : n_tile / n_tiles_seg;
+            const int n0 = pair64 ? 0 : (n_tile % n_tiles_seg) * BN + half * COLS;     // this warp's first channel of the segment
             const int a = tcount % ACC_STAGES;
             if (!mbar_wait_warp(acc_full(a), (uint32_t)((tcount / ACC_STAGES) & 1), p.err, 14)) {
                 ok = false;
@@ -253,14 +258,14 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 ln_a = st.y;
                 ln_b = -st.y * st.x;
             }
-            uint32_t r[2][32];
-            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + half * 64);
-            tmem_ld_32x32(tcol, r[0]);
-            tmem_ld_32x32(tcol + 32, r[1]);
+            uint32_t r[COLS / 32][32];
+            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BNMAX + half * COLS);
+#pragma unroll
+            for (int c = 0; c < COLS / 32; ++c) tmem_ld_32x32(tcol + c * 32, r[c]);
             tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const int n = n0 + half * 64 + c * 32;
+            for (int c = 0; c < COLS / 32; ++c) {
+                const int n = n0 + c * 32;
                 uint32_t packed[16];
                 if (bias) {
 #pragma unroll
@@ -310,7 +315,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                     }
                 }
                 // staging tile: row = lane, 64 bytes per row, 16-byte chunks swizzled as the 64-byte TMA mode
-                const uint32_t stg = stg0 + (uint32_t)c * STG_BYTES;
+                const uint32_t stg = stg0 + (uint32_t)(nstore & 1) * STG_BYTES;
                 if (nstore >= STG_PER_WARP) {
                     if (lane == 0) tma_store_wait_read<STG_PER_WARP - 1>();
                     __syncwarp();
@@ -330,12 +335,10 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
-                        if (chanmajor) {
+                        if (chanmajor)
                             tma_store_3d(omap, stg, row0, b, n);
-                        } else {
-                            const int hh = n / p.head_dim, d0 = n - hh * p.head_dim;
-                            tma_store_3d(omap, stg, row0, d0, b * p.heads + hh);
-                        }
+                        else
+                            tma_store_3d(omap, stg, row0, b * p.seg_n + n, 0);
                         tma_store_commit();
                     }
                     ++nstore;
@@ -343,7 +346,11 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 }
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch) {
-                    const uint32_t addr = stg + (uint32_t)(lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4));
+                    // heads of 8 or 16 channels: [head][row][channel], no swizzle
+                    const uint32_t off = !(FEAT & F_HEADS64) || !head_layout || p.head_dim >= 32 ? (uint32_t)(lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4))
+                                         : p.head_dim == 16 ? (uint32_t)((ch >> 1) * 1024 + lane * 32 + (ch & 1) * 16)
+                                                            : (uint32_t)(ch * 512 + lane * 16);
+                    const uint32_t addr = stg + off;
                     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(packed[4 * ch]),
                                  "r"(packed[4 * ch + 1]), "r"(packed[4 * ch + 2]), "r"(packed[4 * ch + 3])
                                  : "memory");
@@ -352,8 +359,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 __syncwarp();
                 if (lane == 0) {
                     if (head_layout) {
-                        const int hh = n / p.head_dim, d0 = n - hh * p.head_dim;
-                        tma_store_3d(omap, stg, d0, row0, b * p.heads + hh);
+                        const int hh = (b * p.seg_n + n) / p.head_dim;
+                        tma_store_3d(omap, stg, b * p.seg_n + n - hh * p.head_dim, row0, hh);
                     } else {
                         tma_store_3d(omap, stg, n, row0, b);
                     }
@@ -389,22 +396,22 @@ int sm_count()
     return n;
 }
 
-template <int FEAT>
+template <int FEAT, int BN = 128>
 bool launch(cudaStream_t stream, const GemmMaps &maps, const GemmParams &p, const char *name)
 {
     static bool configured = false;
     if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<FEAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        KUTACC_CUDA(cudaFuncSetAttribute(gemm_tcgen05_kernel<FEAT, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         configured = true;
     }
     const int s_tiles = (p.S + BM - 1) / BM;
-    const int64_t tiles = (int64_t)p.B * s_tiles * ((p.seg_n + BN - 1) / BN) * p.nseg;
+    const int n_tiles = p.pair64 ? p.nseg / 2 : ((p.seg_n + BN - 1) / BN) * p.nseg;
+    const int64_t tiles = (int64_t)p.B * s_tiles * n_tiles;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
     GemmParams q = p;
-    const int n_tiles = ((p.seg_n + BN - 1) / BN) * p.nseg;
     q.rotate = (n_tiles > 1 && grid % (unsigned)n_tiles == 0) ? 1 : 0;
     KernelTimer timer__(name, stream);
-    gemm_tcgen05_kernel<FEAT><<<grid, THREADS, SMEM_BYTES, stream>>>(maps, q);
+    gemm_tcgen05_kernel<FEAT, BN><<<grid, THREADS, SMEM_BYTES, stream>>>(maps, q);
     count_launch();
     return true;
 }
@@ -417,7 +424,8 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
                             const float *const *ln_s, const float *const *ln_t)
 {
     const int C = H * D;
-    if (C % 128 != 0 || (D != 32 && D != 64) || C > 256 * 64 || ((uintptr_t)bg & 15u)) return false;
+    if ((C % 128 != 0 && C != 64) || (D != 8 && D != 16 && D != 32 && D != 64) || C > 256 * 64 || ((uintptr_t)bg & 15u)) return false;
+    if (v_transposed && (v_pitch % 8 != 0 || v_pitch < S)) return false;
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     GemmMaps maps;
@@ -425,17 +433,19 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
     void *o[3] = {q, k, v};
     if (!make_tensor_map_bf16_3d(&maps.a, x, C, S, B, C, (uint64_t)S * C, BK, BM, 128)) return false;
     for (int i = 0; i < 4; ++i)
-        if (!make_tensor_map_bf16_3d(&maps.w[i], w[i], C, C, 1, C, (uint64_t)C * C, BK, BN, 128)) return false;
+        if (!make_tensor_map_bf16_3d(&maps.w[i], w[i], C, C, 1, C, (uint64_t)C * C, BK, C == 64 ? 64 : BNMAX, 128)) return false;
     for (int i = 0; i < 3; ++i) {
         if (i == 2 && v_transposed) {
-            // v^T: [B*H][D][S] with row pitch v_pitch (a multiple of 8 elements)
-            if (v_pitch % 8 != 0 || v_pitch < S) return false;
-            if (!make_tensor_map_bf16_3d(&maps.out[i], o[i], S, D, (uint64_t)B * H, (uint64_t)v_pitch,
-                                         (uint64_t)D * v_pitch, 32, 32, 64))
+            // v^T: [B*H*D][S] with row pitch v_pitch (a multiple of 8 elements)
+            if (!make_tensor_map_bf16_3d(&maps.out[i], o[i], S, (uint64_t)B * C, 1, (uint64_t)v_pitch, (uint64_t)B * C * v_pitch,
+                                         32, 32, 64))
                 return false;
             continue;
         }
-        if (!make_tensor_map_bf16_3d(&maps.out[i], o[i], D, S, (uint64_t)B * H, D, (uint64_t)S * D, 32, 32, 64))
+        // [B*H][S][D]; a 32-channel staging tile holds one head, a part of one, or several of 8 or 16 channels
+        const uint32_t box_d = D < 32 ? D : 32;
+        if (!make_tensor_map_bf16_3d(&maps.out[i], o[i], D, S, (uint64_t)B * H, D, (uint64_t)S * D, box_d, 32, D < 32 ? 0 : 64,
+                                     32 / box_d))
             return false;
     }
     if (!make_tensor_map_bf16_3d(&maps.out[3], gate, C, S, B, C, (uint64_t)S * C, 32, 32, 64)) return false;
@@ -455,26 +465,29 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
     p.transposed_mask = v_transposed ? 0x4 : 0;
     p.chanmajor_mask = 0;
     p.w_batched = 0;
-    p.heads = H;
+    p.pair64 = C == 64 ? 1 : 0;
     p.K = C;
     p.S = S;
     p.B = B;
     p.relu = 0;
     p.sigmoid_mask = gate_sigmoid ? 0x8 : 0;
     p.err = ew.device;
+    if (v_transposed != gate_sigmoid || (!v_transposed && (D < 32 || ln_stats))) return false;       // not used together
+    const bool heads64 = C == 64 || D < 32;
     if (ln_stats)
-        return v_transposed && gate_sigmoid ? launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln") : false;
+        return heads64 ? launch<F_TRANSPOSED | F_SIGMOID | F_LN | F_HEADS64>(stream, maps, p, "proj_qkvg_ln")
+                       : launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln");
     if (v_transposed)
-        return gate_sigmoid ? launch<F_TRANSPOSED | F_SIGMOID>(stream, maps, p, "proj_qkvg")
-                            : launch<F_TRANSPOSED>(stream, maps, p, "proj_qkvg");
-    return gate_sigmoid ? launch<F_SIGMOID>(stream, maps, p, "proj_qkvg") : launch<0>(stream, maps, p, "proj_qkvg");
+        return heads64 ? launch<F_TRANSPOSED | F_SIGMOID | F_HEADS64>(stream, maps, p, "proj_qkvg")
+                       : launch<F_TRANSPOSED | F_SIGMOID>(stream, maps, p, "proj_qkvg");
+    return heads64 ? launch<F_HEADS64>(stream, maps, p, "proj_qkvg") : launch<0>(stream, maps, p, "proj_qkvg");
 }
 
 bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w, const float *bias, void *out,
                               int64_t out_row_stride, int B, int S, int N, int K, bool relu, int64_t a_row_stride)
 {
     if (a_row_stride <= 0) a_row_stride = K;
-    if (N % 128 != 0 || K % 64 != 0 || out_row_stride % 8 != 0 || a_row_stride % 8 != 0 || a_row_stride < K ||
+    if ((N % 128 != 0 && (N != 64 || relu)) || K % 64 != 0 || out_row_stride % 8 != 0 || a_row_stride % 8 != 0 || a_row_stride < K ||
         ((uintptr_t)out & 15u) || ((uintptr_t)a & 15u) || ((uintptr_t)w & 15u) || ((uintptr_t)bias & 15u))
         return false;
     KernelErrorWord &ew = kernel_error_word();
@@ -482,7 +495,7 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     GemmMaps maps;
     if (!make_tensor_map_bf16_3d(&maps.a, a, K, S, B, (uint64_t)a_row_stride, (uint64_t)S * a_row_stride, BK, BM, 128))
         return false;
-    if (!make_tensor_map_bf16_3d(&maps.w[0], w, K, N, 1, K, (uint64_t)N * K, BK, BN, 128)) return false;
+    if (!make_tensor_map_bf16_3d(&maps.w[0], w, K, N, 1, K, (uint64_t)N * K, BK, N == 64 ? 64 : BNMAX, 128)) return false;
     if (!make_tensor_map_bf16_3d(&maps.out[0], out, N, S, B, (uint64_t)out_row_stride, (uint64_t)S * out_row_stride, 32,
                                  32, 64))
         return false;
@@ -500,7 +513,7 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     p.transposed_mask = 0;
     p.chanmajor_mask = 0;
     p.w_batched = 0;
-    p.heads = 1;
+    p.pair64 = 0;
     p.K = K;
     p.S = S;
     p.B = B;
@@ -509,6 +522,7 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     p.ln_s[0] = p.ln_s[1] = p.ln_s[2] = p.ln_s[3] = nullptr;
     p.sigmoid_mask = 0;
     p.err = ew.device;
+    if (N == 64) return launch<0, 64>(stream, maps, p, "linear_bias");
     return relu ? launch<F_RELU>(stream, maps, p, "linear_bias_relu") : launch<0>(stream, maps, p, "linear_bias");
 }
 
@@ -530,7 +544,7 @@ bool tcgen05_proj2_chanmajor_bf16(cudaStream_t stream, const void *x, const void
     void *o[2] = {out0, out1};
     if (!make_tensor_map_bf16_3d(&maps.a, x, K, S, B, K, (uint64_t)S * K, BK, BM, 128)) return false;
     for (int i = 0; i < 2; ++i) {
-        if (!make_tensor_map_bf16_3d(&maps.w[i], w[i], K, N, 1, K, (uint64_t)N * K, BK, BN, 128)) return false;
+        if (!make_tensor_map_bf16_3d(&maps.w[i], w[i], K, N, 1, K, (uint64_t)N * K, BK, BNMAX, 128)) return false;
         // [N][B][S]: dims (s, b, n), one 32 (s) x 1 x 32 (n) box per staging tile
         if (!make_tensor_map_bf16_3d(&maps.out[i], o[i], S, B, N, (uint64_t)out_b_stride, (uint64_t)out_c_stride, 32, 1, 64, 32))
             return false;
@@ -550,7 +564,7 @@ bool tcgen05_proj2_chanmajor_bf16(cudaStream_t stream, const void *x, const void
     p.transposed_mask = 0;
     p.chanmajor_mask = 0x3;
     p.w_batched = 0;
-    p.heads = 1;
+    p.pair64 = 0;
     p.K = K;
     p.S = S;
     p.B = B;
@@ -577,7 +591,7 @@ bool tcgen05_batched_nt_bf16(cudaStream_t stream, const void *a, int64_t a_row_s
     if (ew.device == nullptr) return false;
     GemmMaps maps;
     if (!make_tensor_map_bf16_3d(&maps.a, a, K, M, B, (uint64_t)a_row_stride, (uint64_t)a_batch_stride, BK, BM, 128)) return false;
-    if (!make_tensor_map_bf16_3d(&maps.w[0], w, K, N, B, (uint64_t)w_row_stride, (uint64_t)w_batch_stride, BK, BN, 128))
+    if (!make_tensor_map_bf16_3d(&maps.w[0], w, K, N, B, (uint64_t)w_row_stride, (uint64_t)w_batch_stride, BK, BNMAX, 128))
         return false;
     if (!make_tensor_map_bf16_3d(&maps.out[0], out, N, M, B, (uint64_t)out_row_stride, (uint64_t)out_batch_stride, 32, 32, 64))
         return false;
@@ -594,7 +608,7 @@ bool tcgen05_batched_nt_bf16(cudaStream_t stream, const void *a, int64_t a_row_s
     p.transposed_mask = 0;
     p.chanmajor_mask = 0;
     p.w_batched = 1;
-    p.heads = 1;
+    p.pair64 = 0;
     p.K = K;
     p.S = M;
     p.B = B;

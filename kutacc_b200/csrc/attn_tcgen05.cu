@@ -529,18 +529,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
 }
 
-int sm_count_attn()
-{
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
-
 template <int D>
 int smem_bytes(int G, bool has_nb)
 {
@@ -558,7 +546,7 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
                                          smem_bytes<D>(MAXG, HAS_NB)));
         configured = true;
     }
-    const unsigned grid = (unsigned)std::min<int64_t>(p.n_items, std::max(1, sm_count_attn() - runtime().sm_margin));
+    const unsigned grid = (unsigned)std::min<int64_t>(p.n_items, std::max(1, sm_count() - runtime().sm_margin));
     // One pair of counters per STREAM: launches on one stream run one after another, so they can share a pair (the
     // last CTA of a launch zeroes it again), while launches on different streams may overlap and must not. Up to 63
     // streams per device get a pair of their own; further streams share the last pair, which is only safe while they
@@ -672,7 +660,7 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
     p.S = S;
     p.H = H;
     p.B = B;
-    p.G = pick_group(B, n_qt * H, std::max(1, sm_count_attn() - runtime().sm_margin));
+    p.G = pick_group(B, n_qt * H, std::max(1, sm_count() - runtime().sm_margin));
     p.n_qt = (int)n_qt;
     p.n_items = (int)((B + p.G - 1) / p.G * n_qt * H);
     p.scale = scale;

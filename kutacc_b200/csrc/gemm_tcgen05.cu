@@ -32,6 +32,7 @@
 #include "tma_utils.cuh"
 
 #include <algorithm>
+#include <utility>
 
 namespace kutacc {
 namespace dev {
@@ -68,7 +69,6 @@ struct GemmParams {
     int head_dim;           // > 0: segment output is [B*H][S][D] (coords d, s, b*H + h); 0: [B][S][N_seg]
     int head_layout_mask;   // bit i set: segment i uses the head layout
     int transposed_mask;    // bit i set: segment i is stored transposed, [B * N_seg][S] (coords s, b * N_seg + n)
-    int chanmajor_mask;     // bit i set: segment i is stored transposed and channel-major, [N_seg][B][S] (coords s, b, n)
     int w_batched;          // non-zero: W is [B][N_seg][K], one matrix per batch row (coords k, n, b)
     int K;
     int S, B;
@@ -78,6 +78,8 @@ struct GemmParams {
     int rotate;             // non-zero: column tile of tile t is rotated by t / gridDim.x (see tile_of)
     int sigmoid_mask;       // bit i set: segment i stores bf16(sigmoid(bf16(y))) (the gate of the attention, whose
                             // reference rounds the gate to bf16 before the sigmoid: gating_attention.cpp:62-66,134-147)
+    __nv_bfloat16 *direct;  // F_DIRECT: out[b * direct_b + n * direct_n + s]
+    int64_t direct_b, direct_n;
     int *err;
 };
 
@@ -94,6 +96,19 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr)
     d |= (uint64_t)2 << 61;                          // 128-byte swizzle
     return d;
 }
+// MN-major operand (rows of 64 elements = 128 bytes along M or N, one row per k, 128-byte swizzle): 8 k-rows are 1024 bytes
+// apart, the next 64 elements of M or N follow one 64-row block (8 KB) later
+__device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t addr)
+{
+    uint64_t d = 0;
+    d |= (uint64_t)((addr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)((64 * 128) >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
 // 1 / (1 + exp(-g)) of the bf16-rounded g as 0.5 * tanh(g / 2) + 0.5: one MUFU operation (relative error about
 // 2^-11, below the bf16 step of the stored result) instead of an exponential and a division
 __device__ __forceinline__ float sigmoid_of_bf16(float y)
@@ -104,8 +119,13 @@ __device__ __forceinline__ float sigmoid_of_bf16(float y)
 
 // Compile-time feature sets, so that each use of the kernel carries only the epilogue code it needs
 // (the sigmoid and the transposed staging cost registers that the plain linear layer would spill).
+// F_MNMAJOR: both operands are stored with their rows and columns exchanged, X [B][K][S] and W [B][K][N]: the tensor core
+// reads them as they lie (MN-major operands), so a product of transposed matrices needs no transposed copies.
+// F_DIRECT: out[b][n][s] element by element, s along the lanes of a warp (64 contiguous bytes per channel and store): for
+// destinations whose strides no TMA store takes.
 // F_HEADS64: head sizes of 8 or 16 and segments of 64 channels, two of them in a column tile.
-constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16, F_HEADS64 = 32;
+constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16, F_HEADS64 = 32, F_MNMAJOR = 64,
+              F_DIRECT = 128;
 
 // BN: width of a column tile, 128, or 64 for a product with 64 output channels
 template <int FEAT, int BN>
@@ -122,7 +142,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     const uint32_t tmem_slot = bar_base + 8u * NBARS;
 
     constexpr int COLS = BN / 2;                        // columns of an epilogue warp
-    constexpr uint32_t instr_desc = make_instr_desc_bf16(BM, BN);
+    constexpr uint32_t instr_desc = make_instr_desc_bf16(BM, BN) | ((FEAT & F_MNMAJOR) ? (1u << 15) | (1u << 16) : 0u);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int s_tiles = (p.S + BM - 1) / BM;
     const int n_tiles_seg = (p.seg_n + BN - 1) / BN;    // a ragged last tile is zero-filled on load and clipped on store
@@ -183,6 +203,14 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                     }
                     const uint32_t st = smem + (uint32_t)s * STAGE_BYTES;
                     mbar_arrive_expect_tx(full_bar(s), SLAB_BYTES + BN * BK * 2);
+                    if (FEAT & F_MNMAJOR) {
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {            // 64 rows or columns per box
+                            tma_load_3d(st + j * SLAB_BYTES / 2, &maps.a, full_bar(s), s0 + 64 * j, kc * BK, b);
+                            tma_load_3d(st + SLAB_BYTES + j * SLAB_BYTES / 2, wmap, full_bar(s), n0 + 64 * j, kc * BK, b);
+                        }
+                        continue;
+                    }
                     tma_load_3d(st, &maps.a, full_bar(s), kc * BK, s0, b);
                     tma_load_3d(st + SLAB_BYTES, wmap, full_bar(s), kc * BK, n0, (FEAT & F_WBATCH) ? b : 0);
                     if (pair64) tma_load_3d(st + SLAB_BYTES + 64 * BK * 2, wmap + 1, full_bar(s), kc * BK, 0, 0);
@@ -212,8 +240,9 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                     const uint32_t st = smem + (uint32_t)s * STAGE_BYTES;
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
-                        const uint64_t adesc = make_smem_desc(st + k * 32);
-                        const uint64_t bdesc = make_smem_desc(st + SLAB_BYTES + k * 32);
+                        const uint64_t adesc = (FEAT & F_MNMAJOR) ? make_smem_desc_mn(st + k * 2048) : make_smem_desc(st + k * 32);
+                        const uint64_t bdesc = (FEAT & F_MNMAJOR) ? make_smem_desc_mn(st + SLAB_BYTES + k * 2048)
+                                                                  : make_smem_desc(st + SLAB_BYTES + k * 32);
                         tc_mma_bf16(d_tmem, adesc, bdesc, instr_desc, (kc > 0 || k > 0) ? 1u : 0u);
                     }
                     tc_commit(empty_bar(s));                 // slab may be overwritten once these MMAs retire
@@ -244,8 +273,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
             tc_fence_after();
             const float *bias = p.bias[seg];
             const bool head_layout = (p.head_layout_mask >> seg) & 1;
-            const bool chanmajor = (FEAT & F_TRANSPOSED) && ((p.chanmajor_mask >> seg) & 1);
-            const bool transposed = (FEAT & F_TRANSPOSED) && (((p.transposed_mask >> seg) & 1) || chanmajor);
+            const bool transposed = (FEAT & F_TRANSPOSED) && ((p.transposed_mask >> seg) & 1);
             const bool sigmoid = (FEAT & F_SIGMOID) && ((p.sigmoid_mask >> seg) & 1);
             const bool relu = (FEAT & F_RELU) && p.relu;
             const CUtensorMap *omap = &maps.out[seg];
@@ -314,6 +342,20 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                         packed[j] = pack_bf16x2(y0, y1);
                     }
                 }
+                if (FEAT & F_DIRECT) {
+                    __nv_bfloat16 *dst = p.direct + b * p.direct_b + n * p.direct_n + row0 + lane;
+                    if (row0 + lane < p.S) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+                                if (n + 2 * j + e < p.seg_n)
+                                    dst[(2 * j + e) * p.direct_n] =
+                                        __ushort_as_bfloat16((unsigned short)(e ? packed[j] >> 16 : packed[j] & 0xffffu));
+                        }
+                    }
+                    continue;
+                }
                 // staging tile: row = lane, 64 bytes per row, 16-byte chunks swizzled as the 64-byte TMA mode
                 const uint32_t stg = stg0 + (uint32_t)(nstore & 1) * STG_BYTES;
                 if (nstore >= STG_PER_WARP) {
@@ -335,10 +377,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
-                        if (chanmajor)
-                            tma_store_3d(omap, stg, row0, b, n);
-                        else
-                            tma_store_3d(omap, stg, row0, b * p.seg_n + n, 0);
+                        tma_store_3d(omap, stg, row0, b * p.seg_n + n, 0);
                         tma_store_commit();
                     }
                     ++nstore;
@@ -382,18 +421,6 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
         tc_fence_after();
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
-}
-
-int sm_count()
-{
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
 }
 
 template <int FEAT, int BN = 128>
@@ -463,7 +490,6 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
     p.head_dim = D;
     p.head_layout_mask = 0x7;
     p.transposed_mask = v_transposed ? 0x4 : 0;
-    p.chanmajor_mask = 0;
     p.w_batched = 0;
     p.pair64 = C == 64 ? 1 : 0;
     p.K = C;
@@ -511,7 +537,6 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     p.head_dim = 0;
     p.head_layout_mask = 0;
     p.transposed_mask = 0;
-    p.chanmajor_mask = 0;
     p.w_batched = 0;
     p.pair64 = 0;
     p.K = K;
@@ -526,75 +551,43 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     return relu ? launch<F_RELU>(stream, maps, p, "linear_bias_relu") : launch<0>(stream, maps, p, "linear_bias");
 }
 
-// Two projections of x [B, S, K] with row biases, both stored channel-major: out_i[n, b, s] = x[b, s, :] . w_i[n, :]
-// + bias_i[n] (out strides in elements: out_c_stride between channels, out_b_stride between batch rows). The
-// projection and gate products of the triangle multiplication (src/attention/triangle_multiplication.cpp:38-49).
-bool tcgen05_proj2_chanmajor_bf16(cudaStream_t stream, const void *x, const void *w0, const float *bias0, const void *w1,
-                                  const float *bias1, void *out0, void *out1, int64_t out_c_stride, int64_t out_b_stride,
-                                  int B, int S, int N, int K)
+// Batched product with one right-hand matrix per batch: out[b, m, n] = sum_k a[b, m, k] * w[b, n, k], or with
+// `transposed` sum_k a[b, k, m] * w[b, k, n] (a, w, out with row and batch strides in elements). The per-channel products
+// of the triangle multiplication (src/attention/triangle_multiplication.cpp:75-104). An output that no TMA store takes
+// (strides that are not multiples of 8 elements, n not of 8) is computed as its transpose, so that a warp's lanes run along
+// the contiguous index, and stored directly.
+bool tcgen05_batched_bf16(cudaStream_t stream, bool transposed, const void *a, int64_t a_row_stride, int64_t a_batch_stride,
+                          const void *w, int64_t w_row_stride, int64_t w_batch_stride, void *out, int64_t out_row_stride,
+                          int64_t out_batch_stride, int B, int M, int N, int K)
 {
-    if (N % 128 != 0 || K % 64 != 0 || out_c_stride % 8 != 0 || out_b_stride % 8 != 0 || out_b_stride < S ||
-        ((((uintptr_t)x | (uintptr_t)w0 | (uintptr_t)w1 | (uintptr_t)out0 | (uintptr_t)out1 | (uintptr_t)bias0 |
-           (uintptr_t)bias1) & 15u) != 0))
+    if ((a_row_stride | a_batch_stride | w_row_stride | w_batch_stride) % 8 != 0 || a_row_stride < (transposed ? M : K) ||
+        w_row_stride < (transposed ? N : K) || out_row_stride < N || ((((uintptr_t)a | (uintptr_t)w) & 15u) != 0))
         return false;
+    const bool direct = (out_row_stride | out_batch_stride) % 8 != 0 || ((uintptr_t)out & 15u) != 0;
+    if (direct) {
+        std::swap(a, w);
+        std::swap(a_row_stride, w_row_stride);
+        std::swap(a_batch_stride, w_batch_stride);
+        std::swap(M, N);
+    }
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     GemmMaps maps;
-    const void *w[2] = {w0, w1};
-    void *o[2] = {out0, out1};
-    if (!make_tensor_map_bf16_3d(&maps.a, x, K, S, B, K, (uint64_t)S * K, BK, BM, 128)) return false;
-    for (int i = 0; i < 2; ++i) {
-        if (!make_tensor_map_bf16_3d(&maps.w[i], w[i], K, N, 1, K, (uint64_t)N * K, BK, BNMAX, 128)) return false;
-        // [N][B][S]: dims (s, b, n), one 32 (s) x 1 x 32 (n) box per staging tile
-        if (!make_tensor_map_bf16_3d(&maps.out[i], o[i], S, B, N, (uint64_t)out_b_stride, (uint64_t)out_c_stride, 32, 1, 64, 32))
+    if (transposed) {
+        if (!make_tensor_map_bf16_3d(&maps.a, a, M, K, B, (uint64_t)a_row_stride, (uint64_t)a_batch_stride, 64, BK, 128) ||
+            !make_tensor_map_bf16_3d(&maps.w[0], w, N, K, B, (uint64_t)w_row_stride, (uint64_t)w_batch_stride, 64, BK, 128))
+            return false;
+    } else {
+        if (!make_tensor_map_bf16_3d(&maps.a, a, K, M, B, (uint64_t)a_row_stride, (uint64_t)a_batch_stride, BK, BM, 128) ||
+            !make_tensor_map_bf16_3d(&maps.w[0], w, K, N, B, (uint64_t)w_row_stride, (uint64_t)w_batch_stride, BK, BNMAX, 128))
             return false;
     }
-    for (int i = 2; i < 4; ++i) {
-        maps.w[i] = maps.w[0];
-        maps.out[i] = maps.out[0];
+    if (!direct) {
+        if (!make_tensor_map_bf16_3d(&maps.out[0], out, N, M, B, (uint64_t)out_row_stride, (uint64_t)out_batch_stride, 32, 32, 64))
+            return false;
+    } else {
+        maps.out[0] = maps.a;
     }
-    GemmParams p;
-    p.bias[0] = bias0;
-    p.bias[1] = bias1;
-    p.bias[2] = p.bias[3] = nullptr;
-    p.seg_n = N;
-    p.nseg = 2;
-    p.head_dim = 0;
-    p.head_layout_mask = 0;
-    p.transposed_mask = 0;
-    p.chanmajor_mask = 0x3;
-    p.w_batched = 0;
-    p.pair64 = 0;
-    p.K = K;
-    p.S = S;
-    p.B = B;
-    p.relu = 0;
-    p.ln_stats = nullptr;
-    p.ln_s[0] = p.ln_s[1] = p.ln_s[2] = p.ln_s[3] = nullptr;
-    p.sigmoid_mask = 0;
-    p.err = ew.device;
-    return launch<F_TRANSPOSED>(stream, maps, p, "tm_proj");
-}
-
-// Batched product with one right-hand matrix per batch: out[b, m, n] = sum_k a[b, m, k] * w[b, n, k]
-// (a, w, out with row and batch strides in elements). The per-channel products of the triangle multiplication
-// (src/attention/triangle_multiplication.cpp:75-104).
-bool tcgen05_batched_nt_bf16(cudaStream_t stream, const void *a, int64_t a_row_stride, int64_t a_batch_stride,
-                             const void *w, int64_t w_row_stride, int64_t w_batch_stride, void *out,
-                             int64_t out_row_stride, int64_t out_batch_stride, int B, int M, int N, int K)
-{
-    if ((a_row_stride | a_batch_stride | w_row_stride | w_batch_stride | out_row_stride | out_batch_stride) % 8 != 0 ||
-        a_row_stride < K || w_row_stride < K || out_row_stride < N ||
-        ((((uintptr_t)a | (uintptr_t)w | (uintptr_t)out) & 15u) != 0))
-        return false;
-    KernelErrorWord &ew = kernel_error_word();
-    if (ew.device == nullptr) return false;
-    GemmMaps maps;
-    if (!make_tensor_map_bf16_3d(&maps.a, a, K, M, B, (uint64_t)a_row_stride, (uint64_t)a_batch_stride, BK, BM, 128)) return false;
-    if (!make_tensor_map_bf16_3d(&maps.w[0], w, K, N, B, (uint64_t)w_row_stride, (uint64_t)w_batch_stride, BK, BNMAX, 128))
-        return false;
-    if (!make_tensor_map_bf16_3d(&maps.out[0], out, N, M, B, (uint64_t)out_row_stride, (uint64_t)out_batch_stride, 32, 32, 64))
-        return false;
     for (int i = 1; i < 4; ++i) {
         maps.w[i] = maps.w[0];
         maps.out[i] = maps.out[0];
@@ -606,7 +599,6 @@ bool tcgen05_batched_nt_bf16(cudaStream_t stream, const void *a, int64_t a_row_s
     p.head_dim = 0;
     p.head_layout_mask = 0;
     p.transposed_mask = 0;
-    p.chanmajor_mask = 0;
     p.w_batched = 1;
     p.pair64 = 0;
     p.K = K;
@@ -616,8 +608,15 @@ bool tcgen05_batched_nt_bf16(cudaStream_t stream, const void *a, int64_t a_row_s
     p.ln_stats = nullptr;
     p.ln_s[0] = p.ln_s[1] = p.ln_s[2] = p.ln_s[3] = nullptr;
     p.sigmoid_mask = 0;
+    p.direct = (__nv_bfloat16 *)out;
+    p.direct_b = out_batch_stride;
+    p.direct_n = out_row_stride;
     p.err = ew.device;
-    return launch<F_WBATCH>(stream, maps, p, "tm_equation");
+    if (direct)
+        return transposed ? launch<F_WBATCH | F_MNMAJOR | F_DIRECT>(stream, maps, p, "tm_equation")
+                          : launch<F_WBATCH | F_DIRECT>(stream, maps, p, "tm_equation");
+    return transposed ? launch<F_WBATCH | F_MNMAJOR>(stream, maps, p, "tm_equation")
+                      : launch<F_WBATCH>(stream, maps, p, "tm_equation");
 }
 
 }  // namespace dev

@@ -268,18 +268,6 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const SplitArgs args, i
     }
 }
 
-int sm_count_tf32()
-{
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
-
 }  // namespace
 
 bool launch_split_tf32_many(cudaStream_t stream, int count, const void *const *src, int64_t src_ld, void *const *dst,
@@ -294,7 +282,7 @@ bool launch_split_tf32_many(cudaStream_t stream, int count, const void *const *s
         a.dst[i] = (float *)dst[j];
     }
     const int64_t total = rows * (K / 4);
-    const unsigned gx = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count_tf32() * 16);
+    const unsigned gx = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 16);
     KernelTimer timer__("split_tf32", stream);
     split_tf32_kernel<<<dim3(gx, (unsigned)count), 256, 0, stream>>>(a, src_ld, rows, K);
     count_launch();
@@ -342,7 +330,7 @@ bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *c
         configured = true;
     }
     const int64_t tiles = ((M + BM - 1) / BM) * (int64_t)(N / BN) * nseg;
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count_tf32() - runtime().sm_margin));
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
     KernelTimer timer__("gemm_tf32x3_tc", stream);
     gemm_tf32x3_tc_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(maps, p);
     count_launch();

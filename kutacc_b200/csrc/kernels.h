@@ -39,15 +39,17 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
 bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w, const float *bias, void *out,
                               int64_t out_row_stride, int B, int S, int N, int K, bool relu = false,
                               int64_t a_row_stride = 0);
-// out_i[n, b, s] = x[b, s, :] . w_i[n, :] + bias_i[n], i = 0, 1: two projections stored channel-major
-// (N % 128 == 0, K % 64 == 0, strides multiples of 8 elements). False when the shape is not covered.
-bool tcgen05_proj2_chanmajor_bf16(cudaStream_t stream, const void *x, const void *w0, const float *bias0, const void *w1,
-                                  const float *bias1, void *out0, void *out1, int64_t out_c_stride, int64_t out_b_stride,
-                                  int B, int S, int N, int K);
-// out[b, m, n] = sum_k a[b, m, k] * w[b, n, k]: one right-hand matrix per batch (strides multiples of 8 elements).
-bool tcgen05_batched_nt_bf16(cudaStream_t stream, const void *a, int64_t a_row_stride, int64_t a_batch_stride,
-                             const void *w, int64_t w_row_stride, int64_t w_batch_stride, void *out,
-                             int64_t out_row_stride, int64_t out_batch_stride, int B, int M, int N, int K);
+// Projection step of the triangle multiplication (tm_proj.cu): gate[n, b, s] = x[b, s, :] . wg[n, :] + bg[n] and
+// proj[n, b, s] = (x[b, s, :] . wp[n, :] + bp[n]) * mask[b, s] * sigmoid(gate[n, b, s]), any output strides (elements;
+// N % 128 == 0, K % 64 == 0). False when the shape is not covered.
+bool tcgen05_tm_proj_bf16(cudaStream_t stream, const void *x, const void *wp, const float *bp, const void *wg, const float *bg,
+                          const void *mask, int64_t m_s0, void *proj, int64_t p_s0, int64_t p_s1, void *gate, int64_t g_s0,
+                          int64_t g_s1, int B, int S, int N, int K);
+// out[b, m, n] = sum_k a[b, m, k] * w[b, n, k], or with `transposed` sum_k a[b, k, m] * w[b, k, n]: one right-hand matrix
+// per batch (strides of a and w multiples of 8 elements, of out any).
+bool tcgen05_batched_bf16(cudaStream_t stream, bool transposed, const void *a, int64_t a_row_stride, int64_t a_batch_stride,
+                          const void *w, int64_t w_row_stride, int64_t w_batch_stride, void *out, int64_t out_row_stride,
+                          int64_t out_batch_stride, int B, int M, int N, int K);
 
 // fp32 GEMM on tcgen05 (gemm_tf32_tcgen05.cu): operands pre-split into tf32 head and tail, stored as rows
 // [hi(0..K) | lo(0..K)] by launch_split_tf32 (src [rows, K] fp32 with row stride src_ld; dst [rows, 2K] dense).
@@ -73,9 +75,10 @@ bool launch_tm_proj_generic(cudaStream_t stream, const void *x, const void *w0, 
 bool launch_tm_equation_generic(cudaStream_t stream, const void *left, int64_t l_s0, int64_t l_s1, const void *right,
                                 int64_t r_s0, int64_t r_s1, void *center, int64_t c_s0, int64_t c_s1, int64_t c_i,
                                 int64_t n, bool incoming);
-// dst[c, a, k] = src[c, k, a] for every channel c (n x n matrices; dst dense with row pitch d_pitch)
-bool launch_tm_transpose(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
-                         int64_t c_i, int64_t n);
+// dst[c, r, :] = src[c, r, :] for c_i matrices of n x n elements: rows moved from any stride to a pitch that is a multiple of
+// 8 elements (dst dense, 16-byte aligned)
+bool launch_tm_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
+                       int64_t c_i, int64_t n);
 // out[r, :] = bf16(f32(out[r, :]) * sigmoid(f32(gate[r, :]))) for rows of c_o elements
 bool launch_tm_last(cudaStream_t stream, void *out, int64_t o_rs, const void *gate, int64_t g_rs, int64_t rows, int64_t c_o);
 

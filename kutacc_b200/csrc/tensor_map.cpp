@@ -88,6 +88,18 @@ bool make_tensor_map_2d(CUtensorMap *map, const void *base, int elem_bytes, uint
     return r == CUDA_SUCCESS;
 }
 
+int sm_count()
+{
+    static int n = 0;
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 148;
+    }
+    return n;
+}
+
 KernelErrorWord &kernel_error_word()
 {
     static KernelErrorWord w;

@@ -7,6 +7,7 @@
 #include "ptx_utils.cuh"
 
 #include <algorithm>
+#include <climits>
 
 namespace kutacc {
 namespace dev {
@@ -90,22 +91,31 @@ __global__ void tm_equation_generic_kernel(const __nv_bfloat16 *__restrict__ lef
     }
 }
 
-// 32 x 32 tiles through shared memory: dst[c, a, k] = src[c, k, a]
-__global__ void tm_transpose_kernel(const __nv_bfloat16 *__restrict__ src, int64_t s_s0, int64_t s_s1,
-                                    __nv_bfloat16 *__restrict__ dst, int64_t d_pitch, int64_t n)
+// Rows of n elements to a pitch of `vecs` 16-byte vectors. A thread moves one vector: the five aligned 32-bit words that
+// cover it in the source, shifted together when the source starts on an odd element (the words past the row belong to the
+// vector's padding; those past the matrix's last row are not read).
+__global__ void __launch_bounds__(256) tm_repitch_kernel(const __nv_bfloat16 *__restrict__ src, int64_t s_s0, int64_t s_s1,
+                                                         uint4 *__restrict__ dst, int vecs, int c_i, int n)
 {
-    __shared__ __nv_bfloat16 tile[32][33];
-    const int64_t c = blockIdx.z, k0 = (int64_t)blockIdx.y * 32, a0 = (int64_t)blockIdx.x * 32;
-    const __nv_bfloat16 *s = src + c * s_s0;
-    __nv_bfloat16 *d = dst + c * n * d_pitch;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int64_t k = k0 + r, a = a0 + threadIdx.x;
-        tile[r][threadIdx.x] = (k < n && a < n) ? s[k * s_s1 + a] : __float2bfloat16_rn(0.f);
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int64_t a = a0 + r, k = k0 + threadIdx.x;
-        if (a < n && k < n) d[a * d_pitch + k] = tile[threadIdx.x][r];
+    const int64_t total = (int64_t)c_i * n * vecs;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int v = (int)(t % vecs);
+        const int64_t line = t / vecs;
+        const int r = (int)(line % n), c = (int)(line / n);
+        const __nv_bfloat16 *sp = src + c * s_s0 + r * s_s1 + v * 8;
+        const int have = min(8, n - v * 8);               // elements of this vector
+        const uint32_t *wp = reinterpret_cast<const uint32_t *>((uintptr_t)sp & ~(uintptr_t)3);
+        const bool odd = ((uintptr_t)sp & 2) != 0;
+        uint32_t w[5];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) w[i] = 2 * i - (odd ? 1 : 0) < have ? __ldg(wp + i) : 0u;
+        uint4 o;
+        if (odd)
+            o = make_uint4(__funnelshift_r(w[0], w[1], 16), __funnelshift_r(w[1], w[2], 16), __funnelshift_r(w[2], w[3], 16),
+                           __funnelshift_r(w[3], w[4], 16));
+        else
+            o = make_uint4(w[0], w[1], w[2], w[3]);
+        dst[t] = o;
     }
 }
 
@@ -183,14 +193,13 @@ bool launch_tm_equation_generic(cudaStream_t stream, const void *left, int64_t l
     return true;
 }
 
-bool launch_tm_transpose(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
-                         int64_t c_i, int64_t n)
+bool launch_tm_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
+                       int64_t c_i, int64_t n)
 {
-    const int64_t tiles = (n + 31) / 32;
-    if (c_i > 65535 || tiles > 65535) return false;
-    KernelTimer timer__("tm_transpose", stream);
-    dim3 grid((unsigned)tiles, (unsigned)tiles, (unsigned)c_i), block(32, 8);
-    tm_transpose_kernel<<<grid, block, 0, stream>>>((const __nv_bfloat16 *)src, s_s0, s_s1, (__nv_bfloat16 *)dst, d_pitch, n);
+    if (d_pitch % 8 != 0 || d_pitch < n || ((uintptr_t)dst & 15u) || c_i > INT32_MAX || n > INT32_MAX) return false;
+    KernelTimer timer__("tm_repitch", stream);
+    tm_repitch_kernel<<<grid_for(c_i * n * (d_pitch / 8), 256), 256, 0, stream>>>(
+        (const __nv_bfloat16 *)src, s_s0, s_s1, (uint4 *)dst, (int)(d_pitch / 8), (int)c_i, (int)n);
     count_launch();
     return true;
 }

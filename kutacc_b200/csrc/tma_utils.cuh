@@ -25,6 +25,9 @@ bool make_tensor_map_bf16_4d(CUtensorMap *map, const void *base, uint64_t d0, ui
 bool make_tensor_map_2d(CUtensorMap *map, const void *base, int elem_bytes, uint64_t d0, uint64_t d1, uint64_t stride1,
                         uint32_t box0, uint32_t box1, int swizzle_bytes);
 
+// SMs of the current device
+int sm_count();
+
 // Host-visible error word written by kernels whose bounded waits ran out (0 = none). The pointer is a
 // device-accessible alias of pinned host memory; the host reads *host after synchronising.
 struct KernelErrorWord {

@@ -1,8 +1,8 @@
 // The four exported steps of the triangle multiplication (outgoing and incoming edges).
 // Replaces src/attention/triangle_multiplication.cpp:25-262 of the reference. The matrix products run on the
-// tcgen05 projection kernel (channel-major stores for the projections, one right-hand matrix per channel for the
-// per-channel products) where the shape allows it, and on plain CUDA-core kernels otherwise; the mask, gate and
-// sigmoid steps are element-wise kernels. Host or device tensors (host tensors are staged like everywhere else).
+// tensor cores where the shape allows it (tm_proj.cu: both projections with mask and gate in one kernel; gemm_tcgen05.cu: one
+// right-hand matrix per channel, operands read transposed for incoming edges), and on plain CUDA-core kernels otherwise;
+// the final gate is an element-wise kernel. Host or device tensors (host tensors are staged like everywhere else).
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -83,15 +83,14 @@ extern "C" void kutacc_af2_triangle_multiplication_calc_proj(kutacc_af2_tm_act_i
               d_g = resolve_out_keeping_gaps(gate.data_ptr(), g_bytes, g_dense);
     if (kutacc_check_err_set) return;
 
-    bool ok = p_s0 == g_s0 && p_s1 == g_s1 &&
-              dev::tcgen05_proj2_chanmajor_bf16(stream, d_x.dev, d_pw.dev, (const float *)d_pb.dev, d_gw.dev,
-                                                (const float *)d_gb.dev, d_p.dev, d_g.dev, p_s0, p_s1, (int)n_res,
-                                                (int)n_gather, (int)c_i, (int)c_o);
+    bool ok = dev::tcgen05_tm_proj_bf16(stream, d_x.dev, d_pw.dev, (const float *)d_pb.dev, d_gw.dev, (const float *)d_gb.dev,
+                                        d_m.dev, m_s0, d_p.dev, p_s0, p_s1, d_g.dev, g_s0, g_s1, (int)n_res, (int)n_gather,
+                                        (int)c_i, (int)c_o);
     if (kutacc_check_err_set) return;
     if (!ok)
         ok = dev::launch_tm_proj_generic(stream, d_x.dev, d_pw.dev, (const float *)d_pb.dev, d_gw.dev, (const float *)d_gb.dev,
-                                         d_p.dev, d_g.dev, p_s0, p_s1, g_s0, g_s1, n_res, n_gather, c_o, c_i);
-    ok = ok && dev::launch_tm_mask_gate(stream, d_p.dev, d_g.dev, d_m.dev, c_i, n_res, n_gather, p_s0, p_s1, g_s0, g_s1, m_s0);
+                                         d_p.dev, d_g.dev, p_s0, p_s1, g_s0, g_s1, n_res, n_gather, c_o, c_i) &&
+             dev::launch_tm_mask_gate(stream, d_p.dev, d_g.dev, d_m.dev, c_i, n_res, n_gather, p_s0, p_s1, g_s0, g_s1, m_s0);
     KUTACC_CHECK(ok, "triangle_multiplication_calc_proj: no device kernel for c_o=", c_o, " c_i=", c_i);
     finish_out(d_p);
     finish_out(d_g);
@@ -124,26 +123,32 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
     if (!rt.reserve_stage(staged_bytes_needed(left.data_ptr(), l_bytes) + staged_bytes_needed(right.data_ptr(), r_bytes) +
                           staged_bytes_needed(center.data_ptr(), c_bytes)))
         return;
-    const int64_t pitch = (n + 7) / 8 * 8;                           // transposed copies for the incoming product
-    if (is_incoming && !rt.reserve_workspace(2 * ((size_t)c_i * n * pitch * 2 + 256))) return;
+    // The tensor-core product reads rows that start on 16-byte boundaries; operands with other strides (an odd number of
+    // residues) are first moved to padded rows in the workspace, one pass over HBM each.
+    const int64_t pitch = (n + 7) / 8 * 8;
+    const size_t pad_bytes = (size_t)c_i * n * pitch * 2;
+    if (!rt.reserve_workspace(2 * (pad_bytes + 256))) return;
     DeviceArg d_l = resolve_in(left.data_ptr(), l_bytes), d_r = resolve_in(right.data_ptr(), r_bytes);
     DeviceArg d_c = resolve_out_keeping_gaps(center.data_ptr(), c_bytes, dense3(center, n, n));
+    void *pad_l = rt.take_workspace(pad_bytes), *pad_r = rt.take_workspace(pad_bytes);
     if (kutacc_check_err_set) return;
-    bool ok = false;
-    if (!is_incoming) {
-        // center[a, b] = sum_k left[a, k] * right[b, k]
-        ok = dev::tcgen05_batched_nt_bf16(stream, d_l.dev, l_s1, l_s0, d_r.dev, r_s1, r_s0, d_c.dev, c_s1, c_s0, (int)c_i, (int)n,
-                                          (int)n, (int)n);
-    } else {
-        // center[a, b] = sum_k right[k, a] * left[k, b] = sum_k right^T[a, k] * left^T[b, k]: both operands are
-        // transposed once (a pass over HBM each), then the same product runs
-        void *lt = rt.take_workspace((size_t)c_i * n * pitch * 2), *rtp = rt.take_workspace((size_t)c_i * n * pitch * 2);
-        if (kutacc_check_err_set) return;
-        ok = dev::launch_tm_transpose(stream, d_l.dev, l_s0, l_s1, lt, pitch, c_i, n) &&
-             dev::launch_tm_transpose(stream, d_r.dev, r_s0, r_s1, rtp, pitch, c_i, n) &&
-             dev::tcgen05_batched_nt_bf16(stream, rtp, pitch, n * pitch, lt, pitch, n * pitch, d_c.dev, c_s1, c_s0, (int)c_i,
-                                          (int)n, (int)n, (int)n);
-    }
+    struct Operand {
+        const void *p;
+        int64_t s0, s1;
+    };
+    auto aligned_rows = [&](const void *p, int64_t s0, int64_t s1, void *pad, Operand &o) {
+        o = {p, s0, s1};
+        if (((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0) return true;
+        o = {pad, n * pitch, pitch};
+        return dev::launch_tm_repitch(stream, p, s0, s1, pad, pitch, c_i, n);
+    };
+    Operand ol, orr;
+    bool ok = aligned_rows(d_l.dev, l_s0, l_s1, pad_l, ol) && aligned_rows(d_r.dev, r_s0, r_s1, pad_r, orr);
+    // outgoing: center[a, b] = sum_k left[a, k] * right[b, k]; incoming: center[a, b] = sum_k right[k, a] * left[k, b]
+    ok = ok && (is_incoming ? dev::tcgen05_batched_bf16(stream, true, orr.p, orr.s1, orr.s0, ol.p, ol.s1, ol.s0, d_c.dev, c_s1,
+                                                        c_s0, (int)c_i, (int)n, (int)n, (int)n)
+                            : dev::tcgen05_batched_bf16(stream, false, ol.p, ol.s1, ol.s0, orr.p, orr.s1, orr.s0, d_c.dev, c_s1,
+                                                        c_s0, (int)c_i, (int)n, (int)n, (int)n));
     if (kutacc_check_err_set) return;
     if (!ok)
         ok = dev::launch_tm_equation_generic(stream, d_l.dev, l_s0, l_s1, d_r.dev, r_s0, r_s1, d_c.dev, c_s0, c_s1, c_i, n,

@@ -51,6 +51,11 @@ bool tcgen05_batched_bf16(cudaStream_t stream, bool transposed, const void *a, i
                           const void *w, int64_t w_row_stride, int64_t w_batch_stride, void *out, int64_t out_row_stride,
                           int64_t out_batch_stride, int B, int M, int N, int K);
 
+// out = relu(x . w1^T + b1) . w2^T + b2 in one kernel (transition_fused.cu): x, out [M, c_o] dense, w1 [c_i, c_o],
+// w2 [c_o, c_i]. c_o 128 or 256, c_i % 128 == 0. False when the shape is not covered.
+bool tcgen05_transition_bf16(cudaStream_t stream, const void *x, const void *w1, const float *b1, const void *w2, const float *b2,
+                             void *out, int64_t M, int c_o, int c_i);
+
 // fp32 GEMM on tcgen05 (gemm_tf32_tcgen05.cu): operands pre-split into tf32 head and tail, stored as rows
 // [hi(0..K) | lo(0..K)] by launch_split_tf32 (src [rows, K] fp32 with row stride src_ld; dst [rows, 2K] dense).
 // out_i[m, :] = a[m, :] . w_i^T (+ bias_i) for up to four weight matrices [N, K] in one pass over a; out row stride

@@ -1,8 +1,9 @@
 // kutacc_af2_transition: out = relu(x . W1^T + b1) . W2^T + b2, the transition MLP of the Evoformer.
 // Replaces src/attention/transition.cpp:21-61 (two addmm calls with a row bias, the first with ReLU; the
-// intermediate is a bf16 tensor). Both products run on the tcgen05 projection kernel (ReLU in its epilogue);
-// shapes it does not cover take the generic GEMM. The intermediate lives in the library's workspace: the
-// caller's intermediate_act tensor is not written, like the scratch tensors of the attention operators.
+// intermediate is a bf16 tensor). 128 or 256 channels run in one kernel that keeps the hidden activations on the SM
+// (transition_fused.cu); other shapes take two launches of the tcgen05 projection kernel (ReLU in the epilogue of the first)
+// or the generic GEMM, with the intermediate in the library's workspace: the caller's intermediate_act tensor is not
+// written, like the scratch tensors of the attention operators.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -45,32 +46,32 @@ extern "C" void kutacc_af2_transition(kutacc_af2_trans_act_inputs_t *trans_input
                          staged_bytes_needed(w1.data_ptr(), w_bytes) + staged_bytes_needed(w2.data_ptr(), w_bytes) +
                          staged_bytes_needed(b1.data_ptr(), b1_bytes) + staged_bytes_needed(b2.data_ptr(), b2_bytes);
     if (!rt.reserve_stage(stage)) return;
-    if (!rt.reserve_workspace(h_bytes + 256)) return;
     DeviceArg d_x = resolve_in(x.data_ptr(), x_bytes), d_w1 = resolve_in(w1.data_ptr(), w_bytes),
               d_w2 = resolve_in(w2.data_ptr(), w_bytes), d_b1 = resolve_in(b1.data_ptr(), b1_bytes),
               d_b2 = resolve_in(b2.data_ptr(), b2_bytes);
     DeviceArg d_o = resolve_out(o.data_ptr(), x_bytes);
-    void *hid = rt.take_workspace(h_bytes);
     if (kutacc_check_err_set) return;
 
-    // hidden = relu(x . W1^T + b1): W1 is stored [c_i][c_o] (transition.cpp:32, the {c_o, c_i} view with strides {1, c_o})
-    bool ok = dev::tcgen05_linear_bias_bf16(stream, d_x.dev, d_w1.dev, (const float *)d_b1.dev, hid, c_i, (int)batch,
-                                            (int)n_res, (int)c_i, (int)c_o, true);
+    // W1 is stored [c_i][c_o] (transition.cpp:32, the {c_o, c_i} view with strides {1, c_o}), W2 [c_o][c_i] (:36). One kernel
+    // that keeps the hidden activations on the SM, or two products through the workspace.
+    bool ok = dev::tcgen05_transition_bf16(stream, d_x.dev, d_w1.dev, (const float *)d_b1.dev, d_w2.dev, (const float *)d_b2.dev,
+                                           d_o.dev, M, (int)c_o, (int)c_i);
     if (kutacc_check_err_set) return;
     if (!ok) {
-        ok = dev::launch_gemm_generic(stream, dev::kElemBF16, d_x.dev, c_o, d_w1.dev, c_o, (const float *)d_b1.dev, 0.f, hid,
-                                      c_i, M, c_i, c_o) &&
-             dev::launch_relu_bf16(stream, hid, M * c_i);
-    }
-    // out = hidden . W2^T + b2: W2 is stored [c_o][c_i] (transition.cpp:36)
-    if (ok) {
-        bool ok2 = dev::tcgen05_linear_bias_bf16(stream, hid, d_w2.dev, (const float *)d_b2.dev, d_o.dev, c_o, (int)batch,
-                                                 (int)n_res, (int)c_o, (int)c_i, false);
+        if (!rt.reserve_workspace(h_bytes + 256)) return;
+        void *hid = rt.take_workspace(h_bytes);
         if (kutacc_check_err_set) return;
-        if (!ok2)
-            ok2 = dev::launch_gemm_generic(stream, dev::kElemBF16, hid, c_i, d_w2.dev, c_i, (const float *)d_b2.dev, 0.f,
-                                           d_o.dev, c_o, M, c_o, c_i);
-        ok = ok2;
+        ok = dev::tcgen05_linear_bias_bf16(stream, d_x.dev, d_w1.dev, (const float *)d_b1.dev, hid, c_i, (int)batch, (int)n_res,
+                                           (int)c_i, (int)c_o, true) ||
+             (dev::launch_gemm_generic(stream, dev::kElemBF16, d_x.dev, c_o, d_w1.dev, c_o, (const float *)d_b1.dev, 0.f, hid, c_i,
+                                       M, c_i, c_o) &&
+              dev::launch_relu_bf16(stream, hid, M * c_i));
+        if (kutacc_check_err_set) return;
+        ok = ok && (dev::tcgen05_linear_bias_bf16(stream, hid, d_w2.dev, (const float *)d_b2.dev, d_o.dev, c_o, (int)batch,
+                                                  (int)n_res, (int)c_o, (int)c_i, false) ||
+                    dev::launch_gemm_generic(stream, dev::kElemBF16, hid, c_i, d_w2.dev, c_i, (const float *)d_b2.dev, 0.f,
+                                             d_o.dev, c_o, M, c_o, c_i));
+        if (kutacc_check_err_set) return;
     }
     KUTACC_CHECK(ok, "kutacc_af2_transition: no device kernel for c_o=", c_o, " c_i=", c_i);
     finish_out(d_o);

@@ -275,6 +275,7 @@ class Tensor:
         if not self.handle:
             raise_if_error()
             raise KutaccError("tensor descriptor creation failed")
+        self.arg = C.c_void_p(self.handle)     # what the C functions are called with
 
     def __del__(self):
         h = getattr(self, "handle", None)
@@ -318,7 +319,7 @@ def empty_tensor(dtype: int = DTYPE_BF16) -> Tensor:
 
 
 def _h(t) -> C.c_void_p:
-    return C.c_void_p(t.handle if isinstance(t, Tensor) else (t or 0))
+    return t.arg if isinstance(t, Tensor) else C.c_void_p(t or 0)
 
 
 def make_weights(nchannels: int, nheads: int, head_size: int, query_w, key_w, value_w, gating_w, gating_b,

@@ -1,4 +1,5 @@
 // Device runtime: stream, grow-only workspace, staging of host-resident tensors.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -107,9 +108,34 @@ void Runtime::release()
     ws_cap = ws_off = stage_cap = stage_off = 0;
 }
 
+namespace {
+typedef CUresult (*PointerAttributeFn)(void *, CUpointer_attribute, CUdeviceptr);
+PointerAttributeFn pointer_attribute_fn()
+{
+    static const PointerAttributeFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<PointerAttributeFn>(p);
+    }();
+    return fn;
+}
+}  // namespace
+
+// Asked about two dozen times per operator call. The driver's query of the one attribute costs a fraction of
+// cudaPointerGetAttributes, which fetches all of them and stays as the answer for everything the driver does not know.
 bool is_device_pointer(const void *p)
 {
     if (p == nullptr) return false;
+    if (PointerAttributeFn fn = pointer_attribute_fn()) {
+        unsigned type = 0;
+        if (fn(&type, CU_POINTER_ATTRIBUTE_MEMORY_TYPE, (CUdeviceptr)(uintptr_t)p) == CUDA_SUCCESS)
+            return type == CU_MEMORYTYPE_DEVICE;              // managed memory answers "device" too
+    }
     cudaPointerAttributes a;
     cudaError_t e = cudaPointerGetAttributes(&a, p);
     if (e != cudaSuccess) {

@@ -19,6 +19,7 @@
 // strides (nb_stride_h, nb_stride_q, 1) or null.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 
 namespace kutacc {
@@ -60,6 +61,8 @@ __global__ void __launch_bounds__(A_THREADS, 2) attn_f32_kernel(const float *__r
                                                              int n_qt, float scale, float *__restrict__ avg_split)
 {
     __shared__ F32Smem sm;
+    release_successor();
+    wait_for_predecessor();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int item = blockIdx.x;
     const int qt = item % n_qt, h = (item / n_qt) % H, b = item / (n_qt * H);
@@ -277,7 +280,7 @@ bool launch_attn_f32(cudaStream_t stream, const void *q, const void *k, const vo
     const int64_t items = (int64_t)B * H * n_qt;
     if (items > 0x7fffffff) return false;
     KernelTimer timer__("attn_f32", stream);
-    attn_f32_kernel<<<(unsigned)items, A_THREADS, 0, stream>>>(
+    launch_chained(attn_f32_kernel, (unsigned)items, A_THREADS, 0, stream,
         (const float *)q, (const float *)k, (const float *)v, (const float *)gate, (const float *)bias, bias_stride0,
         (const float *)nb, nb_stride_h, nb_stride_q, (float *)avg, S, H, n_qt, scale, (float *)avg_split);
     count_launch();

@@ -42,6 +42,7 @@
 // tail, tensor memory is released, and the host-visible error word carries the site.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -179,6 +180,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    release_successor();
+    wait_for_predecessor();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
     tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);          // warp-uniform
@@ -582,7 +585,7 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
     AttnParams q = p;
     q.counter = counters[dev] + 2 * slot;
     KernelTimer timer__("attn_core", stream);
-    attn_tc_kernel<D, HAS_NB><<<grid, THREADS, smem_bytes<D>(p.G, HAS_NB), stream>>>(tq, tk, tvt, tnb, q);
+    launch_chained(attn_tc_kernel<D, HAS_NB>, grid, THREADS, smem_bytes<D>(p.G, HAS_NB), stream, tq, tk, tvt, tnb, q);
     count_launch();
     return true;
 }

@@ -27,6 +27,7 @@
 // allocation is released and the host-visible error word carries the site.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -179,6 +180,8 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    release_successor();
+    wait_for_predecessor();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
     tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);          // warp-uniform
@@ -438,7 +441,7 @@ bool launch(cudaStream_t stream, const GemmMaps &maps, const GemmParams &p, cons
     GemmParams q = p;
     q.rotate = (n_tiles > 1 && grid % (unsigned)n_tiles == 0) ? 1 : 0;
     KernelTimer timer__(name, stream);
-    gemm_tcgen05_kernel<FEAT, BN><<<grid, THREADS, SMEM_BYTES, stream>>>(maps, q);
+    launch_chained(gemm_tcgen05_kernel<FEAT, BN>, grid, THREADS, SMEM_BYTES, stream, maps, q);
     count_launch();
     return true;
 }

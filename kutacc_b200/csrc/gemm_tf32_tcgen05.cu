@@ -23,6 +23,7 @@
 // released and the host-visible error word carries the site.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -113,6 +114,8 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tf32x3_tc_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    release_successor();
+    wait_for_predecessor();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
 
@@ -242,6 +245,8 @@ struct SplitArgs {
 // dst[r, 0..K) = tf32 head of src[r, :], dst[r, K..2K) = src - head (fp32, at most 12 significant bits)
 __global__ void __launch_bounds__(256) split_tf32_kernel(const SplitArgs args, int64_t src_ld, int64_t rows, int K)
 {
+    release_successor();
+    wait_for_predecessor();
     const float *__restrict__ src = args.src[blockIdx.y];
     float *__restrict__ dst = args.dst[blockIdx.y];
     const int kv = K / 4;
@@ -284,7 +289,7 @@ bool launch_split_tf32_many(cudaStream_t stream, int count, const void *const *s
     const int64_t total = rows * (K / 4);
     const unsigned gx = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 16);
     KernelTimer timer__("split_tf32", stream);
-    split_tf32_kernel<<<dim3(gx, (unsigned)count), 256, 0, stream>>>(a, src_ld, rows, K);
+    launch_chained(split_tf32_kernel, dim3(gx, (unsigned)count), 256, 0, stream, a, src_ld, rows, K);
     count_launch();
     return true;
 }
@@ -332,7 +337,7 @@ bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *c
     const int64_t tiles = ((M + BM - 1) / BM) * (int64_t)(N / BN) * nseg;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
     KernelTimer timer__("gemm_tf32x3_tc", stream);
-    gemm_tf32x3_tc_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(maps, p);
+    launch_chained(gemm_tf32x3_tc_kernel, grid, THREADS, SMEM_BYTES, stream, maps, p);
     count_launch();
     return true;
 }

@@ -7,6 +7,7 @@
 // type (none for fp32).
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 
 #include <algorithm>
@@ -402,6 +403,8 @@ __global__ void __launch_bounds__(256) pair_bias_mma_kernel(const __nv_bfloat16 
     constexpr int ROWB = CZ * 2, CHUNKS = ROWB / 16, TP = 128, STAGES = 3, STAGE_BYTES = TP * ROWB;
     extern __shared__ __align__(128) unsigned char pb_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    release_successor();
+    wait_for_predecessor();
     uint32_t bf[CZ / 16][2];
 #pragma unroll
     for (int ks = 0; ks < CZ / 16; ++ks) {
@@ -481,7 +484,7 @@ bool launch_pair_bias_mma(cudaStream_t stream, const void *z, const void *wb, vo
     }
     const int64_t ntiles = (total + 127) / 128;
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, 148 * 2);
-    pair_bias_mma_kernel<CZ, LN><<<grid, 256, SMEM, stream>>>((const __nv_bfloat16 *)z, (const __nv_bfloat16 *)wb,
+    launch_chained(pair_bias_mma_kernel<CZ, LN>, grid, 256, SMEM, stream, (const __nv_bfloat16 *)z, (const __nv_bfloat16 *)wb,
                                                               (__nv_bfloat16 *)nb, nb_head_stride, total, H,
                                                               (const float2 *)stats, ln_s, ln_t, nk, nb_row_stride);
     return true;

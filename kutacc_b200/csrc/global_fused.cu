@@ -22,6 +22,7 @@
 // them after normalising.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -631,6 +632,15 @@ global_fused_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
         tma_prefetch_desc(&xmap);
         tma_prefetch_desc(&omap);
     }
+    if (warp == K::MMA_WARP) {
+        tmem_alloc(smem_u32(&sm.tmem_base), K::TMEM_COLS);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    release_successor();
+    wait_for_predecessor();
     // weights, once per CTA: 16-byte chunks, swizzled by row for the three 64 x 64 matrices
     for (int idx = tid; idx < FC * 8; idx += K::NTHREADS) {
         const int r = idx >> 3, c = idx & 7;
@@ -654,13 +664,8 @@ global_fused_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
             sm.mask[0][r] = ok ? mask_bits[(int64_t)cluster_id * a.S + row_base + r] : (unsigned short)0;
         }
     }
-    if (warp == K::MMA_WARP) {
-        tmem_alloc(smem_u32(&sm.tmem_base), K::TMEM_COLS);
-        tmem_relinquish();
-    }
-    tc_fence_before();
+    fence_proxy_async();            // the tensor cores read the weights written above
     __syncthreads();
-    tc_fence_after();
     cluster_barrier_all();          // every CTA's barriers exist before a peer arrives on them
 
     if (warp == K::IO_WARP) {
@@ -712,7 +717,9 @@ bool launch_fused(cudaStream_t stream, const void *x, const void *out, int64_t o
         attr_set[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)a.ncta;
     attr[0].val.clusterDim.y = 1;
@@ -737,6 +744,7 @@ bool launch_fused(cudaStream_t stream, const void *x, const void *out, int64_t o
     if (max_clusters[dev][a.ncta] < 1) return false;
     const int nclusters = std::min(a.B, max_clusters[dev][a.ncta]);
     cfg.gridDim = dim3((unsigned)(nclusters * a.ncta));
+    cfg.numAttrs = 2;
 
     CUtensorMap xmap, omap;
     if (!make_tensor_map_bf16_3d(&xmap, x, FC, (uint64_t)a.S, (uint64_t)a.B, FC, (uint64_t)a.S * FC, FC, CH_ROWS, 128))

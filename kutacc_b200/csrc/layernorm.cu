@@ -12,6 +12,7 @@
 // partial sums are added differs (SVE lanes there, warp lanes here).
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 
 #include <algorithm>
@@ -32,6 +33,8 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __nv_bfloat16
                                                              int64_t x_stride, int64_t out_stride, float eps)
 {
     constexpr int RPW = 32 / LPR;                              // rows per warp and step
+    release_successor();
+    wait_for_predecessor();
     const int lane = threadIdx.x & 31, sub = lane / LPR, l = lane % LPR;
     const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -166,7 +169,8 @@ bool launch_layernorm_rows(cudaStream_t stream, const void *x, const float *gamm
     if (vec) {
         const int nv = (int)(size / 8);
 #define KUTACC_LN_LAUNCH(LPR, NVEC)                                                                                   \
-    layernorm_rows_kernel<LPR, NVEC><<<grid, 256, 0, stream>>>(xp, gamma, beta, op, rows, (int)size, x_stride, out_stride, eps)
+    launch_chained(layernorm_rows_kernel<LPR, NVEC>, grid, 256, 0, stream, xp, gamma, beta, op, rows, (int)size, x_stride,    \
+                   out_stride, eps)
         if (nv <= 8)
             KUTACC_LN_LAUNCH(8, 1);
         else if (nv <= 16)

@@ -17,6 +17,7 @@
 //   ln_fold_kernel  : folded weights, s and t for up to four weight matrices (a few hundred KB, once per call)
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 
 #include <algorithm>
@@ -49,6 +50,8 @@ __global__ void __launch_bounds__(256) ln_stats_vec_kernel(const __nv_bfloat16 *
                                                            int64_t x_stride, float eps, float2 *__restrict__ stats)
 {
     constexpr int R = 32 / G;                                    // rows per warp and pass
+    release_successor();
+    wait_for_predecessor();
     const int lane = threadIdx.x & 31, l = lane % G, gi = lane / G;
     const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * R;
@@ -146,6 +149,8 @@ __global__ void __launch_bounds__(256) ln_fold_kernel(const FoldArgs a, const fl
 {
     const int lane = threadIdx.x & 31;
     const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    release_successor();
+    wait_for_predecessor();
     if (warp >= N * nmat) return;
     const int mat = warp / N, n = warp % N;
     const __nv_bfloat16 *wr = a.w[mat] + (int64_t)n * K;
@@ -191,13 +196,13 @@ bool launch_ln_stats(cudaStream_t stream, const void *x, int64_t rows, int64_t s
         const int64_t rows_per_block = 8 * (32 / g) * NR;                   // 8 warps, NR rows in flight per group
         const unsigned grid = (unsigned)std::min<int64_t>((rows + rows_per_block - 1) / rows_per_block, 148 * 8);
         if (g == 4)
-            ln_stats_vec_kernel<4><<<grid, 256, 0, stream>>>(xp, rows, (int)size, x_stride, eps, sp);
+            launch_chained(ln_stats_vec_kernel<4>, grid, 256, 0, stream, xp, rows, (int)size, x_stride, eps, sp);
         else if (g == 8)
-            ln_stats_vec_kernel<8><<<grid, 256, 0, stream>>>(xp, rows, (int)size, x_stride, eps, sp);
+            launch_chained(ln_stats_vec_kernel<8>, grid, 256, 0, stream, xp, rows, (int)size, x_stride, eps, sp);
         else if (g == 16)
-            ln_stats_vec_kernel<16><<<grid, 256, 0, stream>>>(xp, rows, (int)size, x_stride, eps, sp);
+            launch_chained(ln_stats_vec_kernel<16>, grid, 256, 0, stream, xp, rows, (int)size, x_stride, eps, sp);
         else
-            ln_stats_vec_kernel<32><<<grid, 256, 0, stream>>>(xp, rows, (int)size, x_stride, eps, sp);
+            launch_chained(ln_stats_vec_kernel<32>, grid, 256, 0, stream, xp, rows, (int)size, x_stride, eps, sp);
     } else {
         const unsigned grid = (unsigned)std::min<int64_t>((rows + 7) / 8, 148 * 16);
         ln_stats_kernel<<<grid, 256, 0, stream>>>(xp, rows, (int)size, x_stride, eps, sp);
@@ -221,7 +226,7 @@ bool launch_ln_fold(cudaStream_t stream, int nmat, const void *const *w, const f
     }
     const int warps = N * nmat;
     KernelTimer timer__("ln_fold", stream);
-    ln_fold_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>(a, gamma, beta, N, K, nmat);
+    launch_chained(ln_fold_kernel, (unsigned)((warps + 7) / 8), 256, 0, stream, a, gamma, beta, N, K, nmat);
     count_launch();
     return true;
 }

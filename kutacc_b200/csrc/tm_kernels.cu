@@ -4,6 +4,7 @@
 // the shape allows it and on the plain kernels below otherwise.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 
 #include <algorithm>
@@ -98,6 +99,8 @@ __global__ void __launch_bounds__(256) tm_repitch_kernel(const __nv_bfloat16 *__
                                                          uint4 *__restrict__ dst, int vecs, int c_i, int n)
 {
     const int64_t total = (int64_t)c_i * n * vecs;
+    release_successor();
+    wait_for_predecessor();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int v = (int)(t % vecs);
         const int64_t line = t / vecs;
@@ -124,6 +127,8 @@ __global__ void tm_last_kernel(__nv_bfloat16 *__restrict__ out, int64_t o_rs, co
                                int64_t g_rs, int64_t rows, int64_t c_o)
 {
     const int64_t per_row = VEC ? c_o / 8 : c_o;
+    release_successor();
+    wait_for_predecessor();
     const int64_t total = rows * per_row;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = t / per_row, i = (t % per_row) * (VEC ? 8 : 1);
@@ -198,7 +203,7 @@ bool launch_tm_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64
 {
     if (d_pitch % 8 != 0 || d_pitch < n || ((uintptr_t)dst & 15u) || c_i > INT32_MAX || n > INT32_MAX) return false;
     KernelTimer timer__("tm_repitch", stream);
-    tm_repitch_kernel<<<grid_for(c_i * n * (d_pitch / 8), 256), 256, 0, stream>>>(
+    launch_chained(tm_repitch_kernel, grid_for(c_i * n * (d_pitch / 8), 256), 256, 0, stream,
         (const __nv_bfloat16 *)src, s_s0, s_s1, (uint4 *)dst, (int)(d_pitch / 8), (int)c_i, (int)n);
     count_launch();
     return true;
@@ -209,10 +214,10 @@ bool launch_tm_last(cudaStream_t stream, void *out, int64_t o_rs, const void *ga
     const bool vec = c_o % 8 == 0 && o_rs % 8 == 0 && g_rs % 8 == 0 && ((((uintptr_t)out | (uintptr_t)gate) & 15u) == 0);
     KernelTimer timer__("tm_last", stream);
     if (vec)
-        tm_last_kernel<true><<<grid_for(rows * c_o / 8, 256), 256, 0, stream>>>((__nv_bfloat16 *)out, o_rs,
+        launch_chained(tm_last_kernel<true>, grid_for(rows * c_o / 8, 256), 256, 0, stream, (__nv_bfloat16 *)out, o_rs,
                                                                                   (const __nv_bfloat16 *)gate, g_rs, rows, c_o);
     else
-        tm_last_kernel<false><<<grid_for(rows * c_o, 256), 256, 0, stream>>>((__nv_bfloat16 *)out, o_rs,
+        launch_chained(tm_last_kernel<false>, grid_for(rows * c_o, 256), 256, 0, stream, (__nv_bfloat16 *)out, o_rs,
                                                                                (const __nv_bfloat16 *)gate, g_rs, rows, c_o);
     count_launch();
     return true;

@@ -18,6 +18,7 @@
 // and the host-visible error word carries the site.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -80,6 +81,8 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    release_successor();
+    wait_for_predecessor();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
     tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
@@ -232,7 +235,7 @@ bool tcgen05_tm_proj_bf16(cudaStream_t stream, const void *x, const void *wp, co
     const int64_t tiles = (int64_t)B * ((S + BM - 1) / BM) * (N / BN);
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
     KernelTimer timer__("tm_proj", stream);
-    tm_proj_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tx, tp, tg, p);
+    launch_chained(tm_proj_kernel, grid, THREADS, SMEM_BYTES, stream, tx, tp, tg, p);
     count_launch();
     return true;
 }

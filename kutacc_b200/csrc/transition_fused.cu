@@ -21,6 +21,7 @@
 // and the host-visible error word carries the site.
 #include "common.h"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -103,8 +104,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         mbar_init(o_free, 16);
         fence_barrier_init();
     }
-    for (int i = threadIdx.x; i < p.hidden; i += THREADS) bias1[i] = p.b1[i];
-    for (int i = threadIdx.x; i < CO; i += THREADS) bias2[i] = p.b2[i];
     if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
@@ -112,6 +111,11 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    release_successor();
+    wait_for_predecessor();
+    for (int i = threadIdx.x; i < p.hidden; i += THREADS) bias1[i] = p.b1[i];
+    for (int i = threadIdx.x; i < CO; i += THREADS) bias2[i] = p.b2[i];
+    __syncthreads();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
     tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
@@ -412,7 +416,7 @@ bool launch_co(cudaStream_t stream, const CUtensorMap &tx, const CUtensorMap &t1
     const int rows = BM * (CO == 128 ? p.tiles : 1), steps = (p.M + rows - 1) / rows;
     const unsigned grid = (unsigned)std::min(steps, std::max(1, sm_count() - runtime().sm_margin));
     KernelTimer timer__("transition", stream);
-    transition_kernel<CO><<<grid, THREADS, SMEM_BYTES, stream>>>(tx, t1, t2, to, p);
+    launch_chained(transition_kernel<CO>, grid, THREADS, SMEM_BYTES, stream, tx, t1, t2, to, p);
     count_launch();
     return true;
 }

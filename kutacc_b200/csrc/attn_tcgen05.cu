@@ -550,40 +550,9 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
         configured = true;
     }
     const unsigned grid = (unsigned)std::min<int64_t>(p.n_items, std::max(1, sm_count() - runtime().sm_margin));
-    // One pair of counters per STREAM: launches on one stream run one after another, so they can share a pair (the
-    // last CTA of a launch zeroes it again), while launches on different streams may overlap and must not. Up to 63
-    // streams per device get a pair of their own; further streams share the last pair, which is only safe while they
-    // do not run attention kernels at the same time.
-    constexpr int kCounters = 64;
-    static int *counters[64] = {};                       // per device
-    static cudaStream_t owner[64][kCounters] = {};
-    static int owners[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return false;
-    if (counters[dev] == nullptr) {
-        int *c = nullptr;
-        KUTACC_CUDA(cudaMalloc(&c, 2 * kCounters * sizeof(int)));
-        if (c == nullptr) return false;
-        KUTACC_CUDA(cudaMemset(c, 0, 2 * kCounters * sizeof(int)));
-        counters[dev] = c;
-    }
-    int slot = -1;
-    for (int i = 0; i < owners[dev]; ++i)
-        if (owner[dev][i] == stream) {
-            slot = i;
-            break;
-        }
-    if (slot < 0) {
-        if (owners[dev] < kCounters - 1) {
-            slot = owners[dev]++;
-            owner[dev][slot] = stream;
-        } else {
-            slot = kCounters - 1;
-        }
-    }
     AttnParams q = p;
-    q.counter = counters[dev] + 2 * slot;
+    q.counter = work_counter(stream);
+    if (q.counter == nullptr) return false;
     KernelTimer timer__("attn_core", stream);
     launch_chained(attn_tc_kernel<D, HAS_NB>, grid, THREADS, smem_bytes<D>(p.G, HAS_NB), stream, tq, tk, tvt, tnb, q);
     count_launch();

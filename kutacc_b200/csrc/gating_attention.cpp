@@ -91,8 +91,12 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     const bool downloads_in_flight = rt.out_hazard;          // of an earlier enqueue-only call with a HOST result
     if (!rt.reserve_stage(stage, pipelined)) return;
     const int64_t s_pad8 = (S + 7) / 8 * 8;
-    const size_t nb_pad_bytes = has_nb ? (size_t)H * S * s_pad8 * 2 : 0;
-    const size_t v_bytes = std::max(x_bytes, (size_t)B * C * s_pad8 * es);   // v may be stored key-major with padded rows
+    const size_t nb_pad_bytes = has_nb ? (size_t)H * S * s_pad8 * es : 0;
+    // fp32 on the tensor-memory kernels (head size 32): k and v are stored split into tf32 head and tail
+    const bool f32_split = dt == kFP32 && C % 128 == 0 && D == 32 && out_rs % 4 == 0;
+    const size_t k_bytes = f32_split ? 2 * x_bytes : x_bytes;
+    // v may be stored key-major with padded rows
+    const size_t v_bytes = std::max(x_bytes, (size_t)B * C * s_pad8 * es) * (f32_split ? 2 : 1);
     // with LayerNorm: row statistics, four folded weights with their s and t, and (for shapes the folded projection does
     // not cover) a normalised copy of the activations
     const size_t ln_bytes = ln ? (size_t)M * 8 + 4 * (w_bytes + 256) + 8 * (b_bytes + 256) + x_bytes + 1024 : 0;
@@ -100,7 +104,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     // projection and, later, the output projection use in turn; five weights [C, 2C])
     const bool f32_tc = dt == kFP32 && C % 128 == 0 && out_rs % 4 == 0;
     const size_t f32_bytes = f32_tc ? 2 * x_bytes + 256 + 5 * (2 * w_bytes + 256) : 0;
-    if (!rt.reserve_workspace(4 * (x_bytes + 256) + v_bytes + 256 + nb_pad_bytes + 256 + ln_bytes + f32_bytes)) return;
+    if (!rt.reserve_workspace(3 * (x_bytes + 256) + k_bytes + 256 + v_bytes + 256 + nb_pad_bytes + 256 + ln_bytes + f32_bytes)) return;
 
     // The staged output is placed first: its address tells whether downloads of an earlier enqueue-only call, still
     // in flight, read the very block this call will fill. A call of the same shape (same block, same chunks) lets its
@@ -134,7 +138,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         KUTACC_CUDA(cudaStreamWaitEvent((cudaStream_t)cp0.in, (cudaEvent_t)cp0.start, 0));
         KUTACC_CUDA(cudaStreamWaitEvent((cudaStream_t)cp0.out, (cudaEvent_t)cp0.start, 0));
     }
-    char *wq_ = (char *)rt.take_workspace(x_bytes), *wk_ = (char *)rt.take_workspace(x_bytes),
+    char *wq_ = (char *)rt.take_workspace(x_bytes), *wk_ = (char *)rt.take_workspace(k_bytes),
          *wv_ = (char *)rt.take_workspace(v_bytes), *wg_ = (char *)rt.take_workspace(x_bytes),
          *wavg = (char *)rt.take_workspace(x_bytes);
     void *nb_pad = nb_pad_bytes ? rt.take_workspace(nb_pad_bytes) : nullptr;
@@ -174,17 +178,15 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     if (!has_nb || staged_bytes_needed(nonbatched_bias.data_ptr(), nb_bytes) != 0) nb_event = nullptr;   // nothing to wait for / host data
 
     // The TMA loads of the pair bias need 16-byte aligned rows. A pair bias whose strides are not
-    // multiples of 8 elements is first copied into the workspace with padded rows.
+    // multiples of 16 bytes is first copied into the workspace with padded rows.
     const void *nb_dev = has_nb ? d_nb.dev : nullptr;
     int64_t nb_sh = nb_s0, nb_sq = nb_s1;
-    if (fast && has_nb && ((nb_s0 % 8) || (nb_s1 % 8) || !aligned16(d_nb.dev))) {
+    const int64_t nb_unit = dt == kFP32 ? 4 : 8;      // elements of 16 bytes
+    if ((fast || f32_split) && has_nb && ((nb_s0 % nb_unit) || (nb_s1 % nb_unit) || !aligned16(d_nb.dev))) {
         wait_for_pair_bias();                         // the re-pitching copy reads it
-        KUTACC_CUDA(cudaMemcpy2DAsync(nb_pad, (size_t)s_pad8 * 2, d_nb.dev, (size_t)nb_s1 * 2, (size_t)S * 2,
-                                      (size_t)(nb_s0 == S * nb_s1 ? H * S : S), cudaMemcpyDeviceToDevice, stream));
-        for (int64_t hh = 1; nb_s0 != S * nb_s1 && hh < H; ++hh)
-            KUTACC_CUDA(cudaMemcpy2DAsync((char *)nb_pad + (size_t)hh * S * s_pad8 * 2, (size_t)s_pad8 * 2,
-                                          (const char *)d_nb.dev + (size_t)hh * nb_s0 * 2, (size_t)nb_s1 * 2,
-                                          (size_t)S * 2, (size_t)S, cudaMemcpyDeviceToDevice, stream));
+        const bool copied = dev::launch_repitch(stream, d_nb.dev, nb_s0, nb_s1, nb_pad, s_pad8, H, S, (int)es);
+        KUTACC_CHECK(copied, "gating_attention: pair bias could not be re-pitched");
+        if (kutacc_check_err_set) return;
         nb_dev = nb_pad;
         nb_sq = s_pad8;
         nb_sh = S * s_pad8;
@@ -267,24 +269,40 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
             const dev::ElemType et = dt == kFP32 ? dev::kElemF32 : dev::kElemBF16;
             char *v_c = wv_ + b0 * row_bytes;
             char *as_c = f32_tc_ok ? a_split + 2 * b0 * row_bytes : nullptr;
-            bool projected = false;
-            if (f32_tc_ok) {
-                // fp32: all four projections in one pass of the tensor-memory GEMM over the split activations
-                const float *pb[4] = {nullptr, nullptr, nullptr, (const float *)d_bg.dev};
-                void *po[4] = {q_c, k_c, v_c, g_c};
-                projected = dev::launch_split_tf32(stream, x_c, C, as_c, Mc, (int)C) &&
-                            dev::tcgen05_gemm_tf32x3(stream, as_c, w_split, pb, po, C, Mc, (int)C, (int)C, 4);
-            }
-            ok = projected || dev::launch_gemm_generic(stream, et, x_c, C, d_wq.dev, C, nullptr, 0.f, q_c, C, Mc, C, C);
-            ok = ok && (projected || dev::launch_gemm_generic(stream, et, x_c, C, d_wk.dev, C, nullptr, 0.f, k_c, C, Mc, C, C));
-            ok = ok && (projected || dev::launch_gemm_generic(stream, et, x_c, C, d_wv.dev, C, nullptr, 0.f, v_c, C, Mc, C, C));
-            ok = ok && (projected || dev::launch_gemm_generic(stream, et, x_c, C, d_wg.dev, C, (const float *)d_bg.dev, 0.f,
-                                                              g_c, C, Mc, C, C));
-            wait_for_pair_bias();
+            const float *gb_dev = (const float *)d_bg.dev;
             // fp32 with the tensor-memory GEMM after it: the attention core writes its result already split into
             // tf32 head and tail, in the rows of the output projection's operand
-            bool avg_is_split = false;
-            if (ok && dt == kFP32 && f32_tc_ok)
+            bool avg_is_split = false, projected = false;
+            ok = true;
+            if (f32_tc_ok) {
+                // all four projections in one pass of the tensor-memory GEMM over the split activations
+                const float *pb[4] = {nullptr, nullptr, nullptr, gb_dev};
+                const dev::Tf32Layout split[4] = {dev::kTf32Rows, dev::kTf32SplitRows, dev::kTf32SplitTransposed, dev::kTf32Rows};
+                char *k_s = wk_ + 2 * b0 * row_bytes, *v_s = wv_ + (size_t)b0 * 2 * C * s_pad8 * es;
+                void *po[4] = {q_c, f32_split ? k_s : k_c, f32_split ? v_s : v_c, g_c};
+                projected = dev::launch_split_tf32(stream, x_c, C, as_c, Mc, (int)C) &&
+                            dev::tcgen05_gemm_tf32x3(stream, as_c, w_split, pb, po, C, Mc, (int)C, (int)C, 4,
+                                                     f32_split ? split : nullptr, (int)S, s_pad8);
+                wait_for_pair_bias();
+                if (projected && f32_split) {
+                    avg_is_split = dev::tcgen05_attn_f32(stream, q_c, k_s, v_s, s_pad8, g_c, bias_c, bias_s0, nb_dev, nb_sh, nb_sq,
+                                                         as_c, (int)nbr, (int)S, (int)H, (int)D, scale);
+                    // a shape or pair-bias layout that core does not take: k and v once more as plain rows
+                    if (!avg_is_split) {
+                        void *pk[2] = {k_c, v_c};
+                        const float *nobias[2] = {nullptr, nullptr};
+                        projected = dev::tcgen05_gemm_tf32x3(stream, as_c, &w_split[1], nobias, pk, C, Mc, (int)C, (int)C, 2);
+                    }
+                }
+            }
+            if (!projected) {
+                const void *w_dev[4] = {d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev};
+                void *o_dev[4] = {q_c, k_c, v_c, g_c};
+                for (int i = 0; i < 4 && ok; ++i)
+                    ok = dev::launch_gemm_generic(stream, et, x_c, C, w_dev[i], C, i == 3 ? gb_dev : nullptr, 0.f, o_dev[i], C, Mc, C, C);
+            }
+            wait_for_pair_bias();
+            if (ok && dt == kFP32 && f32_tc_ok && !avg_is_split)
                 avg_is_split = dev::launch_attn_f32(stream, q_c, k_c, v_c, g_c, bias_c, bias_s0, has_nb ? d_nb.dev : nullptr,
                                                     nb_s0, nb_s1, a_c, (int)nbr, (int)S, (int)H, (int)D, scale, as_c);
             ok = ok && (avg_is_split ||

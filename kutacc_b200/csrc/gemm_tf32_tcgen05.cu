@@ -6,15 +6,17 @@
 // therefore split beforehand (split_tf32_kernel) into a tf32 head and a tail, x = hi + lo with |lo| <= 2^-11 |x|,
 // stored side by side as one row [hi(0..K) | lo(0..K)] of 2K floats, and the product is taken as
 //   lo(A).hi(W) + hi(A).lo(W) + hi(A).hi(W)        (small terms first; lo.lo, about 2^-22 of the result, is dropped)
-// accumulated in fp32 in tensor memory. With the operands laid out like that the three products are ONE K-loop of
-// 3 * K / 32 slab pairs whose TMA column coordinates pick the head or the tail, so the kernel has the plain GEMM's
-// structure: persistent CTAs (two per SM) walk 128 x 128 output tiles;
-//   warp 0      producer: TMA loads of 128 x 32 fp32 slabs of A' and W' (128-byte swizzle) into a 3-stage ring
-//   warp 1      MMA issuer: one elected lane issues tcgen05.mma kind::tf32 (M = 128, N = 128, K = 8) four times per
-//               slab pair into one of two 128-column TMEM accumulators and commits to mbarriers
-//   warps 2-9   epilogue: each warp owns 32 TMEM lanes x 64 columns: tcgen05.ld, bias add, 16-byte global stores
-//               (a thread writes 256 contiguous bytes of its own output row)
+// accumulated in fp32 in tensor memory. Persistent CTAs, one per SM, walk 128 x 256 output tiles (128 x 128 where there are too
+// few of the wide ones to go round or the columns do not divide):
+//   warp 0      producer: per 32-column slab of K one stage with the heads AND tails of A' and W' (TMA, 128-byte swizzle), so
+//               that the three products read each slab from L2 once
+//   warp 1      MMA issuer: one elected lane issues the 12 tcgen05.mma kind::tf32 (K = 8) of a stage into one of two
+//               TMEM accumulators and commits to mbarriers
+//   warps 2-9   epilogue: each warp owns 32 TMEM lanes x half of the columns: tcgen05.ld, bias add, staging tile (32 x 32),
+//               TMA store
 // Up to four weight matrices share one pass over A (the fused Q/K/V/gate projection of the fp32 attention).
+// What bounds it: the way of the operands from L2. Loading the slab pair of each product by itself with 128 x 128 tiles
+// moves 1.6 GB for 32768 x 1024 x 256 (10 TB/s at its 160 us); sharing the slabs halves that.
 //
 // Replaces addmm -> kutacc_core_bgemm_ex of the reference for fp32 tensors
 // (src/attention/gating_attention.cpp:47-66,152-157; src/linear/mm.cpp:46-86).
@@ -29,40 +31,48 @@
 #include "tma_utils.cuh"
 
 #include <algorithm>
+#include <climits>
 
 namespace kutacc {
 namespace dev {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 32;              // BK floats = one 128-byte swizzle row
-constexpr int NSTAGE = 3;
+constexpr int BM = 128, BK = 32;                        // BK floats = one 128-byte swizzle row
 constexpr int ACC_STAGES = 2;
-constexpr int SLAB_BYTES = BM * BK * 4;                 // 16 KB, A' and W' slabs alike
-constexpr int STAGE_BYTES = 2 * SLAB_BYTES;
+constexpr int SLAB_BYTES = 128 * BK * 4;                // 16 KB: 128 rows of A', or of W'
 constexpr int EPI_WARPS = 8;
-constexpr int BAR_OFF = NSTAGE * STAGE_BYTES;
-constexpr int NBARS = 2 * NSTAGE + 2 * ACC_STAGES;
-constexpr int SMEM_BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;
+constexpr int STG_BYTES = 32 * 32 * 4;                  // one staging tile per epilogue warp
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
-constexpr int TMEM_COLS = ACC_STAGES * BN;              // 256: half of the SM's tensor memory (two CTAs per SM)
+
+template <int BN>
+struct Geo {
+    static constexpr int NB = BN / 128;                              // 128-column blocks of a tile
+    static constexpr int STAGE_BYTES = 2 * (1 + NB) * SLAB_BYTES;    // heads and tails of A' and W'
+    static constexpr int NSTAGE = BN == 256 ? 2 : 3;
+    static constexpr int STG_OFF = NSTAGE * STAGE_BYTES;
+    static constexpr int BAR_OFF = STG_OFF + EPI_WARPS * STG_BYTES;
+    static constexpr int NBARS = 2 * NSTAGE + 2 * ACC_STAGES;
+    static constexpr int SMEM_BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;
+    static constexpr int TMEM_COLS = ACC_STAGES * BN;
+    static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
+};
 
 struct alignas(64) Tf32Maps {
     CUtensorMap a;        // A' [M][2K] fp32, box [32, 128], 128-byte swizzle
     CUtensorMap w[4];     // W' [N][2K] fp32 per segment, box [32, 128], 128-byte swizzle
+    CUtensorMap out[4];   // per segment [M][N] (split rows: [M][2N]), box [32, 32], 128-byte swizzle
 };
 
 struct Tf32Params {
     const float *bias[4];   // per segment, may be null
-    float *out[4];          // per segment, [M][ldo]
-    int64_t ldo;
+    float *out_t[4];        // kTf32SplitTransposed segments: [B][N/32][64][S]
+    int layout[4];          // per segment: Tf32Layout
     int M, N, K, nseg;
+    int S;                  // rows per batch row (transposed segments)
+    int64_t vt_pitch;
     int *err;
 };
-
-// instruction descriptor of tcgen05.mma kind::tf32: D fp32, A and B tf32, both K-major, N = 128, M = 128
-constexpr uint32_t kInstrDescTf32 =
-    (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 
 __device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate)
@@ -77,24 +87,26 @@ __device__ __forceinline__ void tc_mma_tf32(uint32_t d_tmem, uint64_t a_desc, ui
         : "memory");
 }
 
-__global__ void __launch_bounds__(THREADS, 2) gemm_tf32x3_tc_kernel(const __grid_constant__ Tf32Maps maps, const Tf32Params p)
+template <int BN>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tf32x3_tc_kernel(const __grid_constant__ Tf32Maps maps, const __grid_constant__ Tf32Params p)
 {
+    using T = Geo<BN>;
+    constexpr int NSTAGE = T::NSTAGE;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bar_base = smem + BAR_OFF;
+    const uint32_t bar_base = smem + T::BAR_OFF;
     auto full_bar = [&](int s) { return bar_base + 8u * (uint32_t)s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (uint32_t)(NSTAGE + s); };
     auto acc_full = [&](int a) { return bar_base + 8u * (uint32_t)(2 * NSTAGE + a); };
     auto acc_empty = [&](int a) { return bar_base + 8u * (uint32_t)(2 * NSTAGE + ACC_STAGES + a); };
-    const uint32_t tmem_slot = bar_base + 8u * NBARS;
+    const uint32_t tmem_slot = bar_base + 8u * T::NBARS;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int m_tiles = (p.M + BM - 1) / BM;
-    const int n_tiles_seg = p.N / BN;
-    const int n_tiles = n_tiles_seg * p.nseg;
+    const int n_tiles = p.N * p.nseg / BN;
     const int num_tiles = m_tiles * n_tiles;
     const int nk = p.K / BK;
-    const int niter = 3 * nk;                           // slab pairs per tile: lo.hi, hi.lo, hi.hi
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
@@ -108,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tf32x3_tc_kernel(const __grid
         fence_barrier_init();
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, TMEM_COLS);
+        tmem_alloc(tmem_slot, T::TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -118,35 +130,42 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tf32x3_tc_kernel(const __grid
     wait_for_predecessor();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
 
     if (warp == 0) {
         // ================= producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_desc(&maps.a);
             int it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile / n_tiles) * BM, n_tile = tile % n_tiles;
-                const int seg = n_tile / n_tiles_seg, n0 = (n_tile % n_tiles_seg) * BN;
-                const CUtensorMap *wmap = &maps.w[seg];
-                for (int j = 0; j < niter; ++j, ++it) {
+                const int m0 = (tile / n_tiles) * BM, c0 = tile % n_tiles * BN;
+                for (int kc = 0; kc < nk; ++kc, ++it) {
                     const int s = it % NSTAGE;
                     if (it >= NSTAGE && !mbar_wait(empty_bar(s), (uint32_t)((it / NSTAGE - 1) & 1), p.err, 41)) {
                         ok = false;
                         break;
                     }
-                    const int prod = j / nk, kc = (j % nk) * BK;
-                    const int a_col = (prod == 0 ? p.K : 0) + kc;        // product 0 reads the tail of A
-                    const int w_col = (prod == 1 ? p.K : 0) + kc;        // product 1 reads the tail of W
-                    const uint32_t st = smem + (uint32_t)s * STAGE_BYTES;
-                    mbar_arrive_expect_tx(full_bar(s), STAGE_BYTES);
-                    tma_load_2d(st, &maps.a, full_bar(s), a_col, m0);
-                    tma_load_2d(st + SLAB_BYTES, wmap, full_bar(s), w_col, n0);
+                    // [A head | A tail | W heads | W tails]
+                    const uint32_t st = smem + (uint32_t)s * T::STAGE_BYTES;
+                    mbar_arrive_expect_tx(full_bar(s), T::STAGE_BYTES);
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        const int col = t * p.K + kc * BK;
+                        tma_load_2d(st + t * SLAB_BYTES, &maps.a, full_bar(s), col, m0);
+#pragma unroll
+                        for (int j = 0; j < T::NB; ++j) {
+                            const int c = c0 + j * 128;
+                            tma_load_2d(st + (2 + t * T::NB + j) * SLAB_BYTES, &maps.w[c / p.N], full_bar(s), col, c % p.N);
+                        }
+                    }
                 }
             }
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
+        constexpr uint32_t idesc = make_instr_desc_tf32(BM, BN);
+        constexpr uint32_t SLAB16 = SLAB_BYTES >> 4;        // descriptor addresses count in units of 16 bytes
         int it = 0, tcount = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
@@ -157,74 +176,112 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tf32x3_tc_kernel(const __grid
             }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(a * BN);
-            for (int j = 0; j < niter; ++j, ++it) {
+            for (int kc = 0; kc < nk; ++kc, ++it) {
                 const int s = it % NSTAGE;
                 if (!mbar_wait_warp(full_bar(s), (uint32_t)((it / NSTAGE) & 1), p.err, 43)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t st = smem + (uint32_t)s * STAGE_BYTES;
+                if (elect_one()) {
+                    const uint64_t ad = make_smem_desc_kmajor(smem + (uint32_t)s * T::STAGE_BYTES, 128), wd = ad + 2 * SLAB16;
 #pragma unroll
-                    for (int k = 0; k < BK / 8; ++k) {               // 8 tf32 = 32 bytes per instruction
-                        const uint64_t adesc = make_smem_desc_kmajor(st + k * 32, 128);
-                        const uint64_t bdesc = make_smem_desc_kmajor(st + SLAB_BYTES + k * 32, 128);
-                        tc_mma_tf32(d_tmem, adesc, bdesc, kInstrDescTf32, (j > 0 || k > 0) ? 1u : 0u);
-                    }
-                    tc_commit(empty_bar(s));                 // slab pair may be overwritten once these MMAs retire
-                    if (j == niter - 1) tc_commit(acc_full(a));
+                    for (int pr = 0; pr < 3; ++pr)                   // tail.head, head.tail, head.head
+#pragma unroll
+                        for (int k = 0; k < BK / 8; ++k)             // 8 tf32 = 32 bytes per instruction
+                            tc_mma_tf32(d_tmem, ad + (pr == 0 ? SLAB16 : 0u) + 2 * k, wd + (pr == 1 ? T::NB * SLAB16 : 0u) + 2 * k,
+                                        idesc, (kc > 0 || pr > 0 || k > 0) ? 1u : 0u);
+                    tc_commit(empty_bar(s));                 // the stage may be overwritten once these MMAs retire
+                    if (kc == nk - 1) tc_commit(acc_full(a));
                 }
                 __syncwarp();
             }
         }
     } else {
         // ================= epilogue =================
+        constexpr int COLS = BN / 2;
         const int quad = warp & 3;                            // TMEM lanes 32*quad .. 32*quad+31
-        const int half = (warp - 2) >> 2;                     // which 64 columns of the 128-column tile
+        const int ew = warp - 2, half = ew >> 2;              // which half of the tile's columns
+        const uint32_t stg = smem + T::STG_OFF + (uint32_t)ew * STG_BYTES;
         int tcount = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tcount) {
-            const int m0 = (tile / n_tiles) * BM, n_tile = tile % n_tiles;
-            const int seg = n_tile / n_tiles_seg, n0 = (n_tile % n_tiles_seg) * BN;
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++tcount) {
+            const int m0 = (tile / n_tiles) * BM + quad * 32, c0 = tile % n_tiles * BN + half * COLS;
+            const int seg = c0 / p.N, n0 = c0 % p.N;
             const int a = tcount % ACC_STAGES;
-            if (!mbar_wait_warp(acc_full(a), (uint32_t)((tcount / ACC_STAGES) & 1), p.err, 44)) {
-                ok = false;
-                break;
-            }
+            if (!mbar_wait_warp(acc_full(a), (uint32_t)((tcount / ACC_STAGES) & 1), p.err, 44)) break;
             tc_fence_after();
             const float *bias = p.bias[seg];
-            const int m = m0 + quad * 32 + lane;
-            float *orow = p.out[seg] + (int64_t)(m < p.M ? m : 0) * p.ldo + n0 + half * 64;
-            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + half * 64);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            const int layout = p.layout[seg], m = m0 + lane;
+            const CUtensorMap *omap = &maps.out[seg];
+            float *tdst = nullptr;                            // transposed segments: this row's place in the first head
+            if (layout == kTf32SplitTransposed) {
+                const int b = m / p.S;
+                tdst = p.out_t[seg] + ((int64_t)b * (p.N / 32) + n0 / 32) * 64 * p.vt_pitch + (m - b * p.S);
+            }
+            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + half * COLS);
+#pragma unroll 1
+            for (int c = 0; c < COLS / 32; ++c) {
                 uint32_t r[32];
+                __syncwarp();
                 tmem_ld_32x32(tcol + c * 32, r);
                 tmem_ld_wait();
-                if (c == 1) {
-                    // both halves are in registers: the accumulator may be overwritten by the tile after next
+                if (c == COLS / 32 - 1) {
+                    // everything is in registers: the accumulator may be overwritten by the tile after next
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(acc_empty(a));
                 }
-                if (m < p.M) {
+                const int n = n0 + c * 32;
+                if (bias) {
+#pragma unroll
+                    for (int j4 = 0; j4 < 8; ++j4) {
+                        const float4 bv = __ldg(reinterpret_cast<const float4 *>(bias + n) + j4);
+                        r[4 * j4] = __float_as_uint(__uint_as_float(r[4 * j4]) + bv.x);
+                        r[4 * j4 + 1] = __float_as_uint(__uint_as_float(r[4 * j4 + 1]) + bv.y);
+                        r[4 * j4 + 2] = __float_as_uint(__uint_as_float(r[4 * j4 + 2]) + bv.z);
+                        r[4 * j4 + 3] = __float_as_uint(__uint_as_float(r[4 * j4 + 3]) + bv.w);
+                    }
+                }
+                if (layout == kTf32SplitTransposed) {
+                    // one head of 32 channels, split; the lanes of a store run along the sequence
+                    if (m < p.M) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const float v = __uint_as_float(r[j]), h = tf32_head(v);
+                            tdst[j * p.vt_pitch] = h;
+                            tdst[(32 + j) * p.vt_pitch] = v - h;
+                        }
+                    }
+                    tdst += 64 * p.vt_pitch;
+                    continue;
+                }
+                // rows, or rows with every 32 channels as [head | tail]
+                const bool split = layout == kTf32SplitRows;
+                for (int t = 0; t < (split ? 2 : 1); ++t) {
+                    if (lane == 0) tma_store_wait_read<0>();          // the store out of the staging tile has been read
+                    __syncwarp();
 #pragma unroll
                     for (int j4 = 0; j4 < 8; ++j4) {
                         float4 v = make_float4(__uint_as_float(r[4 * j4]), __uint_as_float(r[4 * j4 + 1]),
                                                __uint_as_float(r[4 * j4 + 2]), __uint_as_float(r[4 * j4 + 3]));
-                        if (bias) {
-                            const float4 bv = __ldg(reinterpret_cast<const float4 *>(bias + n0 + half * 64 + c * 32) + j4);
-                            v.x += bv.x;
-                            v.y += bv.y;
-                            v.z += bv.z;
-                            v.w += bv.w;
+                        if (split) {
+                            const float4 h = make_float4(tf32_head(v.x), tf32_head(v.y), tf32_head(v.z), tf32_head(v.w));
+                            v = t == 0 ? h : make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
                         }
-                        reinterpret_cast<float4 *>(orow + c * 32)[j4] = v;
+                        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(stg + (uint32_t)(lane * 128 + ((j4 ^ (lane & 7)) << 4))),
+                                     "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                                     : "memory");
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_2d(omap, stg, split ? 2 * n + 32 * t : n, m0);
+                        tma_store_commit();
                     }
                 }
             }
         }
+        if (lane == 0) tma_store_wait<0>();
     }
 
     // ================= common tail =================
@@ -232,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tf32x3_tc_kernel(const __grid
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc(tmem_base, T::TMEM_COLS);
     }
 }
 
@@ -249,27 +306,26 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const SplitArgs args, i
     wait_for_predecessor();
     const float *__restrict__ src = args.src[blockIdx.y];
     float *__restrict__ dst = args.dst[blockIdx.y];
-    const int kv = K / 4;
-    const int64_t total = rows * kv;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / kv;
-        const int c = (int)(i % kv) * 4;
-        const float4 v = __ldg(reinterpret_cast<const float4 *>(src + r * src_ld + c));
-        float4 hi, lo;
-        const float x[4] = {v.x, v.y, v.z, v.w};
-        float h[4], l[4];
+    const uint32_t kv = (uint32_t)K / 4, total = (uint32_t)rows * kv, step = gridDim.x * blockDim.x;
+    constexpr int U = 4;                                     // loads in flight per thread
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += U * step) {
+        float4 v[U];
+        uint32_t r[U], c[U];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            uint32_t t;
-            asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(t) : "f"(x[e]));
-            h[e] = __uint_as_float(t);
-            l[e] = x[e] - h[e];
+        for (int u = 0; u < U; ++u) {
+            const uint32_t i = i0 + u * step < total ? i0 + u * step : i0;
+            r[u] = i / kv;
+            c[u] = i % kv * 4;
+            v[u] = __ldg(reinterpret_cast<const float4 *>(src + (int64_t)r[u] * src_ld + c[u]));
         }
-        hi = make_float4(h[0], h[1], h[2], h[3]);
-        lo = make_float4(l[0], l[1], l[2], l[3]);
-        float *d = dst + r * 2 * K;
-        *reinterpret_cast<float4 *>(d + c) = hi;
-        *reinterpret_cast<float4 *>(d + K + c) = lo;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i0 + u * step >= total) continue;
+            const float4 h = make_float4(tf32_head(v[u].x), tf32_head(v[u].y), tf32_head(v[u].z), tf32_head(v[u].w));
+            float *d = dst + (int64_t)r[u] * 2 * K + c[u];
+            *reinterpret_cast<float4 *>(d) = h;
+            *reinterpret_cast<float4 *>(d + K) = make_float4(v[u].x - h.x, v[u].y - h.y, v[u].z - h.z, v[u].w - h.w);
+        }
     }
 }
 
@@ -278,7 +334,7 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const SplitArgs args, i
 bool launch_split_tf32_many(cudaStream_t stream, int count, const void *const *src, int64_t src_ld, void *const *dst,
                             int64_t rows, int K)
 {
-    if (count < 1 || count > 8 || rows <= 0 || K <= 0 || K % 4 != 0 || src_ld % 4 != 0) return false;
+    if (count < 1 || count > 8 || rows <= 0 || K <= 0 || K % 4 != 0 || src_ld % 4 != 0 || rows * (K / 4) > INT32_MAX / 2) return false;
     SplitArgs a;
     for (int i = 0; i < 8; ++i) {
         const int j = i < count ? i : 0;
@@ -287,7 +343,7 @@ bool launch_split_tf32_many(cudaStream_t stream, int count, const void *const *s
         a.dst[i] = (float *)dst[j];
     }
     const int64_t total = rows * (K / 4);
-    const unsigned gx = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 16);
+    const unsigned gx = (unsigned)std::min<int64_t>((total + 1023) / 1024, (int64_t)sm_count() * 8);
     KernelTimer timer__("split_tf32", stream);
     launch_chained(split_tf32_kernel, dim3(gx, (unsigned)count), 256, 0, stream, a, src_ld, rows, K);
     count_launch();
@@ -300,9 +356,10 @@ bool launch_split_tf32(cudaStream_t stream, const void *src, int64_t src_ld, voi
 }
 
 bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *const *w_split, const float *const *bias,
-                         void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg)
+                         void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg, const Tf32Layout *layout, int S,
+                         int64_t vt_pitch)
 {
-    if (nseg < 1 || nseg > 4 || M <= 0 || M > INT32_MAX / 2 || N % BN != 0 || K % BK != 0 || K <= 0 || ldo % 4 != 0 ||
+    if (nseg < 1 || nseg > 4 || M <= 0 || M > INT32_MAX / 2 || N % 128 != 0 || K % BK != 0 || K <= 0 || ldo % 4 != 0 ||
         ldo < N || (((uintptr_t)a_split) & 15u))
         return false;
     for (int i = 0; i < nseg; ++i)
@@ -310,34 +367,46 @@ bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *c
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     Tf32Maps maps;
+    Tf32Params p;
     if (!make_tensor_map_2d(&maps.a, a_split, /*elem_bytes=*/4, (uint64_t)2 * K, (uint64_t)M, (uint64_t)2 * K, BK, BM, 128))
         return false;
     for (int i = 0; i < 4; ++i) {
         const int j = i < nseg ? i : 0;
-        if (!make_tensor_map_2d(&maps.w[i], w_split[j], 4, (uint64_t)2 * K, (uint64_t)N, (uint64_t)2 * K, BK, BN, 128))
+        p.bias[i] = bias[j];
+        p.layout[i] = layout ? layout[j] : kTf32Rows;
+        p.out_t[i] = (float *)out[j];
+        if (!make_tensor_map_2d(&maps.w[i], w_split[j], 4, (uint64_t)2 * K, (uint64_t)N, (uint64_t)2 * K, BK, 128, 128))
+            return false;
+        const uint64_t cols = p.layout[i] == kTf32SplitRows ? 2 * (uint64_t)N : (uint64_t)N;
+        if (p.layout[i] == kTf32SplitTransposed)
+            maps.out[i] = maps.a;                            // stored directly
+        else if (!make_tensor_map_2d(&maps.out[i], out[j], 4, cols, (uint64_t)M,
+                                     p.layout[i] == kTf32SplitRows ? cols : (uint64_t)ldo, 32, 32, 128))
             return false;
     }
-    Tf32Params p;
-    for (int i = 0; i < 4; ++i) {
-        const int j = i < nseg ? i : 0;
-        p.bias[i] = bias[j];
-        p.out[i] = (float *)out[j];
-    }
-    p.ldo = ldo;
     p.M = (int)M;
     p.N = N;
     p.K = K;
     p.nseg = nseg;
+    p.S = S > 0 ? S : 1;
+    p.vt_pitch = vt_pitch;
     p.err = ew.device;
     static bool configured = false;
     if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(gemm_tf32x3_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        KUTACC_CUDA(cudaFuncSetAttribute(gemm_tf32x3_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<128>::SMEM_BYTES));
+        KUTACC_CUDA(cudaFuncSetAttribute(gemm_tf32x3_tc_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<256>::SMEM_BYTES));
         configured = true;
     }
-    const int64_t tiles = ((M + BM - 1) / BM) * (int64_t)(N / BN) * nseg;
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
+    const int sms = std::max(1, sm_count() - runtime().sm_margin);
+    const int64_t blocks = ((M + BM - 1) / BM) * (int64_t)(N / 128) * nseg;      // 128 x 128
+    const bool wide = (int64_t)N * nseg % 256 == 0 && blocks / 2 >= sms;
+    const int64_t tiles = wide ? blocks / 2 : blocks;
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, sms);
     KernelTimer timer__("gemm_tf32x3_tc", stream);
-    launch_chained(gemm_tf32x3_tc_kernel, grid, THREADS, SMEM_BYTES, stream, maps, p);
+    if (wide)
+        launch_chained(gemm_tf32x3_tc_kernel<256>, grid, THREADS, Geo<256>::SMEM_BYTES, stream, maps, p);
+    else
+        launch_chained(gemm_tf32x3_tc_kernel<128>, grid, THREADS, Geo<128>::SMEM_BYTES, stream, maps, p);
     count_launch();
     return true;
 }

@@ -64,8 +64,13 @@ bool launch_split_tf32(cudaStream_t stream, const void *src, int64_t src_ld, voi
 // the same for up to eight matrices of one shape in a single launch
 bool launch_split_tf32_many(cudaStream_t stream, int count, const void *const *src, int64_t src_ld, void *const *dst,
                             int64_t rows, int K);
+// `layout` (one per weight matrix, null = rows): how out_i is stored. The attention layouts take 32 channels as a head of
+// batch rows of S positions and split every value into tf32 head and tail: kTf32SplitRows [M, N/32, 64] and
+// kTf32SplitTransposed [M/S, N/32, 64, S] with row pitch vt_pitch.
+enum Tf32Layout { kTf32Rows = 0, kTf32SplitRows = 1, kTf32SplitTransposed = 2 };
 bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *const *w_split, const float *const *bias,
-                         void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg);
+                         void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg, const Tf32Layout *layout = nullptr,
+                         int S = 0, int64_t vt_pitch = 0);
 
 // ---- triangle multiplication: element-wise steps and fallbacks (tm_kernels.cu) ------------------------
 // proj[c, b, i] = bf16((f32(proj) * f32(mask[b, i])) * sigmoid(f32(gate[c, b, i]))) in place; strides in elements.
@@ -80,10 +85,10 @@ bool launch_tm_proj_generic(cudaStream_t stream, const void *x, const void *w0, 
 bool launch_tm_equation_generic(cudaStream_t stream, const void *left, int64_t l_s0, int64_t l_s1, const void *right,
                                 int64_t r_s0, int64_t r_s1, void *center, int64_t c_s0, int64_t c_s1, int64_t c_i,
                                 int64_t n, bool incoming);
-// dst[c, r, :] = src[c, r, :] for c_i matrices of n x n elements: rows moved from any stride to a pitch that is a multiple of
-// 8 elements (dst dense, 16-byte aligned)
-bool launch_tm_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
-                       int64_t c_i, int64_t n);
+// dst[c, r, :] = src[c, r, :] for c_i matrices of n x n elements (2 or 4 bytes): rows moved from any stride to a pitch that is
+// a multiple of 16 bytes (dst dense, 16-byte aligned)
+bool launch_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
+                    int64_t c_i, int64_t n, int elem_bytes = 2);
 // out[r, :] = bf16(f32(out[r, :]) * sigmoid(f32(gate[r, :]))) for rows of c_o elements
 bool launch_tm_last(cudaStream_t stream, void *out, int64_t o_rs, const void *gate, int64_t g_rs, int64_t rows, int64_t c_o);
 
@@ -136,6 +141,13 @@ bool launch_pair_bias_ln(cudaStream_t stream, const void *z, const void *wb_fold
 bool launch_attn_f32(cudaStream_t stream, const void *q, const void *k, const void *v, const void *gate, const void *bias,
                      int64_t bias_stride0, const void *nb, int64_t nb_stride_h, int64_t nb_stride_q, void *avg, int B,
                      int S, int H, int D, float scale, void *avg_split = nullptr);
+
+// The same operator on tcgen05 (attn_f32_tcgen05.cu): q, gate [B, S, H*32] fp32, k_split and vt_split as tcgen05_gemm_tf32x3
+// stores them (kTf32SplitRows, kTf32SplitTransposed), pair-bias strides multiples of 4 elements and its base 16-byte
+// aligned; result as rows [tf32 head | tail] in avg_split. False for other shapes.
+bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, const void *vt_split, int64_t vt_pitch,
+                      const void *gate, const void *bias, int64_t bias_stride0, const void *nb, int64_t nb_stride_h,
+                      int64_t nb_stride_q, void *avg_split, int B, int S, int H, int D, float scale);
 
 // LayerNorm folded into the projection that follows (ln_fold.cu): per-row (mean, rstd) pairs as float2, and
 // for up to four [N, K] weight matrices the folded, centred bf16 weights with the epilogue terms s and t

@@ -155,5 +155,18 @@ __host__ __device__ constexpr uint32_t make_instr_desc_bf16(int M, int N)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// the same for tf32 operands
+__host__ __device__ constexpr uint32_t make_instr_desc_tf32(int M, int N)
+{
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// x rounded to tf32 (11 significant bits)
+__device__ __forceinline__ float tf32_head(float x)
+{
+    uint32_t r;
+    asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(r) : "f"(x));
+    return __uint_as_float(r);
+}
+
 }  // namespace dev
 }  // namespace kutacc

@@ -117,6 +117,23 @@ bool make_tensor_map_bf16_4d(CUtensorMap *map, const void *base, uint64_t d0, ui
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, 4, dims, strides, box, swizzle_bytes);
 }
 
+bool make_tensor_map_f32_4d(CUtensorMap *map, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t d3,
+                            uint64_t stride1, uint64_t stride2, uint64_t stride3, uint32_t box0, uint32_t box1, uint32_t box3,
+                            int swizzle_bytes)
+{
+    const cuuint64_t dims[4] = {d0, d1, d2, d3}, strides[3] = {stride1 * 4, stride2 * 4, stride3 * 4};
+    const cuuint32_t box[4] = {box0, box1, 1, box3};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, 4, dims, strides, box, swizzle_bytes);
+}
+
+bool make_tensor_map_f32_3d(CUtensorMap *map, const void *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1,
+                            uint64_t stride2, uint32_t box0, uint32_t box1, int swizzle_bytes)
+{
+    const cuuint64_t dims[3] = {d0, d1, d2}, strides[2] = {stride1 * 4, stride2 * 4};
+    const cuuint32_t box[3] = {box0, box1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, 3, dims, strides, box, swizzle_bytes);
+}
+
 bool make_tensor_map_2d(CUtensorMap *map, const void *base, int elem_bytes, uint64_t d0, uint64_t d1, uint64_t stride1,
                         uint32_t box0, uint32_t box1, int swizzle_bytes)
 {
@@ -137,6 +154,43 @@ int sm_count()
         if (n <= 0) n = 148;
     }
     return n;
+}
+
+// One pair of counters per STREAM: launches on one stream run one after another, so they can share a pair (the last CTA of a
+// launch zeroes it again), while launches on different streams may overlap and must not. Up to 63 streams per device get a
+// pair of their own; further streams share the last pair, which is only safe while they do not run attention kernels at
+// the same time.
+int *work_counter(cudaStream_t stream)
+{
+    constexpr int kCounters = 64;
+    static int *counters[64] = {};                       // per device
+    static cudaStream_t owner[64][kCounters] = {};
+    static int owners[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return nullptr;
+    if (counters[dev] == nullptr) {
+        int *c = nullptr;
+        KUTACC_CUDA(cudaMalloc(&c, 2 * kCounters * sizeof(int)));
+        if (c == nullptr) return nullptr;
+        KUTACC_CUDA(cudaMemset(c, 0, 2 * kCounters * sizeof(int)));
+        counters[dev] = c;
+    }
+    int slot = -1;
+    for (int i = 0; i < owners[dev]; ++i)
+        if (owner[dev][i] == stream) {
+            slot = i;
+            break;
+        }
+    if (slot < 0) {
+        if (owners[dev] < kCounters - 1) {
+            slot = owners[dev]++;
+            owner[dev][slot] = stream;
+        } else {
+            slot = kCounters - 1;
+        }
+    }
+    return counters[dev] + 2 * slot;
 }
 
 KernelErrorWord &kernel_error_word()

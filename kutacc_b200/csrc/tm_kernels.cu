@@ -95,7 +95,7 @@ __global__ void tm_equation_generic_kernel(const __nv_bfloat16 *__restrict__ lef
 // Rows of n elements to a pitch of `vecs` 16-byte vectors. A thread moves one vector: the five aligned 32-bit words that
 // cover it in the source, shifted together when the source starts on an odd element (the words past the row belong to the
 // vector's padding; those past the matrix's last row are not read).
-__global__ void __launch_bounds__(256) tm_repitch_kernel(const __nv_bfloat16 *__restrict__ src, int64_t s_s0, int64_t s_s1,
+__global__ void __launch_bounds__(256) repitch_bf16_kernel(const __nv_bfloat16 *__restrict__ src, int64_t s_s0, int64_t s_s1,
                                                          uint4 *__restrict__ dst, int vecs, int c_i, int n)
 {
     const int64_t total = (int64_t)c_i * n * vecs;
@@ -119,6 +119,23 @@ __global__ void __launch_bounds__(256) tm_repitch_kernel(const __nv_bfloat16 *__
         else
             o = make_uint4(w[0], w[1], w[2], w[3]);
         dst[t] = o;
+    }
+}
+
+__global__ void __launch_bounds__(256) repitch_f32_kernel(const float *__restrict__ src, int64_t s_s0, int64_t s_s1,
+                                                          float4 *__restrict__ dst, int vecs, int c_i, int n)
+{
+    const int64_t total = (int64_t)c_i * n * vecs;
+    release_successor();
+    wait_for_predecessor();
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+        const int v = (int)(t % vecs);
+        const int64_t line = t / vecs;
+        const float *sp = src + line / n * s_s0 + line % n * s_s1 + v * 4;
+        float w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = v * 4 + i < n ? __ldg(sp + i) : 0.f;
+        dst[t] = make_float4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -198,14 +215,18 @@ bool launch_tm_equation_generic(cudaStream_t stream, const void *left, int64_t l
     return true;
 }
 
-bool launch_tm_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
-                       int64_t c_i, int64_t n)
+// (A copy, like the 2-D device copies of other operands: not counted among the operators' kernels.)
+bool launch_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch, int64_t c_i,
+                    int64_t n, int elem_bytes)
 {
-    if (d_pitch % 8 != 0 || d_pitch < n || ((uintptr_t)dst & 15u) || c_i > INT32_MAX || n > INT32_MAX) return false;
-    KernelTimer timer__("tm_repitch", stream);
-    launch_chained(tm_repitch_kernel, grid_for(c_i * n * (d_pitch / 8), 256), 256, 0, stream,
-        (const __nv_bfloat16 *)src, s_s0, s_s1, (uint4 *)dst, (int)(d_pitch / 8), (int)c_i, (int)n);
-    count_launch();
+    if (d_pitch * elem_bytes % 16 != 0 || d_pitch < n || ((uintptr_t)dst & 15u) || c_i > INT32_MAX || n > INT32_MAX) return false;
+    KernelTimer timer__("repitch", stream);
+    if (elem_bytes == 4)
+        launch_chained(repitch_f32_kernel, grid_for(c_i * n * (d_pitch / 4), 256), 256, 0, stream, (const float *)src, s_s0, s_s1,
+                       (float4 *)dst, (int)(d_pitch / 4), (int)c_i, (int)n);
+    else
+        launch_chained(repitch_bf16_kernel, grid_for(c_i * n * (d_pitch / 8), 256), 256, 0, stream,
+                       (const __nv_bfloat16 *)src, s_s0, s_s1, (uint4 *)dst, (int)(d_pitch / 8), (int)c_i, (int)n);
     return true;
 }
 

@@ -151,6 +151,7 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
 #pragma unroll 1
             for (int c = 0; c < 4; ++c) {
                 uint32_t rp[16], rg[16];
+                __syncwarp();
                 tmem_ld_32x16(tcol + c * 16, rp);
                 tmem_ld_32x16(tcol + BN + c * 16, rg);
                 tmem_ld_wait16(rp);

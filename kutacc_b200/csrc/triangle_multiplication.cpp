@@ -140,7 +140,7 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
         o = {p, s0, s1};
         if (((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0) return true;
         o = {pad, n * pitch, pitch};
-        return dev::launch_tm_repitch(stream, p, s0, s1, pad, pitch, c_i, n);
+        return dev::launch_repitch(stream, p, s0, s1, pad, pitch, c_i, n);
     };
     Operand ol, orr;
     bool ok = aligned_rows(d_l.dev, l_s0, l_s1, pad_l, ol) && aligned_rows(d_r.dev, r_s0, r_s1, pad_r, orr);

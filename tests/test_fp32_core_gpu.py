@@ -1,0 +1,67 @@
+"""fp32 attention core on tensor memory at the edges of its tiles (128 queries, 32 keys, one or two batch rows per work item),
+with pair-bias strides that are and are not multiples of 16 bytes; the fp32 pair-bias projection."""
+import numpy as np
+import pytest
+import torch
+
+from kutacc_b200 import api, runner
+from kutacc_b200 import workloads as W
+from . import helpers
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("with_nb", [True, False])
+@pytest.mark.parametrize("B,S,H", [(1, 1, 4), (2, 31, 4), (3, 33, 8), (2, 64, 4), (5, 129, 4), (81, 130, 4), (40, 257, 8)])
+def test_core_matches_exact_oracle(kutacc_lib, B, S, H, with_nb):
+    w = W.random_gating_case(seed=2000 + S, B=B, S=S, H=H, D=32, dtype="fp32", with_nb=with_nb, full_mask_rows=1 if B > 1 else 0)
+    api.set_profile(True)
+    api.profile_read()
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    names = [n for n, _ in api.profile_read()]
+    api.set_profile(False)
+    assert "attn_f32_tc" in names and np.isfinite(got).all()
+    rows = list(range(B)) if B <= 6 else [0, 1, 2, B - 3, B - 2, B - 1]
+    ref = W.Workload(name="pick", kind="gating", dtype=w.dtype, B=len(rows), S=S, H=H, D=32, seed=0, has_nb=w.has_nb)
+    ref.arrays = dict(w.arrays, x=w.arrays["x"][rows], mask=w.arrays["mask"][rows], bias=w.arrays["bias"][rows])
+    assert helpers.rel_err(got[rows], helpers.oracle_exact(ref)) <= helpers.FP32_TOL / 4
+
+
+def test_running_max_that_grows_late(kutacc_lib):
+    w = W.random_gating_case(seed=31, B=4, S=200, H=4, D=32, dtype="fp32", with_nb=True, mask_frac=0.0)
+    mask = np.ones((4, 200), np.float32)
+    mask[0, :40] = 0.0
+    mask[1, :150] = 0.0
+    mask[2, 5:190] = 0.0
+    w.arrays["mask"], w.arrays["bias"] = mask, (1e9 * (mask - 1.0)).astype(np.float32)
+    w.arrays["nb"] = w.arrays["nb"].copy()
+    w.arrays["nb"][:, :, 100:110] += 40.0
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
+
+
+# 128 x 128 tiles, 128 x 256 tiles (enough of them to go round), ragged rows, K of one and several slabs
+@pytest.mark.parametrize("M,N,K", [(1, 128, 32), (129, 384, 64), (20000, 256, 96), (9600, 512, 32)])
+def test_linear_fp32(kutacc_lib, M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w, b = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g) / K ** 0.5, torch.randn(N, generator=g)
+    ad, wd, bd, r = a.cuda(), w.cuda(), b.cuda(), torch.zeros(M, N, device="cuda")
+    api.linear(api.tensor(ad), api.tensor(wd), bd.data_ptr(), api.tensor(r))
+    torch.cuda.synchronize()
+    ref = a.double() @ w.double().T + b.double()
+    assert (r.cpu().double() - ref).abs().max() <= 4e-6 * ref.abs().max()
+
+
+@pytest.mark.parametrize("R,Nk,Cz,H", [(8, 100, 128, 8), (3, 33, 64, 4), (1, 1, 32, 3), (40, 301, 128, 1)])
+def test_pair_bias_fp32(kutacc_lib, R, Nk, Cz, H):
+    g = torch.Generator().manual_seed(R * Nk + Cz)
+    z, wb = torch.randn(R, Nk, Cz, generator=g), torch.randn(H, Cz, generator=g) / Cz ** 0.5
+    store = torch.full((R, H + 1, Nk), 7.0, device="cuda")
+    nb = torch.zeros(H, R, Nk, device="cuda")
+    zd, wd = z.cuda(), wb.cuda()
+    api.pair_bias(api.tensor(zd), api.tensor(wd), api.tensor(nb))
+    api.pair_bias(api.tensor(zd), api.tensor(wd), api.Tensor(store.data_ptr(), [H, R, Nk], [Nk, (H + 1) * Nk, 1], api.DTYPE_FP32, keep=store))
+    torch.cuda.synchronize()
+    ref = torch.einsum("rkc,hc->hrk", z.double(), wb.double())
+    assert (nb.cpu().double() - ref).abs().max() <= 1e-5 * ref.abs().max()
+    assert torch.equal(store[:, :H].permute(1, 0, 2), nb) and bool((store[:, H] == 7.0).all())

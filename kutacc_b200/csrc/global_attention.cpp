@@ -55,7 +55,8 @@ extern "C" void kutacc_af2_global_attention(kutacc_af2_attention_inputs_t *q_bas
                    staged_bytes_needed(wg.data_ptr(), wcc) + staged_bytes_needed(wo.data_ptr(), wcc) +
                    staged_bytes_needed(bg.data_ptr(), bb) + staged_bytes_needed(bo.data_ptr(), bb);
     if (!rt.reserve_stage(stage)) return;
-    const size_t scratch_bytes = dev::global_attention_scratch_bytes((int)B, (int)S, (int)H, (int)D);
+    const size_t scratch_bytes = std::max(dev::global_attention_scratch_bytes((int)B, (int)S, (int)H, (int)D),
+                                          dev::global_stream_scratch_bytes(B, S));
     if (!rt.reserve_workspace(scratch_bytes + 256)) return;
     // Host-resident activations and result: the batch columns are independent, so they go through in
     // chunks with upload, kernels and download overlapped on three streams (as in the gated attention).
@@ -83,15 +84,15 @@ extern "C" void kutacc_af2_global_attention(kutacc_af2_attention_inputs_t *q_bas
                    (uintptr_t)d_wq.dev | (uintptr_t)d_wk.dev | (uintptr_t)d_wv.dev) & 15u) == 0,
                  "global_attention: q_data, out and the five weights must be 16-byte aligned");
     if (kutacc_check_err_set) return;
-    // one pass over HBM where the shape allows it (a cluster of CTAs holds each column in shared memory),
-    // otherwise three kernels per L2-sized group of columns with the split-softmax state in `scratch`
+    // three streaming kernels for 8 heads x 8 (k, v and partial sums in `scratch`), otherwise three kernels per L2-sized group
+    // of columns with the split-softmax state in `scratch`
     auto run_cols = [&](int64_t b0, int64_t nb) -> bool {
         const char *xc = (const char *)d_x.dev + (size_t)b0 * S * C * 2;
         const char *mc = (const char *)d_m.dev + (size_t)b0 * S * 2;
         char *oc = (char *)d_out.dev + (size_t)b0 * S * out_rs * 2;
-        bool done = dev::launch_global_fused_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
-                                                  (const float *)d_bg.dev, d_wo.dev, (const float *)d_bo.dev, oc, out_rs,
-                                                  (int)nb, (int)S, (int)H, (int)D);
+        bool done = dev::launch_global_stream_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
+                                                   (const float *)d_bg.dev, d_wo.dev, (const float *)d_bo.dev, oc, out_rs,
+                                                   scratch, (int)nb, (int)S, (int)H, (int)D);
         if (kutacc_check_err_set) return false;
         if (!done)
             done = dev::launch_global_attention_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,

@@ -139,71 +139,6 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
     return __all_sync(0xffffffffu, ok);
 }
 
-// ---- device: thread-block clusters and distributed shared memory --------------------------------------
-__device__ __forceinline__ uint32_t cluster_cta_rank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-// address of the same shared-memory location in CTA `rank` of this cluster
-__device__ __forceinline__ uint32_t map_shared_rank(uint32_t addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_shared_cluster_f32(uint32_t addr, float v)
-{
-    asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(addr), "f"(v) : "memory");
-}
-// fire-and-forget store of one word into another CTA's shared memory; the destination CTA's mbarrier
-// receives 4 transaction bytes when the word has landed (it must expect them: mbar_arrive_expect_tx)
-__device__ __forceinline__ void st_async_cluster_f32(uint32_t remote_addr, float v, uint32_t remote_bar)
-{
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(remote_addr),
-                 "r"(__float_as_uint(v)), "r"(remote_bar)
-                 : "memory");
-}
-__device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;\n" ::: "memory"); }
-// arrive on an mbarrier that lives in another CTA of the cluster; releases this thread's earlier writes
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t remote_bar)
-{
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(remote_bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait on a barrier that CTAs of the whole cluster arrive on (acquire at cluster scope).
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int *err, int code)
-{
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait_cluster(bar, parity)) {
-        if (clock64() - t0 > 4000000000LL) {
-            if (err) atomicCAS(err, 0, code);
-            return false;
-        }
-    }
-    return true;
-}
-// Hardware barrier over every thread of the cluster. Only used where all threads are known to arrive.
-__device__ __forceinline__ void cluster_barrier_all()
-{
-    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
-}
-
 // ---- device: TMA -----------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map)
 {
@@ -237,6 +172,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
         : "memory");
+}
+// untiled copy: 16-byte aligned addresses, a size that is a multiple of 16 bytes
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
 }
 // shared -> global tile store (bulk async group)
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int c0, int c1)

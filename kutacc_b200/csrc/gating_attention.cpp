@@ -192,9 +192,11 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         nb_sh = S * s_pad8;
     }
 
-    // LayerNorm in front: folded into the tcgen05 projection where that kernel runs (head sizes up to 32), otherwise the
-    // rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy
-    const bool ln_folded = ln && fast && D <= 32 && (C % 128 == 0 || C == 64);
+    // LayerNorm in front (head sizes up to 32): up to 256 channels the projection normalises its rows itself, on their way to
+    // the tensor cores; wider rows do not fit beside the weights, and there LayerNorm is folded into the weights. Otherwise
+    // the rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy.
+    const bool ln_in_proj = ln && fast && D <= 32 && (C == 64 || C == 128 || C == 256);
+    const bool ln_folded = ln && fast && D <= 32 && C % 128 == 0 && !ln_in_proj;
     if (ln_folded) {
         const void *w_in[4] = {d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev};
         const float *b_in[4] = {nullptr, nullptr, nullptr, (const float *)d_bg.dev};
@@ -215,7 +217,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         const size_t row_bytes = (size_t)S * C * es;                       // one batch row of a [B, S, C]-sized buffer
         const char *x_c = (const char *)d_x.dev + b0 * row_bytes;
         char *st_c = ln ? ln_stats + (size_t)b0 * S * 8 : nullptr;
-        if (ln && !ln_folded) {
+        if (ln && !ln_folded && !ln_in_proj) {
             if (!dev::launch_layernorm_rows(stream, x_c, (const float *)d_lg.dev, (const float *)d_lb.dev, x_norm + b0 * row_bytes,
                                             nbr * S, C, C, C, ln->eps))
                 return false;
@@ -241,12 +243,18 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
                                                  ln_s, ln_t);
                 if (!ok) return false;
                 v_key_major = true;
-            } else if (D <= 32) {
+            } else if (D <= 32 && dev::tcgen05_proj_rows_bf16(stream, x_c, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
+                                                              (const float *)d_bg.dev, q_c, k_c, v_km, s_pad8, g_c, (int)nbr, (int)S,
+                                                              (int)H, (int)D, ln ? (const float *)d_lg.dev : nullptr,
+                                                              ln ? (const float *)d_lb.dev : nullptr, ln ? ln->eps : 0.f)) {
+                ok = v_key_major = true;
+            } else if (D <= 32 && !ln_in_proj) {
                 ok = dev::tcgen05_proj_qkvg_bf16(stream, x_c, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
                                                  (const float *)d_bg.dev, q_c, k_c, v_km, g_c, (int)nbr, (int)S, (int)H,
                                                  (int)D, true, s_pad8, /*gate_sigmoid=*/true);
                 v_key_major = ok;
             }
+            if (ln_in_proj && !ok) return false;
             if (!ok)
                 ok = dev::tcgen05_proj_qkvg_bf16(stream, x_c, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
                                                  (const float *)d_bg.dev, q_c, k_c, v_c, g_c, (int)nbr, (int)S, (int)H,

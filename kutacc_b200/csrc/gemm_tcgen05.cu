@@ -33,6 +33,7 @@
 #include "tma_utils.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <utility>
 
 namespace kutacc {
@@ -516,6 +517,11 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
                               int64_t out_row_stride, int B, int S, int N, int K, bool relu, int64_t a_row_stride)
 {
     if (a_row_stride <= 0) a_row_stride = K;
+    // the rows of all batch rows lie evenly: one long batch row, no tile ends early
+    if ((int64_t)B * S <= INT32_MAX / 2) {
+        S *= B;
+        B = 1;
+    }
     if ((N % 128 != 0 && (N != 64 || relu)) || K % 64 != 0 || out_row_stride % 8 != 0 || a_row_stride % 8 != 0 || a_row_stride < K ||
         ((uintptr_t)out & 15u) || ((uintptr_t)a & 15u) || ((uintptr_t)w & 15u) || ((uintptr_t)bias & 15u))
         return false;

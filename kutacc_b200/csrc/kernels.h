@@ -35,6 +35,12 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
                             int H, int D, bool v_transposed, int64_t v_pitch, bool gate_sigmoid = false,
                             const void *ln_stats = nullptr, const float *const *ln_s = nullptr,
                             const float *const *ln_t = nullptr);
+// The same for up to 256 channels with the rows kept in shared memory while the weights stream past (gemm_proj.cu): q and k
+// [B, H, S, D], v^T [B, H*D, S] with row pitch vt_pitch, gate = bf16(sigmoid(bf16(x.Wg + bg))) [B, S, C]. With ln_gamma the
+// projections are those of LayerNorm(x). C in {64, 128, 256}, D in {8, 16, 32}; false otherwise.
+bool tcgen05_proj_rows_bf16(cudaStream_t stream, const void *x, const void *wq, const void *wk, const void *wv, const void *wg,
+                            const float *bg, void *q, void *k, void *vt, int64_t vt_pitch, void *gate, int B, int S, int H, int D,
+                            const float *ln_gamma, const float *ln_beta, float ln_eps);
 // a_row_stride (elements, 0 = K): row stride of a, whose batch rows are S rows apart.
 bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w, const float *bias, void *out,
                               int64_t out_row_stride, int B, int S, int N, int K, bool relu = false,

@@ -7,12 +7,16 @@
 // persistent CTA (one per SM) loads a block of 256 rows once, all K columns of it, and streams the four weights past it in
 // slabs of 128 channels x 64 columns, each of which serves both 128-row tiles of the block. With a 128 x 128 tile at a time
 // every tile brought its own 64 to 128 KB of operands from L2, which bound the kernel: 146 us for 196608 rows x 256 channels.
-//   warp 0      producer: row blocks (two in flight up to 128 channels), weight slabs (ring)
+//   warp 0      producer: row blocks in slabs of 64 columns (two blocks in flight up to 128 channels), weight slabs (ring)
 //   warp 1      MMA issuer: 128 x 128 accumulators, two row tiles x two column tiles in tensor memory
 //   warps 4-19  epilogue, eight per row tile, 32 rows x 64 columns each: tcgen05.ld, bias and sigmoid for the gate, bf16,
 //               staging tile, TMA store into the destination layout
 // A row tile is four groups of 32 rows, and a group never crosses a batch row: S is padded to 32, not to 128, and the TMA
 // stores of a warp (32 rows) stay inside one batch row. Rows past S are zero-filled on load and clipped on store.
+//
+// What bounds it: at 128 channels the writes to memory (2^20 rows: 238 us without launch, the bytes alone 205); at 256
+// channels the products, whose 128 x 128 instructions read 128 bytes of shared memory per clock (196608 rows: 105 us, of which
+// about 60 on the tensor cores; 77 for the bytes). Before: 266 and 140 us.
 //
 // LayerNorm: the epilogue warps normalise the block where it lies in shared memory (statistics and arithmetic of layernorm.cu,
 // one bf16 rounding), 16 rows each, before the products read it; for 128 channels the next block's turn comes after the
@@ -51,7 +55,7 @@ struct Geo {
     static constexpr int OFF_STG = OFF_A + NBLK * BLOCK_BYTES;
     static constexpr int OFF_VEC = OFF_STG + EPI_WARPS * STG_BYTES;  // gate bias
     static constexpr int OFF_BAR = OFF_VEC + KS * 64 * 4;
-    static constexpr int NBARS = 2 * NW + 3 * NBLK + 8;
+    static constexpr int NBARS = 2 * NW + NBLK * (2 * KS + 1) + 8;
     static constexpr int SMEM_BYTES = OFF_BAR + 8 * NBARS + 16 + 1024;
     static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
 };
@@ -68,8 +72,8 @@ struct ProjParams {
     int S, B, D;
     int s32;              // 32-row groups per batch row
     int rows128;          // S is a multiple of 128: a row tile is one box
-    int R;                // row tiles per block: 1 or 2
-    int nsplit;           // a unit of work is a block x 1 / nsplit of the column tiles
+    int whole;            // a unit of work is a block with all its column tiles, up to this unit;
+    int nsplit;           // after it a unit is 1 / nsplit of a block's column tiles
     int units;
     int *err;
 };
@@ -80,7 +84,8 @@ __device__ __forceinline__ float sigmoid_of_bf16(float y)
     return fmaf(0.5f, tanh_approx(0.5f * round_to_bf16_f32(y)), 0.5f);
 }
 
-template <int KS, bool LN>
+// R: row tiles per block, 1 or 2
+template <int KS, int R, bool LN>
 __global__ void __launch_bounds__(THREADS, 1)
 proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjParams p)
 {
@@ -92,14 +97,22 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
     const uint32_t bar = smem + T::OFF_BAR;
     auto w_full = [&](int s) { return bar + 8u * (uint32_t)s; };
     auto w_empty = [&](int s) { return bar + 8u * (uint32_t)(NW + s); };
-    auto a_full = [&](int s) { return bar + 8u * (uint32_t)(2 * NW + s); };
-    auto a_norm = [&](int s) { return bar + 8u * (uint32_t)(2 * NW + NBLK + s); };
-    auto a_empty = [&](int s) { return bar + 8u * (uint32_t)(2 * NW + 2 * NBLK + s); };
-    auto acc_full = [&](int i) { return bar + 8u * (uint32_t)(2 * NW + 3 * NBLK + i); };        // i = 2 * buffer + row tile
-    auto acc_empty = [&](int i) { return bar + 8u * (uint32_t)(2 * NW + 3 * NBLK + 4 + i); };
+    // the rows arrive and leave in slabs of 64 columns: the next block follows while the last column tile is at work
+    constexpr int BAR_A = 2 * NW, BAR_ACC = BAR_A + NBLK * (2 * KS + 1);
+    auto a_full = [&](int s, int ks) { return bar + 8u * (uint32_t)(BAR_A + s * (2 * KS + 1) + ks); };
+    auto a_empty = [&](int s, int ks) { return bar + 8u * (uint32_t)(BAR_A + s * (2 * KS + 1) + KS + ks); };
+    auto a_norm = [&](int s) { return bar + 8u * (uint32_t)(BAR_A + s * (2 * KS + 1) + 2 * KS); };
+    auto acc_full = [&](int i) { return bar + 8u * (uint32_t)(BAR_ACC + i); };                  // i = 2 * buffer + row tile
+    auto acc_empty = [&](int i) { return bar + 8u * (uint32_t)(BAR_ACC + 4 + i); };
     const uint32_t tmem_slot = bar + 8u * T::NBARS;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int R = p.R, ntp = NT / p.nsplit;
+    // unit u: its block, first column tile and number of column tiles
+    auto unit = [&](int u, int &block, int &t0, int &nt) {
+        const int v = u - p.whole;
+        block = v < 0 ? u : p.whole + v / p.nsplit;
+        nt = v < 0 ? NT : NT / p.nsplit;
+        t0 = v < 0 ? 0 : v % p.nsplit * nt;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NW; ++s) {
@@ -107,9 +120,11 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
             mbar_init(w_empty(s), 1);
         }
         for (int s = 0; s < NBLK; ++s) {
-            mbar_init(a_full(s), 1);
+            for (int ks = 0; ks < KS; ++ks) {
+                mbar_init(a_full(s, ks), 1);
+                mbar_init(a_empty(s, ks), 1);
+            }
             mbar_init(a_norm(s), (uint32_t)(8 * R));
-            mbar_init(a_empty(s), 1);
         }
         for (int i = 0; i < 4; ++i) {
             mbar_init(acc_full(i), 1);
@@ -138,34 +153,36 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
             tma_prefetch_desc(&maps.a);
             bool ok = true;
             int wit = 0;
-            auto load_block = [&](int n) {                             // this CTA's n-th unit
+            auto load_rows = [&](int n, int ks) {                      // a slab of the rows of this CTA's n-th unit
                 const int u = (int)blockIdx.x + n * (int)gridDim.x, s = n % NBLK;
                 if (u >= p.units || !ok) return;
-                if (n >= NBLK) ok = mbar_wait(a_empty(s), (uint32_t)((n / NBLK - 1) & 1), p.err, 101);
+                int block, t0, nt;
+                unit(u, block, t0, nt);
+                if (n >= NBLK) ok = mbar_wait(a_empty(s, ks), (uint32_t)((n / NBLK - 1) & 1), p.err, 101);
                 if (!ok) return;
-                mbar_arrive_expect_tx(a_full(s), (uint32_t)(R * KS * SLAB_BYTES));
+                mbar_arrive_expect_tx(a_full(s, ks), (uint32_t)(R * SLAB_BYTES));
                 for (int r = 0; r < R; ++r) {
-                    const int g0 = (u / p.nsplit * R + r) * 4;
-                    for (int ks = 0; ks < KS; ++ks) {
-                        const uint32_t dst = smem + OFF_A + s * T::BLOCK_BYTES + (r * KS + ks) * SLAB_BYTES;
-                        if (p.rows128) {
-                            tma_load_3d(dst, &maps.a, a_full(s), ks * BK, g0 % p.s32 * 32, g0 / p.s32);
-                        } else {
-                            for (int q = 0; q < 4; ++q)
-                                tma_load_3d(dst + q * 4096, &maps.a, a_full(s), ks * BK, (g0 + q) % p.s32 * 32, (g0 + q) / p.s32);
-                        }
+                    const int g0 = (block * R + r) * 4;
+                    const uint32_t dst = smem + OFF_A + s * T::BLOCK_BYTES + (r * KS + ks) * SLAB_BYTES;
+                    if (p.rows128) {
+                        tma_load_3d(dst, &maps.a, a_full(s, ks), ks * BK, g0 % p.s32 * 32, g0 / p.s32);
+                    } else {
+                        for (int q = 0; q < 4; ++q)
+                            tma_load_3d(dst + q * 4096, &maps.a, a_full(s, ks), ks * BK, (g0 + q) % p.s32 * 32, (g0 + q) / p.s32);
                     }
                 }
             };
-            load_block(0);
+            for (int ks = 0; ks < KS && NBLK == 2; ++ks) load_rows(0, ks);
             for (int n = 0; ok; ++n) {
                 const int u = (int)blockIdx.x + n * (int)gridDim.x;
                 if (u >= p.units) break;
-                const int t0 = u % p.nsplit * ntp;
-                for (int j = 0; j < ntp && ok; ++j) {
+                int block, t0, nt;
+                unit(u, block, t0, nt);
+                for (int j = 0; j < nt && ok; ++j) {
                     for (int ks = 0; ks < KS && ok; ++ks, ++wit) {
+                        if (NBLK == 1 && j == 0) load_rows(n, ks);
                         const int s = wit % NW;
-                        if (wit >= NW) ok = mbar_wait(w_empty(s), (uint32_t)((wit / NW - 1) & 1), p.err, 102);
+                        if (wit >= NW && ok) ok = mbar_wait(w_empty(s), (uint32_t)((wit / NW - 1) & 1), p.err, 102);
                         if (!ok) break;
                         mbar_arrive_expect_tx(w_full(s), SLAB_BYTES);
                         const uint32_t dst = smem + OFF_W + s * SLAB_BYTES;
@@ -173,9 +190,8 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
                         tma_load_3d(dst, &maps.w[col / C], w_full(s), ks * BK, col % C, 0);
                         if (KS == 1) tma_load_3d(dst + SLAB_BYTES / 2, &maps.w[col / C + 1], w_full(s), ks * BK, 0, 0);
                     }
-                    if (NBLK == 2 && j == 0) load_block(n + 1);
+                    for (int ks = 0; ks < KS && NBLK == 2 && j == 0; ++ks) load_rows(n + 1, ks);
                 }
-                if (NBLK == 1) load_block(n + 1);
             }
         }
     } else if (warp == 1) {
@@ -186,21 +202,25 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
         bool ok = true;
         int wit = 0, tc = 0;
         for (int n = 0; ok; ++n) {
-            if ((int)blockIdx.x + n * (int)gridDim.x >= p.units) break;
-            const int sa = n % NBLK;
-            ok = mbar_wait_warp(LN ? a_norm(sa) : a_full(sa), (uint32_t)((n / NBLK) & 1), p.err, 103);
+            const int u = (int)blockIdx.x + n * (int)gridDim.x, sa = n % NBLK;
+            if (u >= p.units) break;
+            int block, t0, nt;
+            unit(u, block, t0, nt);
+            if (LN) ok = mbar_wait_warp(a_norm(sa), (uint32_t)((n / NBLK) & 1), p.err, 103);
             const uint64_t ad = ad0 + (uint32_t)(sa * (T::BLOCK_BYTES >> 4));
-            for (int j = 0; j < ntp && ok; ++j, ++tc) {
+            for (int j = 0; j < nt && ok; ++j, ++tc) {
                 const int buf = tc & 1;
                 for (int r = 0; r < R && tc >= 2 && ok; ++r)
                     ok = mbar_wait_warp(acc_empty(2 * buf + r), (uint32_t)((tc / 2 - 1) & 1), p.err, 104);
                 for (int ks = 0; ks < KS && ok; ++ks, ++wit) {
                     const int s = wit % NW;
-                    ok = mbar_wait_warp(w_full(s), (uint32_t)((wit / NW) & 1), p.err, 105);
+                    if (!LN && j == 0) ok = mbar_wait_warp(a_full(sa, ks), (uint32_t)((n / NBLK) & 1), p.err, 108);
+                    ok = ok && mbar_wait_warp(w_full(s), (uint32_t)((wit / NW) & 1), p.err, 105);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
                         const uint64_t wd = wd0 + (uint32_t)(s * SLAB16);
+#pragma unroll
                         for (int r = 0; r < R; ++r) {
                             const uint64_t a = ad + (uint32_t)((r * KS + ks) * SLAB16);
                             const uint32_t d = tmem_base + (uint32_t)((2 * buf + r) * BN);
@@ -209,7 +229,7 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
                             if (ks == KS - 1) tc_commit(acc_full(2 * buf + r));
                         }
                         tc_commit(w_empty(s));
-                        if (ks == KS - 1 && j == ntp - 1) tc_commit(a_empty(sa));
+                        if (j == nt - 1) tc_commit(a_empty(sa, ks));
                     }
                     __syncwarp();
                 }
@@ -235,7 +255,7 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
         auto normalise = [&](int n) {
             if ((int)blockIdx.x + n * (int)gridDim.x >= p.units || !ok) return;
             const int sa = n % NBLK, sub = lane / LPR, l = lane % LPR;
-            ok = mbar_wait_warp(a_full(sa), (uint32_t)((n / NBLK) & 1), p.err, 106);
+            for (int ks = 0; ks < KS && ok; ++ks) ok = mbar_wait_warp(a_full(sa, ks), (uint32_t)((n / NBLK) & 1), p.err, 106);
             if (!ok) return;
             const uint32_t base = smem + OFF_A + sa * T::BLOCK_BYTES + (rt * KS + l / 8) * SLAB_BYTES;
             constexpr float inv_n = 1.0f / (float)C;
@@ -295,9 +315,11 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
         for (int n = 0; ok; ++n) {
             const int u = (int)blockIdx.x + n * (int)gridDim.x;
             if (u >= p.units) break;
-            const int G = (u / p.nsplit * R + rt) * 4 + quad, b = G / p.s32, row0 = G % p.s32 * 32;
-            for (int j = 0; j < ntp; ++j, ++tc) {
-                const int buf = tc & 1, col = (u % p.nsplit * ntp + j) * BN + half * 64, seg = col / C;
+            int block, t0, nt;
+            unit(u, block, t0, nt);
+            const int G = (block * R + rt) * 4 + quad, b = G / p.s32, row0 = G % p.s32 * 32;
+            for (int j = 0; j < nt; ++j, ++tc) {
+                const int buf = tc & 1, col = (t0 + j) * BN + half * 64, seg = col / C;
                 ok = mbar_wait_warp(acc_full(2 * buf + rt), (uint32_t)((tc / 2) & 1), p.err, 107);
                 if (!ok) break;
                 tc_fence_after();
@@ -377,38 +399,47 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
     }
 }
 
+template <int KS, int R, bool LN>
+void launch_one(cudaStream_t stream, int grid, const ProjMaps &maps, const ProjParams &p)
+{
+    static const cudaError_t attr =
+        cudaFuncSetAttribute(proj_kernel<KS, R, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES);
+    KUTACC_CUDA(attr);
+    launch_chained(proj_kernel<KS, R, LN>, (unsigned)grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
+}
+
 template <int KS>
 bool launch_ks(cudaStream_t stream, const ProjMaps &maps, ProjParams p)
 {
-    static bool configured = false;
-    if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(proj_kernel<KS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES));
-        KUTACC_CUDA(cudaFuncSetAttribute(proj_kernel<KS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES));
-        configured = true;
-    }
-    // How the work is cut: whole blocks of 256 rows where there are many; otherwise blocks of 128 rows, or a part of the column
-    // tiles per unit, whichever leaves the fullest last wave. A unit costs its column tiles plus about one for its rows.
+    // How the work is cut: blocks of 256 rows, or of 128 where that fills the chip better; whole blocks for all full waves, and
+    // the blocks of the last one in 1 / nsplit of their column tiles each, whichever ends first. A unit costs its column tiles
+    // plus about one for its rows.
     constexpr int NT = 4 * KS * 64 / BN;
     const int sms = std::max(1, sm_count() - runtime().sm_margin);
     const int64_t groups = (int64_t)p.B * p.s32;
     double best = 1e30;
-    for (int R = 2; R >= 1; --R)
+    int R = 2;
+    for (int r = 2; r >= 1; --r) {
+        const int64_t blocks = (groups + 4 * r - 1) / (4 * r), whole = blocks / sms * sms;
         for (int ns = 1; ns <= NT; ns *= 2) {
-            const int64_t units = (groups + 4 * R - 1) / (4 * R) * ns;
-            const double cost = (double)((units + sms - 1) / sms) * (R == 2 ? 1.8 : 1.0) * ((double)NT / ns + 1.0);
-            if (cost < best * 0.999 && units <= INT32_MAX / 2) {
+            const int64_t last = (blocks - whole) * ns;
+            const double cost = ((double)(whole / sms) * (NT + 1.0) + (double)((last + sms - 1) / sms) * ((double)NT / ns + 1.0)) *
+                                (r == 2 ? 1.8 : 1.0);
+            if (cost < best * 0.999) {
                 best = cost;
-                p.R = R;
+                R = r;
+                p.whole = (int)whole;
                 p.nsplit = ns;
-                p.units = (int)units;
+                p.units = (int)(whole + last);
             }
         }
-    const unsigned grid = (unsigned)std::min(p.units, sms);
+    }
+    const int grid = std::min(p.units, sms);
     KernelTimer timer__("proj_qkvg", stream);
     if (p.gamma)
-        launch_chained(proj_kernel<KS, true>, grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
+        R == 2 ? launch_one<KS, 2, true>(stream, grid, maps, p) : launch_one<KS, 1, true>(stream, grid, maps, p);
     else
-        launch_chained(proj_kernel<KS, false>, grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
+        R == 2 ? launch_one<KS, 2, false>(stream, grid, maps, p) : launch_one<KS, 1, false>(stream, grid, maps, p);
     count_launch();
     return true;
 }

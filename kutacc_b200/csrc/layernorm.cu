@@ -24,6 +24,12 @@ namespace {
 
 constexpr int LN_MAX_VEC = 4;          // 16-byte vectors per lane: rows of up to 32 * 8 * 4 = 1024 channels in registers
 
+__device__ __forceinline__ void load_params(const float *a, int v, float (&r)[8])
+{
+    const float4 lo = __ldg(reinterpret_cast<const float4 *>(a) + 2 * v), hi = __ldg(reinterpret_cast<const float4 *>(a) + 2 * v + 1);
+    r[0] = lo.x, r[1] = lo.y, r[2] = lo.z, r[3] = lo.w, r[4] = hi.x, r[5] = hi.y, r[6] = hi.z, r[7] = hi.w;
+}
+
 // LPR lanes share a row (32 / LPR rows per warp and step), each lane holds NVEC 16-byte vectors of it.
 template <int LPR, int NVEC>
 __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __nv_bfloat16 *__restrict__ x,
@@ -43,6 +49,17 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __nv_bfloat16
     // the loop bound depends on the warp only, so that all lanes reach the shuffles together; U rows per lane
     // group and step keep 2 x 16 x NVEC bytes per lane in flight
     constexpr int U = 2;
+    // gamma and beta of this lane's channels stay in registers for rows of up to 512 channels: read again for each row they
+    // keep the L1 cache busier than the rows do (147456 rows x 128: 20.8 us, L1 87 % busy; now 18.5)
+    constexpr bool HOLD = NVEC <= 2;
+    float gh[HOLD ? NVEC : 1][8], bh[HOLD ? NVEC : 1][8];
+    if (HOLD) {
+#pragma unroll
+        for (int i = 0; i < NVEC; ++i) {
+            load_params(gamma, l + LPR * i < nv ? l + LPR * i : 0, gh[i]);
+            load_params(beta, l + LPR * i < nv ? l + LPR * i : 0, bh[i]);
+        }
+    }
     for (int64_t row0 = warp * RPW * U; row0 < rows; row0 += nwarps * RPW * U) {
         int64_t row[U];
         bool live[U];
@@ -58,10 +75,10 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __nv_bfloat16
                 const int v = l + LPR * i;
                 raw[u][i] = v < nv ? __ldg(reinterpret_cast<const uint4 *>(xr) + v) : make_uint4(0, 0, 0, 0);
             }
-            delta[u] = __bfloat162float(xr[0]);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
+            delta[u] = bf16lo_to_f32(__shfl_sync(0xffffffffu, raw[u][0].x, sub * LPR));       // the row's first channel
             sum[u] = sum2[u] = 0.f;
 #pragma unroll
             for (int i = 0; i < NVEC; ++i) {
@@ -97,12 +114,13 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const __nv_bfloat16
                 const int v = l + LPR * i;
                 if (live[u] && v < nv) {
                     const uint32_t w[4] = {raw[u][i].x, raw[u][i].y, raw[u][i].z, raw[u][i].w};
-                    const float4 g0 = __ldg(reinterpret_cast<const float4 *>(gamma) + 2 * v),
-                                 g1 = __ldg(reinterpret_cast<const float4 *>(gamma) + 2 * v + 1);
-                    const float4 b0 = __ldg(reinterpret_cast<const float4 *>(beta) + 2 * v),
-                                 b1 = __ldg(reinterpret_cast<const float4 *>(beta) + 2 * v + 1);
-                    const float gs[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-                    const float bs[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+                    float gt[8], bt[8];
+                    if (!HOLD) {
+                        load_params(gamma, v, gt);
+                        load_params(beta, v, bt);
+                    }
+                    const float(&gs)[8] = HOLD ? gh[HOLD ? i : 0] : gt;
+                    const float(&bs)[8] = HOLD ? bh[HOLD ? i : 0] : bt;
                     uint32_t o[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {

@@ -148,7 +148,7 @@ __global__ void tm_last_kernel(__nv_bfloat16 *__restrict__ out, int64_t o_rs, co
     wait_for_predecessor();
     const int64_t total = rows * per_row;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = t / per_row, i = (t % per_row) * (VEC ? 8 : 1);
+        const int64_t r = rows == 1 ? 0 : t / per_row, i = (rows == 1 ? t : t % per_row) * (VEC ? 8 : 1);
         __nv_bfloat16 *op = out + r * o_rs + i;
         const __nv_bfloat16 *gp = gate + r * g_rs + i;
         if (VEC) {
@@ -233,6 +233,12 @@ bool launch_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t 
 bool launch_tm_last(cudaStream_t stream, void *out, int64_t o_rs, const void *gate, int64_t g_rs, int64_t rows, int64_t c_o)
 {
     const bool vec = c_o % 8 == 0 && o_rs % 8 == 0 && g_rs % 8 == 0 && ((((uintptr_t)out | (uintptr_t)gate) & 15u) == 0);
+    if (o_rs == c_o && g_rs == c_o) {
+        // rows without gaps are one long row: no division per vector
+        c_o *= rows;
+        o_rs = g_rs = c_o;
+        rows = 1;
+    }
     KernelTimer timer__("tm_last", stream);
     if (vec)
         launch_chained(tm_last_kernel<true>, grid_for(rows * c_o / 8, 256), 256, 0, stream, (__nv_bfloat16 *)out, o_rs,

@@ -3,16 +3,19 @@
 //   gate[n, b, s] = bf16(x[b, s, :] . Wg[n, :] + bg[n])
 //   proj[n, b, s] = bf16((bf16(x[b, s, :] . Wp[n, :] + bp[n]) * mask[b, s]) * sigmoid(gate[n, b, s]))
 //
-// (src/attention/triangle_multiplication.cpp:38-69). Persistent CTAs, two per SM; a tile is 128 positions x 128 channels
-// of BOTH products, whose accumulators fill 256 columns of tensor memory, so that the epilogue has a position's
-// projection and gate in the same thread and nothing is read back from memory:
-//   warp 0      TMA loads of 128 x 64 slabs of x, Wp and Wg (128-byte swizzle) into a 2-stage ring
-//   warp 1      one elected lane issues both products of a slab
-//   warps 2-9   epilogue, 32 positions x 64 channels each. A lane is a position and the outputs are channel-major, so
-//               the 32 lanes of a store write 64 contiguous bytes of one channel: coalesced whatever the strides are, which
-//               a TMA store (multiples of 16 bytes) or vector stores would not take for an odd number of residues.
-// Bound by HBM (x in, two outputs; 113 MB at 384 x 384 x 128). Where rows of positions follow one another without gaps the
-// batch rows are one row of n_res * n_res_gather positions.
+// (src/attention/triangle_multiplication.cpp:38-69). Persistent CTAs, one per SM; a tile is 128 positions x 128 channels of
+// BOTH products, so that the epilogue has a position's projection and gate in the same thread and nothing is read back from
+// memory:
+//   warp 0      TMA loads of 128 x 64 slabs of x, Wp and Wg (128-byte swizzle) into a 3-stage ring
+//   warp 1      one elected lane issues both products of a slab; two pairs of accumulators fill the tensor memory
+//   warps 4-19  epilogue, 32 channels x 32 positions each, two elements at a time through the packed fp32 operations
+// The outputs are channel-major. Where TMA takes their strides the products are transposed (a lane of the accumulators is a
+// channel): the bias is a register, a lane's positions lie side by side, and the results leave through a staging tile by TMA.
+// For other strides (an odd number of residues) a lane is a position, and the 32 lanes of a 2-byte store write 64 contiguous
+// bytes of a channel; storing words of two positions from staging tiles was slower (301 x 301 x 128: 30 to 34 us against 20 to 25).
+// Bound by HBM (x in, two outputs; 113 MB at 384 x 384 x 128, 17 us) and by the instructions of the epilogue: with one element
+// and one position per lane at a time it took 35 per element and the kernel 34.5 us; now 26. Where rows of positions follow
+// one another without gaps the batch rows are one row of n_res * n_res_gather positions.
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is released
 // and the host-visible error word carries the site.
@@ -31,14 +34,17 @@ namespace dev {
 namespace {
 
 constexpr int BM = 128, BN = 128, BK = 64;
-constexpr int NSTAGE = 2;
+constexpr int NSTAGE = 3;
 constexpr int SLAB_BYTES = 128 * BK * 2;
 constexpr int STAGE_BYTES = 3 * SLAB_BYTES;
-constexpr int EPI_WARPS = 8;
-constexpr int THREADS = 32 * (2 + EPI_WARPS);
-constexpr int BAR_OFF = NSTAGE * STAGE_BYTES;
-constexpr int SMEM_BYTES = BAR_OFF + 64 + 1024;
-constexpr int TMEM_COLS = 2 * BN;               // half of the SM's tensor memory (two CTAs per SM)
+constexpr int EPI_WARPS = 16, EPI_WARP0 = 4;
+constexpr int THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
+constexpr int TILE_BYTES = 32 * 32 * 2;                        // staging tile of a warp, one per output
+constexpr int STG_OFF = NSTAGE * STAGE_BYTES;
+constexpr int MASK_OFF = STG_OFF + EPI_WARPS * 2 * TILE_BYTES;
+constexpr int BAR_OFF = MASK_OFF + EPI_WARPS * 32 * 4;
+constexpr int SMEM_BYTES = BAR_OFF + 128 + 1024;
+constexpr int TMEM_COLS = 4 * BM;               // two pairs of accumulators of 128 channels x 128 positions
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct TmProjParams {
@@ -50,16 +56,40 @@ struct TmProjParams {
     int *err;
 };
 
-__global__ void __launch_bounds__(THREADS, 2)
+// Two elements of the result from their rounded projections, gates and mask values:
+// (proj * mask) * sigmoid(gate), in this order (triangle_multiplication.cpp:60-64)
+__device__ __forceinline__ void gated(uint32_t p16, uint32_t g16, uint64_t mask2, float &y0, float &y1)
+{
+    float e0, e1;
+    unpack_f32x2(mul_f32x2(pack_f32x2(bf16lo_to_f32(g16), bf16hi_to_f32(g16)), pack_f32x2(-kLog2e, -kLog2e)), e0, e1);
+    unpack_f32x2(add_f32x2(pack_f32x2(ex2_approx(e0), ex2_approx(e1)), pack_f32x2(1.f, 1.f)), e0, e1);
+    const uint64_t pm = mul_f32x2(pack_f32x2(bf16lo_to_f32(p16), bf16hi_to_f32(p16)), mask2);
+    unpack_f32x2(mul_f32x2(pm, pack_f32x2(__fdividef(1.f, e0), __fdividef(1.f, e1))), y0, y1);
+}
+
+// bf16 pair of two accumulators plus their biases
+__device__ __forceinline__ uint32_t biased(uint32_t a0, uint32_t a1, uint64_t bias2)
+{
+    float y0, y1;
+    unpack_f32x2(add_f32x2(pack_f32x2(__uint_as_float(a0), __uint_as_float(a1)), bias2), y0, y1);
+    return pack_bf16x2(y0, y1);
+}
+
+// TMA_OUT: the strides of both outputs are multiples of 16 bytes
+template <bool TMA_OUT>
+__global__ void __launch_bounds__(THREADS, 1)
 tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_wp,
-               const __grid_constant__ CUtensorMap tm_wg, const TmProjParams p)
+               const __grid_constant__ CUtensorMap tm_wg, const __grid_constant__ CUtensorMap tm_proj,
+               const __grid_constant__ CUtensorMap tm_gate, const __grid_constant__ TmProjParams p)
 {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bar = smem + BAR_OFF;
     auto full_bar = [&](int s) { return bar + 8u * (uint32_t)s; };
     auto empty_bar = [&](int s) { return bar + 8u * (uint32_t)(NSTAGE + s); };
-    const uint32_t acc_full = bar + 8u * (2 * NSTAGE), acc_empty = acc_full + 8, tmem_slot = acc_full + 16;
+    auto acc_full = [&](int i) { return bar + 8u * (uint32_t)(2 * NSTAGE + i); };
+    auto acc_empty = [&](int i) { return bar + 8u * (uint32_t)(2 * NSTAGE + 2 + i); };
+    const uint32_t tmem_slot = bar + 8u * (2 * NSTAGE + 4);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int s_tiles = (p.S + BM - 1) / BM, n_tiles = (p.N + BN - 1) / BN;
     const int num_tiles = p.B * s_tiles * n_tiles;
@@ -70,8 +100,10 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_empty, EPI_WARPS);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(acc_full(i), 1);
+            mbar_init(acc_empty(i), EPI_WARPS);
+        }
         fence_barrier_init();
     }
     if (warp == 1) {
@@ -109,11 +141,12 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        constexpr uint32_t idesc = make_instr_desc_bf16(BM, BN);
+        constexpr uint32_t idesc = make_instr_desc_bf16(128, 128);
         int it = 0, t = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++t) {
-            if (t > 0 && !mbar_wait_warp(acc_empty, (uint32_t)((t - 1) & 1), p.err, 52)) break;
+            if (t >= 2 && !mbar_wait_warp(acc_empty(t & 1), (uint32_t)((t / 2 - 1) & 1), p.err, 52)) break;
+            const uint32_t d = tmem_base + (uint32_t)((t & 1) * 2 * BM);
             for (int kc = 0; kc < nk; ++kc, ++it) {
                 const int s = it % NSTAGE;
                 if (!mbar_wait_warp(full_bar(s), (uint32_t)((it / NSTAGE) & 1), p.err, 53)) {
@@ -127,61 +160,111 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
                         const uint32_t acc = (kc > 0 || k > 0) ? 1u : 0u;
-                        tc_mma_bf16(tmem_base, xd + 2 * k, xd + SLAB16 + 2 * k, idesc, acc);
-                        tc_mma_bf16(tmem_base + BN, xd + 2 * k, xd + 2 * SLAB16 + 2 * k, idesc, acc);
+                        const uint64_t x = xd + 2 * k, wp = x + SLAB16, wg = x + 2 * SLAB16;
+                        tc_mma_bf16(d, TMA_OUT ? wp : x, TMA_OUT ? x : wp, idesc, acc);
+                        tc_mma_bf16(d + BM, TMA_OUT ? wg : x, TMA_OUT ? x : wg, idesc, acc);
                     }
                     tc_commit(empty_bar(s));
-                    if (kc == nk - 1) tc_commit(acc_full);
+                    if (kc == nk - 1) tc_commit(acc_full(t & 1));
                 }
                 __syncwarp();
             }
         }
-    } else {
-        const int quad = warp & 3, half = (warp - 2) >> 2;
+    } else if (warp >= EPI_WARP0) {
+        // 32 rows (quad) x 32 columns (grp) of both accumulators
+        const int ew = warp - EPI_WARP0, quad = warp & 3, grp = ew >> 2;
+        const uint32_t stg = smem + STG_OFF + (uint32_t)(ew * 2 * TILE_BYTES), mk = smem + MASK_OFF + (uint32_t)(ew * 128);
         int t = 0;
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++t) {
-            const int m_tile = tile / n_tiles, n0 = tile % n_tiles * BN + half * 64;
-            const int b = m_tile / s_tiles, row = m_tile % s_tiles * BM + quad * 32 + lane;
-            const bool live = row < p.S;
-            const float mv = live ? __bfloat162float(p.mask[b * p.m_s0 + row]) : 0.f;
-            __nv_bfloat16 *pr = p.proj + b * p.p_s1 + row, *gr = p.gate + b * p.g_s1 + row;
-            if (!mbar_wait_warp(acc_full, (uint32_t)(t & 1), p.err, 54)) break;
+            const int m_tile = tile / n_tiles, n = tile % n_tiles * BN + (TMA_OUT ? quad : grp) * 32;
+            const int b = m_tile / s_tiles, row0 = m_tile % s_tiles * BM + (TMA_OUT ? grp : quad) * 32, row = row0 + lane;
+            const float mv = row < p.S ? __bfloat162float(p.mask[b * p.m_s0 + row]) : 0.f;
+            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)((t & 1) * 2 * BM + grp * 32);
+            float bp = 0.f, bg = 0.f;
+            if (TMA_OUT) {
+                bp = __ldg(p.bias_p + n + lane);
+                bg = __ldg(p.bias_g + n + lane);
+                asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(mk + lane * 4), "f"(mv) : "memory");
+                if (lane == 0) tma_store_wait_read<0>();           // the staging tiles may be rewritten
+                __syncwarp();
+            }
+            if (!mbar_wait_warp(acc_full(t & 1), (uint32_t)((t / 2) & 1), p.err, 54)) break;
             tc_fence_after();
-            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 64);
-#pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
                 uint32_t rp[16], rg[16];
                 __syncwarp();
                 tmem_ld_32x16(tcol + c * 16, rp);
-                tmem_ld_32x16(tcol + BN + c * 16, rg);
+                tmem_ld_32x16(tcol + BM + c * 16, rg);
                 tmem_ld_wait16(rp);
                 tmem_ld_wait16(rg);
-                if (c == 3) {
-                    // everything is in registers: the next tile may overwrite the accumulators
+                if (c == 1) {
+                    // everything is in registers: the accumulators may be overwritten
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty);
+                    if (lane == 0) mbar_arrive(acc_empty(t & 1));
                 }
-                const int n = n0 + c * 16;
-                if (!live || n >= p.N) continue;
+                if (TMA_OUT) {
+                    uint32_t op[8], og[8];
 #pragma unroll
-                for (int j4 = 0; j4 < 4; ++j4) {
-                    const float4 bp = __ldg(reinterpret_cast<const float4 *>(p.bias_p + n) + j4);
-                    const float4 bg = __ldg(reinterpret_cast<const float4 *>(p.bias_g + n) + j4);
-                    const float bps[4] = {bp.x, bp.y, bp.z, bp.w}, bgs[4] = {bg.x, bg.y, bg.z, bg.w};
+                    for (int j = 0; j < 16; j += 4) {
+                        const float4 m4 = lds128_f32(mk + (uint32_t)((c * 16 + j) * 4));
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int64_t ch = n + j4 * 4 + e;
-                        const float pv = round_to_bf16_f32(__uint_as_float(rp[j4 * 4 + e]) + bps[e]);
-                        const __nv_bfloat16 g16 = __float2bfloat16_rn(__uint_as_float(rg[j4 * 4 + e]) + bgs[e]);
-                        // (proj * mask) * sigmoid(gate), in this order (triangle_multiplication.cpp:60-64)
-                        const float sg = __fdividef(1.0f, 1.0f + ex2_approx(-__bfloat162float(g16) * kLog2e));
-                        gr[ch * p.g_s0] = g16;
-                        pr[ch * p.p_s0] = __float2bfloat16_rn((pv * mv) * sg);
+                        for (int h = 0; h < 4; h += 2) {
+                            float y0, y1;
+                            const uint32_t p16 = biased(rp[j + h], rp[j + h + 1], pack_f32x2(bp, bp));
+                            const uint32_t g16 = biased(rg[j + h], rg[j + h + 1], pack_f32x2(bg, bg));
+                            gated(p16, g16, h == 0 ? pack_f32x2(m4.x, m4.y) : pack_f32x2(m4.z, m4.w), y0, y1);
+                            op[(j + h) >> 1] = pack_bf16x2(y0, y1);
+                            og[(j + h) >> 1] = g16;
+                        }
+                    }
+                    // staging tile: a row of 64 bytes per channel, 64-byte swizzle
+#pragma unroll
+                    for (int v = 0; v < 2; ++v) {
+                        const uint32_t at = stg + (uint32_t)(lane * 64) + ((uint32_t)((c * 2 + v) ^ ((lane >> 1) & 3)) << 4);
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(at), "r"(op[4 * v]), "r"(op[4 * v + 1]),
+                                     "r"(op[4 * v + 2]), "r"(op[4 * v + 3])
+                                     : "memory");
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(at + TILE_BYTES), "r"(og[4 * v]),
+                                     "r"(og[4 * v + 1]), "r"(og[4 * v + 2]), "r"(og[4 * v + 3])
+                                     : "memory");
+                    }
+                } else if (row < p.S) {
+                    uint16_t *po = reinterpret_cast<uint16_t *>(p.proj + b * p.p_s1 + (n + c * 16) * p.p_s0 + row);
+                    uint16_t *go = reinterpret_cast<uint16_t *>(p.gate + b * p.g_s1 + (n + c * 16) * p.g_s0 + row);
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) {
+                        const float4 bp4 = __ldg(reinterpret_cast<const float4 *>(p.bias_p + n + c * 16 + j));
+                        const float4 bg4 = __ldg(reinterpret_cast<const float4 *>(p.bias_g + n + c * 16 + j));
+#pragma unroll
+                        for (int h = 0; h < 4; h += 2) {
+                            float y0, y1;
+                            const uint32_t p16 = biased(rp[j + h], rp[j + h + 1], h == 0 ? pack_f32x2(bp4.x, bp4.y) : pack_f32x2(bp4.z, bp4.w));
+                            const uint32_t g16 = biased(rg[j + h], rg[j + h + 1], h == 0 ? pack_f32x2(bg4.x, bg4.y) : pack_f32x2(bg4.z, bg4.w));
+                            gated(p16, g16, pack_f32x2(mv, mv), y0, y1);
+                            const uint32_t y16 = pack_bf16x2(y0, y1);
+                            po[0] = (uint16_t)y16;
+                            go[0] = (uint16_t)g16;
+                            po[p.p_s0] = (uint16_t)(y16 >> 16);
+                            go[p.g_s0] = (uint16_t)(g16 >> 16);
+                            po += 2 * p.p_s0;
+                            go += 2 * p.g_s0;
+                        }
                     }
                 }
             }
+            if (TMA_OUT) {
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_3d(&tm_proj, stg, row0, n, b);
+                    tma_store_3d(&tm_gate, stg + TILE_BYTES, row0, n, b);
+                    tma_store_commit();
+                }
+            }
         }
+        if (TMA_OUT && lane == 0) tma_store_wait<0>();
     }
 
     tc_fence_before();
@@ -207,12 +290,12 @@ bool tcgen05_tm_proj_bf16(cudaStream_t stream, const void *x, const void *wp, co
     }
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
-    CUtensorMap tx, tp, tg;
+    CUtensorMap tx, tp, tg, op = {}, og = {};
     if (!make_tensor_map_bf16_3d(&tx, x, K, S, B, K, (uint64_t)S * K, BK, BM, 128) ||
         !make_tensor_map_bf16_3d(&tp, wp, K, N, 1, K, (uint64_t)N * K, BK, BN, 128) ||
         !make_tensor_map_bf16_3d(&tg, wg, K, N, 1, K, (uint64_t)N * K, BK, BN, 128))
         return false;
-    TmProjParams p;
+    TmProjParams p = {};
     p.bias_p = bp;
     p.bias_g = bg;
     p.mask = (const __nv_bfloat16 *)mask;
@@ -228,15 +311,21 @@ bool tcgen05_tm_proj_bf16(cudaStream_t stream, const void *x, const void *wp, co
     p.N = N;
     p.K = K;
     p.err = ew.device;
+    // batch rows of one: any stride that TMA takes
+    const int64_t pb = B == 1 ? (int64_t)N * p_s0 : p_s1, gb = B == 1 ? (int64_t)N * g_s0 : g_s1;
+    const bool tma_out = (p_s0 | g_s0 | pb | gb) % 8 == 0 && (((uintptr_t)proj | (uintptr_t)gate) & 15u) == 0 &&
+                         make_tensor_map_bf16_3d(&op, proj, S, N, B, p_s0, pb, 32, 32, 64) &&
+                         make_tensor_map_bf16_3d(&og, gate, S, N, B, g_s0, gb, 32, 32, 64);
     static bool configured = false;
     if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(tm_proj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        KUTACC_CUDA(cudaFuncSetAttribute(tm_proj_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+        KUTACC_CUDA(cudaFuncSetAttribute(tm_proj_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
         configured = true;
     }
     const int64_t tiles = (int64_t)B * ((S + BM - 1) / BM) * (N / BN);
-    const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, std::max(1, sm_count() - runtime().sm_margin));
     KernelTimer timer__("tm_proj", stream);
-    launch_chained(tm_proj_kernel, grid, THREADS, SMEM_BYTES, stream, tx, tp, tg, p);
+    launch_chained(tma_out ? tm_proj_kernel<true> : tm_proj_kernel<false>, grid, THREADS, SMEM_BYTES, stream, tx, tp, tg, op, og, p);
     count_launch();
     return true;
 }

@@ -95,6 +95,9 @@ bool launch_tm_equation_generic(cudaStream_t stream, const void *left, int64_t l
 // a multiple of 16 bytes (dst dense, 16-byte aligned)
 bool launch_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch,
                     int64_t c_i, int64_t n, int elem_bytes = 2);
+// two bf16 operands of the same size in one launch
+bool launch_repitch_pair(cudaStream_t stream, const void *const src[2], const int64_t s_s0[2], const int64_t s_s1[2],
+                         void *const dst[2], int64_t d_pitch, int64_t c_i, int64_t n);
 // out[r, :] = bf16(f32(out[r, :]) * sigmoid(f32(gate[r, :]))) for rows of c_o elements
 bool launch_tm_last(cudaStream_t stream, void *out, int64_t o_rs, const void *gate, int64_t g_rs, int64_t rows, int64_t c_o);
 

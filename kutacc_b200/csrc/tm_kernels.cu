@@ -95,18 +95,29 @@ __global__ void tm_equation_generic_kernel(const __nv_bfloat16 *__restrict__ lef
 // Rows of n elements to a pitch of `vecs` 16-byte vectors. A thread moves one vector: the five aligned 32-bit words that
 // cover it in the source, shifted together when the source starts on an odd element (the words past the row belong to the
 // vector's padding; those past the matrix's last row are not read).
-__global__ void __launch_bounds__(256) repitch_bf16_kernel(const __nv_bfloat16 *__restrict__ src, int64_t s_s0, int64_t s_s1,
-                                                         uint4 *__restrict__ dst, int vecs, int c_i, int n)
+// blockIdx.y: which of up to two operands (both in one launch: 2 x 301 x 301 x 128 in 15.6 instead of 2 x 9.7 us). I: 32-bit
+// indices where the vectors can be counted in them, the two divisions per vector are then a fraction of the 64-bit ones.
+struct RepitchSet {
+    const __nv_bfloat16 *src[2];
+    int64_t s0[2], s1[2];
+    uint4 *dst[2];
+};
+
+template <typename I>
+__global__ void __launch_bounds__(256) repitch_bf16_kernel(const RepitchSet set, int64_t vectors, uint32_t vecs, uint32_t n)
 {
-    const int64_t total = (int64_t)c_i * n * vecs;
     release_successor();
     wait_for_predecessor();
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int v = (int)(t % vecs);
-        const int64_t line = t / vecs;
-        const int r = (int)(line % n), c = (int)(line / n);
+    const int which = blockIdx.y;
+    const __nv_bfloat16 *__restrict__ src = which ? set.src[1] : set.src[0];
+    uint4 *__restrict__ dst = which ? set.dst[1] : set.dst[0];
+    const int64_t s_s0 = which ? set.s0[1] : set.s0[0], s_s1 = which ? set.s1[1] : set.s1[0];
+    const I total = (I)vectors;
+    for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+        const I line = t / vecs, c = line / n;
+        const int v = (int)(t - line * vecs), r = (int)(line - c * n);
         const __nv_bfloat16 *sp = src + c * s_s0 + r * s_s1 + v * 8;
-        const int have = min(8, n - v * 8);               // elements of this vector
+        const int have = min(8, (int)n - v * 8);               // elements of this vector
         const uint32_t *wp = reinterpret_cast<const uint32_t *>((uintptr_t)sp & ~(uintptr_t)3);
         const bool odd = ((uintptr_t)sp & 2) != 0;
         uint32_t w[5];
@@ -215,6 +226,29 @@ bool launch_tm_equation_generic(cudaStream_t stream, const void *left, int64_t l
     return true;
 }
 
+static void launch_repitch_set(cudaStream_t stream, const RepitchSet &set, unsigned count, int64_t d_pitch, int64_t c_i, int64_t n)
+{
+    const int64_t vectors = c_i * n * (d_pitch / 8);
+    launch_chained(vectors < INT32_MAX ? repitch_bf16_kernel<uint32_t> : repitch_bf16_kernel<uint64_t>,
+                   dim3(grid_for(vectors, 256), count), 256, 0, stream, set, vectors, (uint32_t)(d_pitch / 8), (uint32_t)n);
+}
+
+bool launch_repitch_pair(cudaStream_t stream, const void *const src[2], const int64_t s_s0[2], const int64_t s_s1[2],
+                         void *const dst[2], int64_t d_pitch, int64_t c_i, int64_t n)
+{
+    if (d_pitch % 8 != 0 || d_pitch < n || (((uintptr_t)dst[0] | (uintptr_t)dst[1]) & 15u) || c_i > INT32_MAX || n > INT32_MAX) return false;
+    KernelTimer timer__("repitch", stream);
+    RepitchSet set;
+    for (int i = 0; i < 2; ++i) {
+        set.src[i] = (const __nv_bfloat16 *)src[i];
+        set.s0[i] = s_s0[i];
+        set.s1[i] = s_s1[i];
+        set.dst[i] = (uint4 *)dst[i];
+    }
+    launch_repitch_set(stream, set, 2, d_pitch, c_i, n);
+    return true;
+}
+
 // (A copy, like the 2-D device copies of other operands: not counted among the operators' kernels.)
 bool launch_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t s_s1, void *dst, int64_t d_pitch, int64_t c_i,
                     int64_t n, int elem_bytes)
@@ -225,8 +259,7 @@ bool launch_repitch(cudaStream_t stream, const void *src, int64_t s_s0, int64_t 
         launch_chained(repitch_f32_kernel, grid_for(c_i * n * (d_pitch / 4), 256), 256, 0, stream, (const float *)src, s_s0, s_s1,
                        (float4 *)dst, (int)(d_pitch / 4), (int)c_i, (int)n);
     else
-        launch_chained(repitch_bf16_kernel, grid_for(c_i * n * (d_pitch / 8), 256), 256, 0, stream,
-                       (const __nv_bfloat16 *)src, s_s0, s_s1, (uint4 *)dst, (int)(d_pitch / 8), (int)c_i, (int)n);
+        launch_repitch_set(stream, RepitchSet{{(const __nv_bfloat16 *)src}, {s_s0}, {s_s1}, {(uint4 *)dst}}, 1, d_pitch, c_i, n);
     return true;
 }
 

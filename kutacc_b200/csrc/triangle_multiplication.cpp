@@ -136,14 +136,20 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
         const void *p;
         int64_t s0, s1;
     };
-    auto aligned_rows = [&](const void *p, int64_t s0, int64_t s1, void *pad, Operand &o) {
-        o = {p, s0, s1};
-        if (((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0) return true;
-        o = {pad, n * pitch, pitch};
-        return dev::launch_repitch(stream, p, s0, s1, pad, pitch, c_i, n);
-    };
-    Operand ol, orr;
-    bool ok = aligned_rows(d_l.dev, l_s0, l_s1, pad_l, ol) && aligned_rows(d_r.dev, r_s0, r_s1, pad_r, orr);
+    auto aligned_rows = [](const void *p, int64_t s0, int64_t s1) { return ((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0; };
+    const bool l_ok = aligned_rows(d_l.dev, l_s0, l_s1), r_ok = aligned_rows(d_r.dev, r_s0, r_s1);
+    const Operand ol = l_ok ? Operand{d_l.dev, l_s0, l_s1} : Operand{pad_l, n * pitch, pitch};
+    const Operand orr = r_ok ? Operand{d_r.dev, r_s0, r_s1} : Operand{pad_r, n * pitch, pitch};
+    bool ok = true;
+    if (!l_ok && !r_ok) {
+        const void *src[2] = {d_l.dev, d_r.dev};
+        void *dst[2] = {pad_l, pad_r};
+        const int64_t s0[2] = {l_s0, r_s0}, s1[2] = {l_s1, r_s1};
+        ok = dev::launch_repitch_pair(stream, src, s0, s1, dst, pitch, c_i, n);
+    } else {
+        ok = (l_ok || dev::launch_repitch(stream, d_l.dev, l_s0, l_s1, pad_l, pitch, c_i, n)) &&
+             (r_ok || dev::launch_repitch(stream, d_r.dev, r_s0, r_s1, pad_r, pitch, c_i, n));
+    }
     // outgoing: center[a, b] = sum_k left[a, k] * right[b, k]; incoming: center[a, b] = sum_k right[k, a] * left[k, b]
     ok = ok && (is_incoming ? dev::tcgen05_batched_bf16(stream, true, orr.p, orr.s1, orr.s0, ol.p, ol.s1, ol.s0, d_c.dev, c_s1,
                                                         c_s0, (int)c_i, (int)n, (int)n, (int)n)

@@ -27,6 +27,7 @@
 #include "common.h"
 #include "kernels.h"
 #include "launch.cuh"
+#include "ln_utils.cuh"
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
@@ -258,52 +259,16 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
             for (int ks = 0; ks < KS && ok; ++ks) ok = mbar_wait_warp(a_full(sa, ks), (uint32_t)((n / NBLK) & 1), p.err, 106);
             if (!ok) return;
             const uint32_t base = smem + OFF_A + sa * T::BLOCK_BYTES + (rt * KS + l / 8) * SLAB_BYTES;
-            constexpr float inv_n = 1.0f / (float)C;
             constexpr int U = 4;                                       // rows in flight per lane group
 #pragma unroll 1
             for (int p0 = 0; p0 < PASSES; p0 += U) {
-                uint32_t addr[U], w[U][4];
-                float delta[U], sum[U], sum2[U];
+                uint32_t addr[U];
 #pragma unroll
                 for (int i = 0; i < U; ++i) {
                     const int row = (ew & 7) * 16 + (p0 + i) * RPP + sub;
                     addr[i] = base + (uint32_t)(row * 128 + (((l & 7) ^ (row & 7)) << 4));
-                    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n"
-                                 : "=r"(w[i][0]), "=r"(w[i][1]), "=r"(w[i][2]), "=r"(w[i][3]) : "r"(addr[i]) : "memory");
                 }
-#pragma unroll
-                for (int i = 0; i < U; ++i) {
-                    delta[i] = bf16lo_to_f32(__shfl_sync(0xffffffffu, w[i][0], sub * LPR));      // the row's first channel
-                    sum[i] = sum2[i] = 0.f;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float a = bf16lo_to_f32(w[i][e]) - delta[i], b = bf16hi_to_f32(w[i][e]) - delta[i];
-                        sum[i] += a;
-                        sum2[i] = fmaf(a, a, sum2[i]);
-                        sum[i] += b;
-                        sum2[i] = fmaf(b, b, sum2[i]);
-                    }
-                }
-#pragma unroll
-                for (int o = LPR / 2; o > 0; o >>= 1)
-#pragma unroll
-                    for (int i = 0; i < U; ++i) {
-                        sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
-                        sum2[i] += __shfl_xor_sync(0xffffffffu, sum2[i], o);
-                    }
-#pragma unroll
-                for (int i = 0; i < U; ++i) {
-                    const float mean = fmaf(sum[i], inv_n, delta[i]);
-                    const float var = fmaxf((sum2[i] - sum[i] * sum[i] * inv_n) * inv_n, 0.f);
-                    const float rstd = rsqrtf(var + p.eps), shift = -rstd * mean;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        w[i][e] = pack_bf16x2(fmaf(fmaf(bf16lo_to_f32(w[i][e]), rstd, shift), gs[2 * e], bs[2 * e]),
-                                              fmaf(fmaf(bf16hi_to_f32(w[i][e]), rstd, shift), gs[2 * e + 1], bs[2 * e + 1]));
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr[i]), "r"(w[i][0]), "r"(w[i][1]), "r"(w[i][2]),
-                                 "r"(w[i][3])
-                                 : "memory");
-                }
+                layernorm_smem_rows<LPR, U>(addr, gs, bs, p.eps);
             }
             fence_proxy_async();
             __syncwarp();

@@ -8,6 +8,7 @@
 #include "common.h"
 #include "kernels.h"
 #include "launch.cuh"
+#include "ln_utils.cuh"
 #include "ptx_utils.cuh"
 
 #include <algorithm>
@@ -446,14 +447,14 @@ __global__ void __launch_bounds__(256) pair_bias_f32_kernel(const float *__restr
 // bf16 pair bias on tensor cores: a CTA streams 128-position tiles of z through a cp.async ring (16-byte
 // chunks, swizzled by row), each warp multiplies its 16 positions by Wb^T (heads padded to 8) with
 // mma.sync m16n8k16 and writes nb[h, pos]. Bandwidth bound: z is read once, 128-bit loads.
-// With LN the weights are LayerNorm-folded (ln_fold.cu) and a position's result is rstd * (acc - mean * s[h]) + t[h].
+// With LN a warp normalises its 16 positions in shared memory before it multiplies them (a statistics pass over z, a folding
+// of the weights and this kernel were three launches and two reads of z: 301 x 301 x 128 23 us; now 14).
 template <int CZ, bool LN>
 __global__ void __launch_bounds__(256) pair_bias_mma_kernel(const __nv_bfloat16 *__restrict__ z,
                                                             const __nv_bfloat16 *__restrict__ wb,
                                                             __nv_bfloat16 *__restrict__ nb, int64_t nb_head_stride,
-                                                            int64_t total, int H, const float2 *__restrict__ stats,
-                                                            const float *__restrict__ ln_s, const float *__restrict__ ln_t,
-                                                            int64_t nk, int64_t nb_row_stride)
+                                                            int64_t total, int H, const float *__restrict__ gamma,
+                                                            const float *__restrict__ beta, float eps, int64_t nk, int64_t nb_row_stride)
 {
     constexpr int ROWB = CZ * 2, CHUNKS = ROWB / 16, TP = 128, STAGES = 3, STAGE_BYTES = TP * ROWB;
     extern __shared__ __align__(128) unsigned char pb_smem[];
@@ -465,6 +466,14 @@ __global__ void __launch_bounds__(256) pair_bias_mma_kernel(const __nv_bfloat16 
     for (int ks = 0; ks < CZ / 16; ++ks) {
         bf[ks][0] = g < H ? *reinterpret_cast<const uint32_t *>(wb + g * CZ + ks * 16 + 2 * t) : 0u;
         bf[ks][1] = g < H ? *reinterpret_cast<const uint32_t *>(wb + g * CZ + ks * 16 + 8 + 2 * t) : 0u;
+    }
+    float gs[8], bs[8];
+    if (LN) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            gs[e] = gamma[lane % CHUNKS * 8 + e];
+            bs[e] = beta[lane % CHUNKS * 8 + e];
+        }
     }
     const int64_t ntiles = (total + TP - 1) / TP;
     const uint32_t smem0 = smem_u32(pb_smem);
@@ -488,6 +497,20 @@ __global__ void __launch_bounds__(256) pair_bias_mma_kernel(const __nv_bfloat16 
         __syncthreads();                       // tile `it` has landed; the stage refilled below is no longer read
         load_tile(tile + (int64_t)(STAGES - 1) * gridDim.x, (it + STAGES - 1) % STAGES);
         const uint32_t base = smem0 + (it % STAGES) * STAGE_BYTES + warp * 16 * ROWB;
+        if (LN) {
+            constexpr int RPP = 32 / CHUNKS, U = 4;                    // rows per pass, passes in flight
+#pragma unroll
+            for (int q = 0; q < 16; q += RPP * U) {
+                uint32_t addr[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    const int r = q + i * RPP + lane / CHUNKS;
+                    addr[i] = base + r * ROWB + (((lane % CHUNKS) ^ (r & 7)) << 4);
+                }
+                layernorm_smem_rows<CHUNKS, U>(addr, gs, bs, eps);
+            }
+            __syncwarp();
+        }
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int ks = 0; ks < CZ / 16; ++ks) {
@@ -498,15 +521,6 @@ __global__ void __launch_bounds__(256) pair_bias_mma_kernel(const __nv_bfloat16 
         }
         const int64_t p0 = tile * TP + warp * 16 + g, p1 = p0 + 8;
         const int h0 = 2 * t, h1 = 2 * t + 1;
-        if (LN) {
-            const float s0 = h0 < H ? ln_s[h0] : 0.f, s1 = h1 < H ? ln_s[h1] : 0.f;
-            const float t0 = h0 < H ? ln_t[h0] : 0.f, t1 = h1 < H ? ln_t[h1] : 0.f;
-            const float2 st0 = stats[p0 < total ? p0 : 0], st1 = stats[p1 < total ? p1 : 0];
-            acc[0] = fmaf(st0.y, acc[0] - st0.x * s0, t0);
-            acc[1] = fmaf(st0.y, acc[1] - st0.x * s1, t1);
-            acc[2] = fmaf(st1.y, acc[2] - st1.x * s0, t0);
-            acc[3] = fmaf(st1.y, acc[3] - st1.x * s1, t1);
-        }
         // position p = row * nk + key is stored at row * nb_row_stride + key (rows of the output may be further apart
         // than nk: a layout with the heads of a row next to each other, [rows, H, keys], for instance)
         const int64_t o0 = nb_row_stride == nk ? p0 : (p0 / nk) * nb_row_stride + p0 % nk;
@@ -525,8 +539,7 @@ __global__ void __launch_bounds__(256) pair_bias_mma_kernel(const __nv_bfloat16 
 
 template <int CZ, bool LN = false>
 bool launch_pair_bias_mma(cudaStream_t stream, const void *z, const void *wb, void *nb, int64_t nb_head_stride,
-                          int64_t total, int H, const void *stats = nullptr, const float *ln_s = nullptr,
-                          const float *ln_t = nullptr, int64_t nk = 1, int64_t nb_row_stride = 1)
+                          int64_t total, int H, const float *gamma, const float *beta, float eps, int64_t nk, int64_t nb_row_stride)
 {
     constexpr int SMEM = 3 * 128 * CZ * 2;
     static bool configured = false;
@@ -541,7 +554,7 @@ bool launch_pair_bias_mma(cudaStream_t stream, const void *z, const void *wb, vo
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, 148 * 2);
     launch_chained(pair_bias_mma_kernel<CZ, LN>, grid, 256, SMEM, stream, (const __nv_bfloat16 *)z, (const __nv_bfloat16 *)wb,
                                                               (__nv_bfloat16 *)nb, nb_head_stride, total, H,
-                                                              (const float2 *)stats, ln_s, ln_t, nk, nb_row_stride);
+                                                              gamma, beta, eps, nk, nb_row_stride);
     return true;
 }
 
@@ -632,13 +645,13 @@ bool launch_attn_generic(cudaStream_t stream, ElemType t, const void *q, const v
                                                 nb_stride_q, avg, B, S, H, D, scale);
 }
 
-bool launch_pair_bias_ln(cudaStream_t stream, const void *z, const void *wb_folded, const void *stats, const float *ln_s,
-                         const float *ln_t, void *nb, int64_t nb_head_stride, int64_t R, int64_t Nk, int Cz, int H)
+bool launch_pair_bias_ln(cudaStream_t stream, const void *z, const void *wb, const float *gamma, const float *beta, float eps, void *nb,
+                         int64_t nb_head_stride, int64_t R, int64_t Nk, int Cz, int H)
 {
-    if (H > 8 || (Cz != 128 && Cz != 64) || ((uintptr_t)z % 16) != 0 || ((uintptr_t)wb_folded % 4) != 0) return false;
+    if (H > 8 || (Cz != 128 && Cz != 64) || ((uintptr_t)z % 16) != 0 || ((uintptr_t)wb % 4) != 0) return false;
     KernelTimer timer__("pair_bias_ln", stream);
-    const bool ok = Cz == 128 ? launch_pair_bias_mma<128, true>(stream, z, wb_folded, nb, nb_head_stride, R * Nk, H, stats, ln_s, ln_t)
-                              : launch_pair_bias_mma<64, true>(stream, z, wb_folded, nb, nb_head_stride, R * Nk, H, stats, ln_s, ln_t);
+    const bool ok = Cz == 128 ? launch_pair_bias_mma<128, true>(stream, z, wb, nb, nb_head_stride, R * Nk, H, gamma, beta, eps, 1, 1)
+                              : launch_pair_bias_mma<64, true>(stream, z, wb, nb, nb_head_stride, R * Nk, H, gamma, beta, eps, 1, 1);
     if (ok) count_launch();
     return ok;
 }
@@ -656,10 +669,10 @@ bool launch_pair_bias(cudaStream_t stream, ElemType t, const void *z, const void
     const bool pow2 = lanes > 0 && (lanes & (lanes - 1)) == 0 && lanes <= 32 && Cz % 8 == 0;
     if (t == kElemBF16 && H <= 8 && pos_stride == 1 && ((uintptr_t)z % 16) == 0 && ((uintptr_t)wb % 4) == 0 &&
         (Cz == 128 || Cz == 64)) {
-        const bool ok = Cz == 128 ? launch_pair_bias_mma<128>(stream, z, wb, nb, nb_head_stride, pos, H, nullptr, nullptr,
-                                                              nullptr, Nk, nb_row_stride)
-                                  : launch_pair_bias_mma<64>(stream, z, wb, nb, nb_head_stride, pos, H, nullptr, nullptr,
-                                                             nullptr, Nk, nb_row_stride);
+        const bool ok = Cz == 128 ? launch_pair_bias_mma<128>(stream, z, wb, nb, nb_head_stride, pos, H, nullptr, nullptr, 0.f,
+                                                              Nk, nb_row_stride)
+                                  : launch_pair_bias_mma<64>(stream, z, wb, nb, nb_head_stride, pos, H, nullptr, nullptr, 0.f,
+                                                             Nk, nb_row_stride);
         if (ok) {
             count_launch();
             return true;

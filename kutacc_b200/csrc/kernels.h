@@ -137,10 +137,10 @@ bool launch_attn_generic(cudaStream_t stream, ElemType t, const void *q, const v
 bool launch_pair_bias(cudaStream_t stream, ElemType t, const void *z, const void *wb, void *nb,
                       int64_t nb_head_stride, int64_t pos_stride, int64_t R, int64_t Nk, int Cz, int H,
                       int64_t nb_row_stride = 0);
-// The same projection of LayerNorm(z) with folded weights (launch_ln_fold) and per-position statistics: only the
-// tensor-core kernel (bf16, c_z 64 or 128, up to 8 heads, [H, R, Nk] output); false otherwise.
-bool launch_pair_bias_ln(cudaStream_t stream, const void *z, const void *wb_folded, const void *stats, const float *ln_s,
-                         const float *ln_t, void *nb, int64_t nb_head_stride, int64_t R, int64_t Nk, int Cz, int H);
+// The same projection of LayerNorm(z): only the tensor-core kernel (bf16, c_z 64 or 128, up to 8 heads, [H, R, Nk] output);
+// false otherwise.
+bool launch_pair_bias_ln(cudaStream_t stream, const void *z, const void *wb, const float *gamma, const float *beta, float eps, void *nb,
+                         int64_t nb_head_stride, int64_t R, int64_t Nk, int Cz, int H);
 
 // ---- global attention (bf16, C = 64) ---------------------------------------------------------------
 // scratch: qk [B, H, 64] fp32-sized slots and wa [B, 64]; see global_attention.cu

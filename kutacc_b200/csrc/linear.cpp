@@ -159,9 +159,9 @@ extern "C" void kutacc_b200_pair_bias(kutacc_tensor_h z_h, kutacc_tensor_h wb_h,
     end_of_call();
 }
 
-// Pair bias of LayerNorm(z): nb[h, r, k] = LayerNorm(z[r, k, :]) . wb[h, :]. The normalisation is folded into the
-// projection (one read of z for the row statistics, one for the product; the normalised tensor is never written).
-// Shapes the folded tensor-core kernel does not cover normalise into the workspace first.
+// Pair bias of LayerNorm(z): nb[h, r, k] = LayerNorm(z[r, k, :]) . wb[h, :]. The projection kernel normalises its
+// positions itself (one read of z; the normalised tensor is never written). Shapes that kernel does not cover are normalised
+// into the workspace first.
 extern "C" void kutacc_b200_pair_bias_ln(kutacc_tensor_h z_h, const float *ln_gamma, const float *ln_beta, float eps,
                                          kutacc_tensor_h wb_h, kutacc_tensor_h nb_h)
 {
@@ -188,22 +188,13 @@ extern "C" void kutacc_b200_pair_bias_ln(kutacc_tensor_h z_h, const float *ln_ga
     if (!rt.reserve_stage(staged_bytes_needed(z.data_ptr(), z_bytes) + staged_bytes_needed(wb.data_ptr(), w_bytes) +
                           staged_bytes_needed(nb.data_ptr(), nb_bytes) + 2 * staged_bytes_needed(ln_gamma, g_bytes)))
         return;
-    // workspace: statistics, folded weights with s and t, and room for the normalised copy of the fallback
-    if (!rt.reserve_workspace((size_t)P * 8 + w_bytes + 2 * (size_t)H * 4 + z_bytes + 4 * 256)) return;
+    const bool fused = H <= 8 && (Cz == 128 || Cz == 64);
+    if (!rt.reserve_workspace(z_bytes + 256)) return;              // the normalised copy of the fallback
     DeviceArg d_z = resolve_in(z.data_ptr(), z_bytes), d_w = resolve_in(wb.data_ptr(), w_bytes),
               d_g = resolve_in(ln_gamma, g_bytes), d_b = resolve_in(ln_beta, g_bytes), d_n = resolve_out(nb.data_ptr(), nb_bytes);
-    void *stats = rt.take_workspace((size_t)P * 8), *w2 = rt.take_workspace(w_bytes);
-    float *s = (float *)rt.take_workspace((size_t)H * 4), *t = (float *)rt.take_workspace((size_t)H * 4);
     if (kutacc_check_err_set) return;
-    const void *w_in[1] = {d_w.dev};
-    const float *no_bias[1] = {nullptr};
-    void *w_out[1] = {w2};
-    float *s_out[1] = {s}, *t_out[1] = {t};
-    bool ok = H <= 8 && (Cz == 128 || Cz == 64) && ((uintptr_t)d_z.dev % 16) == 0 &&
-              dev::launch_ln_stats(stream, d_z.dev, P, Cz, Cz, eps, stats) &&
-              dev::launch_ln_fold(stream, 1, w_in, no_bias, (const float *)d_g.dev, (const float *)d_b.dev, w_out, s_out, t_out,
-                                  (int)H, (int)Cz) &&
-              dev::launch_pair_bias_ln(stream, d_z.dev, w2, stats, s, t, d_n.dev, hs, R, Nk, (int)Cz, (int)H);
+    bool ok = fused && dev::launch_pair_bias_ln(stream, d_z.dev, d_w.dev, (const float *)d_g.dev, (const float *)d_b.dev, eps, d_n.dev, hs,
+                                                R, Nk, (int)Cz, (int)H);
     if (!ok && !kutacc_check_err_set) {
         void *zn = rt.take_workspace(z_bytes);
         ok = zn != nullptr &&

@@ -180,6 +180,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp == 0 && elect_one()) {                  // kernel parameters: may be fetched before the predecessor ends
+        tma_prefetch_desc(&tm_q);
+        tma_prefetch_desc(&tm_k);
+        tma_prefetch_desc(&tm_vt);
+        if (HAS_NB) tma_prefetch_desc(&tm_nb);
+    }
     release_successor();
     wait_for_predecessor();
     uint32_t tmem_base;
@@ -189,10 +195,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (warp == PRODUCER_WARP) {
         // ================= producer =================
         if (elect_one()) {
-            tma_prefetch_desc(&tm_q);
-            tma_prefetch_desc(&tm_k);
-            tma_prefetch_desc(&tm_vt);
-            if (HAS_NB) tma_prefetch_desc(&tm_nb);
         }
         const uint32_t tx = (uint32_t)(G * (T::K_BYTES + T::VT_TX) + (HAS_NB ? NB_BYTES : 0));
         int g = 0;                                      // tiles issued so far (all items)

@@ -140,6 +140,13 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp == 0 && elect_one()) {                  // kernel parameters: may be fetched before the predecessor ends
+        tma_prefetch_desc(&maps.a);
+        for (int i = 0; i < 4; ++i) {
+            tma_prefetch_desc(&maps.w[i]);
+            tma_prefetch_desc(&maps.out[i]);
+        }
+    }
     release_successor();
     wait_for_predecessor();
     for (int i = threadIdx.x; i < C; i += THREADS) reinterpret_cast<float *>(gen + T::OFF_VEC)[i] = p.bg[i];
@@ -151,7 +158,6 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
     if (warp == 0) {
         // ================= producer =================
         if (elect_one()) {
-            tma_prefetch_desc(&maps.a);
             bool ok = true;
             int wit = 0;
             auto load_rows = [&](int n, int ks) {                      // a slab of the rows of this CTA's n-th unit
@@ -389,7 +395,7 @@ bool launch_ks(cudaStream_t stream, const ProjMaps &maps, ProjParams p)
         for (int ns = 1; ns <= NT; ns *= 2) {
             const int64_t last = (blocks - whole) * ns;
             const double cost = ((double)(whole / sms) * (NT + 1.0) + (double)((last + sms - 1) / sms) * ((double)NT / ns + 1.0)) *
-                                (r == 2 ? 1.8 : 1.0);
+                                (r == 2 ? 1.3 : 1.0);
             if (cost < best * 0.999) {
                 best = cost;
                 R = r;

@@ -181,6 +181,11 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp == 0 && elect_one()) {                  // kernel parameters: may be fetched before the predecessor ends
+        tma_prefetch_desc(&maps.a);
+        tma_prefetch_desc(&maps.w[0]);
+        tma_prefetch_desc(&maps.out[0]);
+    }
     release_successor();
     wait_for_predecessor();
     uint32_t tmem_base;
@@ -190,7 +195,6 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     if (warp == 0) {
         // ================= producer =================
         if (elect_one()) {
-            tma_prefetch_desc(&maps.a);
             int it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {

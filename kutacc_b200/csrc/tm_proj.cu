@@ -113,6 +113,11 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp == 0 && elect_one()) {                  // kernel parameters: may be fetched before the predecessor ends
+        tma_prefetch_desc(&tm_x);
+        tma_prefetch_desc(&tm_wp);
+        tma_prefetch_desc(&tm_wg);
+    }
     release_successor();
     wait_for_predecessor();
     uint32_t tmem_base;

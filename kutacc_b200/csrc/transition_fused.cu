@@ -111,6 +111,12 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (warp == 0 && elect_one()) {                  // kernel parameters: may be fetched before the predecessor ends
+        tma_prefetch_desc(&tm_x);
+        tma_prefetch_desc(&tm_w1);
+        tma_prefetch_desc(&tm_w2);
+        tma_prefetch_desc(&tm_out);
+    }
     release_successor();
     wait_for_predecessor();
     for (int i = threadIdx.x; i < p.hidden; i += THREADS) bias1[i] = p.b1[i];
@@ -123,9 +129,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     if (warp == 0) {
         // ================= producer =================
         if (elect_one()) {
-            tma_prefetch_desc(&tm_x);
-            tma_prefetch_desc(&tm_w1);
-            tma_prefetch_desc(&tm_w2);
             int it = 0;
             bool ok = true;
             auto slab = [&](const CUtensorMap *map, int c0, int c1) {

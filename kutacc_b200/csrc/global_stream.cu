@@ -233,13 +233,15 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
 
 // ---- core: one CTA per column, a warp takes every WARPS-th pair of records -----------------------------------------------
 // A pair is one bulk copy of 2176 bytes into the warp's ring, QN pairs ahead of the arithmetic. (As three copies per record
-// the copies themselves were the bound, 26 us for 61440 records.) Eight warps per column where there are columns for
-// several CTAs per SM, sixteen otherwise.
-constexpr int QN = 4, Q_BYTES = 2 * REC_BYTES;
-constexpr int core_smem(int warps) { return warps * (QN * (Q_BYTES + 8)); }
+// the copies themselves were the bound, 26 us for 61440 records.) Sixteen warps per column whatever the number of columns: a
+// column's sums are split the same way in every batch. More columns than SMs run two CTAs per SM on a shorter ring (250
+// columns x 1500 rows: 41.6 us for the three kernels, with one CTA per SM 44.7); fewer have the longer ring (64 x 5120: 41 us,
+// with the shorter 46).
+constexpr int WARPS = 16, Q_BYTES = 2 * REC_BYTES;
+constexpr int core_smem(int qn) { return WARPS * qn * (Q_BYTES + 8); }
 
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : 1) global_softmax_kernel(const StreamArgs a)
+template <int QN>
+__global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_kernel(const StreamArgs a)
 {
     constexpr int NR = WARPS * 32 / (C + 1);     // row groups of the pooled sums
     extern __shared__ __align__(128) unsigned char core_dyn[];
@@ -711,8 +713,8 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
     static bool configured = false;
     if (!configured) {
         KUTACC_CUDA(cudaFuncSetAttribute(global_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM));
-        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(8)));
-        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(16)));
+        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(3)));
+        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(4)));
         KUTACC_CUDA(cudaFuncSetAttribute(global_stream_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_SMEM));
         configured = true;
     }
@@ -725,10 +727,10 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
     }
     {
         KernelTimer timer__("global_softmax", stream);
-        if (B > 2 * sms)
-            launch_chained(global_softmax_kernel<8>, (unsigned)B, 8 * 32, core_smem(8), stream, a);
+        if (B > sms)
+            launch_chained(global_softmax_kernel<3>, (unsigned)B, WARPS * 32, core_smem(3), stream, a);
         else
-            launch_chained(global_softmax_kernel<16>, (unsigned)B, 16 * 32, core_smem(16), stream, a);
+            launch_chained(global_softmax_kernel<4>, (unsigned)B, WARPS * 32, core_smem(4), stream, a);
     }
     {
         KernelTimer timer__("global_stream_out", stream);

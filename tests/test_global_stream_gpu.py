@@ -31,3 +31,12 @@ def test_rows_whose_logits_grow_late(kutacc_lib):
     w.arrays["x"] = W.as_f32(W.bf16_bits(x))
     got = runner.out_to_f32(runner.DeviceCase(w).run())
     assert helpers.rel_err(got, helpers.oracle_faithful(w)) <= helpers.BF16_TOL
+
+
+def test_a_column_does_not_depend_on_the_number_of_columns(kutacc_lib):
+    # few columns have an SM each, many share one
+    w = W.random_global_case(seed=78, B=300, S=1500)
+    many = runner.out_to_f32(runner.DeviceCase(w).run())
+    few = W.Workload(name="few", kind="global", dtype=w.dtype, B=3, S=w.S, H=w.H, D=w.D, seed=0, has_nb=w.has_nb)
+    few.arrays = dict(w.arrays, x=w.arrays["x"][:3], mask=w.arrays["mask"][:3])
+    assert np.array_equal(many[:3], runner.out_to_f32(runner.DeviceCase(few).run()))

@@ -48,6 +48,7 @@
 #include "tma_utils.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 
 namespace kutacc {
@@ -70,6 +71,7 @@ constexpr int BAR_BYTES = 512;
 constexpr int WG_COLS = 128;          // tensor-memory columns of a warp group: S (then P) 0..63, O from 64
 constexpr int S_COL = 0, O_COL = 64;
 constexpr float kRescaleThreshold = 5.5f;     // P stays below 2^8
+constexpr float kFar = 2147483648.f;          // 2^31: mneg below it is within 64 of -m * log2e
 
 template <int D>
 struct Geo {
@@ -352,8 +354,20 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const uint64_t scale2 = pack_f32x2(p.scale, p.scale), log2e2 = pack_f32x2(kLog2e, kLog2e);
         const uint32_t nb_row = off_nb + (uint32_t)row * 128 + (uint32_t)((row & 7) << 4);   // chunk c lies at ^ (c << 4)
         const uint32_t mb_row = off_mb + (uint32_t)wg * BN * 4;
-        float m = 0.f;                                   // running (possibly stale) max of x
+        // Running (possibly stale) max of x, at least the lowest finite number: keys masked with -inf then weigh nothing, and
+        // a row whose first keys are all of that kind is raised by its first finite one. P = 2^(x * log2e + mneg); the
+        // rounding of mneg is the same for all of a row's keys and cancels in the division, and O is rescaled by the
+        // difference of the very mneg that P was formed with. Past kFar that rounding would leave the range of the
+        // exponential: such rows (masked with the type's lowest value, or masked twice) take x - m first.
+        float m = 0.f, mneg = 0.f;
+        float limit = 0.f;                               // x above it needs a new max; NaN (always) for a far row
         bool ok = true;
+        auto far_row = [&]() { return !(fabsf(mneg) < kFar); };
+        auto set_max = [&](float v) {
+            m = fmaxf(v, -FLT_MAX);
+            mneg = -__fmul_rn(m, kLog2e);
+            limit = far_row() ? __int_as_float(0x7fffffff) : m + kRescaleThreshold;
+        };
 
         // one tile of the softmax: global tile g, tile kt of its item
         auto do_tile = [&](const int g, const int kt) -> bool {
@@ -394,7 +408,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             auto piece = [&](const uint32_t (&r)[16], const int c) {
                 Piece f;
                 fetch(f, c);
-                const uint64_t mneg2 = pack_f32x2(-m * kLog2e, -m * kLog2e);
+                const uint64_t mneg2 = pack_f32x2(mneg, mneg);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const uint64_t x2 = x_pair(r, f, j);
@@ -414,13 +428,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     // first tile of an item: the max of its first 16 keys (key 0 always exists)
                     Piece f;
                     fetch(f, 0);
-                    m = -INFINITY;
+                    float mx = -INFINITY;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         float x0, x1;
                         unpack_f32x2(x_pair(a, f, j), x0, x1);
-                        m = fmax3(m, x0, x1);
+                        mx = fmax3(mx, x0, x1);
                     }
+                    set_max(mx);
                 }
                 tmem_ld_32x16(t_s + 16, b);
                 piece(a, 0);
@@ -432,14 +447,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 piece(a, 2);
                 tmem_ld_wait16(b);
                 piece(b, 3);
-                const bool grow = tmax > m + kRescaleThreshold;
-                if (!__any_sync(0xffffffffu, grow)) break;
+                if (!__any_sync(0xffffffffu, !(tmax <= limit))) break;
                 // rare: the max of some row grew past the threshold. Rescale those rows of O (and their row sums) and form
                 // the tile again against the new max. The product of the previous tile has retired: it was issued
                 // before the logits of this one.
-                const float f = grow ? ex2_approx((m - tmax) * kLog2e) : 1.0f;
-                if (grow) m = tmax;
-                if (kt > 0) {
+                const bool grow = tmax > m + kRescaleThreshold;
+                float f = 1.0f;
+                if (grow) {
+                    const bool was_far = far_row();
+                    const float m_old = m, mneg_old = mneg;
+                    set_max(tmax);
+                    f = ex2_approx(was_far || far_row() ? (m_old - m) * kLog2e : mneg - mneg_old);
+                }
+                if (kt > 0 && __any_sync(0xffffffffu, grow)) {
                     constexpr int OC = D < 16 ? 16 : D;
 #pragma unroll
                     for (int c = 0; c <= OC; c += 16) {
@@ -457,6 +477,23 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         }
                     }
                     tmem_st_wait();
+                }
+                if (__any_sync(0xffffffffu, far_row())) {
+                    const float sub = far_row() ? -m : 0.f, add = far_row() ? 0.f : mneg;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        Piece pc;
+                        fetch(pc, c);
+                        tmem_ld_32x16(t_s + c * 16, a);
+                        tmem_ld_wait16(a);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            float e0, e1;
+                            unpack_f32x2(fma_f32x2(add_f32x2(x_pair(a, pc, j), pack_f32x2(sub, sub)), log2e2, pack_f32x2(add, add)), e0, e1);
+                            pk[c * 8 + j] = pack_bf16x2(ex2_approx(e0), ex2_approx(e1));
+                        }
+                    }
+                    break;
                 }
             }
             tmem_st_32x32(t_s, pk);

@@ -33,3 +33,57 @@ def test_core_matches_faithful_oracle(kutacc_lib, B, S, H, D, with_nb):
         ref.arrays = dict(w.arrays, x=w.arrays["x"][pick], mask=w.arrays["mask"][pick], bias=w.arrays["bias"][pick])
         got, rows = got[pick], slice(0, len(pick))
     assert helpers.rel_err(got[rows], helpers.oracle_faithful(ref)[rows]) <= helpers.BF16_TOL
+
+
+LOWEST = float(np.finfo(np.float32).min)
+LOWEST_BF16 = -float.fromhex("0x1.fep127")
+
+
+def masked_case(value, through_nb, H, D, dtype):
+    """Keys masked with `value` instead of -1e9: the first 70 (more than a tile) of batch row 0, or of all rows through the pair
+    bias; all but the last; scattered ones."""
+    w = W.random_gating_case(seed=77 + D, B=3, S=200, H=H, D=D, dtype=dtype, with_nb=through_nb, mask_frac=0.0)
+    bias, nb = np.zeros((3, 200), np.float32), w.arrays.get("nb")
+    if through_nb:
+        w.arrays["nb"] = nb = nb.copy()
+        nb[:, :, :70] = value
+    else:
+        bias[0, :70] = value
+        bias[1, :199] = value
+        bias[2, np.random.default_rng(1).random(200) < 0.5] = value
+        bias[2, 9] = 0.0
+    w.arrays["bias"] = bias
+    return w
+
+
+@pytest.mark.parametrize("through_nb", [True, False])
+@pytest.mark.parametrize("value", [-np.inf, LOWEST_BF16, -3e9])
+@pytest.mark.parametrize("H,D", [(4, 32), (4, 16), (8, 8)])
+def test_other_mask_values(kutacc_lib, H, D, value, through_nb):
+    w = masked_case(value, through_nb, H, D, "bf16")
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    assert helpers.rel_err(got, helpers.oracle_faithful(w)) <= helpers.BF16_TOL
+
+
+@pytest.mark.parametrize("H,D", [(4, 32), (4, 16), (8, 8)])
+def test_fully_masked_rows_stay_uniform(kutacc_lib, H, D):
+    w = W.random_gating_case(seed=78, B=3, S=200, H=H, D=D, mask_frac=0.0)
+    w.arrays["bias"] = np.stack([np.full(200, v, np.float32) for v in (LOWEST_BF16, -1e9, 0.0)])
+    w.arrays["nb"] = np.zeros_like(w.arrays["nb"])
+    w.arrays["nb"][1] = -2.0e9                 # one head of a row that is masked twice
+    w.arrays["bias"] = W.as_f32(W.bf16_bits(w.arrays["bias"]))
+    w.arrays["nb"] = W.as_f32(W.bf16_bits(w.arrays["nb"]))
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    assert helpers.rel_err(got, helpers.oracle_faithful(w)) <= helpers.BF16_TOL
+
+
+@pytest.mark.parametrize("H,D", [(4, 32), (8, 8)])
+def test_rescaling_of_rows_far_from_zero(kutacc_lib, H, D):
+    # logits are zero, so that every x is exact: 64 keys at b, 66 at b + 6 (just past the threshold of the running max)
+    w = W.random_gating_case(seed=79, B=6, S=130, H=H, D=D, mask_frac=0.0)
+    w.arrays["wq"] = np.zeros_like(w.arrays["wq"])
+    w.arrays["bias"] = W.as_f32(W.bf16_bits(np.repeat(np.array([[-0.7e7], [-0.9e7], [-1.1e7], [-1.3e7], [-1.5e7], [1.2e7]], np.float32), 130, 1)))
+    w.arrays["nb"] = np.zeros_like(w.arrays["nb"])
+    w.arrays["nb"][:, :, 64:] = 6.0
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    assert helpers.rel_err(got, helpers.oracle_faithful(w)) <= helpers.BF16_TOL

@@ -28,6 +28,7 @@
 #include "tma_utils.cuh"
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 
 namespace kutacc {
@@ -308,7 +309,9 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                     tmax = fmax3(tmax, pv[4 * c], pv[4 * c + 1]);
                     tmax = fmax3(tmax, pv[4 * c + 2], pv[4 * c + 3]);
                 }
-                if (kt == 0 && pass == 0) m = tmax;       // the first tile of an item sets the max (key 0 always exists)
+                // the first tile of an item sets the max, at least the lowest finite number: keys masked with -inf weigh nothing,
+                // and a row whose first keys are all of that kind is raised by its first finite one
+                if (kt == 0 && pass == 0) m = fmaxf(tmax, -FLT_MAX);
                 const bool grow = tmax > m + kRescaleThreshold;
                 if (!__any_sync(0xffffffffu, grow)) break;
                 // rare: the max of some row grew past the threshold. Rescale those rows of O (and their row sums); the product
@@ -327,12 +330,14 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 tmem_st_32x1(t_o + D, __float_as_uint(__uint_as_float(osum) * f));
                 tmem_st_wait();
             }
-            const uint64_t mneg2 = pack_f32x2(-m * kLog2e, -m * kLog2e);
+            // x - m first: with m * log2e folded into one multiply-add its rounding would differ from that of the factor that
+            // rescales O, and leave the range of the exponential for masks far below -1e9
+            const uint64_t mneg2 = pack_f32x2(-m, -m);
             uint32_t hi[32], lo[32];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 float e0, e1;
-                unpack_f32x2(fma_f32x2(pack_f32x2(pv[2 * j], pv[2 * j + 1]), log2e2, mneg2), e0, e1);
+                unpack_f32x2(mul_f32x2(add_f32x2(pack_f32x2(pv[2 * j], pv[2 * j + 1]), mneg2), log2e2), e0, e1);
                 const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
                 const float h0 = tf32_head(p0), h1 = tf32_head(p1);
                 hi[2 * j] = __float_as_uint(h0);

@@ -7,6 +7,7 @@ import torch
 from kutacc_b200 import api, runner
 from kutacc_b200 import workloads as W
 from . import helpers
+from .test_attention_core_gpu import LOWEST, masked_case
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +37,25 @@ def test_running_max_that_grows_late(kutacc_lib):
     w.arrays["mask"], w.arrays["bias"] = mask, (1e9 * (mask - 1.0)).astype(np.float32)
     w.arrays["nb"] = w.arrays["nb"].copy()
     w.arrays["nb"][:, :, 100:110] += 40.0
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
+
+
+@pytest.mark.parametrize("through_nb", [True, False])
+@pytest.mark.parametrize("value", [-np.inf, LOWEST, -3e9])
+def test_other_mask_values(kutacc_lib, value, through_nb):
+    w = masked_case(value, through_nb, 4, 32, "fp32")
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
+
+
+def test_rows_far_from_zero(kutacc_lib):
+    # fully masked rows stay uniform; logits are zero in the other rows, so that every x is exact: 64 keys at b, 66 at b + 6
+    w = W.random_gating_case(seed=80, B=5, S=130, H=4, D=32, dtype="fp32", mask_frac=0.0)
+    w.arrays["wq"] = np.zeros_like(w.arrays["wq"])
+    w.arrays["bias"] = np.repeat(np.array([[LOWEST], [-2e9], [-20000.0], [-30000.0], [25000.0]], np.float32), 130, 1)
+    w.arrays["nb"] = np.zeros_like(w.arrays["nb"])
+    w.arrays["nb"][:, :, 64:] = 6.0
     got = runner.out_to_f32(runner.DeviceCase(w).run())
     assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
 

@@ -69,7 +69,7 @@ constexpr int PRODUCER_WARP = SOFTMAX_WARPS, MASK_WARP = SOFTMAX_WARPS + 1, MMA_
 constexpr int THREADS = (SOFTMAX_WARPS + 2 + MMA_WARPS) * 32;
 constexpr int BAR_BYTES = 512;
 constexpr int WG_COLS = 128;          // tensor-memory columns of a warp group: S (then P) 0..63, O from 64
-constexpr int S_COL = 0, O_COL = 64;
+constexpr int S_COL = 0, O_COL = 64, LO_COL = 96;      // LO_COL: tails of P where it is split
 constexpr float kRescaleThreshold = 5.5f;     // P stays below 2^8
 constexpr float kFar = 2147483648.f;          // 2^31: mneg below it is within 64 of -m * log2e
 
@@ -80,6 +80,9 @@ struct Geo {
     static constexpr int VT_ROWS = (D + 16) / 16 * 16;        // channels, the ones row, zero rows
     static constexpr int Q_BYTES = BM * ROWB, K_BYTES = BN * ROWB, VT_BYTES = VT_ROWS * BN * 2;
     static constexpr int VT_TX = D * BN * 2;                  // bytes TMA writes of a V^T tile
+    // Head size 8 keeps 16 bits of P: a bf16 head and a bf16 tail, both multiplied by V^T (beside a product of 16 columns the
+    // second one is cheap, and heads of 8 had unrounded probabilities on the CUDA cores).
+    static constexpr bool SPLIT_P = D < 16;
 };
 
 struct AttnParams {
@@ -325,9 +328,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (elect_one()) {
                         const uint32_t vb = stage_base(s) + off_vt + w * T::VT_BYTES, t0 = tmem_base + w * WG_COLS;
 #pragma unroll
-                        for (int k = 0; k < BN / 16; ++k)
-                            tc_mma_bf16_ts(t0 + O_COL, t0 + S_COL + k * 8, make_smem_desc_kmajor(vb + k * 32, 128), idesc_o,
-                                           (kt > 0 || k > 0) ? 1u : 0u);
+                        for (int part = T::SPLIT_P ? 0 : 1; part < 2; ++part)            // tails, heads
+#pragma unroll
+                            for (int k = 0; k < BN / 16; ++k)
+                                tc_mma_bf16_ts(t0 + O_COL, t0 + (part == 0 ? LO_COL : S_COL) + k * 8,
+                                               make_smem_desc_kmajor(vb + k * 32, 128), idesc_o,
+                                               (kt > 0 || k > 0 || (T::SPLIT_P && part > 0)) ? 1u : 0u);
                         if (last) tc_commit(o_full(w));
                         if (last_w) tc_commit(kv_empty(s));
                     }
@@ -405,8 +411,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (HAS_NB) x2 = add_f32x2(x2, pack_f32x2(bf16lo_to_f32(f.nb[j]), bf16hi_to_f32(f.nb[j])));
                 return x2;
             };
+            // P of the pair of keys j of piece c
+            auto put = [&](const float e0, const float e1, const int c, const int j, uint32_t (&lo)[8]) {
+                const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
+                const uint32_t hi = pack_bf16x2(p0, p1);
+                pk[c * 8 + j] = hi;
+                if (T::SPLIT_P) lo[j] = pack_bf16x2(p0 - bf16lo_to_f32(hi), p1 - bf16hi_to_f32(hi));
+            };
             auto piece = [&](const uint32_t (&r)[16], const int c) {
                 Piece f;
+                uint32_t lo[8];
                 fetch(f, c);
                 const uint64_t mneg2 = pack_f32x2(mneg, mneg);
 #pragma unroll
@@ -416,8 +430,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     unpack_f32x2(x2, x0, x1);
                     tmax = fmax3(tmax, x0, x1);
                     unpack_f32x2(fma_f32x2(x2, log2e2, mneg2), e0, e1);
-                    pk[c * 8 + j] = pack_bf16x2(ex2_approx(e0), ex2_approx(e1));
+                    put(e0, e1, c, j, lo);
                 }
+                if (T::SPLIT_P) tmem_st_32x8(t_s - S_COL + LO_COL + c * 8, lo);
             };
             for (int pass = 0; pass < 2; ++pass) {
                 uint32_t a[16], b[16];
@@ -451,6 +466,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // rare: the max of some row grew past the threshold. Rescale those rows of O (and their row sums) and form
                 // the tile again against the new max. The product of the previous tile has retired: it was issued
                 // before the logits of this one.
+                if (T::SPLIT_P) tmem_st_wait();
                 const bool grow = tmax > m + kRescaleThreshold;
                 float f = 1.0f;
                 if (grow) {
@@ -483,6 +499,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         Piece pc;
+                        uint32_t lo[8];
                         fetch(pc, c);
                         tmem_ld_32x16(t_s + c * 16, a);
                         tmem_ld_wait16(a);
@@ -490,8 +507,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         for (int j = 0; j < 8; ++j) {
                             float e0, e1;
                             unpack_f32x2(fma_f32x2(add_f32x2(x_pair(a, pc, j), pack_f32x2(sub, sub)), log2e2, pack_f32x2(add, add)), e0, e1);
-                            pk[c * 8 + j] = pack_bf16x2(ex2_approx(e0), ex2_approx(e1));
+                            put(e0, e1, c, j, lo);
                         }
+                        if (T::SPLIT_P) tmem_st_32x8(t_s - S_COL + LO_COL + c * 8, lo);
                     }
                     break;
                 }

@@ -86,7 +86,8 @@ struct Geo {
 };
 
 struct AttnParams {
-    const __nv_bfloat16 *gate;        // [B, S, H*D], already bf16(sigmoid(bf16(x.Wg + bg)))
+    const __nv_bfloat16 *gate;        // [B, S, H*D]: bf16(x.Wg + bg), or with gate_is_sigmoid bf16(sigmoid(bf16(x.Wg + bg)))
+    int gate_is_sigmoid;
     const __nv_bfloat16 *bias;        // [B, S] (row stride bias_stride0)
     __nv_bfloat16 *avg;               // [B, S, H*D]
     int64_t bias_stride0;
@@ -561,7 +562,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         // the weighted average is stored as bf16 before gating in the reference (:128-133)
                         const int e = c * 8 + 2 * j;
                         const uint32_t wa = pack_bf16x2(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv);
-                        ow[j] = pack_bf16x2(bf16lo_to_f32(wa) * bf16lo_to_f32(gw[j]), bf16hi_to_f32(wa) * bf16hi_to_f32(gw[j]));
+                        float s0 = bf16lo_to_f32(gw[j]), s1 = bf16hi_to_f32(gw[j]);
+                        if (!p.gate_is_sigmoid) {
+                            s0 = __fdividef(1.0f, 1.0f + ex2_approx(-s0 * kLog2e));
+                            s1 = __fdividef(1.0f, 1.0f + ex2_approx(-s1 * kLog2e));
+                        }
+                        ow[j] = pack_bf16x2(bf16lo_to_f32(wa) * s0, bf16hi_to_f32(wa) * s1);
                     }
                     *(reinterpret_cast<uint4 *>(p.avg + base) + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
                 }
@@ -671,7 +677,7 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
 bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch,
                             const void *gate, const void *bias, int64_t bias_stride0, const void *nb,
                             int64_t nb_stride_h, int64_t nb_stride_q, void *avg, int B, int S, int H, int D,
-                            float scale)
+                            float scale, bool gate_is_sigmoid)
 {
     if ((D != 8 && D != 16 && D != 32) || vt_pitch % 8 != 0) return false;
     if (nb && ((nb_stride_h % 8) || (nb_stride_q % 8) || ((uintptr_t)nb % 16))) return false;
@@ -682,6 +688,7 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
     if (ew.device == nullptr) return false;
     AttnParams p;
     p.gate = (const __nv_bfloat16 *)gate;
+    p.gate_is_sigmoid = gate_is_sigmoid ? 1 : 0;
     p.bias = (const __nv_bfloat16 *)bias;
     p.avg = (__nv_bfloat16 *)avg;
     p.bias_stride0 = bias_stride0;

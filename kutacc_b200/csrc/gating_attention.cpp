@@ -194,6 +194,11 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         nb_sh = S * s_pad8;
     }
 
+    // Layers of 128 n channels with heads of 32: the projection stores the sigmoid of the gate, rounded to bf16, because the
+    // 32 exponentials per query and head are hidden there and not in the core. Narrower heads and layers store the gate itself
+    // and the core applies an fp32 sigmoid.
+    const bool gate_sigmoid = D == 32 && C % 128 == 0;
+
     // LayerNorm in front (head sizes up to 32): up to 256 channels the projection normalises its rows itself, on their way to
     // the tensor cores; wider rows do not fit beside the weights, and there LayerNorm is folded into the weights. Otherwise
     // the rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy.
@@ -241,19 +246,19 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
             if (ln_folded) {
                 ok = dev::launch_ln_stats(stream, x_c, nbr * S, C, C, ln->eps, st_c) &&
                      dev::tcgen05_proj_qkvg_bf16(stream, x_c, ln_w[0], ln_w[1], ln_w[2], ln_w[3], nullptr, q_c, k_c, v_km, g_c,
-                                                 (int)nbr, (int)S, (int)H, (int)D, true, s_pad8, /*gate_sigmoid=*/true, st_c,
+                                                 (int)nbr, (int)S, (int)H, (int)D, true, s_pad8, gate_sigmoid, st_c,
                                                  ln_s, ln_t);
                 if (!ok) return false;
                 v_key_major = true;
             } else if (D <= 32 && dev::tcgen05_proj_rows_bf16(stream, x_c, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
-                                                              (const float *)d_bg.dev, q_c, k_c, v_km, s_pad8, g_c, (int)nbr, (int)S,
-                                                              (int)H, (int)D, ln ? (const float *)d_lg.dev : nullptr,
+                                                              (const float *)d_bg.dev, q_c, k_c, v_km, s_pad8, g_c, gate_sigmoid, (int)nbr,
+                                                              (int)S, (int)H, (int)D, ln ? (const float *)d_lg.dev : nullptr,
                                                               ln ? (const float *)d_lb.dev : nullptr, ln ? ln->eps : 0.f)) {
                 ok = v_key_major = true;
             } else if (D <= 32 && !ln_in_proj) {
                 ok = dev::tcgen05_proj_qkvg_bf16(stream, x_c, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
                                                  (const float *)d_bg.dev, q_c, k_c, v_km, g_c, (int)nbr, (int)S, (int)H,
-                                                 (int)D, true, s_pad8, /*gate_sigmoid=*/true);
+                                                 (int)D, true, s_pad8, gate_sigmoid);
                 v_key_major = ok;
             }
             if (ln_in_proj && !ok) return false;
@@ -267,7 +272,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
             wait_for_pair_bias();
             if (ok && v_key_major)
                 ok = dev::tcgen05_attn_core_bf16(stream, q_c, k_c, v_km, s_pad8, g_c, bias_c, bias_s0, nb_dev, nb_sh,
-                                                 nb_sq, a_c, (int)nbr, (int)S, (int)H, (int)D, scale);
+                                                 nb_sq, a_c, (int)nbr, (int)S, (int)H, (int)D, scale, gate_sigmoid);
             else
                 ok = ok && dev::launch_attn_core_bf16(stream, q_c, k_c, v_c, g_c, bias_c, bias_s0, nb_dev, nb_sh, nb_sq,
                                                       a_c, (int)nbr, (int)S, (int)H, (int)D, scale);

@@ -1,9 +1,9 @@
 // Q/K/V/gate projection of the attention on the fifth-generation tensor cores, with the LayerNorm in front of it where the
 // caller asks for one (up to 256 channels).
 //
-//   q, k [B, H, S, D], v^T [B, H*D, S] (row pitch a multiple of 8), gate = bf16(sigmoid(bf16(x.Wg + bg))) [B, S, C]
+//   q, k [B, H, S, D], v^T [B, H*D, S] (row pitch a multiple of 8), gate = bf16(x.Wg + bg) [B, S, C] or bf16(sigmoid(gate))
 //
-// (src/attention/gating_attention.cpp:47-66; the sigmoid of :134-147 is applied here.) The activations stand still: a
+// (src/attention/gating_attention.cpp:47-66; with gate_sigmoid the sigmoid of :134-147 is applied here.) The activations stand still: a
 // persistent CTA (one per SM) loads a block of 256 rows once, all K columns of it, and streams the four weights past it in
 // slabs of 128 channels x 64 columns, each of which serves both 128-row tiles of the block. With a 128 x 128 tile at a time
 // every tile brought its own 64 to 128 KB of operands from L2, which bound the kernel: 146 us for 196608 rows x 256 channels.
@@ -71,6 +71,7 @@ struct ProjParams {
     const float *bg, *gamma, *beta;     // gamma: null without LayerNorm
     float eps;
     int S, B, D;
+    int gate_sigmoid;     // the stored gate is bf16(sigmoid(bf16(x.Wg + bg)))
     int s32;              // 32-row groups per batch row
     int rows128;          // S is a multiple of 128: a row tile is one box
     int whole;            // a unit of work is a block with all its column tiles, up to this unit;
@@ -310,10 +311,14 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
 #pragma unroll
                         for (int j4 = 0; j4 < 8; ++j4) {
                             const float4 bv = lds128_f32(bg_a + (uint32_t)((nn + 4 * j4) * 4));
-                            packed[2 * j4] = pack_bf16x2(sigmoid_of_bf16(__uint_as_float(r[c][4 * j4]) + bv.x),
-                                                         sigmoid_of_bf16(__uint_as_float(r[c][4 * j4 + 1]) + bv.y));
-                            packed[2 * j4 + 1] = pack_bf16x2(sigmoid_of_bf16(__uint_as_float(r[c][4 * j4 + 2]) + bv.z),
-                                                             sigmoid_of_bf16(__uint_as_float(r[c][4 * j4 + 3]) + bv.w));
+                            float y[4] = {__uint_as_float(r[c][4 * j4]) + bv.x, __uint_as_float(r[c][4 * j4 + 1]) + bv.y,
+                                          __uint_as_float(r[c][4 * j4 + 2]) + bv.z, __uint_as_float(r[c][4 * j4 + 3]) + bv.w};
+                            if (p.gate_sigmoid) {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) y[e] = sigmoid_of_bf16(y[e]);
+                            }
+                            packed[2 * j4] = pack_bf16x2(y[0], y[1]);
+                            packed[2 * j4 + 1] = pack_bf16x2(y[2], y[3]);
                         }
                     } else {
 #pragma unroll
@@ -418,8 +423,8 @@ bool launch_ks(cudaStream_t stream, const ProjMaps &maps, ProjParams p)
 }  // namespace
 
 bool tcgen05_proj_rows_bf16(cudaStream_t stream, const void *x, const void *wq, const void *wk, const void *wv, const void *wg,
-                            const float *bg, void *q, void *k, void *vt, int64_t vt_pitch, void *gate, int B, int S, int H, int D,
-                            const float *ln_gamma, const float *ln_beta, float ln_eps)
+                            const float *bg, void *q, void *k, void *vt, int64_t vt_pitch, void *gate, bool gate_sigmoid, int B, int S,
+                            int H, int D, const float *ln_gamma, const float *ln_beta, float ln_eps)
 {
     const int C = H * D;
     if ((C != 64 && C != 128 && C != 256) || (D != 8 && D != 16 && D != 32) || vt_pitch % 8 != 0 || vt_pitch < S) return false;
@@ -449,6 +454,7 @@ bool tcgen05_proj_rows_bf16(cudaStream_t stream, const void *x, const void *wq, 
     p.S = S;
     p.B = B;
     p.D = D;
+    p.gate_sigmoid = gate_sigmoid ? 1 : 0;
     p.s32 = (int)s32;
     p.err = ew.device;
     return C == 64 ? launch_ks<1>(stream, maps, p) : C == 128 ? launch_ks<2>(stream, maps, p) : launch_ks<4>(stream, maps, p);

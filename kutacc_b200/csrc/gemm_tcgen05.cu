@@ -506,13 +506,14 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
     p.relu = 0;
     p.sigmoid_mask = gate_sigmoid ? 0x8 : 0;
     p.err = ew.device;
-    if (v_transposed != gate_sigmoid || (!v_transposed && (D < 32 || ln_stats))) return false;       // not used together
     const bool heads64 = C == 64 || D < 32;
+    // combinations that no caller uses: the attention core of wide layers with heads of 32 takes the sigmoid, the others the gate
+    if (gate_sigmoid != (v_transposed && !heads64) || (!v_transposed && (D < 32 || ln_stats))) return false;
     if (ln_stats)
-        return heads64 ? launch<F_TRANSPOSED | F_SIGMOID | F_LN | F_HEADS64>(stream, maps, p, "proj_qkvg_ln")
+        return heads64 ? launch<F_TRANSPOSED | F_LN | F_HEADS64>(stream, maps, p, "proj_qkvg_ln")
                        : launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln");
     if (v_transposed)
-        return heads64 ? launch<F_TRANSPOSED | F_SIGMOID | F_HEADS64>(stream, maps, p, "proj_qkvg")
+        return heads64 ? launch<F_TRANSPOSED | F_HEADS64>(stream, maps, p, "proj_qkvg")
                        : launch<F_TRANSPOSED | F_SIGMOID>(stream, maps, p, "proj_qkvg");
     return heads64 ? launch<F_HEADS64>(stream, maps, p, "proj_qkvg") : launch<0>(stream, maps, p, "proj_qkvg");
 }

@@ -36,11 +36,12 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
                             const void *ln_stats = nullptr, const float *const *ln_s = nullptr,
                             const float *const *ln_t = nullptr);
 // The same for up to 256 channels with the rows kept in shared memory while the weights stream past (gemm_proj.cu): q and k
-// [B, H, S, D], v^T [B, H*D, S] with row pitch vt_pitch, gate = bf16(sigmoid(bf16(x.Wg + bg))) [B, S, C]. With ln_gamma the
-// projections are those of LayerNorm(x). C in {64, 128, 256}, D in {8, 16, 32}; false otherwise.
+// [B, H, S, D], v^T [B, H*D, S] with row pitch vt_pitch, gate = bf16(x.Wg + bg) [B, S, C], or with gate_sigmoid
+// bf16(sigmoid(gate)). With ln_gamma the projections are those of LayerNorm(x). C in {64, 128, 256}, D in {8, 16, 32}; false
+// otherwise.
 bool tcgen05_proj_rows_bf16(cudaStream_t stream, const void *x, const void *wq, const void *wk, const void *wv, const void *wg,
-                            const float *bg, void *q, void *k, void *vt, int64_t vt_pitch, void *gate, int B, int S, int H, int D,
-                            const float *ln_gamma, const float *ln_beta, float ln_eps);
+                            const float *bg, void *q, void *k, void *vt, int64_t vt_pitch, void *gate, bool gate_sigmoid, int B, int S,
+                            int H, int D, const float *ln_gamma, const float *ln_beta, float ln_eps);
 // a_row_stride (elements, 0 = K): row stride of a, whose batch rows are S rows apart.
 bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w, const float *bias, void *out,
                               int64_t out_row_stride, int B, int S, int N, int K, bool relu = false,
@@ -110,12 +111,12 @@ bool launch_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, co
                            int64_t nb_stride_q, void *avg, int B, int S, int H, int D, float scale);
 
 // The same operator with both products on tcgen05 and the accumulators in tensor memory (head sizes 8, 16, 32).
-// vt is v transposed, [B, H, D, S] with row pitch vt_pitch, as tcgen05_proj_qkvg_bf16 writes it; `gate` already holds
-// bf16(sigmoid(bf16(x.Wg + bg))) (the projection kernel's gate_sigmoid option): the kernel only multiplies.
+// vt is v transposed, [B, H, D, S] with row pitch vt_pitch, as tcgen05_proj_qkvg_bf16 writes it. With gate_is_sigmoid `gate`
+// already holds bf16(sigmoid(bf16(x.Wg + bg))) (the projection kernels' gate_sigmoid option) and the kernel only multiplies.
 bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch,
                             const void *gate, const void *bias, int64_t bias_stride0, const void *nb,
                             int64_t nb_stride_h, int64_t nb_stride_q, void *avg, int B, int S, int H, int D,
-                            float scale);
+                            float scale, bool gate_is_sigmoid);
 
 // ---- generic (any shape, bf16 or fp32 storage, fp32 math) ------------------------------------------
 // c[m, n] = sum_k a[m, k] * w[n, k] (+ bias[n]) (+ beta * c[m, n]); a row stride lda, w row stride

@@ -5,15 +5,17 @@
 // tcgen05.mma has no fp32 input type; its tf32 kind keeps 11 significant bits of each operand. Every operand is
 // therefore split beforehand (split_tf32_kernel) into a tf32 head and a tail, x = hi + lo with |lo| <= 2^-11 |x|,
 // stored side by side as one row [hi(0..K) | lo(0..K)] of 2K floats, and the product is taken as
-//   lo(A).hi(W) + hi(A).lo(W) + hi(A).hi(W)        (small terms first; lo.lo, about 2^-22 of the result, is dropped)
-// accumulated in fp32 in tensor memory. Persistent CTAs, one per SM, walk 128 x 256 output tiles (128 x 128 where there are too
+//   lo(A).hi(W) + hi(A).lo(W) + hi(A).hi(W)        (lo.lo, about 2^-22 of the result, is dropped)
+// accumulated in fp32 in tensor memory, the small products in an accumulator of their own that the epilogue adds: the tensor
+// core truncates at every accumulation, and with all three products in one accumulator there are three times as many of them
+// at full magnitude (2-norm error at K = 256: 1.7e-6, this way 6.4e-7). Persistent CTAs, one per SM, walk 128 x 256 output tiles (128 x 128 where there are too
 // few of the wide ones to go round or the columns do not divide):
 //   warp 0      producer: per 32-column slab of K one stage with the heads AND tails of A' and W' (TMA, 128-byte swizzle), so
 //               that the three products read each slab from L2 once
-//   warp 1      MMA issuer: one elected lane issues the 12 tcgen05.mma kind::tf32 (K = 8) of a stage into one of two
-//               TMEM accumulators and commits to mbarriers
-//   warps 2-9   epilogue: each warp owns 32 TMEM lanes x half of the columns: tcgen05.ld, bias add, staging tile (32 x 32),
-//               TMA store
+//   warp 1      MMA issuer: one elected lane issues the 12 tcgen05.mma kind::tf32 (K = 8) of a stage into a pair of TMEM
+//               accumulators (two pairs of 128 columns each, or one of 256) and commits to mbarriers
+//   warps 2-9   epilogue: each warp owns 32 TMEM lanes x half of the columns: tcgen05.ld of both accumulators into
+//               registers, which frees them, then bias add, staging tile (32 x 32), TMA store
 // Up to four weight matrices share one pass over A (the fused Q/K/V/gate projection of the fp32 attention).
 // What bounds it: the way of the operands from L2. Loading the slab pair of each product by itself with 128 x 128 tiles
 // moves 1.6 GB for 32768 x 1024 x 256 (10 TB/s at its 160 us); sharing the slabs halves that.
@@ -39,7 +41,6 @@ namespace dev {
 namespace {
 
 constexpr int BM = 128, BK = 32;                        // BK floats = one 128-byte swizzle row
-constexpr int ACC_STAGES = 2;
 constexpr int SLAB_BYTES = 128 * BK * 4;                // 16 KB: 128 rows of A', or of W'
 constexpr int EPI_WARPS = 8;
 constexpr int STG_BYTES = 32 * 32 * 4;                  // one staging tile per epilogue warp
@@ -50,11 +51,12 @@ struct Geo {
     static constexpr int NB = BN / 128;                              // 128-column blocks of a tile
     static constexpr int STAGE_BYTES = 2 * (1 + NB) * SLAB_BYTES;    // heads and tails of A' and W'
     static constexpr int NSTAGE = BN == 256 ? 2 : 3;
+    static constexpr int ACC_STAGES = 256 / BN;                      // pairs of accumulators (hi.hi; the two small products)
     static constexpr int STG_OFF = NSTAGE * STAGE_BYTES;
     static constexpr int BAR_OFF = STG_OFF + EPI_WARPS * STG_BYTES;
     static constexpr int NBARS = 2 * NSTAGE + 2 * ACC_STAGES;
     static constexpr int SMEM_BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;
-    static constexpr int TMEM_COLS = ACC_STAGES * BN;
+    static constexpr int TMEM_COLS = ACC_STAGES * 2 * BN;
     static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
 };
 
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 gemm_tf32x3_tc_kernel(const __grid_constant__ Tf32Maps maps, const __grid_constant__ Tf32Params p)
 {
     using T = Geo<BN>;
-    constexpr int NSTAGE = T::NSTAGE;
+    constexpr int NSTAGE = T::NSTAGE, ACC_STAGES = T::ACC_STAGES;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t bar_base = smem + T::BAR_OFF;
@@ -175,7 +177,7 @@ gemm_tf32x3_tc_kernel(const __grid_constant__ Tf32Maps maps, const __grid_consta
                 break;
             }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + (uint32_t)(a * BN);
+            const uint32_t d_tmem = tmem_base + (uint32_t)(a * 2 * BN);
             for (int kc = 0; kc < nk; ++kc, ++it) {
                 const int s = it % NSTAGE;
                 if (!mbar_wait_warp(full_bar(s), (uint32_t)((it / NSTAGE) & 1), p.err, 43)) {
@@ -189,8 +191,8 @@ gemm_tf32x3_tc_kernel(const __grid_constant__ Tf32Maps maps, const __grid_consta
                     for (int pr = 0; pr < 3; ++pr)                   // tail.head, head.tail, head.head
 #pragma unroll
                         for (int k = 0; k < BK / 8; ++k)             // 8 tf32 = 32 bytes per instruction
-                            tc_mma_tf32(d_tmem, ad + (pr == 0 ? SLAB16 : 0u) + 2 * k, wd + (pr == 1 ? T::NB * SLAB16 : 0u) + 2 * k,
-                                        idesc, (kc > 0 || pr > 0 || k > 0) ? 1u : 0u);
+                            tc_mma_tf32(d_tmem + (pr < 2 ? BN : 0), ad + (pr == 0 ? SLAB16 : 0u) + 2 * k,
+                                        wd + (pr == 1 ? T::NB * SLAB16 : 0u) + 2 * k, idesc, (kc > 0 || pr == 1 || k > 0) ? 1u : 0u);
                     tc_commit(empty_bar(s));                 // the stage may be overwritten once these MMAs retire
                     if (kc == nk - 1) tc_commit(acc_full(a));
                 }
@@ -218,19 +220,28 @@ gemm_tf32x3_tc_kernel(const __grid_constant__ Tf32Maps maps, const __grid_consta
                 const int b = m / p.S;
                 tdst = p.out_t[seg] + ((int64_t)b * (p.N / 32) + n0 / 32) * 64 * p.vt_pitch + (m - b * p.S);
             }
-            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN + half * COLS);
-#pragma unroll 1
+            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * 2 * BN + half * COLS);
+            uint32_t acc[COLS / 32][32];
+#pragma unroll
             for (int c = 0; c < COLS / 32; ++c) {
-                uint32_t r[32];
-                __syncwarp();
-                tmem_ld_32x32(tcol + c * 32, r);
-                tmem_ld_wait();
-                if (c == COLS / 32 - 1) {
-                    // everything is in registers: the accumulator may be overwritten by the tile after next
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty(a));
+                tmem_ld_32x32(tcol + c * 32, acc[c]);
+#pragma unroll
+                for (int q = 0; q < 32; q += 16) {
+                    uint32_t small[16];
+                    tmem_ld_32x16(tcol + BN + c * 32 + q, small);
+                    tmem_ld_wait16(small);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        acc[c][q + j] = __float_as_uint(__uint_as_float(acc[c][q + j]) + __uint_as_float(small[j]));
                 }
+            }
+            // everything is in registers: the accumulators may be overwritten
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty(a));
+#pragma unroll
+            for (int c = 0; c < COLS / 32; ++c) {
+                uint32_t(&r)[32] = acc[c];
                 const int n = n0 + c * 32;
                 if (bias) {
 #pragma unroll

@@ -72,6 +72,19 @@ def test_linear_fp32(kutacc_lib, M, N, K):
     assert (r.cpu().double() - ref).abs().max() <= 4e-6 * ref.abs().max()
 
 
+# The tensor core truncates: each of the K / 8 accumulations of the large product loses half a unit, 2^-24, of a partial sum on
+# average; partial sums are two thirds of the result on average, and lie anywhere in their binade (0.72).
+@pytest.mark.parametrize("M,N,K", [(300, 128, 512), (9600, 512, 512), (2000, 256, 128)])
+def test_linear_fp32_accumulation(kutacc_lib, M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g) / K ** 0.5
+    ad, wd, bd, r = a.cuda(), w.cuda(), torch.zeros(N, device="cuda"), torch.zeros(M, N, device="cuda")
+    api.linear(api.tensor(ad), api.tensor(wd), bd.data_ptr(), api.tensor(r))
+    torch.cuda.synchronize()
+    ref = a.double() @ w.double().T
+    assert (r.cpu().double() - ref).norm() <= K / 8 * 2.0 ** -24 * 0.72 * 2 / 3 * ref.norm()
+
+
 @pytest.mark.parametrize("R,Nk,Cz,H", [(8, 100, 128, 8), (3, 33, 64, 4), (1, 1, 32, 3), (40, 301, 128, 1)])
 def test_pair_bias_fp32(kutacc_lib, R, Nk, Cz, H):
     g = torch.Generator().manual_seed(R * Nk + Cz)

@@ -69,7 +69,7 @@ constexpr int PRODUCER_WARP = SOFTMAX_WARPS, MASK_WARP = SOFTMAX_WARPS + 1, MMA_
 constexpr int THREADS = (SOFTMAX_WARPS + 2 + MMA_WARPS) * 32;
 constexpr int BAR_BYTES = 512;
 constexpr int WG_COLS = 128;          // tensor-memory columns of a warp group: S (then P) 0..63, O from 64
-constexpr int S_COL = 0, O_COL = 64, LO_COL = 96;      // LO_COL: tails of P where it is split
+constexpr int S_COL = 0, O_COL = 64;
 constexpr float kRescaleThreshold = 5.5f;     // P stays below 2^8
 constexpr float kFar = 2147483648.f;          // 2^31: mneg below it is within 64 of -m * log2e
 
@@ -80,14 +80,10 @@ struct Geo {
     static constexpr int VT_ROWS = (D + 16) / 16 * 16;        // channels, the ones row, zero rows
     static constexpr int Q_BYTES = BM * ROWB, K_BYTES = BN * ROWB, VT_BYTES = VT_ROWS * BN * 2;
     static constexpr int VT_TX = D * BN * 2;                  // bytes TMA writes of a V^T tile
-    // Head size 8 keeps 16 bits of P: a bf16 head and a bf16 tail, both multiplied by V^T (beside a product of 16 columns the
-    // second one is cheap, and heads of 8 had unrounded probabilities on the CUDA cores).
-    static constexpr bool SPLIT_P = D < 16;
 };
 
 struct AttnParams {
-    const __nv_bfloat16 *gate;        // [B, S, H*D]: bf16(x.Wg + bg), or with gate_is_sigmoid bf16(sigmoid(bf16(x.Wg + bg)))
-    int gate_is_sigmoid;
+    const __nv_bfloat16 *gate;        // [B, S, H*D]: SPLIT bf16(x.Wg + bg), otherwise bf16(sigmoid(bf16(x.Wg + bg)))
     const __nv_bfloat16 *bias;        // [B, S] (row stride bias_stride0)
     __nv_bfloat16 *avg;               // [B, S, H*D]
     int64_t bias_stride0;
@@ -103,7 +99,14 @@ struct AttnParams {
     float scale;
 };
 
-template <int D, bool HAS_NB>
+// SPLIT: 16 bits of P, a bf16 head and a bf16 tail, both multiplied by V^T, for narrow heads and 64-channel layers: heads of 8
+// had unrounded probabilities on the CUDA cores, and bf16 ones are less exact against a stale maximum than against the true
+// one, where the largest is exactly 1 (error of the layer against 64 bits 1 to 5 % larger; this way 1 % smaller). It costs
+// 129 -> 150 us for 256 x 384 rows of 8 heads of 8, 41 -> 49 us for 256 x 256 rows of 4 heads of 16.
+// Tails of 16 keys from column tail_col(c, D) on: beside O, and for heads of 32 half of them over logits already read.
+__device__ __forceinline__ constexpr int tail_col(int c, int D) { return D < 32 ? 96 + 8 * c : c < 2 ? 112 + 8 * c : 16 + 8 * c; }
+
+template <int D, bool SPLIT, bool HAS_NB>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_vt, const __grid_constant__ CUtensorMap tm_nb,
@@ -329,12 +332,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (elect_one()) {
                         const uint32_t vb = stage_base(s) + off_vt + w * T::VT_BYTES, t0 = tmem_base + w * WG_COLS;
 #pragma unroll
-                        for (int part = T::SPLIT_P ? 0 : 1; part < 2; ++part)            // tails, heads
+                        for (int part = SPLIT ? 0 : 1; part < 2; ++part)            // tails, heads
 #pragma unroll
                             for (int k = 0; k < BN / 16; ++k)
-                                tc_mma_bf16_ts(t0 + O_COL, t0 + (part == 0 ? LO_COL : S_COL) + k * 8,
+                                tc_mma_bf16_ts(t0 + O_COL, t0 + (part == 0 ? tail_col(k, D) : S_COL + k * 8),
                                                make_smem_desc_kmajor(vb + k * 32, 128), idesc_o,
-                                               (kt > 0 || k > 0 || (T::SPLIT_P && part > 0)) ? 1u : 0u);
+                                               (kt > 0 || k > 0 || (SPLIT && part > 0)) ? 1u : 0u);
                         if (last) tc_commit(o_full(w));
                         if (last_w) tc_commit(kv_empty(s));
                     }
@@ -381,7 +384,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             const uint32_t st = stage_base(g % NST);
             if (!mbar_wait_warp(s_full(wg), (uint32_t)(g & 1), p.err, 26)) return false;
             tc_fence_after();
-            uint32_t pk[32];
+            uint32_t pk[32], late[2][8];              // late: tails of keys 32..63 for heads of 32
             float tmax;
             // x = bf16(logit) * scale + bias (+ pair bias) of the pair of keys 2j, 2j + 1 of a 16-key piece
             struct Piece {
@@ -417,7 +420,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
                 const uint32_t hi = pack_bf16x2(p0, p1);
                 pk[c * 8 + j] = hi;
-                if (T::SPLIT_P) lo[j] = pack_bf16x2(p0 - bf16lo_to_f32(hi), p1 - bf16hi_to_f32(hi));
+                if (SPLIT) lo[j] = pack_bf16x2(p0 - bf16lo_to_f32(hi), p1 - bf16hi_to_f32(hi));
+            };
+            auto put_tails = [&](const uint32_t (&lo)[8], const int c) {
+                if (!SPLIT) return;
+                if (D < 32 || c < 2) {
+                    tmem_st_32x8(t_s - S_COL + tail_col(c, D), lo);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) late[c & 1][j] = lo[j];
+                }
             };
             auto piece = [&](const uint32_t (&r)[16], const int c) {
                 Piece f;
@@ -433,7 +445,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     unpack_f32x2(fma_f32x2(x2, log2e2, mneg2), e0, e1);
                     put(e0, e1, c, j, lo);
                 }
-                if (T::SPLIT_P) tmem_st_32x8(t_s - S_COL + LO_COL + c * 8, lo);
+                put_tails(lo, c);
             };
             for (int pass = 0; pass < 2; ++pass) {
                 uint32_t a[16], b[16];
@@ -467,7 +479,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // rare: the max of some row grew past the threshold. Rescale those rows of O (and their row sums) and form
                 // the tile again against the new max. The product of the previous tile has retired: it was issued
                 // before the logits of this one.
-                if (T::SPLIT_P) tmem_st_wait();
+                if (SPLIT) tmem_st_wait();
                 const bool grow = tmax > m + kRescaleThreshold;
                 float f = 1.0f;
                 if (grow) {
@@ -510,12 +522,16 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             unpack_f32x2(fma_f32x2(add_f32x2(x_pair(a, pc, j), pack_f32x2(sub, sub)), log2e2, pack_f32x2(add, add)), e0, e1);
                             put(e0, e1, c, j, lo);
                         }
-                        if (T::SPLIT_P) tmem_st_32x8(t_s - S_COL + LO_COL + c * 8, lo);
+                        put_tails(lo, c);
                     }
                     break;
                 }
             }
             tmem_st_32x32(t_s, pk);
+            if (SPLIT && D == 32) {
+                tmem_st_32x8(t_s - S_COL + tail_col(2, D), late[0]);
+                tmem_st_32x8(t_s - S_COL + tail_col(3, D), late[1]);
+            }
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
@@ -563,7 +579,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         const int e = c * 8 + 2 * j;
                         const uint32_t wa = pack_bf16x2(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv);
                         float s0 = bf16lo_to_f32(gw[j]), s1 = bf16hi_to_f32(gw[j]);
-                        if (!p.gate_is_sigmoid) {
+                        if (SPLIT) {
                             s0 = __fdividef(1.0f, 1.0f + ex2_approx(-s0 * kLog2e));
                             s1 = __fdividef(1.0f, 1.0f + ex2_approx(-s1 * kLog2e));
                         }
@@ -602,13 +618,13 @@ int smem_bytes(int G, bool has_nb)
     return 1024 + 1024 + G * T::Q_BYTES + NST * (G * (T::K_BYTES + T::VT_BYTES) + (has_nb ? NB_BYTES : 0) + MB_BYTES);
 }
 
-template <int D, bool HAS_NB>
+template <int D, bool SPLIT, bool HAS_NB>
 bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tvt,
                 const CUtensorMap &tnb, const AttnParams &p)
 {
     static bool configured = false;
     if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, HAS_NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, SPLIT, HAS_NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_bytes<D>(MAXG, HAS_NB)));
         configured = true;
     }
@@ -617,7 +633,7 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
     q.counter = work_counter(stream);
     if (q.counter == nullptr) return false;
     KernelTimer timer__("attn_core", stream);
-    launch_chained(attn_tc_kernel<D, HAS_NB>, grid, THREADS, smem_bytes<D>(p.G, HAS_NB), stream, tq, tk, tvt, tnb, q);
+    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB>, grid, THREADS, smem_bytes<D>(p.G, HAS_NB), stream, tq, tk, tvt, tnb, q);
     count_launch();
     return true;
 }
@@ -641,7 +657,7 @@ int pick_group(int64_t B, int64_t hq, int sms)
     return best;
 }
 
-template <int D>
+template <int D, bool SPLIT>
 bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch, const void *nb,
               int64_t nb_stride_h, int64_t nb_stride_q, AttnParams &p)
 {
@@ -666,10 +682,10 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
                                             BM, 128)) {
             return false;
         }
-        return launch_one<D, true>(stream, tq, tk, tvt, tnb, p);
+        return launch_one<D, SPLIT, true>(stream, tq, tk, tvt, tnb, p);
     }
     tnb = tk;
-    return launch_one<D, false>(stream, tq, tk, tvt, tnb, p);
+    return launch_one<D, SPLIT, false>(stream, tq, tk, tvt, tnb, p);
 }
 
 }  // namespace
@@ -679,7 +695,7 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
                             int64_t nb_stride_h, int64_t nb_stride_q, void *avg, int B, int S, int H, int D,
                             float scale, bool gate_is_sigmoid)
 {
-    if ((D != 8 && D != 16 && D != 32) || vt_pitch % 8 != 0) return false;
+    if ((D != 8 && D != 16 && D != 32) || (gate_is_sigmoid && D != 32) || vt_pitch % 8 != 0) return false;
     if (nb && ((nb_stride_h % 8) || (nb_stride_q % 8) || ((uintptr_t)nb % 16))) return false;
     if ((((uintptr_t)gate | (uintptr_t)avg) & 15u) != 0) return false;
     const int64_t n_qt = (S + BM - 1) / BM;
@@ -688,7 +704,6 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
     if (ew.device == nullptr) return false;
     AttnParams p;
     p.gate = (const __nv_bfloat16 *)gate;
-    p.gate_is_sigmoid = gate_is_sigmoid ? 1 : 0;
     p.bias = (const __nv_bfloat16 *)bias;
     p.avg = (__nv_bfloat16 *)avg;
     p.bias_stride0 = bias_stride0;
@@ -702,9 +717,11 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
     p.scale = scale;
     p.counter = nullptr;
     switch (D) {
-        case 8: return launch_d<8>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p);
-        case 16: return launch_d<16>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p);
-        default: return launch_d<32>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p);
+        case 8: return launch_d<8, true>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p);
+        case 16: return launch_d<16, true>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p);
+        default:
+            return gate_is_sigmoid ? launch_d<32, false>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p)
+                                   : launch_d<32, true>(stream, q, k, vt, vt_pitch, nb, nb_stride_h, nb_stride_q, p);
     }
 }
 

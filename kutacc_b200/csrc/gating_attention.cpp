@@ -200,10 +200,10 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     const bool gate_sigmoid = D == 32 && C % 128 == 0;
 
     // LayerNorm in front (head sizes up to 32): up to 256 channels the projection normalises its rows itself, on their way to
-    // the tensor cores; wider rows do not fit beside the weights, and there LayerNorm is folded into the weights. Otherwise
-    // the rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy.
+    // the tensor cores; wider rows do not fit beside the weights, and there LayerNorm is folded into the weights (heads of 32).
+    // Otherwise the rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy.
     const bool ln_in_proj = ln && fast && D <= 32 && (C == 64 || C == 128 || C == 256);
-    const bool ln_folded = ln && fast && D <= 32 && C % 128 == 0 && !ln_in_proj;
+    const bool ln_folded = ln && fast && D == 32 && C % 128 == 0 && !ln_in_proj;
     if (ln_folded) {
         const void *w_in[4] = {d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev};
         const float *b_in[4] = {nullptr, nullptr, nullptr, (const float *)d_bg.dev};

@@ -509,9 +509,7 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
     const bool heads64 = C == 64 || D < 32;
     // combinations that no caller uses: the attention core of wide layers with heads of 32 takes the sigmoid, the others the gate
     if (gate_sigmoid != (v_transposed && !heads64) || (!v_transposed && (D < 32 || ln_stats))) return false;
-    if (ln_stats)
-        return heads64 ? launch<F_TRANSPOSED | F_LN | F_HEADS64>(stream, maps, p, "proj_qkvg_ln")
-                       : launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln");
+    if (ln_stats) return heads64 ? false : launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln");
     if (v_transposed)
         return heads64 ? launch<F_TRANSPOSED | F_HEADS64>(stream, maps, p, "proj_qkvg")
                        : launch<F_TRANSPOSED | F_SIGMOID>(stream, maps, p, "proj_qkvg");

@@ -112,7 +112,8 @@ bool launch_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, co
 
 // The same operator with both products on tcgen05 and the accumulators in tensor memory (head sizes 8, 16, 32).
 // vt is v transposed, [B, H, D, S] with row pitch vt_pitch, as tcgen05_proj_qkvg_bf16 writes it. With gate_is_sigmoid `gate`
-// already holds bf16(sigmoid(bf16(x.Wg + bg))) (the projection kernels' gate_sigmoid option) and the kernel only multiplies.
+// already holds bf16(sigmoid(bf16(x.Wg + bg))) (the projection kernels' gate_sigmoid option; heads of 32 only), the kernel only
+// multiplies, and the probabilities are bf16; otherwise the sigmoid is taken here, and the probabilities keep 16 bits.
 bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch,
                             const void *gate, const void *bias, int64_t bias_stride0, const void *nb,
                             int64_t nb_stride_h, int64_t nb_stride_q, void *avg, int B, int S, int H, int D,

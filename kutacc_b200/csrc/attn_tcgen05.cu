@@ -386,6 +386,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             tc_fence_after();
             uint32_t pk[32], late[2][8];              // late: tails of keys 32..63 for heads of 32
             float tmax;
+            bool stored = false;                      // P is already in tensor memory
             // x = bf16(logit) * scale + bias (+ pair bias) of the pair of keys 2j, 2j + 1 of a 16-key piece
             struct Piece {
                 float mb[16];
@@ -415,21 +416,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (HAS_NB) x2 = add_f32x2(x2, pack_f32x2(bf16lo_to_f32(f.nb[j]), bf16hi_to_f32(f.nb[j])));
                 return x2;
             };
-            // P of the pair of keys j of piece c
-            auto put = [&](const float e0, const float e1, const int c, const int j, uint32_t (&lo)[8]) {
+            auto prob = [&](const float e0, const float e1, uint32_t &hi, uint32_t &lo) {
                 const float p0 = ex2_approx(e0), p1 = ex2_approx(e1);
-                const uint32_t hi = pack_bf16x2(p0, p1);
-                pk[c * 8 + j] = hi;
-                if (SPLIT) lo[j] = pack_bf16x2(p0 - bf16lo_to_f32(hi), p1 - bf16hi_to_f32(hi));
-            };
-            auto put_tails = [&](const uint32_t (&lo)[8], const int c) {
-                if (!SPLIT) return;
-                if (D < 32 || c < 2) {
-                    tmem_st_32x8(t_s - S_COL + tail_col(c, D), lo);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) late[c & 1][j] = lo[j];
-                }
+                hi = pack_bf16x2(p0, p1);
+                if (SPLIT) lo = pack_bf16x2(p0 - bf16lo_to_f32(hi), p1 - bf16hi_to_f32(hi));
             };
             auto piece = [&](const uint32_t (&r)[16], const int c) {
                 Piece f;
@@ -443,9 +433,13 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     unpack_f32x2(x2, x0, x1);
                     tmax = fmax3(tmax, x0, x1);
                     unpack_f32x2(fma_f32x2(x2, log2e2, mneg2), e0, e1);
-                    put(e0, e1, c, j, lo);
+                    prob(e0, e1, pk[c * 8 + j], lo[j]);
                 }
-                put_tails(lo, c);
+                if (SPLIT && (D < 32 || c < 2)) tmem_st_32x8(t_s - S_COL + tail_col(c, D), lo);
+                if (SPLIT && D == 32 && c >= 2) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) late[c & 1][j] = lo[j];
+                }
             };
             for (int pass = 0; pass < 2; ++pass) {
                 uint32_t a[16], b[16];
@@ -508,11 +502,12 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     tmem_st_wait();
                 }
                 if (__any_sync(0xffffffffu, far_row())) {
+                    // piece by piece, P over logits already read (a loop, so that the usual path stays short)
                     const float sub = far_row() ? -m : 0.f, add = far_row() ? 0.f : mneg;
-#pragma unroll
+#pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
                         Piece pc;
-                        uint32_t lo[8];
+                        uint32_t hi[8], lo[8];
                         fetch(pc, c);
                         tmem_ld_32x16(t_s + c * 16, a);
                         tmem_ld_wait16(a);
@@ -520,17 +515,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         for (int j = 0; j < 8; ++j) {
                             float e0, e1;
                             unpack_f32x2(fma_f32x2(add_f32x2(x_pair(a, pc, j), pack_f32x2(sub, sub)), log2e2, pack_f32x2(add, add)), e0, e1);
-                            put(e0, e1, c, j, lo);
+                            prob(e0, e1, hi[j], lo[j]);
                         }
-                        put_tails(lo, c);
+                        tmem_st_32x8(t_s + c * 8, hi);
+                        if (SPLIT) tmem_st_32x8(t_s - S_COL + tail_col(c, D), lo);
                     }
+                    stored = true;
                     break;
                 }
             }
-            tmem_st_32x32(t_s, pk);
-            if (SPLIT && D == 32) {
-                tmem_st_32x8(t_s - S_COL + tail_col(2, D), late[0]);
-                tmem_st_32x8(t_s - S_COL + tail_col(3, D), late[1]);
+            if (!stored) {
+                tmem_st_32x32(t_s, pk);
+                if (SPLIT && D == 32) {
+                    tmem_st_32x8(t_s - S_COL + tail_col(2, D), late[0]);
+                    tmem_st_32x8(t_s - S_COL + tail_col(3, D), late[1]);
+                }
             }
             tmem_st_wait();
             tc_fence_before();

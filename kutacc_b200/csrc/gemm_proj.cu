@@ -71,7 +71,6 @@ struct ProjParams {
     const float *bg, *gamma, *beta;     // gamma: null without LayerNorm
     float eps;
     int S, B, D;
-    int gate_sigmoid;     // the stored gate is bf16(sigmoid(bf16(x.Wg + bg)))
     int s32;              // 32-row groups per batch row
     int rows128;          // S is a multiple of 128: a row tile is one box
     int whole;            // a unit of work is a block with all its column tiles, up to this unit;
@@ -86,8 +85,8 @@ __device__ __forceinline__ float sigmoid_of_bf16(float y)
     return fmaf(0.5f, tanh_approx(0.5f * round_to_bf16_f32(y)), 0.5f);
 }
 
-// R: row tiles per block, 1 or 2
-template <int KS, int R, bool LN>
+// R: row tiles per block, 1 or 2. GATE_SIGMOID: the stored gate is bf16(sigmoid(bf16(x.Wg + bg)))
+template <int KS, int R, bool LN, bool GATE_SIGMOID>
 __global__ void __launch_bounds__(THREADS, 1)
 proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjParams p)
 {
@@ -313,7 +312,7 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
                             const float4 bv = lds128_f32(bg_a + (uint32_t)((nn + 4 * j4) * 4));
                             float y[4] = {__uint_as_float(r[c][4 * j4]) + bv.x, __uint_as_float(r[c][4 * j4 + 1]) + bv.y,
                                           __uint_as_float(r[c][4 * j4 + 2]) + bv.z, __uint_as_float(r[c][4 * j4 + 3]) + bv.w};
-                            if (p.gate_sigmoid) {
+                            if (GATE_SIGMOID) {
 #pragma unroll
                                 for (int e = 0; e < 4; ++e) y[e] = sigmoid_of_bf16(y[e]);
                             }
@@ -375,16 +374,16 @@ proj_kernel(const __grid_constant__ ProjMaps maps, const __grid_constant__ ProjP
     }
 }
 
-template <int KS, int R, bool LN>
+template <int KS, int R, bool LN, bool GATE_SIGMOID>
 void launch_one(cudaStream_t stream, int grid, const ProjMaps &maps, const ProjParams &p)
 {
     static const cudaError_t attr =
-        cudaFuncSetAttribute(proj_kernel<KS, R, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES);
+        cudaFuncSetAttribute(proj_kernel<KS, R, LN, GATE_SIGMOID>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES);
     KUTACC_CUDA(attr);
-    launch_chained(proj_kernel<KS, R, LN>, (unsigned)grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
+    launch_chained(proj_kernel<KS, R, LN, GATE_SIGMOID>, (unsigned)grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
 }
 
-template <int KS>
+template <int KS, bool GATE_SIGMOID>
 bool launch_ks(cudaStream_t stream, const ProjMaps &maps, ProjParams p)
 {
     // How the work is cut: blocks of 256 rows, or of 128 where that fills the chip better; whole blocks for all full waves, and
@@ -413,9 +412,9 @@ bool launch_ks(cudaStream_t stream, const ProjMaps &maps, ProjParams p)
     const int grid = std::min(p.units, sms);
     KernelTimer timer__("proj_qkvg", stream);
     if (p.gamma)
-        R == 2 ? launch_one<KS, 2, true>(stream, grid, maps, p) : launch_one<KS, 1, true>(stream, grid, maps, p);
+        R == 2 ? launch_one<KS, 2, true, GATE_SIGMOID>(stream, grid, maps, p) : launch_one<KS, 1, true, GATE_SIGMOID>(stream, grid, maps, p);
     else
-        R == 2 ? launch_one<KS, 2, false>(stream, grid, maps, p) : launch_one<KS, 1, false>(stream, grid, maps, p);
+        R == 2 ? launch_one<KS, 2, false, GATE_SIGMOID>(stream, grid, maps, p) : launch_one<KS, 1, false, GATE_SIGMOID>(stream, grid, maps, p);
     count_launch();
     return true;
 }
@@ -454,10 +453,11 @@ bool tcgen05_proj_rows_bf16(cudaStream_t stream, const void *x, const void *wq, 
     p.S = S;
     p.B = B;
     p.D = D;
-    p.gate_sigmoid = gate_sigmoid ? 1 : 0;
     p.s32 = (int)s32;
     p.err = ew.device;
-    return C == 64 ? launch_ks<1>(stream, maps, p) : C == 128 ? launch_ks<2>(stream, maps, p) : launch_ks<4>(stream, maps, p);
+    if (gate_sigmoid)                    // wide layers with heads of 32
+        return C == 64 ? false : C == 128 ? launch_ks<2, true>(stream, maps, p) : launch_ks<4, true>(stream, maps, p);
+    return C == 64 ? launch_ks<1, false>(stream, maps, p) : C == 128 ? launch_ks<2, false>(stream, maps, p) : launch_ks<4, false>(stream, maps, p);
 }
 
 }  // namespace dev

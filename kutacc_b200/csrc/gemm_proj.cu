@@ -79,12 +79,6 @@ struct ProjParams {
     int *err;
 };
 
-// 1 / (1 + exp(-g)) of the bf16-rounded g as 0.5 * tanh(g / 2) + 0.5 (one MUFU operation, relative error about 2^-11)
-__device__ __forceinline__ float sigmoid_of_bf16(float y)
-{
-    return fmaf(0.5f, tanh_approx(0.5f * round_to_bf16_f32(y)), 0.5f);
-}
-
 // R: row tiles per block, 1 or 2. GATE_SIGMOID: the stored gate is bf16(sigmoid(bf16(x.Wg + bg)))
 template <int KS, int R, bool LN, bool GATE_SIGMOID>
 __global__ void __launch_bounds__(THREADS, 1)

@@ -111,14 +111,6 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t addr)
     return d;
 }
 
-// 1 / (1 + exp(-g)) of the bf16-rounded g as 0.5 * tanh(g / 2) + 0.5: one MUFU operation (relative error about
-// 2^-11, below the bf16 step of the stored result) instead of an exponential and a division
-__device__ __forceinline__ float sigmoid_of_bf16(float y)
-{
-    const float g = round_to_bf16_f32(y);
-    return fmaf(0.5f, tanh_approx(0.5f * g), 0.5f);
-}
-
 // Compile-time feature sets, so that each use of the kernel carries only the epilogue code it needs
 // (the sigmoid and the transposed staging cost registers that the plain linear layer would spill).
 // F_MNMAJOR: both operands are stored with their rows and columns exchanged, X [B][K][S] and W [B][K][N]: the tensor core

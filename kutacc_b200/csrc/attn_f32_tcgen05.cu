@@ -117,7 +117,7 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         }
         for (int w = 0; w < MAXG; ++w) {
             for (int b = 0; b < 2; ++b) {
-                mbar_init(s_full(w, b), 1);
+                mbar_init(s_full(w, b), 2);         // the products' commit, the issuer's own arrival
                 mbar_init(p_full(w, b), 4);
             }
             mbar_init(o_full(w), 1);
@@ -231,6 +231,7 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                     tc_mma_tf32_ts(d, t0 + Q_COL + (pr == 0 ? D : 0) + k * 8, kd + (pr == 1 ? k_tail : 0u) + 2 * k, idesc_s,
                                    (pr > 0 || k > 0) ? 1u : 0u);
             tc_commit(s_full(w, g & 1));
+            mbar_arrive(s_full(w, g & 1));          // passes on that the bias tiles have landed, as in attn_tcgen05.cu
         };
         int g = 0;
         bool ok = w < G;

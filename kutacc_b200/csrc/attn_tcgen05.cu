@@ -163,7 +163,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             mbar_init(kv_empty(s), n_mma);  // each MMA warp's commit after its last P.V^T of the tile
         }
         for (int w = 0; w < MAXG; ++w) {
-            mbar_init(s_full(w), 1);
+            mbar_init(s_full(w), 2);        // the products' commit, the issuer's own arrival
             mbar_init(p_full(w), 4);
             mbar_init(o_full(w), 1);
         }
@@ -293,6 +293,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     tc_mma_bf16(tmem_base + w * WG_COLS + S_COL, make_smem_desc_kmajor(qb + k * 32, T::ROWB),
                                 make_smem_desc_kmajor(kb + k * 32, T::ROWB), idesc_s, k > 0 ? 1u : 0u);
                 tc_commit(s_full(w));
+                // The softmax warps read the tile's pair bias and mask bias, which this thread has seen arrive (kv_full): an
+                // arrival of its own passes that on, a commit answers only for the tensor core. (A second wait in the
+                // softmax warps would cost 1.5 %.)
+                mbar_arrive(s_full(w));
             }
             __syncwarp();
         };

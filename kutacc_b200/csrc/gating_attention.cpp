@@ -90,21 +90,6 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     if (ln) stage += 2 * staged_bytes_needed(ln->gamma, b_bytes);
     const bool downloads_in_flight = rt.out_hazard;          // of an earlier enqueue-only call with a HOST result
     if (!rt.reserve_stage(stage, pipelined)) return;
-    const int64_t s_pad8 = (S + 7) / 8 * 8;
-    const size_t nb_pad_bytes = has_nb ? (size_t)H * S * s_pad8 * es : 0;
-    // fp32 on the tensor-memory kernels (head size 32): k and v are stored split into tf32 head and tail
-    const bool f32_split = dt == kFP32 && C % 128 == 0 && D == 32 && out_rs % 4 == 0;
-    const size_t k_bytes = f32_split ? 2 * x_bytes : x_bytes;
-    // v may be stored key-major with padded rows
-    const size_t v_bytes = std::max(x_bytes, (size_t)B * C * s_pad8 * es) * (f32_split ? 2 : 1);
-    // with LayerNorm: row statistics, four folded weights with their s and t, and (for shapes the folded projection does
-    // not cover) a normalised copy of the activations
-    const size_t ln_bytes = ln ? (size_t)M * 8 + 4 * (w_bytes + 256) + 8 * (b_bytes + 256) + x_bytes + 1024 : 0;
-    // fp32 on the tensor-memory GEMM: operands split into tf32 head and tail (activations: one [M, 2C] buffer that the
-    // projection and, later, the output projection use in turn; five weights [C, 2C])
-    const bool f32_tc = dt == kFP32 && C % 128 == 0 && out_rs % 4 == 0;
-    const size_t f32_bytes = f32_tc ? 2 * x_bytes + 256 + 5 * (2 * w_bytes + 256) : 0;
-    if (!rt.reserve_workspace(3 * (x_bytes + 256) + k_bytes + 256 + v_bytes + 256 + nb_pad_bytes + 256 + ln_bytes + f32_bytes)) return;
 
     // The staged output is placed first: its address tells whether downloads of an earlier enqueue-only call, still
     // in flight, read the very block this call will fill. A call of the same shape (same block, same chunks) lets its
@@ -130,6 +115,39 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
               d_wv = resolve_in(value_w.data_ptr(), w_bytes), d_wg = resolve_in(gating_w.data_ptr(), w_bytes),
               d_wo = resolve_in(output_w.data_ptr(), w_bytes);
     DeviceArg d_bg = resolve_in(gating_b.data_ptr(), b_bytes), d_bo = resolve_in(output_b.data_ptr(), b_bytes);
+
+    const bool fast = dt == kBF16 && (C % 64 == 0) && ((D == 8 && (C % 128 == 0 || C == 64)) || D == 16 || D == 32 || D == 64) && B <= 65535 && H <= 65535 &&
+                      aligned16(d_x.dev) && aligned16(d_wq.dev) && aligned16(d_wk.dev) && aligned16(d_wv.dev) &&
+                      aligned16(d_wg.dev) && aligned16(d_wo.dev) && (out_rs % 2 == 0) &&
+                      (((uintptr_t)d_out.dev & 3u) == 0);
+    // LayerNorm in front (head sizes up to 32): up to 256 channels the projection normalises its rows itself, on their way to
+    // the tensor cores; wider rows do not fit beside the weights, and there LayerNorm is folded into the weights (heads of 32).
+    // Otherwise the rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy.
+    const bool ln_in_proj = ln && fast && D <= 32 && (C == 64 || C == 128 || C == 256);
+    const bool ln_folded = ln && fast && D == 32 && C % 128 == 0 && !ln_in_proj;
+    const bool ln_copied = ln && !ln_in_proj && !ln_folded;
+    // fp32 on the tensor-memory kernels (head size 32): k and v are stored split into tf32 head and tail
+    const bool f32_split = dt == kFP32 && C % 128 == 0 && D == 32 && out_rs % 4 == 0;
+    // fp32 on the tensor-memory GEMM: operands split into tf32 head and tail (activations: one [M, 2C] buffer that the
+    // projection and, later, the output projection use in turn; five weights [C, 2C])
+    const bool f32_tc = dt == kFP32 && C % 128 == 0 && out_rs % 4 == 0;
+    // The TMA loads of the pair bias need 16-byte aligned rows. A pair bias whose strides are not
+    // multiples of 16 bytes is first copied into the workspace with padded rows.
+    const int64_t nb_unit = dt == kFP32 ? 4 : 8;      // elements of 16 bytes
+    const bool nb_repitch = (fast || f32_split) && has_nb && ((nb_s0 % nb_unit) || (nb_s1 % nb_unit) || !aligned16(d_nb.dev));
+
+    // workspace: q, k, v, gate, gated average, and what the path just chosen needs besides
+    const int64_t s_pad8 = (S + 7) / 8 * 8;
+    const size_t k_bytes = f32_split ? 2 * x_bytes : x_bytes;
+    // v may be stored key-major with padded rows
+    const size_t v_bytes = std::max(x_bytes, (size_t)B * C * s_pad8 * es) * (f32_split ? 2 : 1);
+    const size_t nb_pad_bytes = nb_repitch ? (size_t)H * S * s_pad8 * es : 0;
+    const size_t fold_bytes = ln_folded ? (size_t)M * 8 + 256 + 4 * (w_bytes + 256) + 8 * (b_bytes + 256) : 0;
+    const size_t norm_bytes = ln_copied ? x_bytes + 256 : 0;
+    const size_t f32_bytes = f32_tc ? 2 * x_bytes + 256 + 5 * (2 * w_bytes + 256) : 0;
+    if (!rt.reserve_workspace(3 * (x_bytes + 256) + k_bytes + 256 + v_bytes + 256 + nb_pad_bytes + 256 + fold_bytes + norm_bytes + f32_bytes))
+        return;
+
     if (pipelined) {
         // The copy streams start once the previous work on the runtime stream AND the small uploads queued above are
         // done. (Letting the first chunk travel beside the small uploads was tried: the copy engine then served
@@ -145,29 +163,21 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
          *wavg = (char *)rt.take_workspace(x_bytes);
     void *nb_pad = nb_pad_bytes ? rt.take_workspace(nb_pad_bytes) : nullptr;
     DeviceArg d_lg = ln ? resolve_in(ln->gamma, b_bytes) : DeviceArg{}, d_lb = ln ? resolve_in(ln->beta, b_bytes) : DeviceArg{};
-    char *ln_stats = ln ? (char *)rt.take_workspace((size_t)M * 8) : nullptr;
+    char *ln_stats = ln_folded ? (char *)rt.take_workspace((size_t)M * 8) : nullptr;
     void *ln_w[4] = {nullptr, nullptr, nullptr, nullptr};
     float *ln_s[4] = {nullptr, nullptr, nullptr, nullptr}, *ln_t[4] = {nullptr, nullptr, nullptr, nullptr};
-    char *x_norm = nullptr;
-    if (ln) {
-        for (int i = 0; i < 4; ++i) {
-            ln_w[i] = rt.take_workspace(w_bytes);
-            ln_s[i] = (float *)rt.take_workspace(b_bytes);
-            ln_t[i] = (float *)rt.take_workspace(b_bytes);
-        }
-        x_norm = (char *)rt.take_workspace(x_bytes);
+    for (int i = 0; i < 4 && ln_folded; ++i) {
+        ln_w[i] = rt.take_workspace(w_bytes);
+        ln_s[i] = (float *)rt.take_workspace(b_bytes);
+        ln_t[i] = (float *)rt.take_workspace(b_bytes);
     }
+    char *x_norm = ln_copied ? (char *)rt.take_workspace(x_bytes) : nullptr;
     char *a_split = f32_tc ? (char *)rt.take_workspace(2 * x_bytes) : nullptr;
     void *w_split[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     for (int i = 0; i < 5 && f32_tc; ++i) w_split[i] = rt.take_workspace(2 * w_bytes);
     if (kutacc_check_err_set) return;
 
     const float scale = (float)(1 / std::sqrt((double)head_size));  // gating_attention.cpp:68
-
-    const bool fast = dt == kBF16 && (C % 64 == 0) && ((D == 8 && (C % 128 == 0 || C == 64)) || D == 16 || D == 32 || D == 64) && B <= 65535 && H <= 65535 &&
-                      aligned16(d_x.dev) && aligned16(d_wq.dev) && aligned16(d_wk.dev) && aligned16(d_wv.dev) &&
-                      aligned16(d_wg.dev) && aligned16(d_wo.dev) && (out_rs % 2 == 0) &&
-                      (((uintptr_t)d_out.dev & 3u) == 0);
 
     // The pair bias may still be on its way (kutacc_b200_set_pair_bias_event): everything that reads it waits for the
     // event, once. The projections do not read it, so they are queued first where the pair bias is used as it lies.
@@ -179,12 +189,9 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     };
     if (!has_nb || staged_bytes_needed(nonbatched_bias.data_ptr(), nb_bytes) != 0) nb_event = nullptr;   // nothing to wait for / host data
 
-    // The TMA loads of the pair bias need 16-byte aligned rows. A pair bias whose strides are not
-    // multiples of 16 bytes is first copied into the workspace with padded rows.
     const void *nb_dev = has_nb ? d_nb.dev : nullptr;
     int64_t nb_sh = nb_s0, nb_sq = nb_s1;
-    const int64_t nb_unit = dt == kFP32 ? 4 : 8;      // elements of 16 bytes
-    if ((fast || f32_split) && has_nb && ((nb_s0 % nb_unit) || (nb_s1 % nb_unit) || !aligned16(d_nb.dev))) {
+    if (nb_repitch) {
         wait_for_pair_bias();                         // the re-pitching copy reads it
         const bool copied = dev::launch_repitch(stream, d_nb.dev, nb_s0, nb_s1, nb_pad, s_pad8, H, S, (int)es);
         KUTACC_CHECK(copied, "gating_attention: pair bias could not be re-pitched");
@@ -199,11 +206,6 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     // and the core applies an fp32 sigmoid.
     const bool gate_sigmoid = D == 32 && C % 128 == 0;
 
-    // LayerNorm in front (head sizes up to 32): up to 256 channels the projection normalises its rows itself, on their way to
-    // the tensor cores; wider rows do not fit beside the weights, and there LayerNorm is folded into the weights (heads of 32).
-    // Otherwise the rows are normalised into the workspace chunk by chunk and the usual sequence runs on the copy.
-    const bool ln_in_proj = ln && fast && D <= 32 && (C == 64 || C == 128 || C == 256);
-    const bool ln_folded = ln && fast && D == 32 && C % 128 == 0 && !ln_in_proj;
     if (ln_folded) {
         const void *w_in[4] = {d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev};
         const float *b_in[4] = {nullptr, nullptr, nullptr, (const float *)d_bg.dev};
@@ -223,8 +225,8 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     auto run_rows = [&](int64_t b0, int64_t nbr) -> bool {
         const size_t row_bytes = (size_t)S * C * es;                       // one batch row of a [B, S, C]-sized buffer
         const char *x_c = (const char *)d_x.dev + b0 * row_bytes;
-        char *st_c = ln ? ln_stats + (size_t)b0 * S * 8 : nullptr;
-        if (ln && !ln_folded && !ln_in_proj) {
+        char *st_c = ln_folded ? ln_stats + (size_t)b0 * S * 8 : nullptr;
+        if (ln_copied) {
             if (!dev::launch_layernorm_rows(stream, x_c, (const float *)d_lg.dev, (const float *)d_lb.dev, x_norm + b0 * row_bytes,
                                             nbr * S, C, C, C, ln->eps))
                 return false;

@@ -188,14 +188,13 @@ extern "C" void kutacc_b200_pair_bias_ln(kutacc_tensor_h z_h, const float *ln_ga
     if (!rt.reserve_stage(staged_bytes_needed(z.data_ptr(), z_bytes) + staged_bytes_needed(wb.data_ptr(), w_bytes) +
                           staged_bytes_needed(nb.data_ptr(), nb_bytes) + 2 * staged_bytes_needed(ln_gamma, g_bytes)))
         return;
-    const bool fused = H <= 8 && (Cz == 128 || Cz == 64);
-    if (!rt.reserve_workspace(z_bytes + 256)) return;              // the normalised copy of the fallback
     DeviceArg d_z = resolve_in(z.data_ptr(), z_bytes), d_w = resolve_in(wb.data_ptr(), w_bytes),
               d_g = resolve_in(ln_gamma, g_bytes), d_b = resolve_in(ln_beta, g_bytes), d_n = resolve_out(nb.data_ptr(), nb_bytes);
     if (kutacc_check_err_set) return;
-    bool ok = fused && dev::launch_pair_bias_ln(stream, d_z.dev, d_w.dev, (const float *)d_g.dev, (const float *)d_b.dev, eps, d_n.dev, hs,
-                                                R, Nk, (int)Cz, (int)H);
+    bool ok = dev::launch_pair_bias_ln(stream, d_z.dev, d_w.dev, (const float *)d_g.dev, (const float *)d_b.dev, eps, d_n.dev, hs, R, Nk,
+                                       (int)Cz, (int)H);
     if (!ok && !kutacc_check_err_set) {
+        if (!rt.reserve_workspace(z_bytes + 256)) return;
         void *zn = rt.take_workspace(z_bytes);
         ok = zn != nullptr &&
              dev::launch_layernorm_rows(stream, d_z.dev, (const float *)d_g.dev, (const float *)d_b.dev, zn, P, Cz, Cz, Cz, eps) &&

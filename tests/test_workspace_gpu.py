@@ -25,3 +25,11 @@ def test_attention_with_layernorm_in_the_projection(kutacc_lib):
     held = held_after(lambda: api.gating_attention_ln(case.t_x, case.inputs, case.t_bias, case.t_nb, case.weights, g.data_ptr(),
                                                       b.data_ptr(), 1e-5, case.t_out))
     assert held <= 5 * x_bytes * 9 / 8 + (3 << 20)          # q, k, v, gate, average; the pool adds an eighth and rounds up to 2 MB
+
+
+def test_pair_bias_with_layernorm(kutacc_lib):
+    z, wb = torch.randn(64, 64, 128, device="cuda").bfloat16(), torch.randn(4, 128, device="cuda").bfloat16()
+    nb = torch.zeros(4, 64, 64, dtype=torch.bfloat16, device="cuda")
+    g, b = torch.ones(128, device="cuda"), torch.zeros(128, device="cuda")
+    tz, tw, tn = api.tensor(z), api.tensor(wb), api.tensor(nb)
+    assert held_after(lambda: api.pair_bias_ln(tz, g.data_ptr(), b.data_ptr(), 1e-5, tw, tn)) == 0

@@ -123,21 +123,25 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
     if (!rt.reserve_stage(staged_bytes_needed(left.data_ptr(), l_bytes) + staged_bytes_needed(right.data_ptr(), r_bytes) +
                           staged_bytes_needed(center.data_ptr(), c_bytes)))
         return;
-    // The tensor-core product reads rows that start on 16-byte boundaries; operands with other strides (an odd number of
-    // residues) are first moved to padded rows in the workspace, one pass over HBM each.
-    const int64_t pitch = (n + 7) / 8 * 8;
-    const size_t pad_bytes = (size_t)c_i * n * pitch * 2;
-    if (!rt.reserve_workspace(2 * (pad_bytes + 256))) return;
     DeviceArg d_l = resolve_in(left.data_ptr(), l_bytes), d_r = resolve_in(right.data_ptr(), r_bytes);
     DeviceArg d_c = resolve_out_keeping_gaps(center.data_ptr(), c_bytes, dense3(center, n, n));
-    void *pad_l = rt.take_workspace(pad_bytes), *pad_r = rt.take_workspace(pad_bytes);
     if (kutacc_check_err_set) return;
+    // The tensor-core product reads rows that start on 16-byte boundaries; operands with other strides (an
+    // odd number of residues) are first moved to padded rows in the workspace, one pass over HBM.
+    const int64_t pitch = (n + 7) / 8 * 8;
+    const size_t pad_bytes = (size_t)c_i * n * pitch * 2;
     struct Operand {
         const void *p;
         int64_t s0, s1;
     };
-    auto aligned_rows = [](const void *p, int64_t s0, int64_t s1) { return ((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0; };
-    const bool l_ok = aligned_rows(d_l.dev, l_s0, l_s1), r_ok = aligned_rows(d_r.dev, r_s0, r_s1);
+    auto as_is = [&](const void *p, int64_t s0, int64_t s1) {
+        return ((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0;
+    };
+    const bool l_ok = as_is(d_l.dev, l_s0, l_s1), r_ok = as_is(d_r.dev, r_s0, r_s1);
+    const int pads = (l_ok ? 0 : 1) + (r_ok ? 0 : 1);
+    if (pads && !rt.reserve_workspace(pads * (pad_bytes + 256))) return;
+    void *pad_l = l_ok ? nullptr : rt.take_workspace(pad_bytes), *pad_r = r_ok ? nullptr : rt.take_workspace(pad_bytes);
+    if (kutacc_check_err_set) return;
     const Operand ol = l_ok ? Operand{d_l.dev, l_s0, l_s1} : Operand{pad_l, n * pitch, pitch};
     const Operand orr = r_ok ? Operand{d_r.dev, r_s0, r_s1} : Operand{pad_r, n * pitch, pitch};
     bool ok = true;

@@ -33,3 +33,11 @@ def test_pair_bias_with_layernorm(kutacc_lib):
     g, b = torch.ones(128, device="cuda"), torch.zeros(128, device="cuda")
     tz, tw, tn = api.tensor(z), api.tensor(wb), api.tensor(nb)
     assert held_after(lambda: api.pair_bias_ln(tz, g.data_ptr(), b.data_ptr(), 1e-5, tw, tn)) == 0
+
+
+@pytest.mark.parametrize("incoming", [False, True])
+def test_triangle_product_of_aligned_operands(kutacc_lib, incoming):
+    left, right = (torch.randn(8, 64, 64, device="cuda").bfloat16() for _ in range(2))
+    center = torch.zeros(8, 64, 64, dtype=torch.bfloat16, device="cuda")
+    tc, tl, tr = api.tensor(center), api.tensor(left), api.tensor(right)
+    assert held_after(lambda: api.tm_equation(tc, tl, tr, 64, incoming)) == 0

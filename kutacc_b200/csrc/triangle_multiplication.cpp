@@ -126,8 +126,8 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
     DeviceArg d_l = resolve_in(left.data_ptr(), l_bytes), d_r = resolve_in(right.data_ptr(), r_bytes);
     DeviceArg d_c = resolve_out_keeping_gaps(center.data_ptr(), c_bytes, dense3(center, n, n));
     if (kutacc_check_err_set) return;
-    // The tensor-core product reads rows that start on 16-byte boundaries; operands with other strides (an
-    // odd number of residues) are first moved to padded rows in the workspace, one pass over HBM.
+    // The tensor-core product reads rows that start on 16-byte boundaries and do not overlap; operands with other strides (an
+    // odd number of residues, a broadcast channel) are first moved to padded rows in the workspace, one pass over HBM.
     const int64_t pitch = (n + 7) / 8 * 8;
     const size_t pad_bytes = (size_t)c_i * n * pitch * 2;
     struct Operand {
@@ -135,15 +135,17 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
         int64_t s0, s1;
     };
     auto as_is = [&](const void *p, int64_t s0, int64_t s1) {
-        return ((s0 | s1) % 8) == 0 && ((uintptr_t)p & 15u) == 0;
+        return ((s0 | s1) % 8) == 0 && s1 >= n && (c_i == 1 || s0 > 0) && ((uintptr_t)p & 15u) == 0;
     };
     const bool l_ok = as_is(d_l.dev, l_s0, l_s1), r_ok = as_is(d_r.dev, r_s0, r_s1);
     const int pads = (l_ok ? 0 : 1) + (r_ok ? 0 : 1);
     if (pads && !rt.reserve_workspace(pads * (pad_bytes + 256))) return;
     void *pad_l = l_ok ? nullptr : rt.take_workspace(pad_bytes), *pad_r = r_ok ? nullptr : rt.take_workspace(pad_bytes);
     if (kutacc_check_err_set) return;
-    const Operand ol = l_ok ? Operand{d_l.dev, l_s0, l_s1} : Operand{pad_l, n * pitch, pitch};
-    const Operand orr = r_ok ? Operand{d_r.dev, r_s0, r_s1} : Operand{pad_r, n * pitch, pitch};
+    // (the stride between the channels of a single one says nothing)
+    const Operand ol = l_ok ? Operand{d_l.dev, c_i == 1 ? n * l_s1 : l_s0, l_s1} : Operand{pad_l, n * pitch, pitch};
+    const Operand orr = r_ok ? Operand{d_r.dev, c_i == 1 ? n * r_s1 : r_s0, r_s1} : Operand{pad_r, n * pitch, pitch};
+    const int64_t c_b = c_i == 1 ? n * c_s1 : c_s0;
     bool ok = true;
     if (!l_ok && !r_ok) {
         const void *src[2] = {d_l.dev, d_r.dev};
@@ -156,9 +158,9 @@ extern "C" void kutacc_af2_triangle_multiplication_equation(kutacc_tensor_h cent
     }
     // outgoing: center[a, b] = sum_k left[a, k] * right[b, k]; incoming: center[a, b] = sum_k right[k, a] * left[k, b]
     ok = ok && (is_incoming ? dev::tcgen05_batched_bf16(stream, true, orr.p, orr.s1, orr.s0, ol.p, ol.s1, ol.s0, d_c.dev, c_s1,
-                                                        c_s0, (int)c_i, (int)n, (int)n, (int)n)
+                                                        c_b, (int)c_i, (int)n, (int)n, (int)n)
                             : dev::tcgen05_batched_bf16(stream, false, ol.p, ol.s1, ol.s0, orr.p, orr.s1, orr.s0, d_c.dev, c_s1,
-                                                        c_s0, (int)c_i, (int)n, (int)n, (int)n));
+                                                        c_b, (int)c_i, (int)n, (int)n, (int)n));
     if (kutacc_check_err_set) return;
     if (!ok)
         ok = dev::launch_tm_equation_generic(stream, d_l.dev, l_s0, l_s1, d_r.dev, r_s0, r_s1, d_c.dev, c_s0, c_s1, c_i, n,

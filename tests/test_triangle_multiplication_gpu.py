@@ -94,6 +94,21 @@ def test_equation_matches_oracle(kutacc_lib, n, c_i, incoming):
     assert helpers.rel_err(got, O.tm_equation_exact(L, R, incoming)) <= helpers.BF16_TOL
 
 
+@pytest.mark.parametrize("incoming", [False, True])
+@pytest.mark.parametrize("strides", [(0, 40, 1), (64, 8, 1), (0, 0, 1), (640, 16, 1)])
+def test_equation_of_broadcast_and_overlapping_operands(kutacc_lib, strides, incoming):
+    c_i, n = 3, 40
+    rng = np.random.default_rng(650)
+    store = _bf(rng.standard_normal(3 * 1600, dtype=np.float32))
+    right = _bf(rng.standard_normal((c_i, n, n), dtype=np.float32))
+    left = torch.as_strided(store, (c_i, n, n), strides)
+    center = torch.full((c_i, n, n), float("nan"), dtype=torch.bfloat16, device=DEV)
+    api.tm_equation(api.tensor(center), api.tensor(store, sizes=[c_i, n, n], strides=list(strides)), api.tensor(right), n, incoming)
+    torch.cuda.synchronize()
+    want = O.tm_equation_exact(_f32(left.contiguous()), _f32(right), incoming)
+    assert helpers.rel_err(_f32(center), want) <= helpers.BF16_TOL
+
+
 @pytest.mark.parametrize("n,c_o,c_i", [(64, 128, 128), (50, 128, 128), (37, 48, 24)])
 def test_gate_and_out_linear_then_last_match_oracle(kutacc_lib, n, c_o, c_i):
     A = _case(700 + n, n, c_o, c_i)

@@ -2,6 +2,7 @@
 batch rows per work item, head sizes 8, 16 and 32, layers of 64 channels."""
 import numpy as np
 import pytest
+import torch
 
 from kutacc_b200 import api, runner
 from kutacc_b200 import workloads as W
@@ -102,3 +103,22 @@ def test_nearly_closed_gates(kutacc_lib, H, D, low):
     sig = 1 / (1 + np.exp(-w.arrays["bg"].astype(np.float64)))
     got = runner.out_to_f32(runner.DeviceCase(w).run())
     assert helpers.rel_err(got / sig, helpers.oracle_exact(w) / sig) <= helpers.BF16_TOL
+
+
+@pytest.mark.parametrize("H,D,dtype", [(4, 32, "bf16"), (4, 16, "bf16"), (8, 8, "bf16"), (2, 64, "bf16"), (4, 32, "fp32")])
+@pytest.mark.parametrize("strides", [(0, 72, 1), (72, 0, 1), (0, 0, 1)])
+def test_broadcast_pair_bias(kutacc_lib, H, D, dtype, strides):
+    # one head, one query row, or one row for all
+    w = W.random_gating_case(seed=90, B=3, S=72, H=H, D=D, dtype=dtype)
+    case = runner.DeviceCase(w)
+    store = case.nb[:, 0].contiguous() if strides[0] else case.nb[0].contiguous()      # [H, S] or [S, S]
+    view = torch.as_strided(store, (H, 72, 72), strides)
+    nb = api.tensor(store, sizes=[H, 72, 72], strides=list(strides))
+    api.gating_attention(case.t_x, case.inputs, case.t_bias, nb, case.weights, case.t_out, 128)
+    torch.cuda.synchronize()
+    w.arrays["nb"] = view.float().cpu().contiguous().numpy()
+    got = runner.out_to_f32(case.out)
+    if dtype == "fp32":
+        assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
+    else:
+        assert helpers.rel_err(got, helpers.oracle_faithful(w)) <= helpers.BF16_TOL

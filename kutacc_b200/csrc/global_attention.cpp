@@ -55,8 +55,13 @@ extern "C" void kutacc_af2_global_attention(kutacc_af2_attention_inputs_t *q_bas
                    staged_bytes_needed(wg.data_ptr(), wcc) + staged_bytes_needed(wo.data_ptr(), wcc) +
                    staged_bytes_needed(bg.data_ptr(), bb) + staged_bytes_needed(bo.data_ptr(), bb);
     if (!rt.reserve_stage(stage)) return;
-    const size_t scratch_bytes = std::max(dev::global_attention_scratch_bytes((int)B, (int)S, (int)H, (int)D),
-                                          dev::global_stream_scratch_bytes(B, S));
+    // three streaming kernels for 8 heads x 8 (k, v and partial sums in `scratch`, a quarter of the activations' size), over
+    // groups of columns that keep it within 256 MB (a column's result does not depend on its group); otherwise three kernels
+    // per L2-sized group of columns with the split-softmax state in `scratch`
+    const bool streamed = dev::global_stream_covers((int)H, (int)D, out_rs);
+    const int64_t group = streamed ? std::max<int64_t>(1, std::min<int64_t>(B, (int64_t)(((size_t)256 << 20) / dev::global_stream_scratch_bytes(1, S)))) : B;
+    const size_t scratch_bytes = streamed ? dev::global_stream_scratch_bytes(group, S)
+                                          : dev::global_attention_scratch_bytes((int)B, (int)S, (int)H, (int)D);
     if (!rt.reserve_workspace(scratch_bytes + 256)) return;
     // Host-resident activations and result: the batch columns are independent, so they go through in
     // chunks with upload, kernels and download overlapped on three streams (as in the gated attention).
@@ -84,20 +89,21 @@ extern "C" void kutacc_af2_global_attention(kutacc_af2_attention_inputs_t *q_bas
                    (uintptr_t)d_wq.dev | (uintptr_t)d_wk.dev | (uintptr_t)d_wv.dev) & 15u) == 0,
                  "global_attention: q_data, out and the five weights must be 16-byte aligned");
     if (kutacc_check_err_set) return;
-    // three streaming kernels for 8 heads x 8 (k, v and partial sums in `scratch`), otherwise three kernels per L2-sized group
-    // of columns with the split-softmax state in `scratch`
     auto run_cols = [&](int64_t b0, int64_t nb) -> bool {
-        const char *xc = (const char *)d_x.dev + (size_t)b0 * S * C * 2;
-        const char *mc = (const char *)d_m.dev + (size_t)b0 * S * 2;
-        char *oc = (char *)d_out.dev + (size_t)b0 * S * out_rs * 2;
-        bool done = dev::launch_global_stream_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
-                                                   (const float *)d_bg.dev, d_wo.dev, (const float *)d_bo.dev, oc, out_rs,
-                                                   scratch, (int)nb, (int)S, (int)H, (int)D);
-        if (kutacc_check_err_set) return false;
-        if (!done)
-            done = dev::launch_global_attention_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
-                                                     (const float *)d_bg.dev, d_wo.dev, (const float *)d_bo.dev, oc,
-                                                     out_rs, scratch, (int)nb, (int)S, (int)H, (int)D);
+        bool done = true;
+        for (int64_t c0 = b0; c0 < b0 + nb && done; c0 += group) {
+            const int64_t n = std::min(group, b0 + nb - c0);
+            const char *xc = (const char *)d_x.dev + (size_t)c0 * S * C * 2;
+            const char *mc = (const char *)d_m.dev + (size_t)c0 * S * 2;
+            char *oc = (char *)d_out.dev + (size_t)c0 * S * out_rs * 2;
+            done = streamed ? dev::launch_global_stream_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
+                                                             (const float *)d_bg.dev, d_wo.dev, (const float *)d_bo.dev, oc,
+                                                             out_rs, scratch, (int)n, (int)S)
+                            : dev::launch_global_attention_bf16(stream, xc, mc, d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev,
+                                                                (const float *)d_bg.dev, d_wo.dev, (const float *)d_bo.dev, oc,
+                                                                out_rs, scratch, (int)n, (int)S, (int)H, (int)D);
+            if (kutacc_check_err_set) return false;
+        }
         return done;
     };
     bool ok = true;

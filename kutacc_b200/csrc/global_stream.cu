@@ -667,13 +667,18 @@ StreamPlan make_plan(int64_t B, int64_t S)
 
 }  // namespace
 
+bool global_stream_covers(int heads, int head_size, int64_t out_row_stride)
+{
+    return heads == H && head_size == D && (out_row_stride % 8) == 0 && out_row_stride >= C;
+}
+
 size_t global_stream_scratch_bytes(int64_t B, int64_t S) { return make_plan(B, S).bytes; }
 
 bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *mask, const void *wq, const void *wk,
                                const void *wv, const void *wg, const float *bg, const void *wo, const float *bo,
-                               void *out, int64_t out_row_stride, void *scratch, int B, int S, int heads, int head_size)
+                               void *out, int64_t out_row_stride, void *scratch, int B, int S)
 {
-    if (heads != H || head_size != D || B < 1 || S < 1 || (out_row_stride % 8) != 0 || out_row_stride < C) return false;
+    if (B < 1 || S < 1 || !global_stream_covers(H, D, out_row_stride)) return false;
     if ((((uintptr_t)x | (uintptr_t)out | (uintptr_t)wq | (uintptr_t)wg | (uintptr_t)wo | (uintptr_t)scratch) & 15u) != 0) return false;
     if ((((uintptr_t)wk | (uintptr_t)wv) & 3u) != 0) return false;
     KernelErrorWord &ew = kernel_error_word();

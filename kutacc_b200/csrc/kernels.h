@@ -171,12 +171,13 @@ bool launch_ln_fold(cudaStream_t stream, int nmat, const void *const *w, const f
 bool launch_layernorm_rows(cudaStream_t stream, const void *x, const float *gamma, const float *beta, void *out,
                            int64_t rows, int64_t size, int64_t x_stride, int64_t out_stride, float eps);
 
-// Global attention as three streaming kernels with k, v and partial sums in `scratch`; 8 heads x 8 only. Returns false when
-// the shape is not covered.
+// Global attention as three streaming kernels with k, v and partial sums in `scratch`: 8 heads x 8, out row stride a multiple of
+// 8 (global_stream_covers), 16-byte aligned operands.
+bool global_stream_covers(int heads, int head_size, int64_t out_row_stride);
 size_t global_stream_scratch_bytes(int64_t B, int64_t S);
 bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *mask, const void *wq, const void *wk,
                                const void *wv, const void *wg, const float *bg, const void *wo, const float *bo,
-                               void *out, int64_t out_row_stride, void *scratch, int B, int S, int heads, int head_size);
+                               void *out, int64_t out_row_stride, void *scratch, int B, int S);
 size_t global_attention_scratch_bytes(int B, int S, int H, int D);
 bool launch_global_attention_bf16(cudaStream_t stream, const void *x, const void *mask, const void *wq,
                                   const void *wk, const void *wv, const void *wg, const float *bg, const void *wo,

@@ -41,3 +41,32 @@ def test_triangle_product_of_aligned_operands(kutacc_lib, incoming):
     center = torch.zeros(8, 64, 64, dtype=torch.bfloat16, device="cuda")
     tc, tl, tr = api.tensor(center), api.tensor(left), api.tensor(right)
     assert held_after(lambda: api.tm_equation(tc, tl, tr, 64, incoming)) == 0
+
+
+def test_global_attention_of_other_head_shapes(kutacc_lib):
+    w = W.random_global_case(seed=6, B=64, S=4096, H=4, D=16)
+    case = runner.DeviceCase(w)
+    assert held_after(case.run) <= 4 << 20                  # split-softmax state, no k and v (9 MB)
+
+
+def test_global_attention_in_groups_of_columns(kutacc_lib):
+    # 382 MB of k, v and partial sums in groups of 26 columns; a column's result is that of a call of its own
+    B, S, C = 40, 262144, 64
+    g = torch.Generator("cuda").manual_seed(7)
+    x = torch.randn(B, S, C, generator=g, device="cuda").bfloat16()
+    mask = (torch.rand(B, S, generator=g, device="cuda") > 0.2).bfloat16()
+    ws = [torch.randn(n, C, generator=g, device="cuda").bfloat16() / 8 for n in (C, 8, 8, C, C)]
+    bg, bo = torch.ones(C, device="cuda"), torch.zeros(C, device="cuda")
+    weights = api.make_weights(C, 8, 8, *ws[:4], bg, ws[4], bo)
+
+    def run(cols):
+        xs, ms, out = x[cols].contiguous(), mask[cols].contiguous(), torch.empty(len(cols), S, C, dtype=torch.bfloat16, device="cuda")
+        api.global_attention(api.make_inputs(len(cols), S), api.tensor(xs), api.tensor(ms, sizes=[len(cols), S, 1], strides=[S, 1, 1]),
+                             weights, api.tensor(out))
+        torch.cuda.synchronize()
+        return out
+
+    whole = []
+    assert held_after(lambda: whole.append(run(list(range(B))))) <= 256 * 9 / 8 * (1 << 20) + (3 << 20)
+    for c in (0, 25, 26, 39):
+        assert torch.equal(whole[0][c], run([c])[0])

@@ -116,7 +116,10 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
               d_wo = resolve_in(output_w.data_ptr(), w_bytes);
     DeviceArg d_bg = resolve_in(gating_b.data_ptr(), b_bytes), d_bo = resolve_in(output_b.data_ptr(), b_bytes);
 
-    const bool fast = dt == kBF16 && (C % 64 == 0) && ((D == 8 && (C % 128 == 0 || C == 64)) || D == 16 || D == 32 || D == 64) && B <= 65535 && H <= 65535 &&
+    // heads of 8 have no core but the one on tensor memory, whose projection takes up to 256 channels, or up to 16384 with an
+    // aligned gate bias
+    const bool d8 = D == 8 && (C == 64 || C == 128 || C == 256 || (C % 128 == 0 && C <= 16384 && aligned16(d_bg.dev)));
+    const bool fast = dt == kBF16 && (C % 64 == 0) && (d8 || D == 16 || D == 32 || D == 64) && B <= 65535 && H <= 65535 &&
                       aligned16(d_x.dev) && aligned16(d_wq.dev) && aligned16(d_wk.dev) && aligned16(d_wv.dev) &&
                       aligned16(d_wg.dev) && aligned16(d_wo.dev) && (out_rs % 2 == 0) &&
                       (((uintptr_t)d_out.dev & 3u) == 0);

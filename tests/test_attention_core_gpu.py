@@ -122,3 +122,15 @@ def test_broadcast_pair_bias(kutacc_lib, H, D, dtype, strides):
         assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
     else:
         assert helpers.rel_err(got, helpers.oracle_faithful(w)) <= helpers.BF16_TOL
+
+
+@pytest.mark.parametrize("H,D", [(8, 8), (16, 8), (48, 8), (24, 16), (16, 32)])
+def test_unaligned_gate_bias(kutacc_lib, H, D):
+    w = W.random_gating_case(seed=91, B=2, S=40, H=H, D=D)
+    case = runner.DeviceCase(w)
+    store = torch.zeros(w.C + 4, device="cuda")
+    store[1:w.C + 1] = case.bg
+    weights = api.make_weights(w.C, H, D, case.wq, case.wk, case.wv, case.wg, store[1:w.C + 1], case.wo, case.bo)
+    api.gating_attention(case.t_x, case.inputs, case.t_bias, case.t_nb, weights, case.t_out, 128)
+    torch.cuda.synchronize()
+    assert helpers.rel_err(runner.out_to_f32(case.out), helpers.oracle_faithful(w)) <= helpers.BF16_TOL

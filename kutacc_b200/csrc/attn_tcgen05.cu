@@ -702,7 +702,7 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
     if (nb && ((nb_stride_h % 8) || (nb_stride_q % 8) || ((uintptr_t)nb % 16))) return false;
     if ((((uintptr_t)gate | (uintptr_t)avg) & 15u) != 0) return false;
     const int64_t n_qt = (S + BM - 1) / BM;
-    if (n_qt * H * B > INT32_MAX / 64) return false;
+    if (n_qt * H * B > INT32_MAX / 2) return false;          // work items are counted in 32 bits
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     AttnParams p;

@@ -134,3 +134,20 @@ def test_unaligned_gate_bias(kutacc_lib, H, D):
     api.gating_attention(case.t_x, case.inputs, case.t_bias, case.t_nb, weights, case.t_out, 128)
     torch.cuda.synchronize()
     assert helpers.rel_err(runner.out_to_f32(case.out), helpers.oracle_faithful(w)) <= helpers.BF16_TOL
+
+
+def test_more_than_2_25_work_items(kutacc_lib):
+    # one key per row: the result is v times the gate, and with identity weights half of x
+    B, H, D = 33000, 1024, 8
+    C = H * D
+    x = torch.randn(B, 1, C, device="cuda", dtype=torch.bfloat16)
+    eye, zero = torch.eye(C, device="cuda", dtype=torch.bfloat16), torch.zeros(C, C, device="cuda", dtype=torch.bfloat16)
+    vec, out = torch.zeros(C, device="cuda"), torch.empty_like(x)
+    weights = api.make_weights(C, H, D, zero, zero, eye, zero, vec, eye, vec)
+    api.gating_attention(api.tensor(x, sizes=[B, C], strides=[C, 1]), api.make_inputs(B, 1),
+                         api.tensor(torch.zeros(B, 1, device="cuda", dtype=torch.bfloat16)), api.empty_tensor(), weights, api.tensor(out), 128)
+    torch.cuda.synchronize()
+    assert torch.equal(out, x * 0.5)
+    del x, out, eye, zero
+    api.lib().kutacc_b200_release_workspace()
+    torch.cuda.empty_cache()

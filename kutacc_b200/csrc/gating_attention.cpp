@@ -135,10 +135,12 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     // projection and, later, the output projection use in turn; five weights [C, 2C])
     const bool f32_tc = dt == kFP32 && C % 128 == 0 && out_rs % 4 == 0;
     // The TMA loads of the pair bias need 16-byte aligned rows. A pair bias whose strides are not
-    // multiples of 16 bytes, or are zero (one head or one query row for all), is first copied into the workspace with padded rows.
+    // multiples of 16 bytes, or are zero (one head or one query row for all), is first copied into the workspace with padded rows;
+    // for the fp32 core also one with the heads inside its rows.
     const int64_t nb_unit = dt == kFP32 ? 4 : 8;      // elements of 16 bytes
     const bool nb_repitch = (fast || f32_split) && has_nb &&
-                            ((nb_s0 % nb_unit) || (nb_s1 % nb_unit) || nb_s0 <= 0 || nb_s1 <= 0 || !aligned16(d_nb.dev));
+                            ((nb_s0 % nb_unit) || (nb_s1 % nb_unit) || nb_s0 <= 0 || nb_s1 <= 0 || !aligned16(d_nb.dev) ||
+                             (f32_split && nb_s0 < nb_s1));
 
     // workspace: q, k, v, gate, gated average, and what the path just chosen needs besides
     const int64_t s_pad8 = (S + 7) / 8 * 8;

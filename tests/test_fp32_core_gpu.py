@@ -60,6 +60,21 @@ def test_rows_far_from_zero(kutacc_lib):
     assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
 
 
+def test_pair_bias_with_the_heads_inside_its_rows(kutacc_lib):
+    # [S, H, S] storage: copied once, not a second projection of k and v for another core
+    w = W.random_gating_case(seed=82, B=4, S=136, H=4, D=32, dtype="fp32")
+    case = runner.DeviceCase(w)
+    store = case.nb.permute(1, 0, 2).contiguous()
+    nb = api.tensor(store, sizes=[4, 136, 136], strides=[136, 4 * 136, 1])
+    api.set_profile(True)
+    api.profile_read()
+    api.gating_attention(case.t_x, case.inputs, case.t_bias, nb, case.weights, case.t_out, 128)
+    names = [n for n, _ in api.profile_read()]
+    api.set_profile(False)
+    assert names.count("gemm_tf32x3_tc") == 2 and "attn_f32_tc" in names
+    assert helpers.rel_err(runner.out_to_f32(case.out), helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
+
+
 # 128 x 128 tiles, 128 x 256 tiles (enough of them to go round), ragged rows, K of one and several slabs
 @pytest.mark.parametrize("M,N,K", [(1, 128, 32), (129, 384, 64), (20000, 256, 96), (9600, 512, 32)])
 def test_linear_fp32(kutacc_lib, M, N, K):

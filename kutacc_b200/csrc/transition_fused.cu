@@ -424,6 +424,21 @@ bool launch_co(cudaStream_t stream, const CUtensorMap &tx, const CUtensorMap &t1
     return true;
 }
 
+// Whether two products through the workspace are faster. While every SM has at most one row tile the one kernel takes as long as
+// a tile's chain of hidden chunks, whatever the number of rows; two kernels spread few rows over the chip in both directions.
+// Microseconds for h hidden channels (thousands) and m rows (thousands), fitted to 128 to 18944 rows x 256 to 2048 hidden:
+//   256 channels: chain 4.6 + 17.2 h, two kernels 9.7 + 5.2 h + 0.76 h m   (2048 x 1024: 23.0 against 17.0, 12288: 23.8 / 25.0,
+//                 2048 x 2048: 40.6 / 22.8, 12288: 42.1 / 41.2)
+//   128 channels: chain 4.4 +  9.4 h, two kernels 10.5 + 4.6 h + 0.6 h m   (2048 x 2048: 24.0 against 22.2, 4096: 24.1 / 23.9)
+// With more row tiles than SMs one kernel is the faster one (40000 x 1024: 59.9 / 70.2) or as fast within a few us (20000: 41.3 /
+// 36.3). One row tile of up to 1024 hidden channels stays in one launch without a workspace (22 against 15 us).
+bool two_kernels_faster(int64_t M, int c_o, int c_i)
+{
+    if ((M + BM - 1) / BM > sm_count() || (M <= BM && c_i <= 1024)) return false;
+    const double h = c_i * 1e-3, m = (double)M * 1e-3;
+    return c_o == 256 ? 4.6 + 17.2 * h > 9.7 + 5.2 * h + 0.76 * h * m : 4.4 + 9.4 * h > 10.5 + 4.6 * h + 0.6 * h * m;
+}
+
 }  // namespace
 
 bool tcgen05_transition_bf16(cudaStream_t stream, const void *x, const void *w1, const float *b1, const void *w2, const float *b2,
@@ -432,6 +447,8 @@ bool tcgen05_transition_bf16(cudaStream_t stream, const void *x, const void *w1,
     if ((c_o != 128 && c_o != 256) || c_i % BH != 0 || c_i > MAX_HIDDEN || M > INT32_MAX / 2 ||
         ((((uintptr_t)x | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)out) & 15u) != 0))
         return false;
+    // (the two products want aligned biases, this kernel does not)
+    if ((((uintptr_t)b1 | (uintptr_t)b2) & 15u) == 0 && two_kernels_faster(M, c_o, c_i)) return false;
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     CUtensorMap tx, t1, t2, to;

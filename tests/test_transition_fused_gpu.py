@@ -1,6 +1,7 @@
 """The one-kernel transition MLP at the edges of its row tiles (128 or 256 rows per CTA) and hidden chunks (128)."""
 import numpy as np
 import pytest
+import torch
 
 from kutacc_b200 import api
 from kutacc_b200.workloads import as_f32
@@ -22,4 +23,27 @@ def test_matches_oracle(kutacc_lib, rows, c_o, c_i):
     api.set_profile(False)
     assert names == ["transition"]
     assert np.isfinite(got).all()
+    assert helpers.rel_err(got, as_f32(O.transition_bf16(*arrays))) <= helpers.BF16_TOL
+
+
+# few rows and many hidden channels: two products through the workspace, unless their aligned loads do not fit the biases
+@pytest.mark.parametrize("rows,c_o,c_i,unaligned", [(129, 256, 1024, False), (2048, 256, 1024, False), (1, 128, 2048, False),
+                                                    (130, 256, 2048, False), (130, 256, 2048, True)])
+def test_few_rows(kutacc_lib, rows, c_o, c_i, unaligned):
+    arrays = _case(1, rows, c_o, c_i, 7 * rows + c_o)
+    api.set_profile(True)
+    api.profile_read()
+    if unaligned:
+        x, w1, b1, w2, b2 = [torch.from_numpy(a.view(np.int16)).view(torch.bfloat16).cuda() if a.dtype == np.uint16 else torch.from_numpy(a).cuda()
+                             for a in arrays]
+        b1, b2 = (torch.cat([torch.zeros(1, device="cuda"), b])[1:] for b in (b1, b2))
+        out = torch.zeros_like(x)
+        api.transition(1, rows, c_o, c_i, *(api.tensor(t) for t in (x.view(1, rows, c_o), w1, b1, w2, b2, out.view(1, rows, c_o))))
+        torch.cuda.synchronize()
+        got = out.float().cpu().numpy()
+    else:
+        got = _run(1, rows, c_o, c_i, arrays)
+    names = [n for n, _ in api.profile_read()]
+    api.set_profile(False)
+    assert names == (["transition"] if unaligned else ["linear_bias_relu", "linear_bias"])
     assert helpers.rel_err(got, as_f32(O.transition_bf16(*arrays))) <= helpers.BF16_TOL

@@ -54,10 +54,12 @@ struct MlpParams {
     int *err;
 };
 
+// relu of a NaN is 0, as in the epilogue of the two-product path (max.bf16x2 takes the operand that is a number; cvt.relu
+// would keep the NaN)
 __device__ __forceinline__ uint32_t pack_relu_bf16x2(float lo, float hi)
 {
     uint32_t r;
-    asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;\n" : "=r"(r) : "f"(hi), "f"(lo));
+    asm("max.bf16x2 %0, %1, %2;\n" : "=r"(r) : "r"(pack_bf16x2(lo, hi)), "r"(0u));
     return r;
 }
 __device__ __forceinline__ void group_bar(int g) { asm volatile("bar.sync %0, 128;\n" ::"r"(g + 1) : "memory"); }

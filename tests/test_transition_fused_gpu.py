@@ -47,3 +47,15 @@ def test_few_rows(kutacc_lib, rows, c_o, c_i, unaligned):
     api.set_profile(False)
     assert names == (["transition"] if unaligned else ["linear_bias_relu", "linear_bias"])
     assert helpers.rel_err(got, as_f32(O.transition_bf16(*arrays))) <= helpers.BF16_TOL
+
+
+# one kernel and two products
+@pytest.mark.parametrize("rows,c_o,c_i", [(200, 128, 512), (200, 256, 2048), (19100, 256, 256)])
+def test_relu_of_nan_is_zero(kutacc_lib, rows, c_o, c_i):
+    x, w1, b1, w2, b2 = _case(1, rows, c_o, c_i, 3)
+    clean = _run(1, rows, c_o, c_i, (x, w1, b1, w2, b2))
+    x = x.copy()
+    x[7, 3] = 0x7FC0
+    got = _run(1, rows, c_o, c_i, (x, w1, b1, w2, b2))
+    assert (got[7] == torch.from_numpy(b2).bfloat16().float().numpy()).all()
+    assert (np.delete(got, 7, 0) == np.delete(clean, 7, 0)).all()

@@ -382,7 +382,9 @@ bool launch_ks(cudaStream_t stream, const ProjMaps &maps, ProjParams p)
 {
     // How the work is cut: blocks of 256 rows, or of 128 where that fills the chip better; whole blocks for all full waves, and
     // the blocks of the last one in 1 / nsplit of their column tiles each, whichever ends first. A unit costs its column tiles
-    // plus about one for its rows.
+    // plus about one for its rows: a wave of units of 256 rows x 4, 2 and 1 tiles takes 7.0, 3.8 and 2.6 us at 128 channels, of 8, 4
+    // and 2 tiles 18.6, 9.7 and 5.7 us at 256. Units of 128 rows take 4.4, 2.9, 1.7 and 10.5, 6.2, 4.0 us: a block of 256 counts as
+    // 1.3 of them, less than the 1.5 to 1.75 measured, which prefers it in calls of a wave or less.
     constexpr int NT = 4 * KS * 64 / BN;
     const int sms = std::max(1, sm_count() - runtime().sm_margin);
     const int64_t groups = (int64_t)p.B * p.s32;

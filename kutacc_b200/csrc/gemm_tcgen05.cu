@@ -3,9 +3,9 @@
 //
 //   C[b, s, n] = sum_k X[b, s, k] * W[n, k] (+ bias[n])         X [B, S, K] bf16, W [N, K] bf16 (W[out][in])
 //
-// Persistent CTAs (two per SM) walk 128 x 128 output tiles; a row tile never crosses a batch row, so
-// every TMA box lies inside one [S, *] slab and rows past S are zero-filled on load and clipped on
-// store. Warp roles:
+// Persistent CTAs (two per SM) walk 128 x 128 output tiles (128 x 64 for 64 output channels). A row tile never crosses a
+// batch row: every TMA box lies inside one [S, *] slab and rows past S are zero-filled on load and clipped on store; callers
+// whose rows follow one another evenly pass them as one batch row, so that no tile ends early. Warp roles:
 //   warp 0      producer: TMA loads of 128 x 64 slabs of X and W (128-byte swizzle) into a 2-stage ring
 //   warp 1      MMA issuer: one elected lane issues tcgen05.mma (M = 128, N = 128, K = 16) four times per
 //               slab into one of two 128-column TMEM accumulators and commits to mbarriers
@@ -16,9 +16,10 @@
 // eight MMAs, so what hides the rest of the per-tile chain (TMA in, tcgen05.ld, staging, TMA store) is the
 // second CTA resident on the SM (99 KB of shared memory and half of the tensor memory each).
 //
-// For the fused Q/K/V/gate projection the four weights are four tensor maps and the destination maps
-// scatter straight into the attention kernel's [B, H, S, D] layout (q, k, v) and into [B, S, C] (gate,
-// with the gate bias added). The same kernel serves the output projection.
+// It serves the output projection and the other linear layers, the products of the triangle multiplication (one right-hand
+// matrix per batch), and the fused Q/K/V/gate projection of the layers that gemm_proj.cu does not take (more than 256
+// channels, heads of 64): there the four weights are four tensor maps and the destination maps scatter straight into the
+// attention kernel's layouts (q, k, v) and into [B, S, C] (gate, with the gate bias added).
 //
 // Replaces addmm -> kutacc_core_bgemm_ex of the reference
 // (src/attention/gating_attention.cpp:47-66,152-157; src/linear/mm.cpp:46-86).
@@ -67,7 +68,6 @@ struct GemmParams {
     const float *bias[4];   // per segment, may be null
     int seg_n;              // output channels per segment (multiple of 128)
     int nseg;
-    int pair64;             // segments of 64 channels: a column tile holds two of them
     int head_dim;           // > 0: segment output is [B*H][S][D] (coords d, s, b*H + h); 0: [B][S][N_seg]
     int head_layout_mask;   // bit i set: segment i uses the head layout
     int transposed_mask;    // bit i set: segment i is stored transposed, [B * N_seg][S] (coords s, b * N_seg + n)
@@ -117,9 +117,10 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t addr)
 // reads them as they lie (MN-major operands), so a product of transposed matrices needs no transposed copies.
 // F_DIRECT: out[b][n][s] element by element, s along the lanes of a warp (64 contiguous bytes per channel and store): for
 // destinations whose strides no TMA store takes.
-// F_HEADS64: head sizes of 8 or 16 and segments of 64 channels, two of them in a column tile.
-constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16, F_HEADS64 = 32, F_MNMAJOR = 64,
-              F_DIRECT = 128;
+// F_NARROW: head sizes of 8 or 16.
+// F_PAIR64: segments of 64 channels, two of them in a column tile (a layer of one head of 64).
+constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16, F_NARROW = 32, F_MNMAJOR = 64,
+              F_DIRECT = 128, F_PAIR64 = 256;
 
 // BN: width of a column tile, 128, or 64 for a product with 64 output channels
 template <int FEAT, int BN>
@@ -140,7 +141,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int s_tiles = (p.S + BM - 1) / BM;
     const int n_tiles_seg = (p.seg_n + BN - 1) / BN;    // a ragged last tile is zero-filled on load and clipped on store
-    const bool pair64 = (FEAT & F_HEADS64) && p.pair64;
+    constexpr bool pair64 = (FEAT & F_PAIR64) != 0;
     const int n_tiles = pair64 ? p.nseg / 2 : n_tiles_seg * p.nseg;
     const int num_tiles = p.B * s_tiles * n_tiles;
     const int nk = (p.K + BK - 1) / BK;                 // columns past K are zero-filled by TMA
@@ -386,7 +387,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
 #pragma unroll
                 for (int ch = 0; ch < 4; ++ch) {
                     // heads of 8 or 16 channels: [head][row][channel], no swizzle
-                    const uint32_t off = !(FEAT & F_HEADS64) || !head_layout || p.head_dim >= 32 ? (uint32_t)(lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4))
+                    const uint32_t off = !(FEAT & F_NARROW) || !head_layout ? (uint32_t)(lane * 64 + ((ch ^ ((lane >> 1) & 3)) << 4))
                                          : p.head_dim == 16 ? (uint32_t)((ch >> 1) * 1024 + lane * 32 + (ch & 1) * 16)
                                                             : (uint32_t)(ch * 512 + lane * 16);
                     const uint32_t addr = stg + off;
@@ -432,7 +433,7 @@ bool launch(cudaStream_t stream, const GemmMaps &maps, const GemmParams &p, cons
         configured = true;
     }
     const int s_tiles = (p.S + BM - 1) / BM;
-    const int n_tiles = p.pair64 ? p.nseg / 2 : ((p.seg_n + BN - 1) / BN) * p.nseg;
+    const int n_tiles = (FEAT & F_PAIR64) ? p.nseg / 2 : ((p.seg_n + BN - 1) / BN) * p.nseg;
     const int64_t tiles = (int64_t)p.B * s_tiles * n_tiles;
     const unsigned grid = (unsigned)std::min<int64_t>(tiles, 2 * std::max(1, sm_count() - runtime().sm_margin));
     GemmParams q = p;
@@ -491,21 +492,23 @@ bool tcgen05_proj_qkvg_bf16(cudaStream_t stream, const void *x, const void *wq, 
     p.head_layout_mask = 0x7;
     p.transposed_mask = v_transposed ? 0x4 : 0;
     p.w_batched = 0;
-    p.pair64 = C == 64 ? 1 : 0;
     p.K = C;
     p.S = S;
     p.B = B;
     p.relu = 0;
     p.sigmoid_mask = gate_sigmoid ? 0x8 : 0;
     p.err = ew.device;
-    const bool heads64 = C == 64 || D < 32;
-    // combinations that no caller uses: the attention core of wide layers with heads of 32 takes the sigmoid, the others the gate
-    if (gate_sigmoid != (v_transposed && !heads64) || (!v_transposed && (D < 32 || ln_stats))) return false;
-    if (ln_stats) return heads64 ? false : launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln");
-    if (v_transposed)
-        return heads64 ? launch<F_TRANSPOSED | F_HEADS64>(stream, maps, p, "proj_qkvg")
-                       : launch<F_TRANSPOSED | F_SIGMOID>(stream, maps, p, "proj_qkvg");
-    return heads64 ? launch<F_HEADS64>(stream, maps, p, "proj_qkvg") : launch<0>(stream, maps, p, "proj_qkvg");
+    // the combinations that callers use: k, v and the sigmoid of the gate for the attention core on tensor memory, with heads of 32
+    // (with LayerNorm or without), the plain gate with narrower heads; everything as it is for the other core, with heads of 32 or 64
+    if (gate_sigmoid != (v_transposed && D == 32) || (ln_stats && !gate_sigmoid)) return false;
+    if (v_transposed) {
+        if (C == 64 || D == 64) return false;                  // gemm_proj.cu; no such core
+        if (D < 32) return launch<F_TRANSPOSED | F_NARROW>(stream, maps, p, "proj_qkvg");
+        return ln_stats ? launch<F_TRANSPOSED | F_SIGMOID | F_LN>(stream, maps, p, "proj_qkvg_ln")
+                        : launch<F_TRANSPOSED | F_SIGMOID>(stream, maps, p, "proj_qkvg");
+    }
+    if (D < 32) return false;
+    return C == 64 ? launch<F_PAIR64>(stream, maps, p, "proj_qkvg") : launch<0>(stream, maps, p, "proj_qkvg");
 }
 
 bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w, const float *bias, void *out,
@@ -542,7 +545,6 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     p.head_layout_mask = 0;
     p.transposed_mask = 0;
     p.w_batched = 0;
-    p.pair64 = 0;
     p.K = K;
     p.S = S;
     p.B = B;
@@ -604,7 +606,6 @@ bool tcgen05_batched_bf16(cudaStream_t stream, bool transposed, const void *a, i
     p.head_layout_mask = 0;
     p.transposed_mask = 0;
     p.w_batched = 1;
-    p.pair64 = 0;
     p.K = K;
     p.S = M;
     p.B = B;

@@ -10,6 +10,7 @@
 #include "launch.cuh"
 #include "ln_utils.cuh"
 #include "ptx_utils.cuh"
+#include "tma_utils.cuh"
 
 #include <algorithm>
 
@@ -679,7 +680,7 @@ bool launch_pair_bias(cudaStream_t stream, ElemType t, const void *z, const void
         }
     }
     if (t == kElemF32 && H <= 8 && pos_stride == 1 && Cz % 32 == 0 && Cz <= 1024 && (((uintptr_t)z | (uintptr_t)wb) & 15u) == 0) {
-        launch_chained(pair_bias_f32_kernel, (unsigned)std::min<int64_t>((pos + 63) / 64, 148 * 8), 256, (size_t)8 * Cz * 4, stream,
+        launch_chained(pair_bias_f32_kernel, (unsigned)std::min<int64_t>((pos + 63) / 64, (int64_t)sm_count() * 8), 256, (size_t)8 * Cz * 4, stream,
                        (const float *)z, (const float *)wb, (float *)nb, nb_head_stride, pos, Cz, H, Nk, nb_row_stride);
         count_launch();
         return true;

@@ -84,7 +84,7 @@ bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *c
 // proj[c, b, i] = bf16((f32(proj) * f32(mask[b, i])) * sigmoid(f32(gate[c, b, i]))) in place; strides in elements.
 bool launch_tm_mask_gate(cudaStream_t stream, void *proj, const void *gate, const void *mask, int64_t c_i, int64_t n_res,
                          int64_t n_gather, int64_t p_s0, int64_t p_s1, int64_t g_s0, int64_t g_s1, int64_t m_s0);
-// proj and gate of the projection step on CUDA cores (any shape): see tcgen05_proj2_chanmajor_bf16.
+// proj and gate of the projection step on CUDA cores (any shape), without mask and gate (launch_tm_mask_gate follows).
 bool launch_tm_proj_generic(cudaStream_t stream, const void *x, const void *w0, const float *b0, const void *w1,
                             const float *b1, void *out0, void *out1, int64_t p_s0, int64_t p_s1, int64_t g_s0,
                             int64_t g_s1, int64_t n_res, int64_t n_gather, int64_t c_o, int64_t c_i);

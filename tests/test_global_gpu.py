@@ -69,7 +69,7 @@ def test_columns_are_independent_at_full_size(kutacc_lib):
 
 
 def test_many_short_columns_wrap_the_shared_memory_ring(kutacc_lib):
-    # more columns than resident clusters: every CTA walks several columns and reuses its slots
+    # more columns than SMs, short ones: the warps walk chunks of several columns and reuse the slots of their rings
     w = W.random_global_case(seed=23, B=700, S=300, zero_mask_rows=3)
     got = _run(w)
     assert np.isfinite(got).all()

@@ -44,8 +44,8 @@ def test_noalloc_entry_matches_regular_operator_twice_in_a_row(kutacc_lib):
         api.raise_if_error()
         got = out.float().cpu().numpy()
         # the parity tolerance of the other tests (1e-2 relative) is the formal bound; where the regular
-        # operator runs the same three kernels with the same split plan (every shape but 8 heads x 8, which
-        # it computes in one cluster kernel) the results agree to the last bit
+        # operator runs the same kernels with the same split plan (every shape but 8 heads x 8, which
+        # it computes in three streaming kernels) the results agree to the last bit
         assert np.isfinite(got).all()
         assert np.abs(got - want).max() <= 1e-2 * np.abs(want).max()
         if (w.H, w.D) != (8, 8):

@@ -174,6 +174,7 @@ int *work_counter(cudaStream_t stream)
         KUTACC_CUDA(cudaMalloc(&c, 2 * kCounters * sizeof(int)));
         if (c == nullptr) return nullptr;
         KUTACC_CUDA(cudaMemset(c, 0, 2 * kCounters * sizeof(int)));
+        KUTACC_CUDA(cudaStreamSynchronize(nullptr));     // the caller's stream may not wait for the default one
         counters[dev] = c;
     }
     int slot = -1;

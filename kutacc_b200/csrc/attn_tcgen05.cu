@@ -11,7 +11,7 @@
 //               16-column pieces (the next piece is in flight while one is worked on), rounds each raw logit to bf16
 //               as the reference's logits scratch does (src/attention/gating_attention.cpp:97-101), adds the mask and
 //               pair bias in fp32 (:112-117) and keeps P = exp2((x - max) * log2 e) as packed bf16 in 32
-//               registers. P goes back over the logits in tensor memory, where the second product reads it as its A
+//               registers (narrow heads and 64-channel layers: a bf16 head and a bf16 tail, SPLIT below). P goes back over the logits in tensor memory, where the second product reads it as its A
 //               operand: no shared-memory round trip. The running max is the thread's own; it is first taken from the
 //               item's first 16 keys and raised only when a tile exceeds it by 2^8 (a stale max cancels in the final
 //               division): then the row of O is rescaled and the tile formed again.
@@ -22,7 +22,7 @@
 //               tile than the softmax)
 //   warps 18-19 MMA issuers, warp group by warp group (two each): O_w (+)= P_w . V_w^T of tile g, then S_w = Q_w . K_w^T of tile
 //               g + 1. The row of V^T after the last channel is all ones, so the column of O after the last channel
-//               accumulates the row sum of the bf16 probabilities for free
+//               accumulates the row sum of the rounded probabilities for free
 //
 // What bounds it, and why this split: per logit the softmax issues about six instructions (two conversions per pair for
 // the bf16 logit, two packed FMAs, an add, a max3, two unpacks of the pair bias, two exponentials, one pack), so the
@@ -30,12 +30,12 @@
 // keeps a kernel away from them is the latency of the barrier -> tcgen05.ld -> softmax -> tcgen05.st -> barrier ->
 // MMA chain of a tile. Four independent chains per SM hide it: while one warp group waits for its products, the warps
 // of the other three fill the issue slots of the same schedulers. Measured: triangle attention at 1024 residues (4.3 G
-// logits) 2.16 -> 1.57 ms, column attention 384 x 512 x 8 heads 0.41 -> 0.32 ms against two CTAs per SM with one (batch row,
+// logits) 2.16 -> 1.57 ms, column attention 384 x 512 x 8 heads 0.41 -> 0.31 ms against two CTAs per SM with one (batch row,
 // head, 128 queries) each, P through shared memory and two threads per query row. The single-thread cost of the MMA
 // and TMA instructions mattered as much as the split: behind `lane == 0` an instruction took about 70 clocks to
 // issue, behind elect_one() about 33.
 //
-// Fully masked rows stay uniform as in the reference (fp32 absorption of the logit by the -1e9 bias).
+// Fully masked rows stay uniform as in the reference (fp32 absorption of the logit by the -1e9 bias, or by any finite one).
 //
 // mbarrier phases. A parity wait names "the current or the preceding phase", so every barrier here is awaited by each of
 // its waiters once per completion, in order. All waits are bounded; on a timeout the roles fall through to the common

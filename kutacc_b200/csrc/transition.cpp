@@ -1,9 +1,9 @@
 // kutacc_af2_transition: out = relu(x . W1^T + b1) . W2^T + b2, the transition MLP of the Evoformer.
 // Replaces src/attention/transition.cpp:21-61 (two addmm calls with a row bias, the first with ReLU; the
 // intermediate is a bf16 tensor). 128 or 256 channels run in one kernel that keeps the hidden activations on the SM
-// (transition_fused.cu); other shapes take two launches of the tcgen05 projection kernel (ReLU in the epilogue of the first)
-// or the generic GEMM, with the intermediate in the library's workspace: the caller's intermediate_act tensor is not
-// written, like the scratch tensors of the attention operators.
+// (transition_fused.cu); other shapes, and few rows with many hidden channels, take two launches of the tcgen05 projection
+// kernel (ReLU in the epilogue of the first) or the generic GEMM, with the intermediate in the library's workspace: the
+// caller's intermediate_act tensor is not written, like the scratch tensors of the attention operators.
 #include <cuda_runtime.h>
 
 #include <climits>

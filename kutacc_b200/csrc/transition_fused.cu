@@ -14,8 +14,9 @@
 //               epilogue (bias, bf16, staging tile, TMA store). With one group of four warps per chain the conversion of a
 //               chunk took longer than the other chain's products (53 against 50 us at 147456 rows)
 // Two row tiles share every weight slab: the weights stream from L2 once per 256 rows (302 MB instead of 604 MB at 147456
-// rows x 128 channels). Bound by the tensor cores (39 GFLOP at that size) where the two-kernel version was bound by the
-// round trip of the hidden tensor (302 MB through L2 and HBM): 90 -> 46 us there, 0.84 PFLOP/s.
+// rows x 128 channels). Bound by the chain product, conversion, product and by the operands' way through shared memory (tensor
+// pipe 40 % busy) where the two-kernel version was bound by the round trip of the hidden tensor (302 MB through L2 and HBM):
+// 90 -> 44 us there, 0.88 PFLOP/s.
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is released
 // and the host-visible error word carries the site.

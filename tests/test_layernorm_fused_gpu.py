@@ -35,7 +35,7 @@ def _oracle(w, raw, gamma, beta):
     return helpers.oracle_faithful(w2)
 
 
-# head size 32 (normalisation folded into the tcgen05 projection), other shapes (normalised copy in the workspace);
+# head size 32 (the tcgen05 projection normalises its rows), other shapes (normalised copy in the workspace);
 # the last case has row means many standard deviations away from zero
 @pytest.mark.parametrize("B,S,H,D,shift", [(3, 96, 4, 32, 1.0), (2, 200, 8, 32, 2.0), (2, 70, 2, 16, 1.0), (2, 64, 4, 32, 40.0)])
 def test_gating_attention_ln_matches_unfused_oracle(kutacc_lib, B, S, H, D, shift):

@@ -59,10 +59,10 @@ bool tcgen05_batched_bf16(cudaStream_t stream, bool transposed, const void *a, i
                           int64_t out_batch_stride, int B, int M, int N, int K);
 
 // out = relu(x . w1^T + b1) . w2^T + b2 in one kernel (transition_fused.cu): x, out [M, c_o] dense, w1 [c_i, c_o],
-// w2 [c_o, c_i]. c_o 128 or 256, c_i % 128 == 0. False when the shape is not covered, or has so few rows that two products
-// through the workspace are faster.
+// w2 [c_o, c_i]. c_o 128 or 256, c_i % 128 == 0. False when the shape is not covered, or with or_two has so few rows that
+// two products through the workspace are faster.
 bool tcgen05_transition_bf16(cudaStream_t stream, const void *x, const void *w1, const float *b1, const void *w2, const float *b2,
-                             void *out, int64_t M, int c_o, int c_i);
+                             void *out, int64_t M, int c_o, int c_i, bool or_two);
 
 // fp32 GEMM on tcgen05 (gemm_tf32_tcgen05.cu): operands pre-split into tf32 head and tail, stored as rows
 // [hi(0..K) | lo(0..K)] by launch_split_tf32 (src [rows, K] fp32 with row stride src_ld; dst [rows, 2K] dense).

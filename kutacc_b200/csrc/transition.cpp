@@ -54,8 +54,15 @@ extern "C" void kutacc_af2_transition(kutacc_af2_trans_act_inputs_t *trans_input
 
     // W1 is stored [c_i][c_o] (transition.cpp:32, the {c_o, c_i} view with strides {1, c_o}), W2 [c_o][c_i] (:36). One kernel
     // that keeps the hidden activations on the SM, or two products through the workspace.
+    // The workspace cannot grow while the stream is being captured: a call that fits one kernel stays in it then.
+    bool room = rt.ws_cap >= h_bytes + 256;
+    if (!room) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) cudaGetLastError();      // the default stream beside a capture
+        room = capture == cudaStreamCaptureStatusNone;
+    }
     bool ok = dev::tcgen05_transition_bf16(stream, d_x.dev, d_w1.dev, (const float *)d_b1.dev, d_w2.dev, (const float *)d_b2.dev,
-                                           d_o.dev, M, (int)c_o, (int)c_i);
+                                           d_o.dev, M, (int)c_o, (int)c_i, room);
     if (kutacc_check_err_set) return;
     if (!ok) {
         if (!rt.reserve_workspace(h_bytes + 256)) return;

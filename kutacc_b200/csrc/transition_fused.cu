@@ -445,13 +445,13 @@ bool two_kernels_faster(int64_t M, int c_o, int c_i)
 }  // namespace
 
 bool tcgen05_transition_bf16(cudaStream_t stream, const void *x, const void *w1, const float *b1, const void *w2, const float *b2,
-                             void *out, int64_t M, int c_o, int c_i)
+                             void *out, int64_t M, int c_o, int c_i, bool or_two)
 {
     if ((c_o != 128 && c_o != 256) || c_i % BH != 0 || c_i > MAX_HIDDEN || M > INT32_MAX / 2 ||
         ((((uintptr_t)x | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)out) & 15u) != 0))
         return false;
     // (the two products want aligned biases, this kernel does not)
-    if ((((uintptr_t)b1 | (uintptr_t)b2) & 15u) == 0 && two_kernels_faster(M, c_o, c_i)) return false;
+    if (or_two && (((uintptr_t)b1 | (uintptr_t)b2) & 15u) == 0 && two_kernels_faster(M, c_o, c_i)) return false;
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     CUtensorMap tx, t1, t2, to;

@@ -59,3 +59,25 @@ def test_relu_of_nan_is_zero(kutacc_lib, rows, c_o, c_i):
     got = _run(1, rows, c_o, c_i, (x, w1, b1, w2, b2))
     assert (got[7] == torch.from_numpy(b2).bfloat16().float().numpy()).all()
     assert (np.delete(got, 7, 0) == np.delete(clean, 7, 0)).all()
+
+
+def test_few_rows_under_capture_without_a_workspace(kutacc_lib):
+    rows, c_o, c_i = 2048, 256, 1024
+    arrays = _case(1, rows, c_o, c_i, 5)
+    x, w1, b1, w2, b2 = [(torch.from_numpy(a.view(np.int16)).view(torch.bfloat16) if a.dtype == np.uint16 else torch.from_numpy(a)).cuda() for a in arrays]
+    out = torch.zeros_like(x)
+    ts = [api.tensor(t) for t in (x.view(1, rows, c_o), w1, b1, w2, b2, out.view(1, rows, c_o))]
+    torch.cuda.synchronize()
+    api.lib().kutacc_b200_release_workspace()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    api.set_async(True)
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            api.set_stream(stream.cuda_stream)
+            api.transition(1, rows, c_o, c_i, *ts)
+    finally:
+        api.set_stream(0)
+        api.set_async(False)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert helpers.rel_err(out.float().cpu().numpy(), as_f32(O.transition_bf16(*arrays))) <= helpers.BF16_TOL

@@ -50,7 +50,8 @@ constexpr float kRescaleThreshold = 5.5f;       // P stays below 2^8
 struct F32Params {
     const float *q, *gate;            // [B, S, H*D]
     const float *bias;                // [B, S] (row stride bias_stride0)
-    float *avg;                       // [B, S, 2*H*D]: tf32 head | tail of the gated average
+    float *avg;                       // gated average [B, S, H*D], or [B, S, 2*H*D]: its tf32 head | tail
+    int avg_split;
     int64_t bias_stride0;
     int *err;
     int S, H, B, G, n_qt, n_items;
@@ -432,19 +433,19 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             tmem_ld_wait();
             const float inv = 1.0f / __uint_as_float(osum);
             if (live) {
-                float *dst = p.avg + m_row * 2 * C + h * D;
+                float *dst = p.avg + m_row * (p.avg_split ? 2 * C : C) + h * D;
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    float hv[4], lv[4];
+                    float av[4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        // sigmoid with the hardware reciprocal (2 ulp)
-                        const float a = __uint_as_float(o[4 * c + e]) * inv * __fdividef(1.0f, 1.0f + __expf(-gate[4 * c + e]));
-                        hv[e] = tf32_head(a);
-                        lv[e] = a - hv[e];
+                    for (int e = 0; e < 4; ++e)      // sigmoid with the hardware reciprocal (2 ulp)
+                        av[e] = __uint_as_float(o[4 * c + e]) * inv * __fdividef(1.0f, 1.0f + __expf(-gate[4 * c + e]));
+                    float4 hv = make_float4(av[0], av[1], av[2], av[3]);
+                    if (p.avg_split) {
+                        hv = make_float4(tf32_head(av[0]), tf32_head(av[1]), tf32_head(av[2]), tf32_head(av[3]));
+                        *reinterpret_cast<float4 *>(dst + C + 4 * c) = make_float4(av[0] - hv.x, av[1] - hv.y, av[2] - hv.z, av[3] - hv.w);
                     }
-                    *reinterpret_cast<float4 *>(dst + 4 * c) = make_float4(hv[0], hv[1], hv[2], hv[3]);
-                    *reinterpret_cast<float4 *>(dst + C + 4 * c) = make_float4(lv[0], lv[1], lv[2], lv[3]);
+                    *reinterpret_cast<float4 *>(dst + 4 * c) = hv;
                 }
             }
             w = nxt;
@@ -478,11 +479,11 @@ int smem_bytes(int G, bool has_nb)
 
 bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, const void *vt_split, int64_t vt_pitch,
                       const void *gate, const void *bias, int64_t bias_stride0, const void *nb, int64_t nb_stride_h,
-                      int64_t nb_stride_q, void *avg_split, int B, int S, int H, int Dh, float scale)
+                      int64_t nb_stride_q, void *avg, bool avg_split, int B, int S, int H, int Dh, float scale)
 {
     if (Dh != D || vt_pitch % 4 != 0 || vt_pitch < S) return false;
     if (nb && ((nb_stride_h % 4) || (nb_stride_q % 4) || ((uintptr_t)nb % 16) || nb_stride_h < nb_stride_q)) return false;
-    if ((((uintptr_t)q | (uintptr_t)gate | (uintptr_t)avg_split) & 15u) != 0) return false;
+    if ((((uintptr_t)q | (uintptr_t)gate | (uintptr_t)avg) & 15u) != 0) return false;
     const int64_t n_qt = (S + BM - 1) / BM, hq = n_qt * H;
     if (hq * B > INT32_MAX / 64) return false;
     KernelErrorWord &ew = kernel_error_word();
@@ -493,7 +494,8 @@ bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, c
     p.q = (const float *)q;
     p.gate = (const float *)gate;
     p.bias = (const float *)bias;
-    p.avg = (float *)avg_split;
+    p.avg = (float *)avg;
+    p.avg_split = avg_split;
     p.bias_stride0 = bias_stride0;
     p.err = ew.device;
     p.S = S;

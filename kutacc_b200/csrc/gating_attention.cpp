@@ -134,6 +134,9 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     // fp32 on the tensor-memory GEMM: operands split into tf32 head and tail (activations: one [M, 2C] buffer that the
     // projection and, later, the output projection use in turn; five weights [C, 2C])
     const bool f32_tc = dt == kFP32 && C % 128 == 0 && out_rs % 4 == 0;
+    // up to 256 channels the product splits its activations itself, into fp16 heads and tails at twice the rate (128 x 256 rows of
+    // 256 channels: 81 us for the projections, 92 and 20 for the split before them the other way)
+    const bool f32_rows = f32_tc && C <= 256;
     // The TMA loads of the pair bias need 16-byte aligned rows. A pair bias whose strides are not
     // multiples of 16 bytes, or are zero (one head or one query row for all), is first copied into the workspace with padded rows;
     // for the fp32 core also one with the heads inside its rows.
@@ -150,7 +153,8 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     const size_t nb_pad_bytes = nb_repitch ? (size_t)H * S * s_pad8 * es : 0;
     const size_t fold_bytes = ln_folded ? (size_t)M * 8 + 256 + 4 * (w_bytes + 256) + 8 * (b_bytes + 256) : 0;
     const size_t norm_bytes = ln_copied ? x_bytes + 256 : 0;
-    const size_t f32_bytes = f32_tc ? 2 * x_bytes + 256 + 5 * (2 * w_bytes + 256) : 0;
+    const size_t ws_bytes = f32_rows ? w_bytes + b_bytes : 2 * w_bytes;                 // a split weight
+    const size_t f32_bytes = f32_tc ? (f32_rows ? 0 : 2 * x_bytes + 256) + 5 * (ws_bytes + 256) : 0;
     if (!rt.reserve_workspace(3 * (x_bytes + 256) + k_bytes + 256 + v_bytes + 256 + nb_pad_bytes + 256 + fold_bytes + norm_bytes + f32_bytes))
         return;
 
@@ -178,9 +182,9 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         ln_t[i] = (float *)rt.take_workspace(b_bytes);
     }
     char *x_norm = ln_copied ? (char *)rt.take_workspace(x_bytes) : nullptr;
-    char *a_split = f32_tc ? (char *)rt.take_workspace(2 * x_bytes) : nullptr;
+    char *a_split = f32_tc && !f32_rows ? (char *)rt.take_workspace(2 * x_bytes) : nullptr;
     void *w_split[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    for (int i = 0; i < 5 && f32_tc; ++i) w_split[i] = rt.take_workspace(2 * w_bytes);
+    for (int i = 0; i < 5 && f32_tc; ++i) w_split[i] = rt.take_workspace(ws_bytes);
     if (kutacc_check_err_set) return;
 
     const float scale = (float)(1 / std::sqrt((double)head_size));  // gating_attention.cpp:68
@@ -224,7 +228,8 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     bool f32_tc_ok = f32_tc && aligned16(d_x.dev) && aligned16(d_out.dev);
     if (f32_tc_ok) {
         const void *w_in[5] = {d_wq.dev, d_wk.dev, d_wv.dev, d_wg.dev, d_wo.dev};
-        f32_tc_ok = dev::launch_split_tf32_many(stream, 5, w_in, C, w_split, C, (int)C);
+        f32_tc_ok = f32_rows ? dev::split_f32_weights(stream, 5, w_in, C, w_split, (int)C, (int)C)
+                             : dev::launch_split_tf32_many(stream, 5, w_in, C, w_split, C, (int)C);
     }
 
     // kernel sequence for batch rows [b0, b0 + nb): every buffer is batch-major, so a chunk is an offset
@@ -291,11 +296,17 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
         } else {
             const dev::ElemType et = dt == kFP32 ? dev::kElemF32 : dev::kElemBF16;
             char *v_c = wv_ + b0 * row_bytes;
-            char *as_c = f32_tc_ok ? a_split + 2 * b0 * row_bytes : nullptr;
+            char *as_c = f32_tc_ok && !f32_rows ? a_split + 2 * b0 * row_bytes : nullptr;
+            // the tensor-memory product of x_c or, later, a_c (or of their split rows as_c) with up to four weights
+            auto product = [&](const char *a, void *const *w, const float *const *pb, void *const *po, int64_t ldo, int n,
+                               const dev::Tf32Layout *layout) {
+                return f32_rows ? dev::tcgen05_gemm_f32_rows(stream, a, C, w, pb, po, ldo, Mc, (int)C, (int)C, n, layout, (int)S, s_pad8)
+                                : dev::tcgen05_gemm_tf32x3(stream, as_c, w, pb, po, ldo, Mc, (int)C, (int)C, n, layout, (int)S, s_pad8);
+            };
             const float *gb_dev = (const float *)d_bg.dev;
             // fp32 with the tensor-memory GEMM after it: the attention core writes its result already split into
             // tf32 head and tail, in the rows of the output projection's operand
-            bool avg_is_split = false, projected = false;
+            bool avg_is_split = false, avg_done = false, projected = false;
             ok = true;
             if (f32_tc_ok) {
                 // all four projections in one pass of the tensor-memory GEMM over the split activations
@@ -303,18 +314,18 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
                 const dev::Tf32Layout split[4] = {dev::kTf32Rows, dev::kTf32SplitRows, dev::kTf32SplitTransposed, dev::kTf32Rows};
                 char *k_s = wk_ + 2 * b0 * row_bytes, *v_s = wv_ + (size_t)b0 * 2 * C * s_pad8 * es;
                 void *po[4] = {q_c, f32_split ? k_s : k_c, f32_split ? v_s : v_c, g_c};
-                projected = dev::launch_split_tf32(stream, x_c, C, as_c, Mc, (int)C) &&
-                            dev::tcgen05_gemm_tf32x3(stream, as_c, w_split, pb, po, C, Mc, (int)C, (int)C, 4,
-                                                     f32_split ? split : nullptr, (int)S, s_pad8);
+                projected = (f32_rows || dev::launch_split_tf32(stream, x_c, C, as_c, Mc, (int)C)) &&
+                            product(x_c, w_split, pb, po, C, 4, f32_split ? split : nullptr);
                 wait_for_pair_bias();
                 if (projected && f32_split) {
-                    avg_is_split = dev::tcgen05_attn_f32(stream, q_c, k_s, v_s, s_pad8, g_c, bias_c, bias_s0, nb_dev, nb_sh, nb_sq,
-                                                         as_c, (int)nbr, (int)S, (int)H, (int)D, scale);
+                    avg_done = dev::tcgen05_attn_f32(stream, q_c, k_s, v_s, s_pad8, g_c, bias_c, bias_s0, nb_dev, nb_sh, nb_sq,
+                                                     f32_rows ? a_c : as_c, !f32_rows, (int)nbr, (int)S, (int)H, (int)D, scale);
+                    avg_is_split = avg_done && !f32_rows;
                     // a shape or pair-bias layout that core does not take: k and v once more as plain rows
-                    if (!avg_is_split) {
+                    if (!avg_done) {
                         void *pk[2] = {k_c, v_c};
                         const float *nobias[2] = {nullptr, nullptr};
-                        projected = dev::tcgen05_gemm_tf32x3(stream, as_c, &w_split[1], nobias, pk, C, Mc, (int)C, (int)C, 2);
+                        projected = product(x_c, &w_split[1], nobias, pk, C, 2, nullptr);
                     }
                 }
             }
@@ -325,10 +336,10 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
                     ok = dev::launch_gemm_generic(stream, et, x_c, C, w_dev[i], C, i == 3 ? gb_dev : nullptr, 0.f, o_dev[i], C, Mc, C, C);
             }
             wait_for_pair_bias();
-            if (ok && dt == kFP32 && f32_tc_ok && !avg_is_split)
-                avg_is_split = dev::launch_attn_f32(stream, q_c, k_c, v_c, g_c, bias_c, bias_s0, has_nb ? d_nb.dev : nullptr,
+            if (ok && dt == kFP32 && f32_tc_ok && !f32_rows && !avg_done)
+                avg_done = avg_is_split = dev::launch_attn_f32(stream, q_c, k_c, v_c, g_c, bias_c, bias_s0, has_nb ? d_nb.dev : nullptr,
                                                     nb_s0, nb_s1, a_c, (int)nbr, (int)S, (int)H, (int)D, scale, as_c);
-            ok = ok && (avg_is_split ||
+            ok = ok && (avg_done ||
                         (dt == kFP32 && dev::launch_attn_f32(stream, q_c, k_c, v_c, g_c, bias_c, bias_s0,
                                                               has_nb ? d_nb.dev : nullptr, nb_s0, nb_s1, a_c, (int)nbr,
                                                               (int)S, (int)H, (int)D, scale)) ||
@@ -339,8 +350,8 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
             if (ok && f32_tc_ok) {
                 const float *pb[1] = {(const float *)d_bo.dev};
                 void *po[1] = {out_c};
-                out_done = (avg_is_split || dev::launch_split_tf32(stream, a_c, C, as_c, Mc, (int)C)) &&
-                           dev::tcgen05_gemm_tf32x3(stream, as_c, &w_split[4], pb, po, out_rs, Mc, (int)C, (int)C, 1);
+                out_done = (f32_rows || avg_is_split || dev::launch_split_tf32(stream, a_c, C, as_c, Mc, (int)C)) &&
+                           product(a_c, &w_split[4], pb, po, out_rs, 1, nullptr);
             }
             // (when the average exists only in split form, the tensor-memory GEMM is the only kernel that can read it)
             ok = ok && (out_done || (!avg_is_split && dev::launch_gemm_generic(stream, et, a_c, C, d_wo.dev, C,

@@ -80,6 +80,13 @@ bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *c
                          void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg, const Tf32Layout *layout = nullptr,
                          int S = 0, int64_t vt_pitch = 0);
 
+// The same product for K of 128 or 256 (gemm_f32_rows.cu): a [M, K] fp32 with row stride lda, split on the way; the weights split by
+// split_f32_weights into fp16 heads and tails with their rows' scales (each dst rows * K * 4 + rows * 4 bytes).
+bool split_f32_weights(cudaStream_t stream, int count, const void *const *src, int64_t src_ld, void *const *dst, int rows, int K);
+bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, const void *const *w_split, const float *const *bias,
+                           void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg, const Tf32Layout *layout = nullptr,
+                           int S = 0, int64_t vt_pitch = 0);
+
 // ---- triangle multiplication: element-wise steps and fallbacks (tm_kernels.cu) ------------------------
 // proj[c, b, i] = bf16((f32(proj) * f32(mask[b, i])) * sigmoid(f32(gate[c, b, i]))) in place; strides in elements.
 bool launch_tm_mask_gate(cudaStream_t stream, void *proj, const void *gate, const void *mask, int64_t c_i, int64_t n_res,
@@ -156,10 +163,10 @@ bool launch_attn_f32(cudaStream_t stream, const void *q, const void *k, const vo
 
 // The same operator on tcgen05 (attn_f32_tcgen05.cu): q, gate [B, S, H*32] fp32, k_split and vt_split as tcgen05_gemm_tf32x3
 // stores them (kTf32SplitRows, kTf32SplitTransposed), pair-bias strides multiples of 4 elements and its base 16-byte
-// aligned; result as rows [tf32 head | tail] in avg_split. False for other shapes.
+// aligned; result as rows [tf32 head | tail] in avg with avg_split, otherwise plain. False for other shapes.
 bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, const void *vt_split, int64_t vt_pitch,
                       const void *gate, const void *bias, int64_t bias_stride0, const void *nb, int64_t nb_stride_h,
-                      int64_t nb_stride_q, void *avg_split, int B, int S, int H, int D, float scale);
+                      int64_t nb_stride_q, void *avg, bool avg_split, int B, int S, int H, int D, float scale);
 
 // LayerNorm folded into the projection that follows (ln_fold.cu): per-row (mean, rstd) pairs as float2, and
 // for up to four [N, K] weight matrices the folded, centred bf16 weights with the epilogue terms s and t

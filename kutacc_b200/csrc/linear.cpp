@@ -58,14 +58,19 @@ extern "C" void kutacc_af2_linear(kutacc_tensor_h act_h, kutacc_tensor_h weight_
     }
     if (dt == kFP32 && beta == 0 && a16 && k % 32 == 0 && n % 128 == 0 && lda % 4 == 0 && ldw % 4 == 0 && k <= INT32_MAX / 2 &&
         n <= INT32_MAX && (((uintptr_t)d_r.dev | (uintptr_t)d_b.dev) & 15u) == 0) {
-        // fp32 on the tensor-memory GEMM: both operands split into tf32 head and tail in the workspace
-        const size_t as_bytes = (size_t)m * 2 * k * 4, ws_bytes = (size_t)n * 2 * k * 4;
+        // fp32 on the tensor memory: up to 256 columns the product splits its activations itself, beyond that both operands are
+        // split into tf32 head and tail in the workspace
+        const bool rows = k == 128 || k == 256;
+        const size_t as_bytes = rows ? 0 : (size_t)m * 2 * k * 4, ws_bytes = rows ? (size_t)n * (k + 1) * 4 : (size_t)n * 2 * k * 4;
         if (rt.reserve_workspace(as_bytes + ws_bytes + 512)) {
-            void *a_split = rt.take_workspace(as_bytes), *w_split = rt.take_workspace(ws_bytes);
-            const void *wp[1] = {w_split};
+            void *a_split = rows ? nullptr : rt.take_workspace(as_bytes), *w_split = rt.take_workspace(ws_bytes);
+            const void *wp[1] = {w_split}, *const src[1] = {d_w.dev};
+            void *wsp[1] = {w_split};
             const float *bp[1] = {(const float *)d_b.dev};
             void *op[1] = {d_r.dev};
-            ok = a_split && w_split && dev::launch_split_tf32(stream, d_a.dev, lda, a_split, m, (int)k) &&
+            ok = rows ? w_split && dev::split_f32_weights(stream, 1, src, ldw, wsp, (int)n, (int)k) &&
+                            dev::tcgen05_gemm_f32_rows(stream, d_a.dev, lda, wp, bp, op, n, m, (int)n, (int)k, 1)
+                      : a_split && w_split && dev::launch_split_tf32(stream, d_a.dev, lda, a_split, m, (int)k) &&
                  dev::launch_split_tf32(stream, d_w.dev, ldw, w_split, n, (int)k) &&
                  dev::tcgen05_gemm_tf32x3(stream, a_split, wp, bp, op, n, m, (int)n, (int)k, 1);
         }

@@ -120,3 +120,21 @@ def test_pair_bias_written_with_the_heads_inside_the_rows(kutacc_lib, R, Nk, Cz,
     torch.cuda.synchronize()
     assert torch.equal(store[:, :H, :].permute(1, 0, 2), dense)
     assert (store[:, H, :] == 7.0).all()
+
+
+# rows around the 128-row block, calls of more blocks than SMs (whole blocks, then parts of blocks), one to three column tiles
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (127, 128, 256), (129, 384, 128), (300, 256, 256), (19200, 384, 128), (19201, 128, 256)])
+def test_linear_fp32_rows_of_any_magnitude(kutacc_lib, M, N, K):
+    # powers of two up to 2^60 between rows, channels and columns (the latter against their weights), a row of zeros
+    rng = np.random.default_rng(M + N + K)
+    col = np.exp2(rng.integers(-12, 13, K)).astype(np.float32)
+    a = (rng.standard_normal((M, K)) * np.exp2(rng.integers(-60, 61, (M, 1)))).astype(np.float32) * col
+    w = (rng.standard_normal((N, K)) * np.exp2(rng.integers(-20, 21, (N, 1)))).astype(np.float32) / col
+    a[M // 2] = 0
+    ta, tw = torch.from_numpy(a).to(DEV), torch.from_numpy(w).to(DEV)
+    tr = torch.full((M, N), 7.0, dtype=torch.float32, device=DEV)
+    api.linear(api.tensor(ta), api.tensor(tw), None, api.tensor(tr), 0)
+    torch.cuda.synchronize()
+    ref, terms = ta.double() @ tw.double().T, ta.double().abs() @ tw.double().abs().T
+    # operands to 2^-23 each, the product of the tails dropped (2^-24): 3 * 2^-23; up to 2 K / 16 accumulations that truncate at 2^-23
+    assert ((tr.double() - ref).abs() <= (3 + K / 8) * 2.0 ** -23 * terms).all()

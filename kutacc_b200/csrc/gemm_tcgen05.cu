@@ -60,6 +60,7 @@ constexpr int TMEM_COLS = ACC_STAGES * BNMAX;              // 256: half of the S
 
 struct alignas(64) GemmMaps {
     CUtensorMap a;        // X  [B][S][K], box [64, 128, 1], 128-byte swizzle
+    CUtensorMap a2;       // F_TWO: X of segment 1
     CUtensorMap w[4];     // W  [1][N_seg][K], box [64, 128 (segments of 64 channels and 64-wide tiles: 64), 1], 128-byte swizzle
     CUtensorMap out[4];   // destination per segment, box [32, 32, 1], 64-byte swizzle; head sizes below 32: box [D, 32, 32 / D]
 };
@@ -118,9 +119,11 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t addr)
 // F_DIRECT: out[b][n][s] element by element, s along the lanes of a warp (64 contiguous bytes per channel and store): for
 // destinations whose strides no TMA store takes.
 // F_NARROW: head sizes of 8 or 16.
+// F_TWO: two linear layers of one shape in one launch, segment i reads its own X (the gate and output layers of the triangle
+// multiplication: 384 x 384 x 128 27 us as two launches, 25 as one; 301 x 301 22 and 17, as one fills the last wave).
 // F_PAIR64: segments of 64 channels, two of them in a column tile (a layer of one head of 64).
 constexpr int F_SIGMOID = 1, F_TRANSPOSED = 2, F_RELU = 4, F_WBATCH = 8, F_LN = 16, F_NARROW = 32, F_MNMAJOR = 64,
-              F_DIRECT = 128, F_PAIR64 = 256;
+              F_DIRECT = 128, F_PAIR64 = 256, F_TWO = 512;
 
 // BN: width of a column tile, 128, or 64 for a product with 64 output channels
 template <int FEAT, int BN>
@@ -195,7 +198,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 tile_of(tile, m_tile, n_tile);
                 const int b = m_tile / s_tiles, s0 = (m_tile % s_tiles) * BM;
                 const int seg = pair64 ? 2 * n_tile : n_tile / n_tiles_seg, n0 = pair64 ? 0 : (n_tile % n_tiles_seg) * BN;
-                const CUtensorMap *wmap = &maps.w[seg];
+                const CUtensorMap *wmap = &maps.w[seg], *amap = (FEAT & F_TWO) && seg == 1 ? &maps.a2 : &maps.a;
                 for (int kc = 0; kc < nk; ++kc, ++it) {
                     const int s = it % NSTAGE;
                     if (it >= NSTAGE && !mbar_wait(empty_bar(s), (uint32_t)((it / NSTAGE - 1) & 1), p.err, 11)) {
@@ -212,7 +215,7 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                         }
                         continue;
                     }
-                    tma_load_3d(st, &maps.a, full_bar(s), kc * BK, s0, b);
+                    tma_load_3d(st, amap, full_bar(s), kc * BK, s0, b);
                     tma_load_3d(st + SLAB_BYTES, wmap, full_bar(s), kc * BK, n0, (FEAT & F_WBATCH) ? b : 0);
                     if (pair64) tma_load_3d(st + SLAB_BYTES + 64 * BK * 2, wmap + 1, full_bar(s), kc * BK, 0, 0);
                 }
@@ -555,6 +558,39 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     p.err = ew.device;
     if (N == 64) return launch<0, 64>(stream, maps, p, "linear_bias");
     return relu ? launch<F_RELU>(stream, maps, p, "linear_bias_relu") : launch<0>(stream, maps, p, "linear_bias");
+}
+
+// Two linear layers of one shape in one launch: out_i = a_i . w_i^T + bias_i
+bool tcgen05_linear_pair_bf16(cudaStream_t stream, const LinearOperands (&l)[2], int64_t rows, int N, int K)
+{
+    if (N % 128 != 0 || K % 64 != 0 || rows > INT32_MAX / 2) return false;
+    KernelErrorWord &ew = kernel_error_word();
+    if (ew.device == nullptr) return false;
+    GemmMaps maps;
+    GemmParams p = {};
+    for (int i = 0; i < 2; ++i) {
+        if (l[i].out_row_stride % 8 != 0 || l[i].a_row_stride % 8 != 0 || l[i].a_row_stride < K ||
+            ((((uintptr_t)l[i].out | (uintptr_t)l[i].a | (uintptr_t)l[i].w | (uintptr_t)l[i].bias) & 15u) != 0))
+            return false;
+        if (!make_tensor_map_bf16_3d(i ? &maps.a2 : &maps.a, l[i].a, K, rows, 1, (uint64_t)l[i].a_row_stride, (uint64_t)rows * l[i].a_row_stride,
+                                     BK, BM, 128) ||
+            !make_tensor_map_bf16_3d(&maps.w[i], l[i].w, K, N, 1, K, (uint64_t)N * K, BK, BNMAX, 128) ||
+            !make_tensor_map_bf16_3d(&maps.out[i], l[i].out, N, rows, 1, (uint64_t)l[i].out_row_stride, (uint64_t)rows * l[i].out_row_stride, 32, 32,
+                                     64))
+            return false;
+        p.bias[i] = l[i].bias;
+    }
+    for (int i = 2; i < 4; ++i) {
+        maps.w[i] = maps.w[0];
+        maps.out[i] = maps.out[0];
+    }
+    p.seg_n = N;
+    p.nseg = 2;
+    p.K = K;
+    p.S = (int)rows;
+    p.B = 1;
+    p.err = ew.device;
+    return launch<F_TWO>(stream, maps, p, "linear_pair");
 }
 
 // Batched product with one right-hand matrix per batch: out[b, m, n] = sum_k a[b, m, k] * w[b, n, k], or with

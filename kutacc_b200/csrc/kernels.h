@@ -52,6 +52,17 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
 bool tcgen05_tm_proj_bf16(cudaStream_t stream, const void *x, const void *wp, const float *bp, const void *wg, const float *bg,
                           const void *mask, int64_t m_s0, void *proj, int64_t p_s0, int64_t p_s1, void *gate, int64_t g_s0,
                           int64_t g_s1, int B, int S, int N, int K);
+// Two linear layers of one shape (rows of the same number of channels in and out) in one launch.
+struct LinearOperands {
+    const void *a;
+    int64_t a_row_stride;
+    const void *w;              // [N, K]
+    const float *bias;          // [N], may be null
+    void *out;
+    int64_t out_row_stride;
+};
+bool tcgen05_linear_pair_bf16(cudaStream_t stream, const LinearOperands (&l)[2], int64_t rows, int N, int K);
+
 // out[b, m, n] = sum_k a[b, m, k] * w[b, n, k], or with `transposed` sum_k a[b, k, m] * w[b, k, n]: one right-hand matrix
 // per batch (strides of a and w multiples of 8 elements, of out any).
 bool tcgen05_batched_bf16(cudaStream_t stream, bool transposed, const void *a, int64_t a_row_stride, int64_t a_batch_stride,

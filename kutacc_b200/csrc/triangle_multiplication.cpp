@@ -27,6 +27,12 @@ DeviceArg resolve_out_keeping_gaps(void *p, size_t bytes, bool dense)
     return dense ? resolve_out(p, bytes) : resolve_in(p, bytes);
 }
 
+// two ranges without a common byte
+bool apart(const void *a, size_t a_bytes, const void *b, size_t b_bytes)
+{
+    return (uintptr_t)a + a_bytes <= (uintptr_t)b || (uintptr_t)b + b_bytes <= (uintptr_t)a;
+}
+
 }  // namespace
 }  // namespace kutacc
 
@@ -224,14 +230,22 @@ extern "C" void kutacc_af2_triangle_multiplication_gate_and_out_linear(kutacc_te
     DeviceArg d_g = resolve_out_keeping_gaps(gate.data_ptr(), g_bytes, g_rs == c_o),
               d_o = resolve_out_keeping_gaps(out.data_ptr(), o_bytes, o_rs == c_o);
     if (kutacc_check_err_set) return;
-    bool ok = dev::tcgen05_linear_bias_bf16(stream, d_x.dev, d_gw.dev, (const float *)d_gb.dev, d_g.dev, g_rs, (int)n_res,
-                                            (int)n_gather, (int)c_o, (int)c_o, false, c_o);
+    // both layers in one launch where they have one shape; their order then is not fixed, so neither may write what the other reads
+    bool both = false;
+    if (c_o == c_i && apart(d_g.dev, g_bytes, d_c.dev, c_bytes) && apart(d_g.dev, g_bytes, d_o.dev, o_bytes) && apart(d_o.dev, o_bytes, d_x.dev, x_bytes)) {
+        const dev::LinearOperands layers[2] = {{d_x.dev, c_o, d_gw.dev, (const float *)d_gb.dev, d_g.dev, g_rs},
+                                               {d_c.dev, c_rs, d_ow.dev, (const float *)d_ob.dev, d_o.dev, o_rs}};
+        both = dev::tcgen05_linear_pair_bf16(stream, layers, P, (int)c_o, (int)c_o);
+        if (kutacc_check_err_set) return;
+    }
+    bool ok = both || dev::tcgen05_linear_bias_bf16(stream, d_x.dev, d_gw.dev, (const float *)d_gb.dev, d_g.dev, g_rs, (int)n_res,
+                                                    (int)n_gather, (int)c_o, (int)c_o, false, c_o);
     if (kutacc_check_err_set) return;
     if (!ok)
         ok = dev::launch_gemm_generic(stream, dev::kElemBF16, d_x.dev, c_o, d_gw.dev, c_o, (const float *)d_gb.dev, 0.f, d_g.dev,
                                       g_rs, P, c_o, c_o);
-    bool ok2 = ok && dev::tcgen05_linear_bias_bf16(stream, d_c.dev, d_ow.dev, (const float *)d_ob.dev, d_o.dev, o_rs, (int)n_res,
-                                                   (int)n_gather, (int)c_o, (int)c_i, false, c_rs);
+    bool ok2 = both || (ok && dev::tcgen05_linear_bias_bf16(stream, d_c.dev, d_ow.dev, (const float *)d_ob.dev, d_o.dev, o_rs, (int)n_res,
+                                                            (int)n_gather, (int)c_o, (int)c_i, false, c_rs));
     if (kutacc_check_err_set) return;
     if (ok && !ok2)
         ok2 = dev::launch_gemm_generic(stream, dev::kElemBF16, d_c.dev, c_rs, d_ow.dev, c_i, (const float *)d_ob.dev, 0.f, d_o.dev,

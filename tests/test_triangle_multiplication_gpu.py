@@ -200,3 +200,26 @@ def test_null_arguments_are_reported(kutacc_lib):
     L.kutacc_af2_triangle_multiplication_last(None, None, 2, 2, 2)
     assert api.error_set() and "input args nullptr error" in api.last_error()
     api.clear_error()
+
+
+@pytest.mark.parametrize("n,c_o,c_i", [(9, 128, 128), (33, 256, 256), (40, 128, 64)])
+def test_gate_and_out_linear_with_an_output_over_its_input(kutacc_lib, n, c_o, c_i):
+    """Both layers run in one launch where they have one shape; an output in the place of the other layer's input keeps the order
+    of the reference (the gate first)."""
+    A = _case(950 + n, n, c_o, c_i)
+    cen = _bf(np.random.default_rng(n).standard_normal((n, n, c_i)).astype(np.float32))
+    weights = api.make_tm_linear_weights(c_o, c_i, _bf(A["gating_w"]), torch.from_numpy(A["gating_b"]).to(DEV), _bf(A["out_w"]),
+                                         torch.from_numpy(A["out_b"]).to(DEV))
+
+    def run(x, out):
+        gate = torch.zeros((n, n, c_o), dtype=torch.bfloat16, device=DEV)
+        api.tm_gate_and_out_linear(api.tensor(gate), api.tensor(out), api.make_tm_acts(n, n, None, x, None), api.tensor(cen), weights)
+        torch.cuda.synchronize()
+        return gate, out
+
+    x = _bf(A["x"])
+    gate, out = run(x, torch.zeros((n, n, c_o), dtype=torch.bfloat16, device=DEV))
+    gate2, out2 = run(x, x)
+    assert torch.equal(gate, gate2) and torch.equal(out, out2)
+    want = O.linear_bf16(W.bf16_bits(A["x"]).reshape(-1, c_o), W.bf16_bits(A["gating_w"]), A["gating_b"])
+    assert helpers.rel_err(_f32(gate).reshape(-1, c_o), W.as_f32(want)) <= 2.0 ** -7

@@ -295,6 +295,10 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
 #pragma unroll
             for (int c = 0; c < COLS / 32; ++c) tmem_ld_32x32(tcol + c * 32, r[c]);
             tmem_ld_wait();
+            // everything is in registers: the accumulator may be overwritten
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty(a));
 #pragma unroll
             for (int c = 0; c < COLS / 32; ++c) {
                 const int n = n0 + c * 32;
@@ -411,9 +415,6 @@ gemm_tcgen05_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p)
                 }
                 ++nstore;
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty(a));
         }
         if (lane == 0) tma_store_wait<0>();
     }

@@ -15,7 +15,9 @@
 // bytes of a channel; storing words of two positions from staging tiles was slower (301 x 301 x 128: 30 to 34 us against 20 to 25).
 // Bound by HBM (x in, two outputs; 113 MB at 384 x 384 x 128, 17 us) and by the instructions of the epilogue: with one element
 // and one position per lane at a time it took 35 per element and the kernel 34.5 us; now 26. Where rows of positions follow
-// one another without gaps the batch rows are one row of n_res * n_res_gather positions.
+// one another without gaps the batch rows are one row of n_res * n_res_gather positions. The clocks of a CTA showed 2000 of a
+// tile's 3700 between two tiles' arithmetic: mask and biases on their way from memory and the wait for the staging tiles, both now
+// out of that path (384 x 384 x 128: 25 -> 22 us).
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is released
 // and the host-visible error word carries the site.
@@ -179,18 +181,37 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
         // 32 rows (quad) x 32 columns (grp) of both accumulators
         const int ew = warp - EPI_WARP0, quad = warp & 3, grp = ew >> 2;
         const uint32_t stg = smem + STG_OFF + (uint32_t)(ew * 2 * TILE_BYTES), mk = smem + MASK_OFF + (uint32_t)(ew * 128);
-        int t = 0;
-        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++t) {
-            const int m_tile = tile / n_tiles, n = tile % n_tiles * BN + (TMA_OUT ? quad : grp) * 32;
-            const int b = m_tile / s_tiles, row0 = m_tile % s_tiles * BM + (TMA_OUT ? grp : quad) * 32, row = row0 + lane;
-            const float mv = row < p.S ? __bfloat162float(p.mask[b * p.m_s0 + row]) : 0.f;
-            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)((t & 1) * 2 * BM + grp * 32);
-            float bp = 0.f, bg = 0.f;
+        int t = 0, b, row0, row, n;
+        // where this warp's part of a tile lies, and its mask value and biases, which are loaded a tile ahead: their way from memory
+        // (and the wait for the staging tiles, which comes as late as it can) was half of a tile's time
+        auto place = [&](int tile) {
+            const int m_tile = tile / n_tiles;
+            n = tile % n_tiles * BN + (TMA_OUT ? quad : grp) * 32;
+            b = m_tile / s_tiles;
+            row0 = m_tile % s_tiles * BM + (TMA_OUT ? grp : quad) * 32;
+            row = row0 + lane;
+        };
+        __nv_bfloat16 mask_next = __float2bfloat16(0.f);
+        float bp = 0.f, bg = 0.f, bp_next = 0.f, bg_next = 0.f;
+        auto load_next = [&](int tile) {
+            if (tile >= num_tiles) return;
+            place(tile);
+            mask_next = row < p.S ? p.mask[b * p.m_s0 + row] : __float2bfloat16(0.f);
             if (TMA_OUT) {
-                bp = __ldg(p.bias_p + n + lane);
-                bg = __ldg(p.bias_g + n + lane);
+                bp_next = __ldg(p.bias_p + n + lane);
+                bg_next = __ldg(p.bias_g + n + lane);
+            }
+        };
+        load_next(blockIdx.x);
+        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++t) {
+            const float mv = __bfloat162float(mask_next);
+            bp = bp_next;
+            bg = bg_next;
+            load_next(tile + gridDim.x);
+            place(tile);
+            const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)((t & 1) * 2 * BM + grp * 32);
+            if (TMA_OUT) {
                 asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(mk + lane * 4), "f"(mv) : "memory");
-                if (lane == 0) tma_store_wait_read<0>();           // the staging tiles may be rewritten
                 __syncwarp();
             }
             if (!mbar_wait_warp(acc_full(t & 1), (uint32_t)((t / 2) & 1), p.err, 54)) break;
@@ -223,6 +244,10 @@ tm_proj_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__
                             op[(j + h) >> 1] = pack_bf16x2(y0, y1);
                             og[(j + h) >> 1] = g16;
                         }
+                    }
+                    if (c == 0) {                                  // the staging tiles may be rewritten
+                        if (lane == 0) tma_store_wait_read<0>();
+                        __syncwarp();
                     }
                     // staging tile: a row of 64 bytes per channel, 64-byte swizzle
 #pragma unroll

@@ -6,7 +6,8 @@
 //
 // A work item is (two batch rows, head h, 128 queries); persistent CTAs, one per SM, take items from an atomic counter.
 //   warps 0-7   softmax: warp group w (four warps, 128 tensor-memory lanes) owns batch row w of the item; one thread per
-//               query row. The thread splits its row of Q and keeps it in tensor memory, where the first product reads
+//               query row. The warp's rows of Q and of the gate come by TMA into tiles of its own, from the latter of
+//               which the result leaves; the thread splits its row of Q and keeps it in tensor memory, where the first product reads
 //               it; per 32-key tile it reads 32 logits, adds mask and pair bias, forms P = exp(x - max), and writes the head
 //               of P over the logits and the tail beside them: the A operand of the second product. The logits are
 //               double-buffered, so the products of one tile run under the softmax of the other.
@@ -17,6 +18,8 @@
 // What bounds it: 24 MMA instructions per 32-key tile and warp group, about 55 clocks each at these widths (N = 32 and 48),
 // beside a softmax of two warps per scheduler (tensor memory holds no third warp group). The version on mma.sync split K
 // and V anew in every CTA and was bound by its shared-memory fragment loads: 269 -> 103 us at 128 x 256 rows, 8 heads.
+// Between two items the clocks of a CTA showed 11000, as many as its eight tiles took: rows of Q, gate and result read and written
+// by the threads they belong to, 32 lines an instruction. With TMA tiles, the next item's number and first operands early: -> 82 us.
 //
 // mbarrier conventions as in attn_tcgen05.cu: every barrier is awaited by each of its waiters once per completion, in order;
 // all waits are bounded and fall through to the common tail.
@@ -40,18 +43,17 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr int D = 32, BM = 128, BN = 32;        // head size, queries per item, keys per tile
 constexpr int MAXG = 2, NST = 3;
 constexpr int VT_ROWS = 48;                     // channels, the ones row, zero rows
-constexpr int K_BYTES = BN * 128, VT_BYTES = VT_ROWS * 128, NB_BYTES = BM * 128;    // one head or tail tile
+constexpr int K_BYTES = BN * 128, NB_BYTES = BM * 128;       // one head or tail tile of K
+constexpr int VT_HEAD = VT_ROWS * 128, VT_BYTES = VT_HEAD + D * 128;      // V^T: head tile, tail tile (channels only)
 constexpr int SOFTMAX_WARPS = 4 * MAXG, PRODUCER_WARP = SOFTMAX_WARPS, MASK_WARP = PRODUCER_WARP + 1, MMA_WARP = PRODUCER_WARP + 2;
 constexpr int THREADS = (SOFTMAX_WARPS + 4) * 32;
 constexpr int WG_COLS = 256, Q_COL = 0, S_COL = 64, O_COL = 192;     // tensor memory of a warp group; S of buffer b at + 64 b
-constexpr int OFF_STAGE = 1024;
+constexpr int ROWS_BYTES = 32 * 128;            // a warp's 32 rows of one head: Q, the gate, the result
 constexpr float kRescaleThreshold = 5.5f;       // P stays below 2^8
 
 struct F32Params {
-    const float *q, *gate;            // [B, S, H*D]
     const float *bias;                // [B, S] (row stride bias_stride0)
-    float *avg;                       // gated average [B, S, H*D], or [B, S, 2*H*D]: its tf32 head | tail
-    int avg_split;
+    int avg_split;                    // the result is [B, S, 2*H*D], tf32 heads | tails, instead of [B, S, H*D]
     int64_t bias_stride0;
     int *err;
     int S, H, B, G, n_qt, n_items;
@@ -75,16 +77,19 @@ __device__ __forceinline__ void tc_mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem,
 template <bool HAS_NB>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_vt,
-                   const __grid_constant__ CUtensorMap tm_nb, const F32Params p)
+                   const __grid_constant__ CUtensorMap tm_nb, const __grid_constant__ CUtensorMap tm_q,
+                   const __grid_constant__ CUtensorMap tm_gate, const __grid_constant__ CUtensorMap tm_avg, const F32Params p)
 {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *smem_gen = smem_raw + (smem - smem_u32(smem_raw));
     const int G = p.G;
     // stage: K heads x G, K tails x G, then per batch row V^T head and tail, pair bias, mask bias
-    const uint32_t off_vt = (uint32_t)(2 * G * K_BYTES), off_nb = off_vt + (uint32_t)(2 * G * VT_BYTES),
+    const uint32_t off_vt = (uint32_t)(2 * G * K_BYTES), off_nb = off_vt + (uint32_t)(G * VT_BYTES),
                    off_mb = off_nb + (HAS_NB ? NB_BYTES : 0), stage_bytes = off_mb + 1024;
-    auto stage_base = [&](int s) { return smem + OFF_STAGE + (uint32_t)s * stage_bytes; };
+    // before it the warps' tiles of Q and, later, of the gate and the result
+    const uint32_t off_stage = 1024u + (uint32_t)(2 * 4 * G * ROWS_BYTES);
+    auto stage_base = [&](int s) { return smem + off_stage + (uint32_t)s * stage_bytes; };
     const uint32_t bar = smem;
     auto kv_full = [&](int s) { return bar + 8u * (uint32_t)s; };
     auto kv_empty = [&](int s) { return bar + 8u * (uint32_t)(NST + s); };
@@ -92,7 +97,8 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     auto p_full = [&](int w, int b) { return bar + 8u * (uint32_t)(2 * NST + 2 * MAXG + 2 * w + b); };
     auto o_full = [&](int w) { return bar + 8u * (uint32_t)(2 * NST + 4 * MAXG + w); };
     auto q_full = [&](int w) { return bar + 8u * (uint32_t)(2 * NST + 5 * MAXG + w); };
-    const uint32_t it_base = bar + 8u * (2 * NST + 6 * MAXG);
+    auto rows_full = [&](int which, int softmax_warp) { return bar + 8u * (uint32_t)(2 * NST + 6 * MAXG + which * SOFTMAX_WARPS + softmax_warp); };
+    const uint32_t it_base = bar + 8u * (2 * NST + 6 * MAXG + 2 * SOFTMAX_WARPS);
     auto it_full = [&](int i) { return it_base + 8u * (uint32_t)(i & 3); };
     const uint32_t item_ring = it_base + 32u, tmem_slot = it_base + 48u;
 
@@ -124,15 +130,16 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             mbar_init(o_full(w), 1);
             mbar_init(q_full(w), 4);
         }
+        for (int i = 0; i < 2 * SOFTMAX_WARPS; ++i) mbar_init(rows_full(0, i), 1);       // Q, gate
         for (int i = 0; i < 4; ++i) mbar_init(it_full(i), 1);
         fence_barrier_init();
     }
-    // static rows 32..47 of every V^T tile: row 32 of a head tile = 1.0, everything else = 0
-    for (int i = threadIdx.x; i < NST * 2 * G * 128; i += THREADS) {
+    // static rows 32..47 of every head tile of V^T: row 32 = 1.0, the others = 0
+    for (int i = threadIdx.x; i < NST * G * 128; i += THREADS) {
         const int t = i / 128, rem = i % 128, row = 32 + rem / 8, ch = rem % 8;
-        const float v = row == 32 && (t & 1) == 0 ? 1.0f : 0.0f;
-        *reinterpret_cast<float4 *>(smem_gen + OFF_STAGE + (t / (2 * G)) * stage_bytes + off_vt + (t % (2 * G)) * VT_BYTES +
-                                    row * 128 + ch * 16) = make_float4(v, v, v, v);
+        const float v = row == 32 ? 1.0f : 0.0f;
+        *reinterpret_cast<float4 *>(smem_gen + off_stage + (t / G) * stage_bytes + off_vt + (t % G) * VT_BYTES + row * 128 + ch * 16) =
+            make_float4(v, v, v, v);
     }
     fence_proxy_async();
     if (warp == MMA_WARP) {
@@ -151,9 +158,7 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     if (warp == PRODUCER_WARP) {
         // ================= producer =================
         const uint32_t tx = (uint32_t)(2 * G * (K_BYTES + D * 128) + (HAS_NB ? NB_BYTES : 0));
-        int g = 0;
-        bool ok = true;
-        for (int i = 0; ok; ++i) {
+        auto take = [&](int i) -> int {                                // as in attn_tcgen05.cu
             int w = 0;
             if (lane == 0) {
                 w = atomicAdd(p.counter, 1);
@@ -161,9 +166,20 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(item_ring + 4u * (uint32_t)(i & 3)), "r"(w) : "memory");
                 mbar_arrive(it_full(i));
             }
-            w = __shfl_sync(0xffffffffu, w, 0);
-            if (w < 0) break;
-            int q0, h, b0;
+            return __shfl_sync(0xffffffffu, w, 0);
+        };
+        auto prefetch_tile = [&](int kt, int q0, int h, int b0) {      // into L2, by the elected lane
+            const int k0 = kt * BN;
+            for (int t = 0; t < 2; ++t) tma_prefetch_4d(&tm_k, t * D, k0, h, b0);
+            for (int r = 0; r < G; ++r)
+                for (int t = 0; t < 2; ++t) tma_prefetch_4d(&tm_vt, k0, t * D, h, b0 + r);
+            if (HAS_NB) tma_prefetch_3d(&tm_nb, k0, q0, h);
+        };
+        int g = 0;
+        bool ok = true;
+        int w = take(0);
+        for (int i = 0; ok && w >= 0; ++i) {
+            int q0, h, b0, next = -1;
             decode(w, q0, h, b0);
             for (int kt = 0; kt < nkt; ++kt, ++g) {
                 const int s = g % NST;
@@ -178,13 +194,25 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                     tma_load_4d(st, &tm_k, kv_full(s), 0, k0, h, b0);
                     tma_load_4d(st + G * K_BYTES, &tm_k, kv_full(s), D, k0, h, b0);
                     for (int r = 0; r < G; ++r) {
-                        tma_load_4d(st + off_vt + 2 * r * VT_BYTES, &tm_vt, kv_full(s), k0, 0, h, b0 + r);
-                        tma_load_4d(st + off_vt + (2 * r + 1) * VT_BYTES, &tm_vt, kv_full(s), k0, D, h, b0 + r);
+                        tma_load_4d(st + off_vt + r * VT_BYTES, &tm_vt, kv_full(s), k0, 0, h, b0 + r);
+                        tma_load_4d(st + off_vt + r * VT_BYTES + VT_HEAD, &tm_vt, kv_full(s), k0, D, h, b0 + r);
                     }
                     if (HAS_NB) tma_load_3d(st + off_nb, &tm_nb, kv_full(s), k0, q0, h);
                 }
                 __syncwarp();
+                // the next item's number early, and its first operands on their way to L2
+                if (kt == max(nkt - 2, 0)) {
+                    next = take(i + 1);
+                    if (next >= 0) {
+                        int q1, h1, b1;
+                        decode(next, q1, h1, b1);
+                        if (elect_one())
+                            for (int t = 0; t < min(nkt, 2); ++t) prefetch_tile(t, q1, h1, b1);
+                        __syncwarp();
+                    }
+                }
             }
+            w = next;
         }
     } else if (warp == MASK_WARP) {
         // ================= mask bias =================
@@ -219,8 +247,8 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         constexpr uint32_t idesc_s = make_instr_desc_tf32(BM, BN), idesc_o = make_instr_desc_tf32(BM, VT_ROWS);
         const uint32_t t0 = tmem_base + (uint32_t)(w * WG_COLS);
         const uint64_t kd0 = make_smem_desc_kmajor(stage_base(0) + w * K_BYTES, 128),
-                       vd0 = make_smem_desc_kmajor(stage_base(0) + off_vt + 2 * w * VT_BYTES, 128);
-        const uint32_t k_tail = (uint32_t)(G * K_BYTES) >> 4, v_tail = VT_BYTES >> 4;
+                       vd0 = make_smem_desc_kmajor(stage_base(0) + off_vt + w * VT_BYTES, 128);
+        const uint32_t k_tail = (uint32_t)(G * K_BYTES) >> 4, v_tail = VT_HEAD >> 4;
         // S = Q . K^T of global tile g: tail.head + head.tail + head.head (k steps of 8 elements = 32 bytes, 8 columns)
         auto issue_qk = [&](int g) {
             const uint64_t kd = kd0 + (uint32_t)((g % NST) * (int)(stage_bytes >> 4));
@@ -258,7 +286,7 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                     for (int pr = 0; pr < 3; ++pr)
 #pragma unroll
                         for (int k = 0; k < BN / 8; ++k)
-                            tc_mma_tf32_ts(t0 + O_COL, a + (pr == 0 ? BN : 0) + k * 8, vd + (pr == 1 ? v_tail : 0u) + 2 * k, idesc_o,
+                            tc_mma_tf32_ts(t0 + O_COL, a + (pr == 0 ? BN : 0) + k * 8, vd + (pr == 1 ? v_tail : 0u) + 2 * k, pr == 1 ? idesc_s : idesc_o,
                                            (kt > 0 || pr > 0 || k > 0) ? 1u : 0u);
                     tc_commit(kv_empty(g % NST));
                     if (kt == nkt - 1) tc_commit(o_full(w));
@@ -281,10 +309,15 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         float m = 0.f;                                   // running (possibly stale) max of x
         bool ok = true;
 
-        auto do_tile = [&](const int g, const int kt) -> bool {
+        // a warp whose 32 rows all lie past the item's end only passes on the barriers
+        auto do_tile = [&](const int g, const int kt, const bool idle) -> bool {
             const uint32_t st = stage_base(g % NST);
             const uint32_t t_s = t_w + S_COL + (uint32_t)(g & 1) * 64;
             if (!mbar_wait_warp(s_full(wg, g & 1), (uint32_t)((g >> 1) & 1), p.err, 79)) return false;
+            if (idle) {
+                if (lane == 0) mbar_arrive(p_full(wg, g & 1));
+                return true;
+            }
             tc_fence_after();
             float pv[32];
             float tmax;
@@ -356,34 +389,54 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             return true;
         };
 
-        // this thread's row of Q of item w, kept in registers until the products with the previous Q have all been formed
-        float qreg[32];
-        auto fetch_q = [&](int w) {
+        // This warp's rows of Q and of the gate come by TMA into its two tiles; the result leaves from the gate's. (Read row by row
+        // by the threads they came to, with 32 lines an instruction, they were half of the kernel's time at 256 keys.)
+        const uint32_t q_rows = smem + 1024u + (uint32_t)(warp * 2 * ROWS_BYTES), g_rows = q_rows + ROWS_BYTES;
+        auto load_rows = [&](const CUtensorMap *map, int which, int w) {
             int q0, h, b0;
             decode(w, q0, h, b0);
-            const int qi = q0 + row, bb = b0 + wg;
-            const bool live = qi < S && bb < p.B;
-            const float4 *src = reinterpret_cast<const float4 *>(p.q + (live ? ((int64_t)bb * S + qi) * C + h * D : 0));
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float4 v = live ? __ldg(src + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-                qreg[4 * c] = v.x;
-                qreg[4 * c + 1] = v.y;
-                qreg[4 * c + 2] = v.z;
-                qreg[4 * c + 3] = v.w;
+            if (lane == 0) {
+                if (which == 1) tma_store_wait_read<0>();
+                mbar_arrive_expect_tx(rows_full(which, warp), ROWS_BYTES);
+                tma_load_3d(which == 0 ? q_rows : g_rows, map, rows_full(which, warp), h * D, q0 + quad * 32, b0 + wg);
             }
+            __syncwarp();
         };
-        auto publish_q = [&]() {
-            uint32_t hi[32], lo[32];
+        uint32_t loads[2] = {0, 0}, waits[2] = {0, 0};                // tiles of Q and of the gate
+        auto row_chunk = [&](uint32_t rows, int c) { return rows + (uint32_t)(lane * 128 + ((c ^ (lane & 7)) << 4)); };
+        auto idle_in = [&](int w) {
+            int q0, h, b0;
+            decode(w, q0, h, b0);
+            return q0 + quad * 32 >= S || b0 + wg >= p.B;
+        };
+        auto fetch_q = [&](int w) {
+            if (idle_in(w)) return;
+            load_rows(&tm_q, 0, w);
+            ++loads[0];
+        };
+        // split into tensor memory, once the products with the previous Q have all been formed
+        auto publish_q = [&](const bool idle) {
+            if (!idle) {
+                if (!mbar_wait_warp(rows_full(0, warp), waits[0]++ & 1u, p.err, 84)) {
+                    ok = false;
+                    return;
+                }
+                uint32_t hi[32], lo[32];
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                const float h = tf32_head(qreg[e]);
-                hi[e] = __float_as_uint(h);
-                lo[e] = __float_as_uint(qreg[e] - h);
+                for (int c = 0; c < 8; ++c) {
+                    const float4 v = lds128_f32(row_chunk(q_rows, c));
+                    const float q4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float h = tf32_head(q4[e]);
+                        hi[4 * c + e] = __float_as_uint(h);
+                        lo[4 * c + e] = __float_as_uint(q4[e] - h);
+                    }
+                }
+                tmem_st_32x32(t_w + Q_COL, hi);
+                tmem_st_32x32(t_w + Q_COL + D, lo);
+                tmem_st_wait();
             }
-            tmem_st_32x32(t_w + Q_COL, hi);
-            tmem_st_32x32(t_w + Q_COL + D, lo);
-            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(q_full(wg));
@@ -393,63 +446,77 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         int w = item_of(0, 81);
         if (w >= 0) {
             fetch_q(w);
-            publish_q();
+            publish_q(idle_in(w));
         }
         for (int i = 0; w >= 0; ++i) {
             int q0, h, b0, nxt = -1;
             decode(w, q0, h, b0);
+            const bool idle = idle_in(w);
+            if (!idle) {
+                load_rows(&tm_gate, 1, w);
+                ++loads[1];
+            }
             for (int kt = 0; kt < nkt && ok; ++kt, ++g) {
-                if (kt == nkt - 1) {
+                if (kt == max(nkt - 2, 0)) {
                     nxt = item_of(i + 1, 82);
                     ok = nxt != -2;
                     if (nxt >= 0) fetch_q(nxt);
                 }
-                ok = ok && do_tile(g, kt);
+                ok = ok && do_tile(g, kt, idle);
             }
             if (!ok) break;
             // every product with this Q has been formed (the logits of its last tile have been read)
-            if (nxt >= 0) publish_q();
+            if (nxt >= 0) publish_q(idle_in(nxt));
+            if (!ok) break;
 
             // ---- item epilogue: one row of 32 channels per thread ----
-            const int qi = q0 + row, bb = b0 + wg;
-            const bool live = qi < S && bb < p.B;
-            const int64_t m_row = live ? (int64_t)bb * S + qi : 0;
-            // all of the gate row is in flight while the last product retires
-            const float4 *gp = reinterpret_cast<const float4 *>(p.gate + m_row * C + h * D);
-            float gate[32];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const float4 v = __ldg(gp + c);
-                gate[4 * c] = v.x;
-                gate[4 * c + 1] = v.y;
-                gate[4 * c + 2] = v.z;
-                gate[4 * c + 3] = v.w;
-            }
             if (!mbar_wait_warp(o_full(wg), (uint32_t)(i & 1), p.err, 83)) break;
+            w = nxt;
+            if (idle) continue;
             tc_fence_after();
             uint32_t o[32];
             tmem_ld_32x32(t_o, o);
             const uint32_t osum = tmem_ld_32x1(t_o + D);
             tmem_ld_wait();
             const float inv = 1.0f / __uint_as_float(osum);
-            if (live) {
-                float *dst = p.avg + m_row * (p.avg_split ? 2 * C : C) + h * D;
+            ok = mbar_wait_warp(rows_full(1, warp), waits[1]++ & 1u, p.err, 85);
+            if (!ok) break;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const float4 gv = lds128_f32(row_chunk(g_rows, c));
+                const float gate[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)      // sigmoid with the hardware reciprocal (2 ulp)
+                    o[4 * c + e] = __float_as_uint(__uint_as_float(o[4 * c + e]) * inv * __fdividef(1.0f, 1.0f + __expf(-gate[e])));
+            }
+            // the result, or its tf32 heads and then, with the same tile, its tails
+            for (int t = 0; t < (p.avg_split ? 2 : 1); ++t) {
+                if (t == 1) {
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                }
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    float av[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)      // sigmoid with the hardware reciprocal (2 ulp)
-                        av[e] = __uint_as_float(o[4 * c + e]) * inv * __fdividef(1.0f, 1.0f + __expf(-gate[4 * c + e]));
-                    float4 hv = make_float4(av[0], av[1], av[2], av[3]);
+                    float4 v = make_float4(__uint_as_float(o[4 * c]), __uint_as_float(o[4 * c + 1]), __uint_as_float(o[4 * c + 2]),
+                                           __uint_as_float(o[4 * c + 3]));
                     if (p.avg_split) {
-                        hv = make_float4(tf32_head(av[0]), tf32_head(av[1]), tf32_head(av[2]), tf32_head(av[3]));
-                        *reinterpret_cast<float4 *>(dst + C + 4 * c) = make_float4(av[0] - hv.x, av[1] - hv.y, av[2] - hv.z, av[3] - hv.w);
+                        const float4 hv = make_float4(tf32_head(v.x), tf32_head(v.y), tf32_head(v.z), tf32_head(v.w));
+                        v = t == 0 ? hv : make_float4(v.x - hv.x, v.y - hv.y, v.z - hv.z, v.w - hv.w);
                     }
-                    *reinterpret_cast<float4 *>(dst + 4 * c) = hv;
+                    asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(row_chunk(g_rows, c)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {                 // rows past S are clipped
+                    tma_store_3d(&tm_avg, g_rows, h * D + t * C, q0 + quad * 32, b0 + wg);
+                    tma_store_commit();
                 }
             }
-            w = nxt;
         }
+        // after a wait that ran out: no copy may still be on its way when the CTA exits
+        for (int t = 0; t < 2; ++t)
+            if (loads[t] != waits[t]) mbar_wait_warp(rows_full(t, warp), waits[t] & 1u, p.err, 86);
+        if (lane == 0) tma_store_wait<0>();
     }
 
     // ================= common tail =================
@@ -472,7 +539,7 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
 int smem_bytes(int G, bool has_nb)
 {
-    return OFF_STAGE + 1024 + NST * (2 * G * (K_BYTES + VT_BYTES) + (has_nb ? NB_BYTES : 0) + 1024);
+    return 1024 + 1024 + 2 * 4 * G * ROWS_BYTES + NST * (G * (2 * K_BYTES + VT_BYTES) + (has_nb ? NB_BYTES : 0) + 1024);
 }
 
 }  // namespace
@@ -491,10 +558,7 @@ bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, c
     if (ew.device == nullptr || counter == nullptr) return false;
     const int sms = std::max(1, sm_count() - runtime().sm_margin);
     F32Params p;
-    p.q = (const float *)q;
-    p.gate = (const float *)gate;
     p.bias = (const float *)bias;
-    p.avg = (float *)avg;
     p.avg_split = avg_split;
     p.bias_stride0 = bias_stride0;
     p.err = ew.device;
@@ -507,7 +571,12 @@ bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, c
     p.counter = counter;
     p.scale = scale;
     const uint64_t Su = (uint64_t)S, Hu = (uint64_t)H, vp = (uint64_t)vt_pitch;
-    CUtensorMap tk, tvt, tnb;
+    CUtensorMap tk, tvt, tnb, tq, tg, ta;
+    const uint64_t Cu = Hu * D, ca = avg_split ? 2 * Cu : Cu;
+    if (!make_tensor_map_f32_3d(&tq, q, Cu, Su, (uint64_t)B, Cu, Su * Cu, D, 32, 128) ||
+        !make_tensor_map_f32_3d(&tg, gate, Cu, Su, (uint64_t)B, Cu, Su * Cu, D, 32, 128) ||
+        !make_tensor_map_f32_3d(&ta, avg, ca, Su, (uint64_t)B, ca, Su * ca, D, 32, 128))
+        return false;
     if (!make_tensor_map_f32_4d(&tk, k_split, 2 * D, Su, Hu, (uint64_t)B, 2 * D * Hu, 2 * D, Su * 2 * D * Hu, D, BN,
                                 (uint32_t)p.G, 128) ||
         !make_tensor_map_f32_4d(&tvt, vt_split, Su, 2 * D, Hu, (uint64_t)B, vp, 2 * D * vp, 2 * D * vp * Hu, BN, D, 1, 128))
@@ -523,9 +592,9 @@ bool tcgen05_attn_f32(cudaStream_t stream, const void *q, const void *k_split, c
     const unsigned grid = (unsigned)std::min(p.n_items, sms);
     KernelTimer timer__("attn_f32_tc", stream);
     if (nb)
-        launch_chained(attn_f32_tc_kernel<true>, grid, THREADS, smem_bytes(p.G, true), stream, tk, tvt, tnb, p);
+        launch_chained(attn_f32_tc_kernel<true>, grid, THREADS, smem_bytes(p.G, true), stream, tk, tvt, tnb, tq, tg, ta, p);
     else
-        launch_chained(attn_f32_tc_kernel<false>, grid, THREADS, smem_bytes(p.G, false), stream, tk, tvt, tnb, p);
+        launch_chained(attn_f32_tc_kernel<false>, grid, THREADS, smem_bytes(p.G, false), stream, tk, tvt, tnb, tq, tg, ta, p);
     count_launch();
     return true;
 }

@@ -16,7 +16,7 @@
 // Two row tiles share every weight slab: the weights stream from L2 once per 256 rows (302 MB instead of 604 MB at 147456
 // rows x 128 channels). Bound by the chain product, conversion, product and by the operands' way through shared memory (tensor
 // pipe 40 % busy) where the two-kernel version was bound by the round trip of the hidden tensor (302 MB through L2 and HBM):
-// 90 -> 44 us there, 0.88 PFLOP/s.
+// 90 -> 42 us there, 0.92 PFLOP/s.
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is released
 // and the host-visible error word carries the site.
@@ -35,13 +35,13 @@ namespace dev {
 namespace {
 
 constexpr int BM = 128, BH = 128, BK = 64;      // rows of a tile, hidden channels of a chunk, k columns of a slab
-constexpr int NSLAB = 7;
+constexpr int RING_SLABS = 7;
 constexpr int SLAB_BYTES = 128 * BK * 2;
 constexpr int X_BYTES = 4 * SLAB_BYTES;         // two tiles of 128 channels or one of 256
 constexpr int STG_TILE = 128 * 64;              // output staging, 128 rows x 32 channels per group
 constexpr int STG_BYTES = 4 * STG_TILE;
 constexpr int MAX_HIDDEN = 2048;
-constexpr int OFF_RING = X_BYTES, OFF_STG = OFF_RING + NSLAB * SLAB_BYTES, OFF_BAR = OFF_STG + STG_BYTES;
+constexpr int OFF_RING = X_BYTES, OFF_STG = OFF_RING + RING_SLABS * SLAB_BYTES, OFF_BAR = OFF_STG + STG_BYTES;
 constexpr int OFF_BIAS = OFF_BAR + 256;
 constexpr int SMEM_BYTES = OFF_BIAS + (MAX_HIDDEN + 256) * 4 + 1024;
 constexpr int THREADS = 20 * 32;
@@ -70,6 +70,10 @@ __global__ void __launch_bounds__(THREADS, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w1,
                   const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_out, const MlpParams p)
 {
+    // The weight ring counts in units of SPU slabs. With 128 channels a chunk of W1 or W2 is two slabs that come and go together: half
+    // the waits and commits on the issuing warp's path (160000 rows x 512 hidden: 56.3 -> 52.3 us). With 256 channels it is four, and
+    // a ring that moves in twos is too short for them (160000 rows x 1024: 189 us by single slabs, 196 in twos).
+    constexpr int SPU = CO == 128 ? 2 : 1, NUNIT = RING_SLABS / SPU;
     constexpr int KX = CO / BK;                 // slabs of an x tile, and of a chunk of W1
     constexpr int NO = CO / 128;                // 128-row blocks of W2
     extern __shared__ unsigned char smem_raw[];
@@ -77,13 +81,13 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     unsigned char *smem_gen = smem_raw + (smem - smem_u32(smem_raw));
     const uint32_t bar = smem + OFF_BAR;
     auto w_full = [&](int s) { return bar + 8u * (uint32_t)s; };
-    auto w_empty = [&](int s) { return bar + 8u * (uint32_t)(NSLAB + s); };
-    auto x_full = [&](int r) { return bar + 8u * (uint32_t)(2 * NSLAB + r); };
-    auto x_empty = [&](int r) { return bar + 8u * (uint32_t)(2 * NSLAB + 2 + r); };
-    auto s_full = [&](int c) { return bar + 8u * (uint32_t)(2 * NSLAB + 4 + c); };
-    auto p_full = [&](int c) { return bar + 8u * (uint32_t)(2 * NSLAB + 6 + c); };
-    auto o_full = [&](int r) { return bar + 8u * (uint32_t)(2 * NSLAB + 8 + r); };
-    const uint32_t o_free = bar + 8u * (2 * NSLAB + 10), tmem_slot = o_free + 8;
+    auto w_empty = [&](int s) { return bar + 8u * (uint32_t)(NUNIT + s); };
+    auto x_full = [&](int r) { return bar + 8u * (uint32_t)(2 * NUNIT + r); };
+    auto x_empty = [&](int r) { return bar + 8u * (uint32_t)(2 * NUNIT + 2 + r); };
+    auto s_full = [&](int c) { return bar + 8u * (uint32_t)(2 * NUNIT + 4 + c); };
+    auto p_full = [&](int c) { return bar + 8u * (uint32_t)(2 * NUNIT + 6 + c); };
+    auto o_full = [&](int r) { return bar + 8u * (uint32_t)(2 * NUNIT + 8 + r); };
+    const uint32_t o_free = bar + 8u * (2 * NUNIT + 10), tmem_slot = o_free + 8;
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int R = CO == 128 ? p.tiles : 1;
@@ -93,7 +97,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     float *bias1 = reinterpret_cast<float *>(smem_gen + OFF_BIAS), *bias2 = bias1 + MAX_HIDDEN;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NSLAB; ++s) {
+        for (int s = 0; s < NUNIT; ++s) {
             mbar_init(w_full(s), 1);
             mbar_init(w_empty(s), 1);
         }
@@ -132,15 +136,23 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     if (warp == 0) {
         // ================= producer =================
         if (elect_one()) {
-            int it = 0;
+            int s = 0, round = 0;                                  // next unit's slot, times the ring has gone round
             bool ok = true;
+            int filled = 0;                                        // slabs of the unit that have been asked for
             auto slab = [&](const CUtensorMap *map, int c0, int c1) {
-                const int s = it % NSLAB;
-                if (it >= NSLAB && ok) ok = mbar_wait(w_empty(s), (uint32_t)((it / NSLAB - 1) & 1), p.err, 61);
+                if (filled == 0) {
+                    if (round > 0 && ok) ok = mbar_wait(w_empty(s), (uint32_t)((round - 1) & 1), p.err, 61);
+                    if (!ok) return;
+                    mbar_arrive_expect_tx(w_full(s), SPU * SLAB_BYTES);
+                }
                 if (!ok) return;
-                mbar_arrive_expect_tx(w_full(s), SLAB_BYTES);
-                tma_load_3d(smem + OFF_RING + s * SLAB_BYTES, map, w_full(s), c0, c1, 0);
-                ++it;
+                tma_load_3d(smem + OFF_RING + (s * SPU + filled) * SLAB_BYTES, map, w_full(s), c0, c1, 0);
+                if (++filled < SPU) return;
+                filled = 0;
+                if (++s == NUNIT) {
+                    s = 0;
+                    ++round;
+                }
             };
             auto load_w1 = [&](int j) {
                 for (int k = 0; k < KX; ++k) slab(&tm_w1, k * BK, j * BH);
@@ -189,60 +201,77 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         constexpr uint32_t idesc_h = make_instr_desc_bf16(BM, BH);
         constexpr uint32_t SLAB16 = SLAB_BYTES >> 4;               // descriptor addresses count in units of 16 bytes
         const uint64_t xd = make_smem_desc_kmajor(smem, 128), wd = make_smem_desc_kmajor(smem + OFF_RING, 128);
-        int it = 0;                                                // slabs taken so far
         bool ok = true;
-        auto wait_slabs = [&](int first, int n) {
-            for (int i = first; i < first + n && ok; ++i)
-                ok = mbar_wait_warp(w_full(i % NSLAB), (uint32_t)((i / NSLAB) & 1), p.err, 63);
+        // place of a unit in the ring; its barrier's parity
+        struct Pos {
+            int s;
+            uint32_t par;
         };
-        auto free_slabs = [&](int first, int n) {                  // by the elected lane
-            for (int i = first; i < first + n; ++i) tc_commit(w_empty(i % NSLAB));
+        auto advance = [](Pos q, int n) {
+            q.s += n;
+            if (q.s >= NUNIT) {
+                q.s -= NUNIT;
+                q.par ^= 1u;
+            }
+            return q;
         };
-        // S_c = x_r . W1_chunk^T with the slabs from `first` on
-        auto mma1 = [&](int c, int r, int first) {
+        Pos it = {0, 0};
+        auto wait_units = [&](Pos q, int n) {
+            for (int i = 0; i < n && ok; ++i, q = advance(q, 1)) ok = mbar_wait_warp(w_full(q.s), q.par, p.err, 63);
+        };
+        auto free_units = [&](Pos q, int n) {                      // by the elected lane
+            for (int i = 0; i < n; ++i, q = advance(q, 1)) tc_commit(w_empty(q.s));
+        };
+        // descriptor of the i-th slab from the unit `q` on
+        auto slab_desc = [&](Pos q, int i) {
+            q = advance(q, i / SPU);
+            return wd + (uint32_t)((q.s * SPU + i % SPU) * SLAB16);
+        };
+        // S_c = x_r . W1_chunk^T with the units from `q` on
+        auto mma1 = [&](int c, int r, Pos q) {
 #pragma unroll
             for (int k = 0; k < KX; ++k) {
-                const uint64_t a = xd + (uint32_t)((r * KX + k) * SLAB16), b = wd + (uint32_t)(((first + k) % NSLAB) * SLAB16);
+                const uint64_t a = xd + (uint32_t)((r * KX + k) * SLAB16), b = slab_desc(q, k);
 #pragma unroll
-                for (int q = 0; q < BK / 16; ++q)
-                    tc_mma_bf16(tmem_base + S_COL + c * BH, a + 2 * q, b + 2 * q, idesc_h, (k > 0 || q > 0) ? 1u : 0u);
+                for (int e = 0; e < BK / 16; ++e)
+                    tc_mma_bf16(tmem_base + S_COL + c * BH, a + 2 * e, b + 2 * e, idesc_h, (k > 0 || e > 0) ? 1u : 0u);
             }
             tc_commit(s_full(c));
         };
         // O_r += P_c . W2_chunk^T
-        auto mma2 = [&](int c, int r, int first, bool fresh) {
+        auto mma2 = [&](int c, int r, Pos q, bool fresh) {
 #pragma unroll
             for (int k = 0; k < BH / BK; ++k)
 #pragma unroll
                 for (int o = 0; o < NO; ++o) {
-                    const uint64_t b = wd + (uint32_t)(((first + k * NO + o) % NSLAB) * SLAB16);
+                    const uint64_t b = slab_desc(q, k * NO + o);
 #pragma unroll
-                    for (int q = 0; q < BK / 16; ++q)
-                        tc_mma_bf16_ts(tmem_base + O_COL + (r * NO + o) * 128, tmem_base + S_COL + c * BH + k * 64 + q * 8, b + 2 * q,
-                                       idesc_h, (!fresh || k > 0 || q > 0) ? 1u : 0u);
+                    for (int e = 0; e < BK / 16; ++e)
+                        tc_mma_bf16_ts(tmem_base + O_COL + (r * NO + o) * 128, tmem_base + S_COL + c * BH + k * 64 + e * 8, b + 2 * e,
+                                       idesc_h, (!fresh || k > 0 || e > 0) ? 1u : 0u);
                 }
         };
         const int total = mine * nch;
-        constexpr int W1N = KX, W2N = BH / BK * NO;
+        constexpr int W1N = KX / SPU, W2N = BH / BK * NO / SPU;
         if constexpr (CO == 128) {
             if (total > 0) {
                 for (int r = 0; r < R && ok; ++r) ok = mbar_wait_warp(x_full(r), 0, p.err, 64);
-                wait_slabs(0, W1N);
+                wait_units(it, W1N);
                 tc_fence_after();
                 if (ok && elect_one()) {
                     for (int r = 0; r < R; ++r) {
-                        mma1(r, r, 0);
+                        mma1(r, r, it);
                         if (nch == 1) tc_commit(x_empty(r));
                     }
-                    free_slabs(0, W1N);
+                    free_units(it, W1N);
                 }
                 __syncwarp();
-                it = W1N;
+                it = advance(it, W1N);
             }
             for (int c = 0; c < total && ok; ++c) {
                 const int j = c % nch, n = c + 1;                  // chunk c with its W2, then chunk n with its W1
                 const bool more = n < total;
-                wait_slabs(it, W2N);
+                wait_units(it, W2N);
                 for (int r = 0; r < R && ok; ++r) {
                     ok = ok && mbar_wait_warp(p_full(r), (uint32_t)(c & 1), p.err, 65);
                     if (!ok) break;
@@ -250,40 +279,41 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                     if (elect_one()) {
                         mma2(r, r, it, j == 0);
                         if (j == nch - 1) tc_commit(o_full(r));
-                        if (r == R - 1) free_slabs(it, W2N);
+                        if (r == R - 1) free_units(it, W2N);
                     }
                     __syncwarp();
                     if (!more) continue;
-                    if (r == 0) wait_slabs(it + W2N, W1N);
+                    if (r == 0) wait_units(advance(it, W2N), W1N);
                     if (n % nch == 0) ok = ok && mbar_wait_warp(x_full(r), (uint32_t)((n / nch) & 1), p.err, 64);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        mma1(r, r, it + W2N);                      // overwrites P: the products run in the order of issue
+                        mma1(r, r, advance(it, W2N));                      // overwrites P: the products run in the order of issue
                         if (n % nch == nch - 1) tc_commit(x_empty(r));
-                        if (r == R - 1) free_slabs(it + W2N, W1N);
+                        if (r == R - 1) free_units(advance(it, W2N), W1N);
                     }
                     __syncwarp();
                 }
-                it += W2N + (more ? W1N : 0);
+                it = advance(it, W2N);
+                if (more) it = advance(it, W1N);
             }
         } else {
-            auto first_product = [&](int n, int first) {           // chunk n into chain n & 1
-                wait_slabs(first, W1N);
+            auto first_product = [&](int n, Pos first) {           // chunk n into chain n & 1
+                wait_units(first, W1N);
                 if (ok && n % nch == 0) ok = mbar_wait_warp(x_full(0), (uint32_t)((n / nch) & 1), p.err, 64);
                 if (!ok) return;
                 tc_fence_after();
                 if (elect_one()) {
                     mma1(n & 1, 0, first);
                     if (n % nch == nch - 1) tc_commit(x_empty(0));
-                    free_slabs(first, W1N);
+                    free_units(first, W1N);
                 }
                 __syncwarp();
             };
-            for (int n = 0; n < 2 && n < total && ok; ++n, it += W1N) first_product(n, it);
+            for (int n = 0; n < 2 && n < total && ok; ++n, it = advance(it, W1N)) first_product(n, it);
             for (int c = 0; c < total && ok; ++c) {
                 const int j = c % nch, t = c / nch;
-                wait_slabs(it, W2N);
+                wait_units(it, W2N);
                 // the first product into O of a tile: both groups have read the tile before
                 if (ok && j == 0 && t > 0) ok = mbar_wait_warp(o_free, (uint32_t)((t - 1) & 1), p.err, 66);
                 ok = ok && mbar_wait_warp(p_full(c & 1), (uint32_t)((c >> 1) & 1), p.err, 65);
@@ -292,13 +322,13 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 if (elect_one()) {
                     mma2(c & 1, 0, it, j == 0);
                     if (j == nch - 1) tc_commit(o_full(0));
-                    free_slabs(it, W2N);
+                    free_units(it, W2N);
                 }
                 __syncwarp();
-                it += W2N;
+                it = advance(it, W2N);
                 if (c + 2 < total) {
                     first_product(c + 2, it);
-                    it += W1N;
+                    it = advance(it, W1N);
                 }
             }
         }

@@ -15,13 +15,13 @@
 // The activations stand still, as in gemm_proj.cu: a persistent CTA (one per SM) loads 128 rows, all K columns, as fp32; the
 // epilogue warps split them where they lie (the head and tail of a row take just the bytes of its fp32 values), and the
 // weights, split by a kernel of their own (a row of them is used by every CTA), stream past in slabs of 128 channels x 64 columns.
-//   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (head and tail, a ring of two stages)
-//   warp 1      MMA issuer: 12 instructions a stage into a pair of 128 x 128 accumulators (two pairs in tensor memory)
+//   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (tail and head in turn, a ring of five or eight)
+//   warp 1      MMA issuer: 12 instructions a tail and head into a pair of 128 x 128 accumulators (two pairs in tensor memory)
 //   warps 4-11  split the rows, 16 each; epilogue, 32 rows x 64 columns each: tcgen05.ld of both accumulators, scaling, bias,
-//               staging tile (32 x 32), TMA store
+//               staging tile (32 x 16), TMA store
 // What bounds it: the products (128 x 128 instructions, each weight slab used for one block of rows) and, twice per CTA at the size
 // below, the way of a block into shared memory and its split, which nothing overlaps. 32768 rows x 256 channels, four projections:
-// 81 us (HBM 31, products 31); as a split of the activations and tf32 products 20 + 92. Error against 64 bits at K = 128 and 256
+// 80 us (HBM 31, products 31); as a split of the activations and tf32 products 20 + 92. Error against 64 bits at K = 128 and 256
 // (2-norm): 2.0e-7 and 3.5e-7, before 3.4e-7 and 6.4e-7. The fp32 layer of 128 x 256 rows: 288 -> 227 us.
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is
@@ -45,18 +45,18 @@ namespace {
 
 constexpr int BM = 128, BN = 128;
 constexpr int SLAB_BYTES = 128 * 128;                   // 128 rows (or channels) x 32 fp32 or 64 fp16 columns
-constexpr int NW = 2;                                   // weight ring; a stage is a head and a tail slab
 constexpr int EPI_WARPS = 8, EPI_WARP0 = 4;
 constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
-constexpr int STG_BYTES = 32 * 32 * 4;
+constexpr int STG_BYTES = 32 * 16 * 4;
 constexpr float kTail = 1.0f / 2048;                    // weight of the small products
 
 // KS: 64-column slabs of a row
 template <int KS>
 struct Geo {
-    static constexpr int OFF_A = NW * 2 * SLAB_BYTES;
+    static constexpr int NW = KS == 4 ? 4 : 8;                                   // slabs of the weight ring
+    static constexpr int OFF_A = NW * SLAB_BYTES;
     static constexpr int OFF_STG = OFF_A + 2 * KS * SLAB_BYTES;
-    static constexpr int OFF_SCALE = OFF_STG + EPI_WARPS * STG_BYTES;            // of the rows of two blocks
+    static constexpr int OFF_SCALE = OFF_STG + EPI_WARPS * 2 * STG_BYTES;            // of the rows of two blocks
     static constexpr int OFF_BAR = OFF_SCALE + 2 * BM * 4;
     static constexpr int NBARS = 2 * NW + 2 * KS + 5;
     static constexpr int SMEM_BYTES = OFF_BAR + 8 * NBARS + 16 + 1024;
@@ -66,7 +66,7 @@ struct Geo {
 struct alignas(64) RowsMaps {
     CUtensorMap a;        // A [M][K] fp32, box [32, 128], 128-byte swizzle
     CUtensorMap w[4];     // W' [N][2K] fp16 (head | tail) per segment, box [64, 128], 128-byte swizzle
-    CUtensorMap out[4];   // per segment [M][N] (split rows: [M][2N]) fp32, box [32, 32], 128-byte swizzle
+    CUtensorMap out[4];   // per segment [M][N] (split rows: [M][2N]) fp32, box [16, 32], 64-byte swizzle
 };
 
 struct RowsParams {
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ RowsParams p)
 {
     using T = Geo<KS>;
-    constexpr int K = 64 * KS;
+    constexpr int K = 64 * KS, NW = T::NW;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *gen = smem_raw + (smem - smem_u32(smem_raw));
@@ -171,7 +171,7 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
         // ================= producer =================
         if (elect_one()) {
             bool ok = true;
-            int wit = 0;
+            int s = 0, round = 0;                                      // next slab's slot, times the ring has gone round
             for (int n = 0; ok; ++n) {
                 const int u = (int)blockIdx.x + n * (int)gridDim.x;
                 if (u >= p.units) break;
@@ -187,14 +187,15 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                 }
                 for (int j = 0; j < nt && ok; ++j) {
                     const int col = (t0 + j) * BN, seg = col / p.N;
-                    for (int ks = 0; ks < KS; ++ks, ++wit) {
-                        const int s = wit % NW;
-                        if (wit >= NW) ok = mbar_wait(w_empty(s), (uint32_t)((wit / NW - 1) & 1), p.err, 112);
+                    for (int h = 0; h < 2 * KS; ++h) {                 // tails and heads in turn
+                        if (round > 0) ok = mbar_wait(w_empty(s), (uint32_t)((round - 1) & 1), p.err, 112);
                         if (!ok) break;
-                        mbar_arrive_expect_tx(w_full(s), 2 * SLAB_BYTES);
-                        const uint32_t dst = smem + (uint32_t)(s * 2 * SLAB_BYTES);
-                        tma_load_2d(dst, &maps.w[seg], w_full(s), ks * 64, col % p.N);
-                        tma_load_2d(dst + SLAB_BYTES, &maps.w[seg], w_full(s), K + ks * 64, col % p.N);
+                        mbar_arrive_expect_tx(w_full(s), SLAB_BYTES);
+                        tma_load_2d(smem + (uint32_t)(s * SLAB_BYTES), &maps.w[seg], w_full(s), (h & 1 ? 0 : K) + (h >> 1) * 64, col % p.N);
+                        if (++s == NW) {
+                            s = 0;
+                            ++round;
+                        }
                     }
                 }
             }
@@ -205,7 +206,14 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
         constexpr uint32_t SLAB16 = SLAB_BYTES >> 4;                   // descriptor addresses count in units of 16 bytes
         const uint64_t wd0 = make_smem_desc_kmajor(smem, 128), ad0 = make_smem_desc_kmajor(smem + T::OFF_A, 128);
         bool ok = true;
-        int wit = 0, tc = 0;
+        int s = 0, tc = 0;
+        uint32_t par = 0;
+        auto next_slab = [&]() {
+            if (++s == NW) {
+                s = 0;
+                par ^= 1u;
+            }
+        };
         for (int n = 0; ok; ++n) {
             const int u = (int)blockIdx.x + n * (int)gridDim.x;
             if (u >= p.units) break;
@@ -216,31 +224,44 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                 const int buf = tc & 1;
                 if (tc >= 2) ok = mbar_wait_warp(acc_empty(buf), (uint32_t)((tc / 2 - 1) & 1), p.err, 114);
                 const uint32_t d = tmem_base + (uint32_t)(buf * 2 * BN);
-                for (int ks = 0; ks < KS && ok; ++ks, ++wit) {
-                    const int s = wit % NW;
-                    ok = mbar_wait_warp(w_full(s), (uint32_t)((wit / NW) & 1), p.err, 115);
+                for (int ks = 0; ks < KS && ok; ++ks) {
+                    // head.tail, then tail.head and head.head: each slab is freed as soon as it can be
+                    ok = mbar_wait_warp(w_full(s), par, p.err, 115);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t a = ad0 + (uint32_t)(ks * 2 * SLAB16);
+                    if (elect_one()) {
+                        const uint64_t w = wd0 + (uint32_t)(s * SLAB16);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)                    // 16 columns = 32 bytes an instruction
+                            tc_mma_bf16(d + BN, a + 2 * k, w + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+                        tc_commit(w_empty(s));
+                    }
+                    __syncwarp();
+                    next_slab();
+                    ok = mbar_wait_warp(w_full(s), par, p.err, 115);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
-                        const uint64_t a = ad0 + (uint32_t)(ks * 2 * SLAB16), w = wd0 + (uint32_t)(s * 2 * SLAB16);
+                        const uint64_t w = wd0 + (uint32_t)(s * SLAB16);
 #pragma unroll
-                        for (int pr = 0; pr < 3; ++pr)                 // tail.head, head.tail, head.head
+                        for (int k = 0; k < 4; ++k) tc_mma_bf16(d + BN, a + SLAB16 + 2 * k, w + 2 * k, idesc, 1u);
 #pragma unroll
-                            for (int k = 0; k < 4; ++k)                // 16 columns = 32 bytes an instruction
-                                tc_mma_bf16(d + (pr < 2 ? BN : 0), a + (pr == 0 ? SLAB16 : 0u) + 2 * k, w + (pr == 1 ? SLAB16 : 0u) + 2 * k,
-                                            idesc, (ks > 0 || pr == 1 || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < 4; ++k) tc_mma_bf16(d, a + 2 * k, w + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
                         tc_commit(w_empty(s));
                         if (j == nt - 1) tc_commit(a_empty(ks));
                         if (ks == KS - 1) tc_commit(acc_full(buf));
                     }
                     __syncwarp();
+                    next_slab();
                 }
             }
         }
     } else if (warp >= EPI_WARP0) {
         // ================= split, epilogue =================
         const int ew = warp - EPI_WARP0, half = ew >> 2, quad = warp & 3;
-        const uint32_t stg = smem + T::OFF_STG + (uint32_t)(ew * STG_BYTES);
+        const uint32_t stg0 = smem + T::OFF_STG + (uint32_t)(ew * 2 * STG_BYTES);
+        uint32_t nstore = 0;
         bool ok = true;
 
         // 16 rows of the block: LPR lanes share a row, eight columns each
@@ -368,25 +389,28 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                     }
                     // rows, or rows with every 32 channels as [head | tail]
                     const bool split = layout == kTf32SplitRows;
-                    for (int t = 0; t < (split ? 2 : 1); ++t) {
-                        if (lane == 0) tma_store_wait_read<0>();          // the store out of the staging tile has been read
+                    for (int t = 0; t < (split ? 4 : 2); ++t) {               // 16 columns each, heads and tails in turn
+                        const int hf = split ? t >> 1 : t;
+                        const uint32_t stg = stg0 + (nstore++ & 1) * STG_BYTES;
+                        if (lane == 0) tma_store_wait_read<1>();          // the last but one store has been read
                         __syncwarp();
 #pragma unroll
-                        for (int j4 = 0; j4 < 8; ++j4) {
-                            float4 v = make_float4(__uint_as_float(r[4 * j4]), __uint_as_float(r[4 * j4 + 1]),
-                                                   __uint_as_float(r[4 * j4 + 2]), __uint_as_float(r[4 * j4 + 3]));
-                            if (split) {
-                                const float4 h = make_float4(tf32_head(v.x), tf32_head(v.y), tf32_head(v.z), tf32_head(v.w));
-                                v = t == 0 ? h : make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+                        for (int j4 = 0; j4 < 4; ++j4) {
+                            float v[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                v[e] = __uint_as_float(hf ? r[16 + 4 * j4 + e] : r[4 * j4 + e]);
+                                const float h = tf32_head(v[e]);
+                                if (split) v[e] = (t & 1) == 0 ? h : v[e] - h;
                             }
-                            asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(stg + (uint32_t)(lane * 128 + ((j4 ^ (lane & 7)) << 4))),
-                                         "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                            asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};\n" ::"r"(stg + (uint32_t)(lane * 64 + ((j4 ^ ((lane >> 1) & 3)) << 4))),
+                                         "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
                                          : "memory");
                         }
                         fence_proxy_async();
                         __syncwarp();
                         if (lane == 0) {
-                            tma_store_2d(omap, stg, split ? 2 * nn + 32 * t : nn, m0);
+                            tma_store_2d(omap, stg, (split ? 2 * nn + 32 * (t & 1) : nn) + 16 * hf, m0);
                             tma_store_commit();
                         }
                     }
@@ -498,7 +522,7 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
         const uint64_t cols = p.layout[i] == kTf32SplitRows ? 2 * (uint64_t)N : (uint64_t)N;
         if (p.layout[i] == kTf32SplitTransposed)
             maps.out[i] = maps.a;                            // stored directly
-        else if (!make_tensor_map_2d(&maps.out[i], out[j], 4, cols, (uint64_t)M, p.layout[i] == kTf32SplitRows ? cols : (uint64_t)ldo, 32, 32, 128))
+        else if (!make_tensor_map_2d(&maps.out[i], out[j], 4, cols, (uint64_t)M, p.layout[i] == kTf32SplitRows ? cols : (uint64_t)ldo, 16, 32, 64))
             return false;
     }
     p.M = (int)M;

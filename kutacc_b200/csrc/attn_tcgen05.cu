@@ -73,14 +73,27 @@ constexpr int S_COL = 0, O_COL = 64;
 constexpr float kRescaleThreshold = 5.5f;     // P stays below 2^8
 constexpr float kFar = 2147483648.f;          // 2^31: mneg below it is within 64 of -m * log2e
 
-template <int D>
+// Without a pair bias there is room (STAGED): a warp's rows of the gate come by TMA into a tile of its own, where the result takes
+// their place; the next item's number and first operands are asked for early. The clocks of a CTA showed 6000 between two items of
+// eight tiles of 2700: Q and the first tile from memory (3400), rows of gate and result read and written by the threads they belong to,
+// 32 lines an instruction. 384 x 512 rows x 8 heads: 300 -> 267 us. With a pair bias the same (rows straight to memory, they do
+// not fit) made no difference at 301 and 1024 residues, and a call of 4 x 192 rows 9 % slower.
+template <int D, bool STAGED>
 struct Geo {
+    static constexpr int ROWS_BYTES = STAGED ? 32 * D * 2 : 0;
     static constexpr int KD = D < 16 ? 16 : D;                // K extent of Q.K^T; TMA zero-fills past D
     static constexpr int ROWB = KD * 2;                       // bytes of a q/k row = swizzle width
     static constexpr int VT_ROWS = (D + 16) / 16 * 16;        // channels, the ones row, zero rows
     static constexpr int Q_BYTES = BM * ROWB, K_BYTES = BN * ROWB, VT_BYTES = VT_ROWS * BN * 2;
     static constexpr int VT_TX = D * BN * 2;                  // bytes TMA writes of a V^T tile
 };
+
+template <bool STAGED>
+struct RowMaps {                      // [B][S][C], box [D, 32]
+    CUtensorMap gate, avg;
+};
+template <>
+struct RowMaps<false> {};
 
 struct AttnParams {
     const __nv_bfloat16 *gate;        // [B, S, H*D]: SPLIT bf16(x.Wg + bg), otherwise bf16(sigmoid(bf16(x.Wg + bg)))
@@ -110,16 +123,17 @@ template <int D, bool SPLIT, bool HAS_NB>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_vt, const __grid_constant__ CUtensorMap tm_nb,
-               const AttnParams p)
+               const __grid_constant__ RowMaps<!HAS_NB> tm_rows, const AttnParams p)
 {
-    using T = Geo<D>;
+    constexpr bool STAGED = !HAS_NB;
+    using T = Geo<D, STAGED>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *smem_gen = smem_raw + (smem - smem_u32(smem_raw));
     const int G = p.G;
-    // shared memory: barriers, Q tiles, ring of [K x G | V^T x G | pair bias | mask bias]
+    // shared memory: barriers, Q tiles, rows of the gate, ring of [K x G | V^T x G | pair bias | mask bias]
     const uint32_t off_q = 1024;
-    const uint32_t off_stage = off_q + (uint32_t)(G * T::Q_BYTES);
+    const uint32_t off_rows = off_q + (uint32_t)(G * T::Q_BYTES), off_stage = off_rows + (uint32_t)(G * 4 * T::ROWS_BYTES);
     const uint32_t off_vt = (uint32_t)(G * T::K_BYTES), off_nb = off_vt + (uint32_t)(G * T::VT_BYTES),
                    off_mb = off_nb + (HAS_NB ? NB_BYTES : 0), stage_bytes = off_mb + MB_BYTES;
     auto stage_base = [&](int s) { return smem + off_stage + (uint32_t)s * stage_bytes; };
@@ -133,7 +147,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     auto it_full = [&](int i) { return q_full + 16u + 8u * (uint32_t)(i & 3); };      // item number i has been written
     const uint32_t item_ring = q_full + 48u;                                         // four ints
     const uint32_t tmem_slot = q_full + 64u;
-    static_assert(8 * (2 * NST + 3 * MAXG) + 68 <= BAR_BYTES, "barriers fit their block");
+    auto g_full = [&](int softmax_warp) { return q_full + 72u + 8u * (uint32_t)softmax_warp; };
+    static_assert(8 * (2 * NST + 3 * MAXG) + 72 + 8 * SOFTMAX_WARPS <= BAR_BYTES, "barriers fit their block");
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int S = p.S;
@@ -170,6 +185,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         mbar_init(q_full, 1);
         mbar_init(q_empty, n_mma);
         for (int i = 0; i < 4; ++i) mbar_init(it_full(i), 1);
+        for (int i = 0; i < SOFTMAX_WARPS && STAGED; ++i) mbar_init(g_full(i), 1);
         fence_barrier_init();
     }
     // static rows of every V^T tile: row D = 1.0 (row-sum column of O), the rows after it = 0
@@ -194,6 +210,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_vt);
         if (HAS_NB) tma_prefetch_desc(&tm_nb);
+        if constexpr (STAGED) {
+            tma_prefetch_desc(&tm_rows.gate);
+            tma_prefetch_desc(&tm_rows.avg);
+        }
     }
     release_successor();
     wait_for_predecessor();
@@ -204,9 +224,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     if (warp == PRODUCER_WARP) {
         // ================= producer =================
         const uint32_t tx = (uint32_t)(G * (T::K_BYTES + T::VT_TX) + (HAS_NB ? NB_BYTES : 0));
-        int g = 0;                                      // tiles issued so far (all items)
-        bool ok = true;
-        for (int i = 0; ok; ++i) {
+        // number of this CTA's i-th item, published to the other roles
+        auto take = [&](int i) -> int {
             int w = 0;
             if (lane == 0) {
                 w = atomicAdd(p.counter, 1);
@@ -214,22 +233,28 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(item_ring + 4u * (uint32_t)(i & 3)), "r"(w) : "memory");
                 mbar_arrive(it_full(i));                               // releases the store above
             }
-            w = __shfl_sync(0xffffffffu, w, 0);
-            if (w < 0) break;
-            int q0, h, b0;
-            decode(w, q0, h, b0);
-            if (i >= 1 && !mbar_wait_warp(q_empty, (uint32_t)((i - 1) & 1), p.err, 20)) break;
+            return __shfl_sync(0xffffffffu, w, 0);
+        };
+        auto load_q = [&](int i, int q0, int h, int b0) -> bool {
+            if (i >= 1 && !mbar_wait_warp(q_empty, (uint32_t)((i - 1) & 1), p.err, 20)) return false;
             if (elect_one()) {
                 mbar_arrive_expect_tx(q_full, (uint32_t)(G * T::Q_BYTES));
                 tma_load_4d(smem + off_q, &tm_q, q_full, 0, q0, h, b0);
             }
             __syncwarp();
-            for (int kt = 0; kt < nkt; ++kt, ++g) {
+            return true;
+        };
+        int g = 0;                                      // tiles issued so far (all items)
+        bool ok = true;
+        int w = take(0);
+        for (int i = 0; w >= 0; ++i) {
+            int q0, h, b0, next = -1;
+            decode(w, q0, h, b0);
+            if (!STAGED) ok = load_q(i, q0, h, b0);
+            for (int kt = 0; kt < nkt && ok; ++kt, ++g) {
                 const int s = g % NST;
-                if (g >= NST && !mbar_wait_warp(kv_empty(s), (uint32_t)((g / NST - 1) & 1), p.err, 21)) {
-                    ok = false;
-                    break;
-                }
+                ok = g < NST || mbar_wait_warp(kv_empty(s), (uint32_t)((g / NST - 1) & 1), p.err, 21);
+                if (!ok) break;
                 if (elect_one()) {
                     const uint32_t st = stage_base(s);
                     const int k0 = kt * BN;
@@ -240,7 +265,27 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     if (HAS_NB) tma_load_3d(st + off_nb, &tm_nb, kv_full(s), k0, p.nb_head_inner ? h : q0, p.nb_head_inner ? q0 : h);
                 }
                 __syncwarp();
+                if (!STAGED) continue;
+                // Q after the item's first tile, whose stage is free earlier than the tile of the Q before it
+                if (kt == 0) ok = load_q(i, q0, h, b0);
+                // The next item's number two tiles before this one's loads end, its Q and first tile on their way to L2. Ring slot
+                // i & 3: every role has read the number of item i - 4, as this tile's stage was free.
+                if (kt == max(nkt - 2, 0)) {
+                    next = take(i + 1);
+                    if (next >= 0) {
+                        int q1, h1, b1;
+                        decode(next, q1, h1, b1);
+                        if (elect_one()) {
+                            tma_prefetch_4d(&tm_q, 0, q1, h1, b1);
+                            tma_prefetch_4d(&tm_k, 0, 0, h1, b1);
+                            for (int r = 0; r < G; ++r) tma_prefetch_4d(&tm_vt, 0, 0, h1, b1 + r);
+                        }
+                        __syncwarp();
+                    }
+                }
             }
+            if (!ok) break;
+            w = STAGED ? next : take(i + 1);
         }
     } else if (warp == MASK_WARP) {
         // ================= mask bias: fp32 copies of the keys' bias values beside the tile =================
@@ -540,22 +585,34 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             return true;
         };
 
+        const uint32_t rows = smem + off_rows + (uint32_t)(warp * T::ROWS_BYTES);
+        uint32_t gates = 0, gate_loads = 0;              // tiles of gate rows waited for, and asked for
         int g = 0;
         for (int i = 0; ok; ++i) {
             const int w = item_of(i, 34);
             if (w < 0) break;
             int q0, h, b0;
             decode(w, q0, h, b0);
+            if constexpr (STAGED) {
+                const bool any = q0 + quad * 32 < S && b0 + wg < p.B;
+                gate_loads += any ? 1u : 0u;
+                if (any && lane == 0) {
+                    tma_store_wait_read<0>();
+                    mbar_arrive_expect_tx(g_full(warp), (uint32_t)T::ROWS_BYTES);
+                    tma_load_3d(rows, &tm_rows.gate, g_full(warp), h * D, q0 + quad * 32, b0 + wg);
+                }
+                __syncwarp();
+            }
             for (int kt = 0; kt < nkt && ok; ++kt, ++g) ok = do_tile(g, kt);
             if (!ok) break;
 
             // ---- item epilogue: one row of D channels per thread ----
             const int qi = q0 + row, bb = b0 + wg;
-            const bool live = qi < S && bb < p.B;
-            const int64_t base = live ? ((int64_t)bb * S + qi) * (p.H * D) + h * D : 0;
+            const bool live = STAGED ? q0 + quad * 32 < S && bb < p.B : qi < S && bb < p.B;      // (STAGED: the warp has a row)
+            const int64_t base = live && !STAGED ? ((int64_t)bb * S + qi) * (p.H * D) + h * D : 0;
             uint4 gv[D / 8];
 #pragma unroll
-            for (int c = 0; c < D / 8; ++c) gv[c] = __ldg(reinterpret_cast<const uint4 *>(p.gate + base) + c);   // in flight
+            for (int c = 0; c < D / 8 && !STAGED; ++c) gv[c] = __ldg(reinterpret_cast<const uint4 *>(p.gate + base) + c);   // in flight
             if (!mbar_wait_warp(o_full(wg), (uint32_t)(i & 1), p.err, 29)) break;
             tc_fence_after();
             uint32_t o[D < 16 ? 16 : D], osum;
@@ -570,8 +627,15 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             if (D < 16) osum = o[D];
             const float inv = 1.0f / __uint_as_float(osum);
             if (live) {
+                if (STAGED && !mbar_wait_warp(g_full(warp), gates++ & 1u, p.err, 30)) break;
 #pragma unroll
                 for (int c = 0; c < D / 8; ++c) {
+                    // chunk c of this thread's row, in the swizzle of the tensor map
+                    const uint32_t at = rows + (uint32_t)(lane * (D * 2) + ((c ^ (D == 32 ? (lane >> 1) & 3 : D == 16 ? (lane >> 2) & 1 : 0)) << 4));
+                    if (STAGED)
+                        asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n"
+                                     : "=r"(gv[c].x), "=r"(gv[c].y), "=r"(gv[c].z), "=r"(gv[c].w)
+                                     : "r"(at));
                     const uint32_t gw[4] = {gv[c].x, gv[c].y, gv[c].z, gv[c].w};
                     uint32_t ow[4];
 #pragma unroll
@@ -586,9 +650,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                         }
                         ow[j] = pack_bf16x2(bf16lo_to_f32(wa) * s0, bf16hi_to_f32(wa) * s1);
                     }
-                    *(reinterpret_cast<uint4 *>(p.avg + base) + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                    if (STAGED)
+                        asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(at), "r"(ow[0]), "r"(ow[1]), "r"(ow[2]), "r"(ow[3]) : "memory");
+                    else
+                        *(reinterpret_cast<uint4 *>(p.avg + base) + c) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+                }
+                if constexpr (STAGED) {
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {                     // rows past S are clipped
+                        tma_store_3d(&tm_rows.avg, rows, h * D, q0 + quad * 32, bb);
+                        tma_store_commit();
+                    }
                 }
             }
+        }
+        if (STAGED) {
+            // after a wait that ran out: no copy may still be on its way when the CTA exits
+            if (gates != gate_loads) mbar_wait_warp(g_full(warp), gates & 1u, p.err, 31);
+            if (lane == 0) tma_store_wait<0>();
         }
     }
 
@@ -612,21 +692,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
 }
 
-template <int D>
-int smem_bytes(int G, bool has_nb)
+template <int D, bool HAS_NB>
+int smem_bytes(int G)
 {
-    using T = Geo<D>;
-    return 1024 + 1024 + G * T::Q_BYTES + NST * (G * (T::K_BYTES + T::VT_BYTES) + (has_nb ? NB_BYTES : 0) + MB_BYTES);
+    using T = Geo<D, !HAS_NB>;
+    return 1024 + 1024 + G * (T::Q_BYTES + 4 * T::ROWS_BYTES) + NST * (G * (T::K_BYTES + T::VT_BYTES) + (HAS_NB ? NB_BYTES : 0) + MB_BYTES);
 }
 
 template <int D, bool SPLIT, bool HAS_NB>
 bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tvt,
-                const CUtensorMap &tnb, const AttnParams &p)
+                const CUtensorMap &tnb, const RowMaps<!HAS_NB> &rows, const AttnParams &p)
 {
     static bool configured = false;
     if (!configured) {
         KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, SPLIT, HAS_NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem_bytes<D>(MAXG, HAS_NB)));
+                                         smem_bytes<D, HAS_NB>(MAXG)));
         configured = true;
     }
     const unsigned grid = (unsigned)std::min<int64_t>(p.n_items, std::max(1, sm_count() - runtime().sm_margin));
@@ -634,7 +714,7 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
     q.counter = work_counter(stream);
     if (q.counter == nullptr) return false;
     KernelTimer timer__("attn_core", stream);
-    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB>, grid, THREADS, smem_bytes<D>(p.G, HAS_NB), stream, tq, tk, tvt, tnb, q);
+    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB>, grid, THREADS, smem_bytes<D, HAS_NB>(p.G), stream, tq, tk, tvt, tnb, rows, q);
     count_launch();
     return true;
 }
@@ -664,7 +744,7 @@ template <int D, bool SPLIT>
 bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch, const void *nb,
               int64_t nb_stride_h, int64_t nb_stride_q, AttnParams &p)
 {
-    using T = Geo<D>;
+    using T = Geo<D, false>;
     const uint64_t Su = (uint64_t)p.S;
     CUtensorMap tq, tk, tvt, tnb;
     const uint64_t H = (uint64_t)p.H, B = (uint64_t)p.B, vp = (uint64_t)vt_pitch;
@@ -685,10 +765,15 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
                                             BM, 128)) {
             return false;
         }
-        return launch_one<D, SPLIT, true>(stream, tq, tk, tvt, tnb, p);
+        return launch_one<D, SPLIT, true>(stream, tq, tk, tvt, tnb, RowMaps<false>{}, p);
     }
     tnb = tk;
-    return launch_one<D, SPLIT, false>(stream, tq, tk, tvt, tnb, p);
+    RowMaps<true> rows;
+    const int swizzle = D == 8 ? 0 : D * 2;
+    if (!make_tensor_map_bf16_3d(&rows.gate, p.gate, H * D, Su, B, H * D, Su * H * D, D, 32, swizzle) ||
+        !make_tensor_map_bf16_3d(&rows.avg, p.avg, H * D, Su, B, H * D, Su * H * D, D, 32, swizzle))
+        return false;
+    return launch_one<D, SPLIT, false>(stream, tq, tk, tvt, tnb, rows, p);
 }
 
 }  // namespace

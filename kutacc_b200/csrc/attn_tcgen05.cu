@@ -73,11 +73,13 @@ constexpr int S_COL = 0, O_COL = 64;
 constexpr float kRescaleThreshold = 5.5f;     // P stays below 2^8
 constexpr float kFar = 2147483648.f;          // 2^31: mneg below it is within 64 of -m * log2e
 
-// Without a pair bias there is room (STAGED): a warp's rows of the gate come by TMA into a tile of its own, where the result takes
-// their place; the next item's number and first operands are asked for early. The clocks of a CTA showed 6000 between two items of
-// eight tiles of 2700: Q and the first tile from memory (3400), rows of gate and result read and written by the threads they belong to,
-// 32 lines an instruction. 384 x 512 rows x 8 heads: 300 -> 267 us. With a pair bias the same (rows straight to memory, they do
-// not fit) made no difference at 301 and 1024 residues, and a call of 4 x 192 rows 9 % slower.
+// STAGED: a warp's rows of the gate come by TMA into a tile of its own, where the result takes their place; the next item's number and
+// first operands are asked for early. The clocks of a CTA showed 6000 between two items of eight tiles of 2700: Q and the first
+// tile from memory (3400), rows of gate and result read and written by the threads they belong to, 32 lines an instruction. 384 x 512
+// rows x 8 heads: 300 -> 267 us; with a pair bias 512 x 512 x 4 338 -> 317 us (the whole call), 1024 residues 2030 -> 1988. Beside the
+// pair bias of heads of 32 there is room for two of its tiles, a ring of their own, and they come one tile after K and V, which a CTA with
+// a single short item feels: 4 x 192 rows 20.5 against 22.2 us, 64 residues 28.7 against 30.7. So there, and for narrow heads, whose
+// rows are short, everything stays in one ring of three.
 template <int D, bool STAGED>
 struct Geo {
     static constexpr int ROWS_BYTES = STAGED ? 32 * D * 2 : 0;
@@ -119,13 +121,12 @@ struct AttnParams {
 // Tails of 16 keys from column tail_col(c, D) on: beside O, and for heads of 32 half of them over logits already read.
 __device__ __forceinline__ constexpr int tail_col(int c, int D) { return D < 32 ? 96 + 8 * c : c < 2 ? 112 + 8 * c : 16 + 8 * c; }
 
-template <int D, bool SPLIT, bool HAS_NB>
+template <int D, bool SPLIT, bool HAS_NB, bool STAGED>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_vt, const __grid_constant__ CUtensorMap tm_nb,
-               const __grid_constant__ RowMaps<!HAS_NB> tm_rows, const AttnParams p)
+               const __grid_constant__ RowMaps<STAGED> tm_rows, const AttnParams p)
 {
-    constexpr bool STAGED = !HAS_NB;
     using T = Geo<D, STAGED>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -135,8 +136,9 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const uint32_t off_q = 1024;
     const uint32_t off_rows = off_q + (uint32_t)(G * T::Q_BYTES), off_stage = off_rows + (uint32_t)(G * 4 * T::ROWS_BYTES);
     const uint32_t off_vt = (uint32_t)(G * T::K_BYTES), off_nb = off_vt + (uint32_t)(G * T::VT_BYTES),
-                   off_mb = off_nb + (HAS_NB ? NB_BYTES : 0), stage_bytes = off_mb + MB_BYTES;
+                   off_mb = off_nb + (HAS_NB && !STAGED ? NB_BYTES : 0), stage_bytes = off_mb + MB_BYTES;
     auto stage_base = [&](int s) { return smem + off_stage + (uint32_t)s * stage_bytes; };
+    auto nb_ring = [&](int g) { return smem + off_stage + NST * stage_bytes + (uint32_t)((g & 1) * NB_BYTES); };     // STAGED
     const uint32_t bar = smem;
     auto kv_full = [&](int s) { return bar + 8u * (uint32_t)s; };
     auto kv_empty = [&](int s) { return bar + 8u * (uint32_t)(NST + s); };
@@ -247,6 +249,10 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         int g = 0;                                      // tiles issued so far (all items)
         bool ok = true;
         int w = take(0);
+        int nb_g = -1, nb_k0 = 0, nb_q0 = 0, nb_h = 0;  // the tile whose pair bias has not been asked for
+        auto load_nb = [&]() {                          // by the elected lane
+            tma_load_3d(nb_ring(nb_g), &tm_nb, kv_full(nb_g % NST), nb_k0, p.nb_head_inner ? nb_h : nb_q0, p.nb_head_inner ? nb_q0 : nb_h);
+        };
         for (int i = 0; w >= 0; ++i) {
             int q0, h, b0, next = -1;
             decode(w, q0, h, b0);
@@ -255,16 +261,25 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const int s = g % NST;
                 ok = g < NST || mbar_wait_warp(kv_empty(s), (uint32_t)((g / NST - 1) & 1), p.err, 21);
                 if (!ok) break;
+                const int k0 = kt * BN;
+                auto this_nb = [&]() {
+                    nb_g = g;
+                    nb_k0 = k0;
+                    nb_q0 = q0;
+                    nb_h = h;
+                };
                 if (elect_one()) {
                     const uint32_t st = stage_base(s);
-                    const int k0 = kt * BN;
                     mbar_arrive_expect_tx(kv_full(s), tx);
                     // K, V^T and Q of batch rows past B are filled with zeros
                     tma_load_4d(st, &tm_k, kv_full(s), 0, k0, h, b0);
                     for (int r = 0; r < G; ++r) tma_load_4d(st + off_vt + r * T::VT_BYTES, &tm_vt, kv_full(s), k0, 0, h, b0 + r);
-                    if (HAS_NB) tma_load_3d(st + off_nb, &tm_nb, kv_full(s), k0, p.nb_head_inner ? h : q0, p.nb_head_inner ? q0 : h);
+                    if (HAS_NB && !STAGED) tma_load_3d(st + off_nb, &tm_nb, kv_full(s), k0, p.nb_head_inner ? h : q0, p.nb_head_inner ? q0 : h);
+                    // (the stage waited for above belonged to tile g - 3, whose pair bias lay where that of tile g - 1 goes)
+                    if (HAS_NB && STAGED && nb_g >= 0) load_nb();
                 }
                 __syncwarp();
+                if (HAS_NB && STAGED) this_nb();
                 if (!STAGED) continue;
                 // Q after the item's first tile, whose stage is free earlier than the tile of the Q before it
                 if (kt == 0) ok = load_q(i, q0, h, b0);
@@ -279,6 +294,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                             tma_prefetch_4d(&tm_q, 0, q1, h1, b1);
                             tma_prefetch_4d(&tm_k, 0, 0, h1, b1);
                             for (int r = 0; r < G; ++r) tma_prefetch_4d(&tm_vt, 0, 0, h1, b1 + r);
+                            if (HAS_NB) tma_prefetch_3d(&tm_nb, 0, p.nb_head_inner ? h1 : q1, p.nb_head_inner ? q1 : h1);
                         }
                         __syncwarp();
                     }
@@ -286,6 +302,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             }
             if (!ok) break;
             w = STAGED ? next : take(i + 1);
+        }
+        if (HAS_NB && STAGED && ok && nb_g >= 0 &&
+            (nb_g < 2 || mbar_wait_warp(kv_empty((nb_g - 2) % NST), (uint32_t)(((nb_g - 2) / NST) & 1), p.err, 19))) {
+            if (elect_one()) load_nb();
+            __syncwarp();
         }
     } else if (warp == MASK_WARP) {
         // ================= mask bias: fp32 copies of the keys' bias values beside the tile =================
@@ -409,7 +430,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const uint32_t t_s = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(wg * WG_COLS + S_COL);
         const uint32_t t_o = t_s - S_COL + O_COL;
         const uint64_t scale2 = pack_f32x2(p.scale, p.scale), log2e2 = pack_f32x2(kLog2e, kLog2e);
-        const uint32_t nb_row = off_nb + (uint32_t)row * 128 + (uint32_t)((row & 7) << 4);   // chunk c lies at ^ (c << 4)
+        const uint32_t nb_row = (STAGED ? 0u : off_nb) + (uint32_t)row * 128 + (uint32_t)((row & 7) << 4);   // chunk c lies at ^ (c << 4)
         const uint32_t mb_row = off_mb + (uint32_t)wg * BN * 4;
         // Running (possibly stale) max of x, at least the lowest finite number: keys masked with -inf then weigh nothing, and
         // a row whose first keys are all of that kind is raised by its first finite one. P = 2^(x * log2e + mneg); the
@@ -453,7 +474,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                     for (int i = 0; i < 2; ++i)
                         asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];\n"
                                      : "=r"(f.nb[4 * i]), "=r"(f.nb[4 * i + 1]), "=r"(f.nb[4 * i + 2]), "=r"(f.nb[4 * i + 3])
-                                     : "r"((st + nb_row) ^ (uint32_t)((2 * c + i) << 4)));
+                                     : "r"(((STAGED ? nb_ring(g) : st) + nb_row) ^ (uint32_t)((2 * c + i) << 4)));
                 }
             };
             auto x_pair = [&](const uint32_t (&r)[16], const Piece &f, const int j) -> uint64_t {
@@ -692,21 +713,22 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     }
 }
 
-template <int D, bool HAS_NB>
+template <int D, bool HAS_NB, bool STAGED>
 int smem_bytes(int G)
 {
-    using T = Geo<D, !HAS_NB>;
-    return 1024 + 1024 + G * (T::Q_BYTES + 4 * T::ROWS_BYTES) + NST * (G * (T::K_BYTES + T::VT_BYTES) + (HAS_NB ? NB_BYTES : 0) + MB_BYTES);
+    using T = Geo<D, STAGED>;
+    return 1024 + 1024 + G * (T::Q_BYTES + 4 * T::ROWS_BYTES) + NST * (G * (T::K_BYTES + T::VT_BYTES) + MB_BYTES) +
+           (!HAS_NB ? 0 : STAGED ? 2 : NST) * NB_BYTES;
 }
 
-template <int D, bool SPLIT, bool HAS_NB>
+template <int D, bool SPLIT, bool HAS_NB, bool STAGED>
 bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tvt,
-                const CUtensorMap &tnb, const RowMaps<!HAS_NB> &rows, const AttnParams &p)
+                const CUtensorMap &tnb, const RowMaps<STAGED> &rows, const AttnParams &p)
 {
     static bool configured = false;
     if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, SPLIT, HAS_NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem_bytes<D, HAS_NB>(MAXG)));
+        KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, SPLIT, HAS_NB, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem_bytes<D, HAS_NB, STAGED>(MAXG)));
         configured = true;
     }
     const unsigned grid = (unsigned)std::min<int64_t>(p.n_items, std::max(1, sm_count() - runtime().sm_margin));
@@ -714,7 +736,7 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
     q.counter = work_counter(stream);
     if (q.counter == nullptr) return false;
     KernelTimer timer__("attn_core", stream);
-    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB>, grid, THREADS, smem_bytes<D, HAS_NB>(p.G), stream, tq, tk, tvt, tnb, rows, q);
+    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB, STAGED>, grid, THREADS, smem_bytes<D, HAS_NB, STAGED>(p.G), stream, tq, tk, tvt, tnb, rows, q);
     count_launch();
     return true;
 }
@@ -744,7 +766,7 @@ template <int D, bool SPLIT>
 bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt, int64_t vt_pitch, const void *nb,
               int64_t nb_stride_h, int64_t nb_stride_q, AttnParams &p)
 {
-    using T = Geo<D, false>;
+    using T = Geo<D, true>;
     const uint64_t Su = (uint64_t)p.S;
     CUtensorMap tq, tk, tvt, tnb;
     const uint64_t H = (uint64_t)p.H, B = (uint64_t)p.B, vp = (uint64_t)vt_pitch;
@@ -752,6 +774,15 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
     if (!make_tensor_map_bf16_4d(&tq, q, D, Su, H, B, D, Su * D, Su * D * H, T::KD, BM, G, T::ROWB)) return false;
     if (!make_tensor_map_bf16_4d(&tk, k, D, Su, H, B, D, Su * D, Su * D * H, T::KD, BN, G, T::ROWB)) return false;
     if (!make_tensor_map_bf16_4d(&tvt, vt, Su, D, H, B, vp, D * vp, D * vp * H, BN, D, 1, 128)) return false;
+    // with a pair bias where a CTA has several items (see Geo)
+    const bool staged = !nb || (D == 32 && p.n_items > std::max(1, sm_count() - runtime().sm_margin));
+    RowMaps<true> rows;
+    if (staged) {
+        const int swizzle = D == 8 ? 0 : D * 2;
+        if (!make_tensor_map_bf16_3d(&rows.gate, p.gate, H * D, Su, B, H * D, Su * H * D, D, 32, swizzle) ||
+            !make_tensor_map_bf16_3d(&rows.avg, p.avg, H * D, Su, B, H * D, Su * H * D, D, 32, swizzle))
+            return false;
+    }
     p.nb_head_inner = 0;
     if (nb) {
         if (nb_stride_h < nb_stride_q) {
@@ -765,15 +796,13 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
                                             BM, 128)) {
             return false;
         }
-        return launch_one<D, SPLIT, true>(stream, tq, tk, tvt, tnb, RowMaps<false>{}, p);
+        if constexpr (D == 32) {
+            if (staged) return launch_one<D, SPLIT, true, true>(stream, tq, tk, tvt, tnb, rows, p);
+        }
+        return launch_one<D, SPLIT, true, false>(stream, tq, tk, tvt, tnb, RowMaps<false>{}, p);
     }
     tnb = tk;
-    RowMaps<true> rows;
-    const int swizzle = D == 8 ? 0 : D * 2;
-    if (!make_tensor_map_bf16_3d(&rows.gate, p.gate, H * D, Su, B, H * D, Su * H * D, D, 32, swizzle) ||
-        !make_tensor_map_bf16_3d(&rows.avg, p.avg, H * D, Su, B, H * D, Su * H * D, D, 32, swizzle))
-        return false;
-    return launch_one<D, SPLIT, false>(stream, tq, tk, tvt, tnb, rows, p);
+    return launch_one<D, SPLIT, false, true>(stream, tq, tk, tvt, tnb, rows, p);
 }
 
 }  // namespace

@@ -60,6 +60,7 @@ struct StreamArgs {
     float *hwa;                              // [B, 64]: weighted average / 2
     int B, S, nrec;                          // nrec: records per column
     int chunk_rows, chunks;                  // rows per partial sum (32 or 64) and their number per column
+    int keep_from;                           // units from here on should stay in L2 for the out kernel
     int *err;
 };
 
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
     auto rows_of = [&](int c) { return min(a.chunk_rows, a.S - c * a.chunk_rows); };
 
     // the copies run ahead of the work: unit, its first row and rows, row within it
+    const uint64_t first = l2_evict_first(), normal = l2_evict_normal();
     int iu = u0, ir = 0, irows = 0, issued = 0;
     int64_t irow = 0;
     auto enter_issue = [&]() {
@@ -115,7 +117,7 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
         if (lane == 0) {
             const uint32_t slot = (uint32_t)(issued % NS), bytes = (uint32_t)min(16, irows - ir) * (C * 2);
             mbar_arrive_expect_tx(bars + 8 * slot, bytes);
-            bulk_load(slots + slot * STEP_BYTES, a.x + (irow + ir) * C, bytes, bars + 8 * slot);
+            bulk_load(slots + slot * STEP_BYTES, a.x + (irow + ir) * C, bytes, bars + 8 * slot, iu < a.keep_from ? first : normal);
         }
         ++issued;
         ir += 16;
@@ -259,12 +261,13 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
     }
     __syncwarp();
     wait_for_predecessor();
+    const uint64_t policy = l2_evict_first();    // read once, and x should stay
     auto issue = [&](int i) {                    // this warp's i-th pair
         const int r0 = 2 * (warp + i * WARPS);
         if (lane == 0 && r0 < nrec) {
             const uint32_t slot = (uint32_t)(i % QN), bytes = (uint32_t)min(2, nrec - r0) * REC_BYTES;
             mbar_arrive_expect_tx(bars + 8 * slot, bytes);
-            bulk_load(slots + slot * Q_BYTES, a.rec + ((int64_t)b * nrec + r0) * REC_BYTES, bytes, bars + 8 * slot);
+            bulk_load(slots + slot * Q_BYTES, a.rec + ((int64_t)b * nrec + r0) * REC_BYTES, bytes, bars + 8 * slot, policy);
         }
     };
     for (int i = 0; i < QN; ++i) issue(i);
@@ -484,13 +487,14 @@ global_stream_out_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_
             tma_prefetch_desc(&xmap);
             tma_prefetch_desc(&omap);
             int issued = 0, freed = 0, b, row0;
+            const uint64_t policy = l2_evict_first();            // of what is left of x, and of the result
             bool ok = true;
             auto issue_loads = [&]() {
                 while (issued < mine && issued - NSLOT < freed) {
                     tile_of(issued, b, row0);
                     const int s = issued % NSLOT;
                     mbar_arrive_expect_tx(full(s), SLOT_BYTES);
-                    tma_load_3d(smem + s * SLOT_BYTES, &xmap, full(s), 0, row0, b);
+                    tma_load_3d(smem + s * SLOT_BYTES, &xmap, full(s), 0, row0, b, policy);
                     ++issued;
                 }
             };
@@ -502,7 +506,7 @@ global_stream_out_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_
                     break;
                 }
                 tile_of(t, b, row0);
-                tma_store_3d(&omap, smem + s * SLOT_BYTES, 0, row0, b);
+                tma_store_3d(&omap, smem + s * SLOT_BYTES, 0, row0, b, policy);
                 tma_store_commit();
                 tma_store_wait_read<1>();                        // all but the newest store have left their slots
                 freed = t;
@@ -665,6 +669,15 @@ StreamPlan make_plan(int64_t B, int64_t S)
     return p;
 }
 
+// x is read twice. What the kv kernel reads last should still be in L2 when the out kernel starts from there, beside the records that
+// the softmax kernel reads in between (L2 126 MB): the units before go first when room is made, like everything that is not read again.
+// 384 x 5120 rows: 179.5 -> 173.7 us; all of x first 176, nothing first 178.
+int keep_from(int64_t B, int64_t S, const StreamPlan &p)
+{
+    const int64_t x_bytes = B * S * C * 2, keep = std::max<int64_t>(0, ((int64_t)90 << 20) - (int64_t)p.bytes), units = B * p.chunks;
+    return keep >= x_bytes ? 0 : (int)(units - units * keep / x_bytes);
+}
+
 }  // namespace
 
 bool global_stream_covers(int heads, int head_size, int64_t out_row_stride)
@@ -699,6 +712,7 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
     a.nrec = pl.nrec;
     a.chunk_rows = pl.chunk_rows;
     a.chunks = pl.chunks;
+    a.keep_from = keep_from(B, S, pl);
     a.err = ew.device;
     OutArgs o;
     o.bg = bg;

@@ -106,7 +106,8 @@ struct AttnParams {
     int S, H, B;
     int G;                            // batch rows per item: 1, 2 or 4
     int n_qt;                         // query tiles per (b, h)
-    int n_items;                      // ceil(B / G) * H * n_qt
+    int n_whole, parts;               // narrow heads: items of G batch rows; each one after them is cut into this many items
+    int n_items;
     int nb_head_inner;                // pair-bias tensor map has the dimensions (key, head, query): the heads of a
                                       // query row lie closer together than the rows (a [S, H, S] storage)
     int *counter;                     // [0] next work item of this launch, [1] CTAs that have finished (both zero at
@@ -160,11 +161,19 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // item number, publishes it to the other roles through a ring of four shared-memory words (one mbarrier each),
     // and publishes -1 when the list is exhausted. Ring depth: slot i & 3 is written when the products of item i - 2
     // have all been issued, by which time every role has long read the number of item i - 4.
+    constexpr bool CUT = D < 32;
+    auto rows_of = [&](int w) { return CUT && w >= p.n_whole ? G / p.parts : G; };
     auto decode = [&](int w, int &q0, int &h, int &b0) {
+        int sub = 0;
+        if (CUT && w >= p.n_whole) {
+            const int v = w - p.n_whole;
+            sub = v % p.parts * (G / p.parts);
+            w = p.n_whole + v / p.parts;
+        }
         const int qt = w % p.n_qt, hb = w / p.n_qt;
         q0 = qt * BM;
         h = hb % p.H;
-        b0 = hb / p.H * G;
+        b0 = hb / p.H * G + sub;
     };
     // item number of this CTA's i-th item, or -1 (bounded wait; -2 on a timeout)
     auto item_of = [&](int i, int code) -> int {
@@ -615,7 +624,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             int q0, h, b0;
             decode(w, q0, h, b0);
             if constexpr (STAGED) {
-                const bool any = q0 + quad * 32 < S && b0 + wg < p.B;
+                const bool any = q0 + quad * 32 < S && b0 + wg < p.B && (!CUT || wg < rows_of(w));
                 gate_loads += any ? 1u : 0u;
                 if (any && lane == 0) {
                     tma_store_wait_read<0>();
@@ -624,12 +633,21 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 }
                 __syncwarp();
             }
-            for (int kt = 0; kt < nkt && ok; ++kt, ++g) ok = do_tile(g, kt);
+            const bool mine = !CUT || wg < rows_of(w);
+            if (mine) {
+                for (int kt = 0; kt < nkt && ok; ++kt, ++g) ok = do_tile(g, kt);
+            } else {                                     // a cut item has no row for this group, which only passes on the barriers
+                for (int kt = 0; kt < nkt && ok; ++kt, ++g) {
+                    ok = mbar_wait_warp(s_full(wg), (uint32_t)(g & 1), p.err, 26);
+                    tc_fence_before();
+                    if (ok && lane == 0) mbar_arrive(p_full(wg));
+                }
+            }
             if (!ok) break;
 
             // ---- item epilogue: one row of D channels per thread ----
             const int qi = q0 + row, bb = b0 + wg;
-            const bool live = STAGED ? q0 + quad * 32 < S && bb < p.B : qi < S && bb < p.B;      // (STAGED: the warp has a row)
+            const bool live = mine && bb < p.B && (STAGED ? q0 + quad * 32 < S : qi < S);      // (STAGED: the warp has a row)
             const int64_t base = live && !STAGED ? ((int64_t)bb * S + qi) * (p.H * D) + h * D : 0;
             uint4 gv[D / 8];
 #pragma unroll
@@ -741,25 +759,31 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
     return true;
 }
 
-// Batch rows per item. More rows per CTA overlap more chains and share the pair-bias tile, fewer rows spread a small
-// problem over more SMs: the choice minimises waves x (relative time of an item with that many rows). Measured per full wave
+// How the work is cut into items. More batch rows per CTA overlap more chains and share the pair-bias tile, fewer rows spread a
+// small problem over more SMs: the choice minimises waves x (relative time of an item with that many rows). Measured per full wave
 // against one row, at 128, 256, 384 and 1024 positions: four rows 2.4 (with pair bias 3.2), 2.3, 2.1, 1.8 with heads of 32, 1.4 to
-// 2.1 with narrower ones; two rows 1.3 to 1.6 and 1.0 to 1.5.
-int pick_group(int64_t B, int64_t hq, int sms)
+// 2.1 with narrower ones; two rows 1.3 to 1.6 and 1.0 to 1.5. Narrow heads: what is left for the last wave is cut into items of two
+// or one batch rows where that ends sooner: 256 x 256 rows of 4 heads of 16, the whole call, 63.7 -> 62.5 us (with heads of 32 the
+// kernel that can do this lost 1 to 3 % and gained nothing).
+void plan_items(AttnParams &p, int64_t sms, bool cut)
 {
     const int groups[3] = {4, 2, 1};
     const double t[3] = {2.03, 1.36, 1.0};
-    int best = 4;
-    double cost = 1e30;
+    double best = 1e30;
     for (int i = 0; i < 3; ++i) {
-        const int64_t items = (B + groups[i] - 1) / groups[i] * hq;
-        const double c = (double)((items + sms - 1) / sms) * t[i];
-        if (c < cost) {
-            cost = c;
-            best = groups[i];
+        const int64_t items = (int64_t)(p.B + groups[i] - 1) / groups[i] * p.H * p.n_qt, whole = items / sms * sms, last = items - whole;
+        for (int j = i; j < (cut ? 3 : i + 1); ++j) {
+            const int parts = groups[i] / groups[j];
+            const double cost = (double)(whole / sms) * t[i] + (double)((last * parts + sms - 1) / sms) * t[j];
+            if (cost < (j > i ? best * 0.99 : best)) {
+                best = cost;
+                p.G = groups[i];
+                p.parts = parts;
+                p.n_whole = (int)(parts == 1 ? items : whole);
+                p.n_items = (int)(parts == 1 ? items : whole + last * parts);
+            }
         }
     }
-    return best;
 }
 
 template <int D, bool SPLIT>
@@ -828,9 +852,8 @@ bool tcgen05_attn_core_bf16(cudaStream_t stream, const void *q, const void *k, c
     p.S = S;
     p.H = H;
     p.B = B;
-    p.G = pick_group(B, n_qt * H, std::max(1, sm_count() - runtime().sm_margin));
     p.n_qt = (int)n_qt;
-    p.n_items = (int)((B + p.G - 1) / p.G * n_qt * H);
+    plan_items(p, std::max(1, sm_count() - runtime().sm_margin), D < 32);
     p.scale = scale;
     p.counter = nullptr;
     switch (D) {

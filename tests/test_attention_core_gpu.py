@@ -151,3 +151,20 @@ def test_more_than_2_25_work_items(kutacc_lib):
     del x, out, eye, zero
     api.lib().kutacc_b200_release_workspace()
     torch.cuda.empty_cache()
+
+
+# (batch rows, positions): last query tile with one, two or three warps at work and its items at the end of the list; a last wave of
+# items cut in two or in four; last key tiles of one to four pieces; a batch that does not fill its last item
+@pytest.mark.parametrize("B,S,H,D,nb", [(301, 140, 4, 32, True), (75, 192, 4, 32, True), (161, 257, 4, 32, True), (298, 230, 2, 32, True),
+                                        (77, 131, 8, 16, True), (150, 333, 8, 8, True), (160, 49, 4, 32, True), (297, 112, 8, 8, True),
+                                        (600, 17, 2, 32, True), (299, 140, 4, 32, False), (101, 257, 4, 16, False)])
+def test_rows_do_not_depend_on_the_item_list(kutacc_lib, B, S, H, D, nb):
+    w = W.random_gating_case(seed=5 + S, B=B, S=S, H=H, D=D, with_nb=nb, full_mask_rows=1)
+    got = runner.out_to_f32(runner.DeviceCase(w).run())
+    pick = [0, 1, 2, 3, B // 2, B - 5, B - 4, B - 3, B - 2, B - 1]
+    for rows in (pick[:1], pick[3:6], pick):                          # one row an item, three items, ...
+        few = W.Workload(name="few", kind="gating", dtype=w.dtype, B=len(rows), S=S, H=H, D=D, seed=0, has_nb=nb)
+        few.arrays = dict(w.arrays, x=w.arrays["x"][rows], mask=w.arrays["mask"][rows], bias=w.arrays["bias"][rows])
+        assert np.array_equal(runner.out_to_f32(runner.DeviceCase(few).run()), got[rows])
+    few.B, few.arrays = 3, {k: v[:3] if k in ("x", "mask", "bias") else v for k, v in few.arrays.items()}
+    assert helpers.rel_err(got[:3], helpers.oracle_faithful(few)) <= helpers.BF16_TOL

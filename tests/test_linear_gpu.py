@@ -32,6 +32,22 @@ def test_linear_bf16(kutacc_lib, M, N, K, bias, beta):
     assert helpers.rel_err(got, ref) <= 5e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (129, 256, 256), (4700, 256, 128), (4736, 256, 128), (4737, 256, 128)])
+def test_linear_bf16_rows_do_not_depend_on_the_column_split(kutacc_lib, M, N, K):
+    # few tiles are cut into halves of their columns: the same rows as in a call of many
+    rng = np.random.default_rng(M)
+    w = W.as_f32(W.bf16_bits(rng.standard_normal((N, K)).astype(np.float32) / np.sqrt(K)))
+    tw, tb = _bf16_cuda(w), torch.randn(N, device=DEV)
+    many = _bf16_cuda(rng.standard_normal((20000, K)).astype(np.float32))
+    out = [torch.full((m + 1, N), 7.0, dtype=torch.bfloat16, device=DEV) for m in (20000, M)]
+    for t in out:
+        m = t.shape[0] - 1
+        api.linear(api.tensor(many[:m].clone()), api.tensor(tw), tb.data_ptr(), api.tensor(t[:m]), 0)
+    assert torch.equal(out[0][:M], out[1][:M]) and bool((out[1][M] == 7.0).all())
+    ref = many[:M].float() @ tw.float().T + tb
+    assert float((out[1][:M].float() - ref).abs().max()) <= 2.0 ** -8 * float(ref.abs().max()) * 1.01
+
+
 def test_linear_fp32(kutacc_lib):
     rng = np.random.default_rng(5)
     a = rng.standard_normal((200, 96)).astype(np.float32)

@@ -29,6 +29,7 @@ namespace {
 
 constexpr int C = 64, H = 8, D = 8;
 constexpr int REC_BYTES = 512 + 512 + 64;
+constexpr float kLog2e = 1.4426950408889634f;
 constexpr int POOL_PITCH = C + 4;            // floats per partial sum: 64 channels, the mask sum, padding
 
 __device__ __forceinline__ float rbf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
@@ -238,7 +239,8 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
 // the copies themselves were the bound, 26 us for 61440 records.) Sixteen warps per column whatever the number of columns: a
 // column's sums are split the same way in every batch. More columns than SMs run two CTAs per SM on a shorter ring (250
 // columns x 1500 rows: 41.6 us for the three kernels, with one CTA per SM 44.7); fewer have the longer ring (64 x 5120: 41 us,
-// with the shorter 46).
+// with the shorter 46). Half of a long column's time is issue slots (about 250 instructions a record with single values; two rows
+// a packed operation and a flushed exponential now: 384 x 5120, the three kernels 164.7 -> 162.9 us).
 constexpr int WARPS = 16, Q_BYTES = 2 * REC_BYTES;
 constexpr int core_smem(int qn) { return WARPS * qn * (Q_BYTES + 8); }
 
@@ -311,32 +313,40 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
 
     // thread (g, t) owns head g: logits^T [8 heads x 16] = q.k^T, wa [8 x 8] += P.v
     const uint32_t aq = pack_bf16x2(q_s[g * D + 2 * t], q_s[g * D + 2 * t + 1]);
-    float m_run = -INFINITY, l_run = 0.f, wa[4] = {0.f, 0.f, 0.f, 0.f};
-    // logits of the record at `src`; its v stays in registers
-    auto logits = [&](uint32_t src, float (&xv)[8], uint4 &vq) -> float {
+    float m_run = -INFINITY, wa[4] = {0.f, 0.f, 0.f, 0.f};
+    uint64_t l2 = 0;                             // sums of the even and of the odd rows' probabilities
+    const uint64_t scale2 = pack_f32x2(scale, scale), big2 = pack_f32x2(1e9f, 1e9f), nbig2 = pack_f32x2(-1e9f, -1e9f);
+    const uint64_t log2e2 = pack_f32x2(kLog2e, kLog2e);
+    // logits of the record at `src`, two rows at a time; its v stays in registers
+    auto logits = [&](uint32_t src, uint64_t (&xv)[4], uint4 &vq) -> float {
         const uint4 kq = lds128_u32(src + lane * 16), mq = lds128_u32(src + 1024 + t * 16);
         vq = lds128_u32(src + 512 + lane * 16);
         const uint32_t kk[4] = {kq.x, kq.y, kq.z, kq.w}, mm[4] = {mq.x, mq.y, mq.z, mq.w};
         float tmax = -INFINITY;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float l[4] = {0.f, 0.f, 0.f, 0.f};
+            float l[4] = {0.f, 0.f, 0.f, 0.f}, x0, x1;
             mma_1688(l, aq, 0u, kk[j]);
-            xv[2 * j] = rbf(l[0]) * scale + fmaf(bf16lo_to_f32(mm[j]), 1e9f, -1e9f);
-            xv[2 * j + 1] = rbf(l[1]) * scale + fmaf(bf16hi_to_f32(mm[j]), 1e9f, -1e9f);
-            tmax = fmax3(tmax, xv[2 * j], xv[2 * j + 1]);
+            xv[j] = fma_f32x2(pack_f32x2(round_to_bf16_f32(l[0]), round_to_bf16_f32(l[1])), scale2,
+                              fma_f32x2(pack_f32x2(bf16lo_to_f32(mm[j]), bf16hi_to_f32(mm[j])), big2, nbig2));
+            unpack_f32x2(xv[j], x0, x1);
+            tmax = fmax3(tmax, x0, x1);
         }
         return tmax;
     };
-    auto accumulate = [&](const float (&xv)[8], const uint4 &vq) {
-        float pv[8];
+    auto accumulate = [&](const uint64_t (&xv)[4], const uint4 &vq) {
+        const uint64_t neg2 = pack_f32x2(-m_run, -m_run);
+        uint32_t pk[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            pv[i] = __expf(xv[i] - m_run);
-            l_run += pv[i];
+        for (int j = 0; j < 4; ++j) {
+            float e0, e1;
+            unpack_f32x2(mul_f32x2(add_f32x2(xv[j], neg2), log2e2), e0, e1);
+            e0 = ex2_approx(e0);
+            e1 = ex2_approx(e1);
+            l2 = add_f32x2(l2, pack_f32x2(e0, e1));
+            pk[j] = pack_bf16x2(e0, e1);
         }
-        const uint32_t pa[4] = {pack_bf16x2(pv[0], pv[1]), 0u, pack_bf16x2(pv[2], pv[3]), 0u};
-        const uint32_t pb[4] = {pack_bf16x2(pv[4], pv[5]), 0u, pack_bf16x2(pv[6], pv[7]), 0u};
+        const uint32_t pa[4] = {pk[0], 0u, pk[1], 0u}, pb[4] = {pk[2], 0u, pk[3], 0u};
         mma_bf16_16816(wa, pa, vq.x, vq.y);
         mma_bf16_16816(wa, pb, vq.z, vq.w);
     };
@@ -345,7 +355,7 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
     // The running max may be stale by up to 5.5 (P below 2^8; it cancels in the division): a step needs a vote and no
     // exchange of maxima unless some row exceeds it by more.
     for (; 2 * (warp + n * WARPS) < nrec; ++n) {
-        float x0[8], x1[8];
+        uint64_t x0[4], x1[4];
         uint4 v0, v1;
         const uint32_t slot = (uint32_t)(n % QN), src = slots + slot * Q_BYTES;
         ok = mbar_wait_warp(bars + 8 * slot, (uint32_t)((n / QN) & 1), a.err, 99);
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
             const float m_new = fmaxf(m_run, tmax);                  // finite: every record holds a row
             const float corr = __expf(m_run - m_new);                // first step: exp(-inf) = 0
             m_run = m_new;
-            l_run *= corr;
+            l2 = mul_f32x2(l2, pack_f32x2(corr, corr));
             wa[0] *= corr;
             wa[1] *= corr;
         }
@@ -372,6 +382,9 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
     if (!ok)
         for (int i = n; i < n + QN && 2 * (warp + i * WARPS) < nrec; ++i)
             mbar_wait_warp(bars + 8 * (uint32_t)(i % QN), (uint32_t)((i / QN) & 1), a.err, 100);
+    float l_run, l_odd;
+    unpack_f32x2(l2, l_run, l_odd);
+    l_run += l_odd;
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
     if (t == 0) {

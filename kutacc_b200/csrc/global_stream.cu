@@ -234,24 +234,28 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
         for (int i = step; i < issued; ++i) mbar_wait_warp(bars + 8 * (uint32_t)(i % NS), (uint32_t)((i / NS) & 1), a.err, 98);
 }
 
-// ---- core: one CTA per column, a warp takes every WARPS-th pair of records -----------------------------------------------
+// ---- core: one CTA per column, whose pairs of records are dealt to SLICES slices -----------------------------------------------
 // A pair is one bulk copy of 2176 bytes into the warp's ring, QN pairs ahead of the arithmetic. (As three copies per record
-// the copies themselves were the bound, 26 us for 61440 records.) Sixteen warps per column whatever the number of columns: a
+// the copies themselves were the bound, 26 us for 61440 records.) Sixteen slices per column whatever the number of columns: a
 // column's sums are split the same way in every batch. More columns than SMs run two CTAs per SM on a shorter ring (250
 // columns x 1500 rows: 41.6 us for the three kernels, with one CTA per SM 44.7); fewer have the longer ring (64 x 5120: 41 us,
-// with the shorter 46). Half of a long column's time is issue slots (about 250 instructions a record with single values; two rows
-// a packed operation and a flushed exponential now: 384 x 5120, the three kernels 164.7 -> 162.9 us).
-constexpr int WARPS = 16, Q_BYTES = 2 * REC_BYTES;
-constexpr int core_smem(int qn) { return WARPS * qn * (Q_BYTES + 8); }
+// with the shorter 46). Where those come in two waves and the columns are short, up to 2048 rows, four CTAs per SM of eight
+// warps, each with two slices one after the other: one wave of the chain from the partial sums to the query instead of two
+// (297 x 128: 17.2 -> 15.7 us, 384 x 512: 31.3 -> 29.7, 384 x 2000: 77.4 -> 77.2; but 384 x 5120: 162.9 -> 163.4, 592 x 3000: 150.6 -> 155.5).
+// Half of a long column's time is issue slots (about 250 instructions a record with single values; two rows a packed operation
+// and a flushed exponential now: 384 x 5120, the three kernels 164.7 -> 162.9 us).
+constexpr int SLICES = 16, Q_BYTES = 2 * REC_BYTES;
+constexpr int core_smem(int warps, int qn) { return warps * qn * (Q_BYTES + 8); }
 
-template <int QN>
-__global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_kernel(const StreamArgs a)
+template <int WARPS, int QN>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 4 : QN == 3 ? 2 : 1) global_softmax_kernel(const StreamArgs a)
 {
-    constexpr int NR = WARPS * 32 / (C + 1);     // row groups of the pooled sums
+    constexpr int NR = 7;                        // row groups of the pooled sums: a thread for each and channel in sixteen warps
+    static_assert(NR * (C + 1) <= SLICES * 32 && SLICES % WARPS == 0, "");
     extern __shared__ __align__(128) unsigned char core_dyn[];
     __shared__ float red[NR][C + 1], qa[C];
     __shared__ __align__(16) float q_s[C];
-    __shared__ float s_m[WARPS][H], s_part[WARPS][H][1 + D];
+    __shared__ float s_m[SLICES][H], s_part[SLICES][H][1 + D];
     release_successor();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.x, nrec = a.nrec;
@@ -264,8 +268,13 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
     __syncwarp();
     wait_for_predecessor();
     const uint64_t policy = l2_evict_first();    // read once, and x should stay
-    auto issue = [&](int i) {                    // this warp's i-th pair
-        const int r0 = 2 * (warp + i * WARPS);
+    const int n_first = max(0, ((nrec + 1) / 2 - warp + SLICES - 1) / SLICES);         // pairs of slice `warp`; slice warp + WARPS follows
+    static_assert(SLICES <= 2 * WARPS, "at most two slices a warp");
+    auto first_record = [&](int i) {             // of this warp's i-th pair; from nrec on there is none
+        return 2 * (WARPS == SLICES || i < n_first ? warp + i * SLICES : warp + WARPS + (i - n_first) * SLICES);
+    };
+    auto issue = [&](int i) {
+        const int r0 = first_record(i);
         if (lane == 0 && r0 < nrec) {
             const uint32_t slot = (uint32_t)(i % QN), bytes = (uint32_t)min(2, nrec - r0) * REC_BYTES;
             mbar_arrive_expect_tx(bars + 8 * slot, bytes);
@@ -274,8 +283,8 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
     };
     for (int i = 0; i < QN; ++i) issue(i);
     const float scale = 1.0f / sqrtf((float)D);
-    if (tid < NR * (C + 1)) {
-        const int grp = tid / (C + 1), ch = tid % (C + 1);
+    for (int i = tid; i < NR * (C + 1); i += WARPS * 32) {
+        const int grp = i / (C + 1), ch = i % (C + 1);
         const float *pp = a.pool + (int64_t)b * a.chunks * POOL_PITCH + ch;
         float s = 0.f;
 #pragma unroll 8
@@ -313,8 +322,8 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
 
     // thread (g, t) owns head g: logits^T [8 heads x 16] = q.k^T, wa [8 x 8] += P.v
     const uint32_t aq = pack_bf16x2(q_s[g * D + 2 * t], q_s[g * D + 2 * t + 1]);
-    float m_run = -INFINITY, wa[4] = {0.f, 0.f, 0.f, 0.f};
-    uint64_t l2 = 0;                             // sums of the even and of the odd rows' probabilities
+    float m_run, wa[4];
+    uint64_t l2;                                 // sums of the even and of the odd rows' probabilities
     const uint64_t scale2 = pack_f32x2(scale, scale), big2 = pack_f32x2(1e9f, 1e9f), nbig2 = pack_f32x2(-1e9f, -1e9f);
     const uint64_t log2e2 = pack_f32x2(kLog2e, kLog2e);
     // logits of the record at `src`, two rows at a time; its v stays in registers
@@ -352,56 +361,62 @@ __global__ void __launch_bounds__(WARPS * 32, QN == 3 ? 2 : 1) global_softmax_ke
     };
     bool ok = true;
     int n = 0;
-    // The running max may be stale by up to 5.5 (P below 2^8; it cancels in the division): a step needs a vote and no
-    // exchange of maxima unless some row exceeds it by more.
-    for (; 2 * (warp + n * WARPS) < nrec; ++n) {
-        uint64_t x0[4], x1[4];
-        uint4 v0, v1;
-        const uint32_t slot = (uint32_t)(n % QN), src = slots + slot * Q_BYTES;
-        ok = mbar_wait_warp(bars + 8 * slot, (uint32_t)((n / QN) & 1), a.err, 99);
-        if (!ok) break;
-        const bool two = 2 * (warp + n * WARPS) + 1 < nrec;
-        float tmax = logits(src, x0, v0);
-        if (two) tmax = fmaxf(tmax, logits(src + REC_BYTES, x1, v1));
-        __syncwarp();
-        issue(n + QN);                           // refills the slot
-        if (__any_sync(0xffffffffu, tmax > m_run + 5.5f)) {
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-            tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-            const float m_new = fmaxf(m_run, tmax);                  // finite: every record holds a row
-            const float corr = __expf(m_run - m_new);                // first step: exp(-inf) = 0
-            m_run = m_new;
-            l2 = mul_f32x2(l2, pack_f32x2(corr, corr));
-            wa[0] *= corr;
-            wa[1] *= corr;
+#pragma unroll 1
+    for (int slice = warp; slice < SLICES && ok; slice += WARPS) {
+        m_run = -INFINITY;
+        l2 = 0;
+        wa[0] = wa[1] = wa[2] = wa[3] = 0.f;
+        // The running max may be stale by up to 5.5 (P below 2^8; it cancels in the division): a step needs a vote and no
+        // exchange of maxima unless some row exceeds it by more.
+        for (int r0 = 2 * slice; r0 < nrec; r0 += 2 * SLICES, ++n) {
+            uint64_t x0[4], x1[4];
+            uint4 v0, v1;
+            const uint32_t slot = (uint32_t)(n % QN), src = slots + slot * Q_BYTES;
+            ok = mbar_wait_warp(bars + 8 * slot, (uint32_t)((n / QN) & 1), a.err, 99);
+            if (!ok) break;
+            const bool two = r0 + 1 < nrec;
+            float tmax = logits(src, x0, v0);
+            if (two) tmax = fmaxf(tmax, logits(src + REC_BYTES, x1, v1));
+            __syncwarp();
+            issue(n + QN);                       // refills the slot
+            if (__any_sync(0xffffffffu, tmax > m_run + 5.5f)) {
+                tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
+                tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
+                const float m_new = fmaxf(m_run, tmax);              // finite: every record holds a row
+                const float corr = __expf(m_run - m_new);            // first step: exp(-inf) = 0
+                m_run = m_new;
+                l2 = mul_f32x2(l2, pack_f32x2(corr, corr));
+                wa[0] *= corr;
+                wa[1] *= corr;
+            }
+            accumulate(x0, v0);
+            if (two) accumulate(x1, v1);
         }
-        accumulate(x0, v0);
-        if (two) accumulate(x1, v1);
+        float l_run, l_odd;
+        unpack_f32x2(l2, l_run, l_odd);
+        l_run += l_odd;
+        l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
+        l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
+        if (t == 0) {
+            s_m[slice][g] = m_run;
+            s_part[slice][g][0] = l_run;
+        }
+        s_part[slice][g][1 + 2 * t] = wa[0];
+        s_part[slice][g][2 + 2 * t] = wa[1];
     }
     // after a wait that ran out: no copy may still be on its way when the CTA exits
     if (!ok)
-        for (int i = n; i < n + QN && 2 * (warp + i * WARPS) < nrec; ++i)
-            mbar_wait_warp(bars + 8 * (uint32_t)(i % QN), (uint32_t)((i / QN) & 1), a.err, 100);
-    float l_run, l_odd;
-    unpack_f32x2(l2, l_run, l_odd);
-    l_run += l_odd;
-    l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
-    l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-    if (t == 0) {
-        s_m[warp][g] = m_run;
-        s_part[warp][g][0] = l_run;
-    }
-    s_part[warp][g][1 + 2 * t] = wa[0];
-    s_part[warp][g][2 + 2 * t] = wa[1];
+        for (int i = n; i < n + QN; ++i)
+            if (first_record(i) < nrec) mbar_wait_warp(bars + 8 * (uint32_t)(i % QN), (uint32_t)((i / QN) & 1), a.err, 100);
     __syncthreads();
     if (tid < C) {
         const int h = tid >> 3, d = tid & 7;
         float mx = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) mx = fmaxf(mx, s_m[w][h]);
+        for (int w = 0; w < SLICES; ++w) mx = fmaxf(mx, s_m[w][h]);
         float l = 0.f, av = 0.f;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
+        for (int w = 0; w < SLICES; ++w) {
             const float f = s_m[w][h] == -INFINITY ? 0.f : __expf(s_m[w][h] - mx);
             l += s_part[w][h][0] * f;
             av += s_part[w][h][1 + d] * f;
@@ -745,8 +760,9 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
     static bool configured = false;
     if (!configured) {
         KUTACC_CUDA(cudaFuncSetAttribute(global_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM));
-        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(3)));
-        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(4)));
+        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(8, 3)));
+        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(16, 3)));
+        KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(16, 4)));
         KUTACC_CUDA(cudaFuncSetAttribute(global_stream_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_SMEM));
         configured = true;
     }
@@ -759,10 +775,13 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
     }
     {
         KernelTimer timer__("global_softmax", stream);
-        if (B > sms)
-            launch_chained(global_softmax_kernel<3>, (unsigned)B, WARPS * 32, core_smem(3), stream, a);
+        const int w16 = (B + 2 * sms - 1) / (2 * sms), w8 = (B + 4 * sms - 1) / (4 * sms);       // waves
+        if (2 * w8 <= w16 && pl.nrec <= 64)
+            launch_chained(global_softmax_kernel<8, 3>, (unsigned)B, 8 * 32, core_smem(8, 3), stream, a);
+        else if (B > sms)
+            launch_chained(global_softmax_kernel<16, 3>, (unsigned)B, 16 * 32, core_smem(16, 3), stream, a);
         else
-            launch_chained(global_softmax_kernel<4>, (unsigned)B, WARPS * 32, core_smem(4), stream, a);
+            launch_chained(global_softmax_kernel<16, 4>, (unsigned)B, 16 * 32, core_smem(16, 4), stream, a);
     }
     {
         KernelTimer timer__("global_stream_out", stream);

@@ -390,11 +390,13 @@ __global__ void __launch_bounds__(256) pair_bias_vec_kernel(const __nv_bfloat16 
     }
 }
 
-// fp32, up to 8 heads: eight lanes share a position, four positions per warp and step, two steps in flight. A lane takes every
+// fp32, up to 8 heads: eight lanes share a position, four positions per warp and step, four steps at once. A lane takes every
 // eighth float4 of the row (the eight lanes read 128 contiguous bytes), weights come from shared memory, and the eight heads'
-// partial sums are reduced by halves, so that lane l ends with head l after seven shuffles instead of 24. Bound by the read
-// of z: 35 -> 19 us (5 of them the timing events) for 256 x 256 positions of 128 channels against one position per warp.
-__global__ void __launch_bounds__(256) pair_bias_f32_kernel(const float *__restrict__ z, const float *__restrict__ wb,
+// partial sums are reduced by halves, so that lane l ends with head l after seven shuffles instead of 24: 35 -> 19 us (5 of them
+// the timing events) for 256 x 256 positions of 128 channels against one position per warp. Bound by the reads of the weights from
+// shared memory (64 to 75 % of what that path can do with two steps at once) more than by z (5 us): four steps share a read, and
+// the next columns are on their way meanwhile. The fp32 layer of 100 x 333 rows 256 -> 252 us, of 128 x 256 rows alone 228 -> 225.5.
+__global__ void __launch_bounds__(256, 2) pair_bias_f32_kernel(const float *__restrict__ z, const float *__restrict__ wb,
                                                             float *__restrict__ nb, int64_t nb_head_stride, int64_t total,
                                                             int Cz, int H, int64_t nk, int64_t nb_row_stride)
 {
@@ -405,21 +407,26 @@ __global__ void __launch_bounds__(256) pair_bias_f32_kernel(const float *__restr
     __syncthreads();
     const int lane = threadIdx.x & 31, l = lane & 7, sub = lane >> 3;
     const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    constexpr int U = 2;
+    constexpr int U = 4;
     for (int64_t p0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (4 * U); p0 < total; p0 += nwarps * (4 * U)) {
         float v[U][8];
         const float4 *zr[U];
+        float4 a[U], next[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int64_t pos = p0 + u * 4 + sub;
-            zr[u] = reinterpret_cast<const float4 *>(z + (pos < total ? pos : 0) * Cz);
+            zr[u] = reinterpret_cast<const float4 *>(z + (pos < total ? pos : 0) * Cz) + l;
+            next[u] = __ldg(zr[u]);
 #pragma unroll
             for (int h = 0; h < 8; ++h) v[u][h] = 0.f;
         }
         for (int c = l; c < Cz / 4; c += 8) {
-            float4 a[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) a[u] = __ldg(zr[u] + c);
+            for (int u = 0; u < U; ++u) {
+                a[u] = next[u];
+                zr[u] += 8;
+                if (c + 8 < Cz / 4) next[u] = __ldg(zr[u]);
+            }
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
                 const float4 w = *reinterpret_cast<const float4 *>(pbw + h * Cz + c * 4);
@@ -680,7 +687,7 @@ bool launch_pair_bias(cudaStream_t stream, ElemType t, const void *z, const void
         }
     }
     if (t == kElemF32 && H <= 8 && pos_stride == 1 && Cz % 32 == 0 && Cz <= 1024 && (((uintptr_t)z | (uintptr_t)wb) & 15u) == 0) {
-        launch_chained(pair_bias_f32_kernel, (unsigned)std::min<int64_t>((pos + 63) / 64, (int64_t)sm_count() * 8), 256, (size_t)8 * Cz * 4, stream,
+        launch_chained(pair_bias_f32_kernel, (unsigned)std::min<int64_t>((pos + 127) / 128, (int64_t)sm_count() * 2), 256, (size_t)8 * Cz * 4, stream,
                        (const float *)z, (const float *)wb, (float *)nb, nb_head_stride, pos, Cz, H, Nk, nb_row_stride);
         count_launch();
         return true;

@@ -122,7 +122,7 @@ struct AttnParams {
 // Tails of 16 keys from column tail_col(c, D) on: beside O, and for heads of 32 half of them over logits already read.
 __device__ __forceinline__ constexpr int tail_col(int c, int D) { return D < 32 ? 96 + 8 * c : c < 2 ? 112 + 8 * c : 16 + 8 * c; }
 
-template <int D, bool SPLIT, bool HAS_NB, bool STAGED>
+template <int D, bool SPLIT, bool HAS_NB, bool STAGED, bool CUT>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_vt, const __grid_constant__ CUtensorMap tm_nb,
@@ -161,7 +161,6 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // item number, publishes it to the other roles through a ring of four shared-memory words (one mbarrier each),
     // and publishes -1 when the list is exhausted. Ring depth: slot i & 3 is written when the products of item i - 2
     // have all been issued, by which time every role has long read the number of item i - 4.
-    constexpr bool CUT = D < 32;
     auto rows_of = [&](int w) { return CUT && w >= p.n_whole ? G / p.parts : G; };
     auto decode = [&](int w, int &q0, int &h, int &b0) {
         int sub = 0;
@@ -739,13 +738,15 @@ int smem_bytes(int G)
            (!HAS_NB ? 0 : STAGED ? 2 : NST) * NB_BYTES;
 }
 
-template <int D, bool SPLIT, bool HAS_NB, bool STAGED>
+template <int D, bool SPLIT, bool HAS_NB, bool STAGED, bool CUT = false>
 bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap &tvt,
                 const CUtensorMap &tnb, const RowMaps<STAGED> &rows, const AttnParams &p)
 {
+    if constexpr (D < 32 && !CUT)
+        if (p.parts > 1) return launch_one<D, SPLIT, HAS_NB, STAGED, true>(stream, tq, tk, tvt, tnb, rows, p);
     static bool configured = false;
     if (!configured) {
-        KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, SPLIT, HAS_NB, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        KUTACC_CUDA(cudaFuncSetAttribute(attn_tc_kernel<D, SPLIT, HAS_NB, STAGED, CUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_bytes<D, HAS_NB, STAGED>(MAXG)));
         configured = true;
     }
@@ -754,7 +755,7 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
     q.counter = work_counter(stream);
     if (q.counter == nullptr) return false;
     KernelTimer timer__("attn_core", stream);
-    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB, STAGED>, grid, THREADS, smem_bytes<D, HAS_NB, STAGED>(p.G), stream, tq, tk, tvt, tnb, rows, q);
+    launch_chained(attn_tc_kernel<D, SPLIT, HAS_NB, STAGED, CUT>, grid, THREADS, smem_bytes<D, HAS_NB, STAGED>(p.G), stream, tq, tk, tvt, tnb, rows, q);
     count_launch();
     return true;
 }
@@ -764,7 +765,9 @@ bool launch_one(cudaStream_t stream, const CUtensorMap &tq, const CUtensorMap &t
 // against one row, at 128, 256, 384 and 1024 positions: four rows 2.4 (with pair bias 3.2), 2.3, 2.1, 1.8 with heads of 32, 1.4 to
 // 2.1 with narrower ones; two rows 1.3 to 1.6 and 1.0 to 1.5. Narrow heads: what is left for the last wave is cut into items of two
 // or one batch rows where that ends sooner: 256 x 256 rows of 4 heads of 16, the whole call, 63.7 -> 62.5 us (with heads of 32 the
-// kernel that can do this lost 1 to 3 % and gained nothing).
+// kernel that can do this lost 1 to 3 % and gained nothing; narrow ones whose items stay whole run without it, 85 x 85 rows of 4
+// heads of 16 24.4 against 24.1 us; without a full wave before them fewer rows for all items do the same for less, 64 x 64 rows 19.6
+// against 18.9 us, 16 x 48 rows of 8 heads of 8 18.9 against 18.4).
 void plan_items(AttnParams &p, int64_t sms, bool cut)
 {
     const int groups[3] = {4, 2, 1};
@@ -772,7 +775,7 @@ void plan_items(AttnParams &p, int64_t sms, bool cut)
     double best = 1e30;
     for (int i = 0; i < 3; ++i) {
         const int64_t items = (int64_t)(p.B + groups[i] - 1) / groups[i] * p.H * p.n_qt, whole = items / sms * sms, last = items - whole;
-        for (int j = i; j < (cut ? 3 : i + 1); ++j) {
+        for (int j = i; j < (cut && whole > 0 ? 3 : i + 1); ++j) {
             const int parts = groups[i] / groups[j];
             const double cost = (double)(whole / sms) * t[i] + (double)((last * parts + sms - 1) / sms) * t[j];
             if (cost < (j > i ? best * 0.99 : best)) {

@@ -43,7 +43,7 @@ namespace dev {
 
 namespace {
 
-constexpr int BM = 128, BN = 128;
+constexpr int BM = 128;
 constexpr int SLAB_BYTES = 128 * 128;                   // 128 rows (or channels) x 32 fp32 or 64 fp16 columns
 constexpr int EPI_WARPS = 8, EPI_WARP0 = 4;
 constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
@@ -103,7 +103,8 @@ __device__ __forceinline__ uint32_t magnitude_bits(const float4 &v)
     return max(a, max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
 }
 
-template <int KS>
+// BN: channels of a column tile, 128 or 64
+template <int KS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ RowsParams p)
 {
@@ -190,7 +191,7 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                     for (int h = 0; h < 2 * KS; ++h) {                 // tails and heads in turn
                         if (round > 0) ok = mbar_wait(w_empty(s), (uint32_t)((round - 1) & 1), p.err, 112);
                         if (!ok) break;
-                        mbar_arrive_expect_tx(w_full(s), SLAB_BYTES);
+                        mbar_arrive_expect_tx(w_full(s), BN * 128);
                         tma_load_2d(smem + (uint32_t)(s * SLAB_BYTES), &maps.w[seg], w_full(s), (h & 1 ? 0 : K) + (h >> 1) * 64, col % p.N);
                         if (++s == NW) {
                             s = 0;
@@ -327,14 +328,14 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
             const bool a_large = a_scale > 1.0f;
             const int m0 = block * BM + quad * 32, m = m0 + lane;
             for (int j = 0; j < nt; ++j, ++tc) {
-                const int buf = tc & 1, col = (t0 + j) * BN + half * 64, seg = col / p.N, n0 = col % p.N;
+                const int buf = tc & 1, col = (t0 + j) * BN + half * (BN / 2), seg = col / p.N, n0 = col % p.N;
                 ok = mbar_wait_warp(acc_full(buf), (uint32_t)((tc / 2) & 1), p.err, 117);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 2 * BN + half * 64);
-                uint32_t acc[2][32];
+                const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 2 * BN + half * (BN / 2));
+                uint32_t acc[BN / 64][32];
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                for (int c = 0; c < BN / 64; ++c) {
                     tmem_ld_32x32(tcol + c * 32, acc[c]);
 #pragma unroll
                     for (int q = 0; q < 32; q += 16) {
@@ -359,7 +360,7 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                     tdst = p.out_t[seg] + ((int64_t)b * (p.N / 32) + n0 / 32) * 64 * p.vt_pitch + (m - b * p.S);
                 }
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                for (int c = 0; c < BN / 64; ++c) {
                     uint32_t(&r)[32] = acc[c];
                     const int nn = n0 + c * 32;
 #pragma unroll
@@ -467,12 +468,12 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const SplitArgs args
     if (lane == 0) args.scale[blockIdx.y][row] = down;
 }
 
-template <int KS>
+template <int KS, int BN>
 void launch_ks(cudaStream_t stream, const RowsMaps &maps, const RowsParams &p, int grid)
 {
-    static const cudaError_t attr = cudaFuncSetAttribute(gemm_f32_rows_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES);
+    static const cudaError_t attr = cudaFuncSetAttribute(gemm_f32_rows_kernel<KS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES);
     KUTACC_CUDA(attr);
-    launch_chained(gemm_f32_rows_kernel<KS>, (unsigned)grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
+    launch_chained(gemm_f32_rows_kernel<KS, BN>, (unsigned)grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
 }
 
 }  // namespace
@@ -509,6 +510,12 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
         if ((((uintptr_t)w_split[i] | (uintptr_t)out[i] | (uintptr_t)bias[i]) & 15u) != 0) return false;
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
+    // Few rows: column tiles of half the width where those of four such products run at once; a product is then as long as one
+    // tile's chain: fp32 layer of 8 x 48 rows 34.5 -> 32.6 us, of 8 x 130 rows 45.0 -> 39.0. The rule does not look at nseg, so that a
+    // layer's projections and output run the same code: an output product alone in half tiles cost 40 x 60 rows 44.9 -> 48.9 us.
+    const int sms = std::max(1, sm_count() - runtime().sm_margin);
+    const int64_t blocks = (M + BM - 1) / BM;
+    const int BN = blocks * (N / 64) * 4 <= sms ? 64 : 128;
     RowsMaps maps;
     RowsParams p = {};
     if (!make_tensor_map_2d(&maps.a, a, /*elem_bytes=*/4, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 32, BM, 128)) return false;
@@ -518,7 +525,7 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
         p.w_scale[i] = (const float *)((const char *)w_split[j] + (size_t)N * K * 4);
         p.layout[i] = layout ? layout[j] : kTf32Rows;
         p.out_t[i] = (float *)out[j];
-        if (!make_tensor_map_2d(&maps.w[i], w_split[j], 2, (uint64_t)2 * K, (uint64_t)N, (uint64_t)2 * K, 64, 128, 128)) return false;
+        if (!make_tensor_map_2d(&maps.w[i], w_split[j], 2, (uint64_t)2 * K, (uint64_t)N, (uint64_t)2 * K, 64, BN, 128)) return false;
         const uint64_t cols = p.layout[i] == kTf32SplitRows ? 2 * (uint64_t)N : (uint64_t)N;
         if (p.layout[i] == kTf32SplitTransposed)
             maps.out[i] = maps.a;                            // stored directly
@@ -533,8 +540,7 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
     p.err = ew.device;
     // As in gemm_proj.cu: whole blocks for all full waves, the blocks of the last one in 1 / nsplit of their column tiles each. A
     // unit costs its column tiles and about two for the way of its rows into shared memory and their split.
-    const int sms = std::max(1, sm_count() - runtime().sm_margin);
-    const int64_t blocks = (M + BM - 1) / BM, whole = blocks / sms * sms;
+    const int64_t whole = blocks / sms * sms;
     double best = 1e30;
     for (int ns = 1; ns <= p.tiles; ++ns) {
         if (p.tiles % ns != 0 || (blocks - whole) * ns + whole > INT32_MAX / 2) continue;
@@ -549,7 +555,10 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
     }
     const int grid = std::min(p.units, sms);
     KernelTimer timer__("gemm_tf32x3_tc", stream);           // the name of the fp32 tensor-memory products, whichever kernel
-    K == 128 ? launch_ks<2>(stream, maps, p, grid) : launch_ks<4>(stream, maps, p, grid);
+    if (BN == 64)
+        K == 128 ? launch_ks<2, 64>(stream, maps, p, grid) : launch_ks<4, 64>(stream, maps, p, grid);
+    else
+        K == 128 ? launch_ks<2, 128>(stream, maps, p, grid) : launch_ks<4, 128>(stream, maps, p, grid);
     count_launch();
     return true;
 }

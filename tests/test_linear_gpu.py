@@ -138,8 +138,10 @@ def test_pair_bias_written_with_the_heads_inside_the_rows(kutacc_lib, R, Nk, Cz,
     assert (store[:, H, :] == 7.0).all()
 
 
-# rows around the 128-row block, calls of more blocks than SMs (whole blocks, then parts of blocks), one to three column tiles
-@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (127, 128, 256), (129, 384, 128), (300, 256, 256), (19200, 384, 128), (19201, 128, 256)])
+# rows around the 128-row block, calls of more blocks than SMs (whole blocks, then parts of blocks), one to three column tiles, the last
+# size with tiles of half the width and the first without
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (127, 128, 256), (129, 384, 128), (300, 256, 256), (1152, 256, 256), (1153, 256, 128),
+                                   (19200, 384, 128), (19201, 128, 256)])
 def test_linear_fp32_rows_of_any_magnitude(kutacc_lib, M, N, K):
     # powers of two up to 2^60 between rows, channels and columns (the latter against their weights), a row of zeros
     rng = np.random.default_rng(M + N + K)

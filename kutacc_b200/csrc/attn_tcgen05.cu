@@ -31,7 +31,8 @@
 // MMA chain of a tile. Four independent chains per SM hide it: while one warp group waits for its products, the warps
 // of the other three fill the issue slots of the same schedulers. Measured: triangle attention at 1024 residues (4.3 G
 // logits) 2.16 -> 1.57 ms, column attention 384 x 512 x 8 heads 0.41 -> 0.31 ms against two CTAs per SM with one (batch row,
-// head, 128 queries) each, P through shared memory and two threads per query row. The single-thread cost of the MMA
+// head, 128 queries) each, P through shared memory and two threads per query row. (Now 1.49 and 0.27 ms, see STAGED.) A share of the
+// exponentials on the FMA units, 1 to 4 of 8 pairs, made the call 5 to 22 % longer: instructions are what is short. The single-thread cost of the MMA
 // and TMA instructions mattered as much as the split: behind `lane == 0` an instruction took about 70 clocks to
 // issue, behind elect_one() about 33.
 //

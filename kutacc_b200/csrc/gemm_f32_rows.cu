@@ -15,14 +15,17 @@
 // The activations stand still, as in gemm_proj.cu: a persistent CTA (one per SM) loads 128 rows, all K columns, as fp32; the
 // epilogue warps split them where they lie (the head and tail of a row take just the bytes of its fp32 values), and the
 // weights, split by a kernel of their own (a row of them is used by every CTA), stream past in slabs of 128 channels x 64 columns.
-//   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (tail and head in turn, a ring of five or eight)
-//   warp 1      MMA issuer: 12 instructions a tail and head into a pair of 128 x 128 accumulators (two pairs in tensor memory)
+//   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (tail and head in turn, a ring of four or eight)
+//   warp 1      MMA issuer: 12 instructions a tail and head into a pair of 128 x 128 accumulators (two pairs in tensor memory;
+//               128 x 64 for few rows)
 //   warps 4-11  split the rows, 16 each; epilogue, 32 rows x 64 columns each: tcgen05.ld of both accumulators, scaling, bias,
-//               staging tile (32 x 16), TMA store
-// What bounds it: the products (128 x 128 instructions, each weight slab used for one block of rows) and, twice per CTA at the size
-// below, the way of a block into shared memory and its split, which nothing overlaps. 32768 rows x 256 channels, four projections:
-// 80 us (HBM 31, products 31); as a split of the activations and tf32 products 20 + 92. Error against 64 bits at K = 128 and 256
-// (2-norm): 2.0e-7 and 3.5e-7, before 3.4e-7 and 6.4e-7. The fp32 layer of 128 x 256 rows: 288 -> 227 us.
+//               one of two staging tiles (32 x 16), TMA store
+// What bounds it: the way of the results out of the SM beside the products, and, twice per CTA at the size below, the way of a block
+// into shared memory and its split, which nothing overlaps. With parts taken out of copies, 32768 x 1024 x 256: complete 96 us, without
+// stores 82, without products 87, without both 57, without the split 92, with an eighth of the weights' bytes 93. 32768 rows x 256
+// channels, four projections: 80 us (HBM 31, products 31); as a split of the activations and tf32 products 20 + 92. Error
+// against 64 bits at K = 128 and 256 (2-norm): 2.0e-7 and 3.5e-7, before 3.4e-7 and 6.4e-7. The fp32 layer of 128 x 256 rows: 288 -> 227 us (now 214, with the
+// slabs freed one by one, the second staging tile and a faster attention core).
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is
 // released and the host-visible error word carries the site.

@@ -4,7 +4,7 @@
 // output needs the softmax over all its rows: two passes over x that nothing can join. A single kernel that holds each
 // column in the shared memory of a thread-block cluster reads x once, but its stages (pool, exchange, softmax, exchange,
 // output) run one after another with two columns per SM, and it is bound by that chain: 235 us at 384 x 5120 rows where
-// its bytes take 77 (166 us here). Here every stage is a stream with enough independent work in flight:
+// its bytes take 77 (163 us here). Here every stage is a stream with enough independent work in flight:
 //   kv    x once: masked partial sums of every 32 or 64 rows, k = x.Wk^T and v = x.Wv^T (bf16, 32 bytes per row)        (:44-89)
 //   core  one CTA per column: q from the partial sums, logits, softmax, weighted v from k and v                      (:76-133)
 //   out   x again, last rows first (what the kv kernel read last is still in L2): gate, gated average, output     (:90-94, :134-163)
@@ -242,8 +242,8 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
 // with the shorter 46). Where those come in two waves and the columns are short, up to 2048 rows, four CTAs per SM of eight
 // warps, each with two slices one after the other: one wave of the chain from the partial sums to the query instead of two
 // (297 x 128: 17.2 -> 15.7 us, 384 x 512: 31.3 -> 29.7, 384 x 2000: 77.4 -> 77.2; but 384 x 5120: 162.9 -> 163.4, 592 x 3000: 150.6 -> 155.5).
-// Half of a long column's time is issue slots (about 250 instructions a record with single values; two rows a packed operation
-// and a flushed exponential now: 384 x 5120, the three kernels 164.7 -> 162.9 us).
+// Half of a long column's time is issue slots (two rows a packed operation and a flushed exponential: 141 instructions a record
+// of 32 rows; 384 x 5120, the three kernels 164.7 -> 162.9 us).
 constexpr int SLICES = 16, Q_BYTES = 2 * REC_BYTES;
 constexpr int core_smem(int warps, int qn) { return warps * qn * (Q_BYTES + 8); }
 

@@ -40,3 +40,15 @@ def test_a_column_does_not_depend_on_the_number_of_columns(kutacc_lib):
     few = W.Workload(name="few", kind="global", dtype=w.dtype, B=3, S=w.S, H=w.H, D=w.D, seed=0, has_nb=w.has_nb)
     few.arrays = dict(w.arrays, x=w.arrays["x"][:3], mask=w.arrays["mask"][:3])
     assert np.array_equal(many[:3], runner.out_to_f32(runner.DeviceCase(few).run()))
+
+
+# sixteen warps a column in one wave; eight where two waves become one, up to their longest column; sixteen past it and in three waves
+@pytest.mark.parametrize("B,S", [(200, 700), (297, 31), (297, 2048), (297, 2049), (593, 40)])
+def test_columns_do_not_depend_on_the_warps_they_share(kutacc_lib, B, S):
+    w = W.random_global_case(seed=79 + S, B=B, S=S, zero_mask_rows=1)
+    many = runner.out_to_f32(runner.DeviceCase(w).run())
+    pick = [0, 1, B // 2, B - 1]
+    few = W.Workload(name="few", kind="global", dtype=w.dtype, B=len(pick), S=S, H=w.H, D=w.D, seed=0, has_nb=w.has_nb)
+    few.arrays = dict(w.arrays, x=w.arrays["x"][pick], mask=w.arrays["mask"][pick])
+    assert np.array_equal(many[pick], runner.out_to_f32(runner.DeviceCase(few).run()))
+    assert helpers.rel_err(many[pick], helpers.oracle_faithful(few)) <= helpers.BF16_TOL

@@ -132,10 +132,10 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     // fp32 on the tensor-memory kernels (head size 32): k and v are stored split into tf32 head and tail
     const bool f32_split = dt == kFP32 && C % 128 == 0 && D == 32 && out_rs % 4 == 0;
     // fp32 on the tensor-memory GEMM: operands split into tf32 head and tail (activations: one [M, 2C] buffer that the
-    // projection and, later, the output projection use in turn; five weights [C, 2C])
+    // projection and, later, the output projection use in turn; five weights [C, 2C]);
     const bool f32_tc = dt == kFP32 && C % 128 == 0 && out_rs % 4 == 0;
-    // up to 256 channels the product splits its activations itself, into fp16 heads and tails at twice the rate (128 x 256 rows of
-    // 256 channels: 81 us for the projections, 92 and 20 for the split before them the other way)
+    // up to 256 channels the product splits its activations itself, into three bf16 pieces (128 x 256 rows of 256 channels: 68 us for the
+    // projections, 92 and 20 for the split before them the other way)
     const bool f32_rows = f32_tc && C <= 256;
     // The TMA loads of the pair bias need 16-byte aligned rows. A pair bias whose strides are not
     // multiples of 16 bytes, or are zero (one head or one query row for all), is first copied into the workspace with padded rows;
@@ -153,7 +153,7 @@ static void gating_attention_impl(Tensor &input, int64_t batch, int64_t seq_len,
     const size_t nb_pad_bytes = nb_repitch ? (size_t)H * S * s_pad8 * es : 0;
     const size_t fold_bytes = ln_folded ? (size_t)M * 8 + 256 + 4 * (w_bytes + 256) + 8 * (b_bytes + 256) : 0;
     const size_t norm_bytes = ln_copied ? x_bytes + 256 : 0;
-    const size_t ws_bytes = f32_rows ? w_bytes + b_bytes : 2 * w_bytes;                 // a split weight
+    const size_t ws_bytes = f32_rows ? w_bytes / 2 * 3 : 2 * w_bytes;                 // a split weight
     const size_t f32_bytes = f32_tc ? (f32_rows ? 0 : 2 * x_bytes + 256) + 5 * (ws_bytes + 256) : 0;
     if (!rt.reserve_workspace(3 * (x_bytes + 256) + k_bytes + 256 + v_bytes + 256 + nb_pad_bytes + 256 + fold_bytes + norm_bytes + f32_bytes))
         return;

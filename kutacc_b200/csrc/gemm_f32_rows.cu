@@ -3,29 +3,29 @@
 //   C[m, n] = sum_k A[m, k] * W[n, k] (+ bias[n])         A [M, K] fp32, W [N, K] fp32 (W[out][in]), C fp32, K = 128 or 256
 //
 // (the four projections of the fp32 attention in one pass, its output projection, kutacc_af2_linear on fp32 tensors;
-// src/attention/gating_attention.cpp:47-66,152-157; src/linear/mm.cpp:46-86.) tcgen05.mma has no fp32 input type. Every row of A and of
-// W is brought to a largest element in [2^14, 2^15) by a power of two and split into an fp16 head and an fp16 tail, the tail
-// times 2^11 so that it has the range of the head: x * 2^s = hi + lo * 2^-11 with 22 bits, for elements down to 2^-29 of their row's
-// largest, and an error of 2^-51 of that one below. The product is
-//   hi(A).hi(W) + 2^-11 (lo(A).hi(W) + hi(A).lo(W))        (lo.lo, about 2^-22 of the result, is dropped)
-// with the small products in an accumulator of their own, and the powers of two are taken back in the epilogue. Against tf32
-// heads and tails (gemm_tf32_tcgen05.cu, which keeps all other K) an operand has half the bytes and the tensor cores twice
-// the rate, and there are half as many accumulations, each of which truncates.
+// src/attention/gating_attention.cpp:47-66,152-157; src/linear/mm.cpp:46-86.) tcgen05.mma has no fp32 input type. An element is
+// split into three bf16 pieces, x = x0 + x1 + x2: each has eight bits and the exponent range of fp32, together they are x itself, whatever
+// the other elements of its row are. The product is
+//   x0.w0 + (x0.w1 + x1.w0 + x1.w1 + x0.w2 + x2.w0)        (the other three, below 2^-22 of the first, are dropped)
+// with the five small products in an accumulator of their own, which the epilogue adds: the tensor core truncates at every
+// accumulation, and only K / 16 of them are at full magnitude. Against tf32 heads and tails (gemm_tf32_tcgen05.cu, which keeps all
+// other K: three products at half the rate) the tensor cores have the same work, but an operand 6 bytes instead of 8, its activations
+// are read once, and half as many accumulations count. (fp16 heads and tails with a power of two per row need half the
+// work, three products at the full rate, but hold elements below 2^-29 of their row's largest in fewer bits and from 2^-51 on not at all.)
 //
 // The activations stand still, as in gemm_proj.cu: a persistent CTA (one per SM) loads 128 rows, all K columns, as fp32; the
-// epilogue warps split them where they lie (the head and tail of a row take just the bytes of its fp32 values), and the
-// weights, split by a kernel of their own (a row of them is used by every CTA), stream past in slabs of 128 channels x 64 columns.
-//   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (tail and head in turn, a ring of four or eight)
-//   warp 1      MMA issuer: 12 instructions a tail and head into a pair of 128 x 128 accumulators (two pairs in tensor memory;
-//               128 x 64 for few rows)
-//   warps 4-11  split the rows, 16 each; epilogue, 32 rows x 64 columns each: tcgen05.ld of both accumulators, scaling, bias,
-//               one of two staging tiles (32 x 16), TMA store
-// What bounds it: the way of the results out of the SM beside the products, and, twice per CTA at the size below, the way of a block
-// into shared memory and its split, which nothing overlaps. With parts taken out of copies, 32768 x 1024 x 256: complete 96 us, without
-// stores 82, without products 87, without both 57, without the split 92, with an eighth of the weights' bytes 93. 32768 rows x 256
-// channels, four projections: 80 us (HBM 31, products 31); as a split of the activations and tf32 products 20 + 92. Error
-// against 64 bits at K = 128 and 256 (2-norm): 2.0e-7 and 3.5e-7, before 3.4e-7 and 6.4e-7. The fp32 layer of 128 x 256 rows: 288 -> 227 us (now 214, with the
-// slabs freed one by one, the second staging tile and a faster attention core).
+// epilogue warps split them, the first two pieces into tensor memory, where two thirds of the products read them without a byte of
+// shared memory, the third where the fp32 values were; and the weights, split by a kernel of their own (a row of them
+// is used by every CTA), stream past in slabs of 128 channels x 64 columns.
+//   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (third, second, first pieces of 64 columns, a ring of five or eight)
+//   warp 1      MMA issuer: 24 instructions of 16 columns for every 64, into two 128 x 128 accumulators (128 x 64 for few rows), of which the
+//               epilogue takes the small products first: the next tile begins while it waits for the large ones
+//   warps 4-11  split the rows, a thread half a row; epilogue, 32 rows x 64 columns each: tcgen05.ld of both accumulators, which frees them,
+//               the split of the next block once the last tile of this one is in registers, bias, staging tile (32 x 16), TMA store
+// What bounds it: the tensor cores and the power they take. 32768 rows x 1024 channels x 256 columns: 68 us, 117000 clocks of a CTA (for
+// its 14 tiles of 6144 clocks of products, and 14000 before the first, whose rows come from HBM), at 1.75 GHz under the power limit; with fp16
+// pairs 65. As a split of the activations and tf32 products 20 + 92. x 128 columns 45 us. Error against 64 bits at K = 128 and 256 (2-norm):
+// 1.3e-7 and 2.4e-7 (tf32 3.4e-7 and 6.4e-7, fp16 pairs 2.0e-7 and 3.5e-7). The fp32 layer of 128 x 256 rows: 290 us with tf32, 234 (fp16 pairs 217).
 //
 // All mbarrier waits are bounded; on a timeout the roles fall through to the common tail, the TMEM allocation is
 // released and the host-visible error word carries the site.
@@ -35,8 +35,6 @@
 #include "ptx_utils.cuh"
 #include "tcgen05_utils.cuh"
 #include "tma_utils.cuh"
-
-#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <climits>
@@ -51,59 +49,49 @@ constexpr int SLAB_BYTES = 128 * 128;                   // 128 rows (or channels
 constexpr int EPI_WARPS = 8, EPI_WARP0 = 4;
 constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
 constexpr int STG_BYTES = 32 * 16 * 4;
-constexpr float kTail = 1.0f / 2048;                    // weight of the small products
 
-// KS: 64-column slabs of a row
-template <int KS>
+// KS: 64-column slabs of a row, BN: channels of a column tile
+template <int KS, int BN>
 struct Geo {
-    static constexpr int NW = KS == 4 ? 4 : 8;                                   // slabs of the weight ring
+    static constexpr int NW = KS == 4 ? 5 : 8;                                   // slabs of the weight ring
+    static constexpr int NSTG = KS == 4 ? 1 : 2;                                 // staging tiles of a warp
+    static constexpr int ACC_COL = 64 * KS;                                      // after the first and second pieces of the rows
     static constexpr int OFF_A = NW * SLAB_BYTES;
     static constexpr int OFF_STG = OFF_A + 2 * KS * SLAB_BYTES;
-    static constexpr int OFF_SCALE = OFF_STG + EPI_WARPS * 2 * STG_BYTES;            // of the rows of two blocks
-    static constexpr int OFF_BAR = OFF_SCALE + 2 * BM * 4;
-    static constexpr int NBARS = 2 * NW + 2 * KS + 5;
+    static constexpr int OFF_BAR = OFF_STG + EPI_WARPS * NSTG * STG_BYTES;
+    static constexpr int NBARS = 2 * NW + 3 * KS + 4;
+    static_assert(ACC_COL + 2 * BN <= 512, "tensor memory");
     static constexpr int SMEM_BYTES = OFF_BAR + 8 * NBARS + 16 + 1024;
     static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA");
 };
 
 struct alignas(64) RowsMaps {
     CUtensorMap a;        // A [M][K] fp32, box [32, 128], 128-byte swizzle
-    CUtensorMap w[4];     // W' [N][2K] fp16 (head | tail) per segment, box [64, 128], 128-byte swizzle
+    CUtensorMap w[4];     // W' [N][3K] bf16 (the three pieces one after another) per segment, box [64, BN], 128-byte swizzle
     CUtensorMap out[4];   // per segment [M][N] (split rows: [M][2N]) fp32, box [16, 32], 64-byte swizzle
 };
 
 struct RowsParams {
     const float *bias[4];   // per segment, may be null
-    const float *w_scale[4];
     float *out_t[4];        // kTf32SplitTransposed segments: [B][N/32][64][S]
     int layout[4];          // per segment: Tf32Layout
     int M, N, tiles;        // column tiles of all segments
     int S;                  // rows per batch row (transposed segments)
     int64_t vt_pitch;
-    int whole, nsplit, units;       // as in gemm_proj.cu: blocks with all their column tiles, then parts of blocks
+    int whole;              // blocks with all their column tiles, full waves of them
+    int rest, per, units;   // the tiles of the blocks after them, how many of these in a row are a unit, and whole blocks and units
     int *err;
 };
 
-// exponent that brings the largest magnitude (its bits) to [2^14, 2^15), as the bits of 2^s and of 2^-s
-__device__ __forceinline__ void scale_of(uint32_t max_bits, float &up, float &down)
+// Two elements in three packed bf16 pieces each, x = x0 + x1 + x2: x0 the upper half of the bits, x1 the rest rounded, x2 what is left,
+// which has eight bits.
+__device__ __forceinline__ void split_bf16(float a, float b, uint32_t &x0, uint32_t &x1, uint32_t &x2)
 {
-    const int s = min(268 - (int)(max_bits >> 23), 253);           // biased; rows below 2^-112 keep 2^126
-    up = __int_as_float(s << 23);
-    down = __int_as_float((254 - s) << 23);
-}
-// two elements, already scaled: packed heads and packed tails
-__device__ __forceinline__ void split_f16(float x0, float x1, uint32_t &hi, uint32_t &lo)
-{
-    const __half2 h = __floats2half2_rn(x0, x1);
-    const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn((x0 - f.x) * 2048.f, (x1 - f.y) * 2048.f);
-    hi = *reinterpret_cast<const uint32_t *>(&h);
-    lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-__device__ __forceinline__ uint32_t magnitude_bits(const float4 &v)
-{
-    const uint32_t a = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
-    return max(a, max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
+    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+    x0 = __byte_perm(ua, ub, 0x7632);
+    const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
+    x1 = pack_bf16x2(ra, rb);
+    x2 = __byte_perm(__float_as_uint(ra - bf16lo_to_f32(x1)), __float_as_uint(rb - bf16hi_to_f32(x1)), 0x7632);
 }
 
 // BN: channels of a column tile, 128 or 64
@@ -111,28 +99,33 @@ template <int KS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constant__ RowsParams p)
 {
-    using T = Geo<KS>;
+    using T = Geo<KS, BN>;
     constexpr int K = 64 * KS, NW = T::NW;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    unsigned char *gen = smem_raw + (smem - smem_u32(smem_raw));
     const uint32_t bar = smem + T::OFF_BAR;
     auto w_full = [&](int s) { return bar + 8u * (uint32_t)s; };
     auto w_empty = [&](int s) { return bar + 8u * (uint32_t)(NW + s); };
     auto a_full = [&](int ks) { return bar + 8u * (uint32_t)(2 * NW + ks); };
     auto a_empty = [&](int ks) { return bar + 8u * (uint32_t)(2 * NW + KS + ks); };
-    const uint32_t a_split = bar + 8u * (2 * NW + 2 * KS);
-    auto acc_full = [&](int b) { return a_split + 8u + 8u * (uint32_t)b; };
-    auto acc_empty = [&](int b) { return a_split + 24u + 8u * (uint32_t)b; };
+    auto a_split = [&](int ks) { return bar + 8u * (uint32_t)(2 * NW + 2 * KS + ks); };
+    const uint32_t small_full = bar + 8u * (uint32_t)(2 * NW + 3 * KS), small_empty = small_full + 8u, large_full = small_full + 16u,
+                   large_empty = small_full + 24u;
     const uint32_t tmem_slot = bar + 8u * T::NBARS;
-    float *const row_scale = reinterpret_cast<float *>(gen + T::OFF_SCALE);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    // unit u: its block, first column tile and number of column tiles
-    auto unit = [&](int u, int &block, int &t0, int &nt) {
-        const int v = u - p.whole;
-        block = v < 0 ? u : p.whole + v / p.nsplit;
-        nt = v < 0 ? p.tiles : p.tiles / p.nsplit;
-        t0 = v < 0 ? 0 : v % p.nsplit * nt;
+    // This CTA's next part of its units: a block, its first column tile and how many. u: the unit, at: tiles of it handed out
+    auto next_part = [&](int &u, int &at, int &block, int &t0, int &nt) -> bool {
+        if (u >= p.units) return false;
+        const int v = u - p.whole, first = v * p.per, n = v < 0 ? p.tiles : min(p.per, p.rest - first);
+        block = v < 0 ? u : p.whole + (first + at) / p.tiles;
+        t0 = v < 0 ? 0 : (first + at) % p.tiles;
+        nt = min(p.tiles - t0, n - at);
+        at += nt;
+        if (at == n) {
+            at = 0;
+            u += (int)gridDim.x;
+        }
+        return true;
     };
 
     if (threadIdx.x == 0) {
@@ -143,12 +136,12 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
         for (int ks = 0; ks < KS; ++ks) {
             mbar_init(a_full(ks), 1);
             mbar_init(a_empty(ks), 1);
+            mbar_init(a_split(ks), 4);
         }
-        mbar_init(a_split, EPI_WARPS);
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(acc_full(b), 1);
-            mbar_init(acc_empty(b), EPI_WARPS);
-        }
+        mbar_init(small_full, 1);
+        mbar_init(small_empty, EPI_WARPS);
+        mbar_init(large_full, 1);
+        mbar_init(large_empty, EPI_WARPS);
         fence_barrier_init();
     }
     if (warp == 1) {
@@ -176,11 +169,9 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
         if (elect_one()) {
             bool ok = true;
             int s = 0, round = 0;                                      // next slab's slot, times the ring has gone round
-            for (int n = 0; ok; ++n) {
-                const int u = (int)blockIdx.x + n * (int)gridDim.x;
-                if (u >= p.units) break;
+            for (int n = 0, u = (int)blockIdx.x, at = 0; ok; ++n) {
                 int block, t0, nt;
-                unit(u, block, t0, nt);
+                if (!next_part(u, at, block, t0, nt)) break;
                 for (int ks = 0; ks < KS && ok; ++ks) {
                     if (n > 0) ok = mbar_wait(a_empty(ks), (uint32_t)((n - 1) & 1), p.err, 111);
                     if (!ok) break;
@@ -191,170 +182,167 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                 }
                 for (int j = 0; j < nt && ok; ++j) {
                     const int col = (t0 + j) * BN, seg = col / p.N;
-                    for (int h = 0; h < 2 * KS; ++h) {                 // tails and heads in turn
+                    for (int h = 0; h < 3 * KS; ++h) {                 // of every 64 columns the third, second, first pieces
                         if (round > 0) ok = mbar_wait(w_empty(s), (uint32_t)((round - 1) & 1), p.err, 112);
                         if (!ok) break;
                         mbar_arrive_expect_tx(w_full(s), BN * 128);
-                        tma_load_2d(smem + (uint32_t)(s * SLAB_BYTES), &maps.w[seg], w_full(s), (h & 1 ? 0 : K) + (h >> 1) * 64, col % p.N);
+                        tma_load_2d(smem + (uint32_t)(s * SLAB_BYTES), &maps.w[seg], w_full(s), (2 - h % 3) * K + h / 3 * 64, col % p.N);
                         if (++s == NW) {
                             s = 0;
                             ++round;
                         }
+                    }
+                    if (j == 0) {                                      // the next block's rows on their way to L2
+                        int u2 = u, at2 = at, next, nt0, nnt;
+                        if (next_part(u2, at2, next, nt0, nnt))
+                            for (int c = 0; c < 2 * KS; ++c) tma_prefetch_2d(&maps.a, c * 32, next * BM);
                     }
                 }
             }
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        constexpr uint32_t idesc = make_instr_desc_f16(BM, BN);
+        constexpr uint32_t idesc = make_instr_desc_bf16(BM, BN);
         constexpr uint32_t SLAB16 = SLAB_BYTES >> 4;                   // descriptor addresses count in units of 16 bytes
         const uint64_t wd0 = make_smem_desc_kmajor(smem, 128), ad0 = make_smem_desc_kmajor(smem + T::OFF_A, 128);
         bool ok = true;
         int s = 0, tc = 0;
         uint32_t par = 0;
-        auto next_slab = [&]() {
-            if (++s == NW) {
-                s = 0;
-                par ^= 1u;
-            }
-        };
-        for (int n = 0; ok; ++n) {
-            const int u = (int)blockIdx.x + n * (int)gridDim.x;
-            if (u >= p.units) break;
+        for (int n = 0, u = (int)blockIdx.x, at = 0; ok; ++n) {
             int block, t0, nt;
-            unit(u, block, t0, nt);
-            ok = mbar_wait_warp(a_split, (uint32_t)(n & 1), p.err, 113);
+            if (!next_part(u, at, block, t0, nt)) break;
             for (int j = 0; j < nt && ok; ++j, ++tc) {
-                const int buf = tc & 1;
-                if (tc >= 2) ok = mbar_wait_warp(acc_empty(buf), (uint32_t)((tc / 2 - 1) & 1), p.err, 114);
-                const uint32_t d = tmem_base + (uint32_t)(buf * 2 * BN);
+                if (tc > 0) ok = mbar_wait_warp(small_empty, (uint32_t)((tc - 1) & 1), p.err, 114);
+                const uint32_t large = tmem_base + (uint32_t)T::ACC_COL, small = large + BN;
                 for (int ks = 0; ks < KS && ok; ++ks) {
-                    // head.tail, then tail.head and head.head: each slab is freed as soon as it can be
-                    ok = mbar_wait_warp(w_full(s), par, p.err, 115);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint64_t a = ad0 + (uint32_t)(ks * 2 * SLAB16);
-                    if (elect_one()) {
-                        const uint64_t w = wd0 + (uint32_t)(s * SLAB16);
+                    if (j == 0) ok = mbar_wait_warp(a_split(ks), (uint32_t)(n & 1), p.err, 113);
+                    const uint32_t a0 = tmem_base + (uint32_t)(ks * 64), a1 = a0 + 32;
+                    const uint64_t a2 = ad0 + (uint32_t)(ks * 2 * SLAB16);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)                    // 16 columns = 32 bytes an instruction
-                            tc_mma_bf16(d + BN, a + 2 * k, w + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
-                        tc_commit(w_empty(s));
+                    for (int piece = 2; piece >= 0; --piece) {         // of W
+                        ok = ok && mbar_wait_warp(w_full(s), par, p.err, 115);
+                        if (ks == 0 && piece == 0 && tc > 0) ok = ok && mbar_wait_warp(large_empty, (uint32_t)((tc - 1) & 1), p.err, 118);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {
+                            // 16 columns an instruction: 32 bytes, or 8 columns of tensor memory
+                            const uint64_t w = wd0 + (uint32_t)(s * SLAB16);
+                            if (piece > 0) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) tc_mma_bf16_ts(small, a0 + 8 * k, w + 2 * k, idesc, piece == 1 || ks > 0 || k > 0 ? 1u : 0u);
+                            }
+                            if (piece < 2) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) tc_mma_bf16_ts(small, a1 + 8 * k, w + 2 * k, idesc, 1u);
+                            }
+                            if (piece == 0) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) tc_mma_bf16(small, a2 + 2 * k, w + 2 * k, idesc, 1u);
+                                if (ks == KS - 1) tc_commit(small_full);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) tc_mma_bf16_ts(large, a0 + 8 * k, w + 2 * k, idesc, ks > 0 || k > 0 ? 1u : 0u);
+                                if (j == nt - 1) tc_commit(a_empty(ks));
+                                if (ks == KS - 1) tc_commit(large_full);
+                            }
+                            tc_commit(w_empty(s));
+                        }
+                        __syncwarp();
+                        if (++s == NW) {
+                            s = 0;
+                            par ^= 1u;
+                        }
                     }
-                    __syncwarp();
-                    next_slab();
-                    ok = mbar_wait_warp(w_full(s), par, p.err, 115);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (elect_one()) {
-                        const uint64_t w = wd0 + (uint32_t)(s * SLAB16);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) tc_mma_bf16(d + BN, a + SLAB16 + 2 * k, w + 2 * k, idesc, 1u);
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) tc_mma_bf16(d, a + 2 * k, w + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
-                        tc_commit(w_empty(s));
-                        if (j == nt - 1) tc_commit(a_empty(ks));
-                        if (ks == KS - 1) tc_commit(acc_full(buf));
-                    }
-                    __syncwarp();
-                    next_slab();
                 }
             }
         }
     } else if (warp >= EPI_WARP0) {
         // ================= split, epilogue =================
         const int ew = warp - EPI_WARP0, half = ew >> 2, quad = warp & 3;
-        const uint32_t stg0 = smem + T::OFF_STG + (uint32_t)(ew * 2 * STG_BYTES);
+        const uint32_t stg0 = smem + T::OFF_STG + (uint32_t)(ew * T::NSTG * STG_BYTES);
         uint32_t nstore = 0;
         bool ok = true;
 
-        // 16 rows of the block: LPR lanes share a row, eight columns each
-        constexpr int LPR = K / 8, RPP = 32 / LPR, U = 4;
+        // a thread's row, of every 64 columns that this half of the warps takes: the fp32 values make way for the first pieces (where
+        // columns 0..31 lay) and the second pieces, the third go to tensor memory
         auto split_rows = [&](int n) {
-            for (int ks = 0; ks < KS && ok; ++ks) ok = mbar_wait_warp(a_full(ks), (uint32_t)(n & 1), p.err, 116);
-            if (!ok) return;
-            const int l = lane % LPR, sub = lane / LPR;
-            const uint32_t src = smem + T::OFF_A + (l >> 2) * SLAB_BYTES;           // slab of 32 columns, chunks 2 (l & 3) and + 1
-            const uint32_t dst = smem + T::OFF_A + (l >> 3) * 2 * SLAB_BYTES;       // slab of 64 columns, chunk l & 7
-            const int swap = (l >> 2) & 1;                                          // so that eight lanes read eight banks' worth
+            constexpr int CH = 8;                                      // chunks of 16 bytes (4 columns) at a time
+            const int row = quad * 32 + lane;
 #pragma unroll 1
-            for (int r0 = 0; r0 < 16; r0 += U * RPP) {
-                float4 v[U][2];
-                uint32_t mx[U];
+            for (int ks = half * (KS / 2); ks < (half + 1) * (KS / 2); ++ks) {
+                ok = mbar_wait_warp(a_full(ks), (uint32_t)(n & 1), p.err, 116);
+                if (!ok) return;
+                tc_fence_after();
+                const uint32_t slab = smem + T::OFF_A + (uint32_t)(ks * 2 * SLAB_BYTES + row * 128);
+                auto chunk = [&](int c) { return slab + (uint32_t)((c >> 3) * SLAB_BYTES + (((c & 7) ^ (row & 7)) << 4)); };
+                const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ks * 64);
 #pragma unroll
-                for (int i = 0; i < U; ++i) {
-                    const int row = ew * 16 + r0 + i * RPP + sub;
+                for (int c = 0; c < 16; c += CH) {                     // no chunk is written before it has been read
+                    float4 v[CH];
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        v[i][j] = lds128_f32(src + (uint32_t)(row * 128 + (((2 * (l & 3) + (j ^ swap)) ^ (row & 7)) << 4)));
-                    mx[i] = max(magnitude_bits(v[i][0]), magnitude_bits(v[i][1]));
+                    for (int e = 0; e < CH; ++e) v[e] = lds128_f32(chunk(c + e));
+#pragma unroll
+                    for (int e = 0; e < CH; e += 4) {
+                        uint32_t x0[8], x1[8], x2[8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            split_bf16(v[e + i].x, v[e + i].y, x0[2 * i], x1[2 * i], x2[2 * i]);
+                            split_bf16(v[e + i].z, v[e + i].w, x0[2 * i + 1], x1[2 * i + 1], x2[2 * i + 1]);
+                        }
+                        tmem_st_32x8(t_row + (c + e) * 2, x0);
+                        tmem_st_32x8(t_row + 32 + (c + e) * 2, x1);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(chunk((c + e) / 2 + i)), "r"(x2[4 * i]), "r"(x2[4 * i + 1]),
+                                         "r"(x2[4 * i + 2]), "r"(x2[4 * i + 3])
+                                         : "memory");
+                    }
                 }
-#pragma unroll
-                for (int o = LPR / 2; o > 0; o >>= 1)
-#pragma unroll
-                    for (int i = 0; i < U; ++i) mx[i] = max(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
-#pragma unroll
-                for (int i = 0; i < U; ++i) {
-                    const int row = ew * 16 + r0 + i * RPP + sub;
-                    float up, down;
-                    scale_of(mx[i], up, down);
-                    const float4 c0 = swap ? v[i][1] : v[i][0], c1 = swap ? v[i][0] : v[i][1];
-                    uint32_t hi[4], lo[4];
-                    split_f16(c0.x * up, c0.y * up, hi[0], lo[0]);
-                    split_f16(c0.z * up, c0.w * up, hi[1], lo[1]);
-                    split_f16(c1.x * up, c1.y * up, hi[2], lo[2]);
-                    split_f16(c1.z * up, c1.w * up, hi[3], lo[3]);
-                    // (the shuffles above come after every lane's loads of these rows)
-                    const uint32_t d = dst + (uint32_t)(row * 128 + (((l & 7) ^ (row & 7)) << 4));
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(d), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
-                    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(d + SLAB_BYTES), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3])
-                                 : "memory");
-                    if (l == 0) row_scale[(n & 1) * BM + row] = down;
-                }
+                tmem_st_wait();
+                tc_fence_before();
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(a_split(ks));
             }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(a_split);
         };
 
         int tc = 0;
-        for (int n = 0; ok; ++n) {
-            const int u = (int)blockIdx.x + n * (int)gridDim.x;
-            if (u >= p.units) break;
+        for (int n = 0, u = (int)blockIdx.x, at = 0; ok; ++n) {
             int block, t0, nt;
-            unit(u, block, t0, nt);
-            split_rows(n);
-            // the scales of the other warps' rows; every warp comes by here once per block
-            if (ok) ok = mbar_wait_warp(a_split, (uint32_t)(n & 1), p.err, 118);
+            if (!next_part(u, at, block, t0, nt)) break;
+            if (n == 0) split_rows(0);
             if (!ok) break;
-            const float a_scale = row_scale[(n & 1) * BM + quad * 32 + lane];
-            const bool a_large = a_scale > 1.0f;
             const int m0 = block * BM + quad * 32, m = m0 + lane;
             for (int j = 0; j < nt; ++j, ++tc) {
-                const int buf = tc & 1, col = (t0 + j) * BN + half * (BN / 2), seg = col / p.N, n0 = col % p.N;
-                ok = mbar_wait_warp(acc_full(buf), (uint32_t)((tc / 2) & 1), p.err, 117);
+                const int col = (t0 + j) * BN + half * (BN / 2), seg = col / p.N, n0 = col % p.N;
+                const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(T::ACC_COL + half * (BN / 2));
+                uint32_t acc[BN / 64][32], small[BN / 64][32];
+                // out of tensor memory, so that the next tile's small products may begin, and then its large ones
+                ok = mbar_wait_warp(small_full, (uint32_t)(tc & 1), p.err, 119);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t tcol = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * 2 * BN + half * (BN / 2));
-                uint32_t acc[BN / 64][32];
 #pragma unroll
-                for (int c = 0; c < BN / 64; ++c) {
-                    tmem_ld_32x32(tcol + c * 32, acc[c]);
-#pragma unroll
-                    for (int q = 0; q < 32; q += 16) {
-                        uint32_t small[16];
-                        tmem_ld_32x16(tcol + BN + c * 32 + q, small);
-                        tmem_ld_wait16(small);
-#pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            acc[c][q + e] = __float_as_uint(fmaf(__uint_as_float(small[e]), kTail, __uint_as_float(acc[c][q + e])));
-                    }
-                }
-                // everything is in registers: the accumulators may be overwritten
+                for (int c = 0; c < BN / 64; ++c) tmem_ld_32x32(tcol + BN + c * 32, small[c]);
+                tmem_ld_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty(buf));
-                const float *bias = p.bias[seg], *ws = p.w_scale[seg];
+                if (lane == 0) mbar_arrive(small_empty);
+                ok = mbar_wait_warp(large_full, (uint32_t)(tc & 1), p.err, 117);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < BN / 64; ++c) tmem_ld_32x32(tcol + c * 32, acc[c]);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(large_empty);
+#pragma unroll
+                for (int c = 0; c < BN / 64; ++c)
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) acc[c][e] = __float_as_uint(__uint_as_float(acc[c][e]) + __uint_as_float(small[c][e]));
+                // the next block's products wait for its split
+                if (j == nt - 1 && u < p.units) split_rows(n + 1);
+                if (!ok) break;
+                const float *bias = p.bias[seg];
                 const int layout = p.layout[seg];
                 const CUtensorMap *omap = &maps.out[seg];
                 float *tdst = nullptr;                            // transposed segments: this row's place in the first head
@@ -366,16 +354,14 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                 for (int c = 0; c < BN / 64; ++c) {
                     uint32_t(&r)[32] = acc[c];
                     const int nn = n0 + c * 32;
+                    if (bias) {
 #pragma unroll
-                    for (int j4 = 0; j4 < 8; ++j4) {
-                        const float4 sv = __ldg(reinterpret_cast<const float4 *>(ws + nn) + j4);
-                        const float4 bv = bias ? __ldg(reinterpret_cast<const float4 *>(bias + nn) + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float s4[4] = {sv.x, sv.y, sv.z, sv.w}, b4[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            // the factor that may be large last: the powers of two of a row and a channel can be far apart
-                            const float t = __uint_as_float(r[4 * j4 + e]) * (a_large ? s4[e] : a_scale);
-                            r[4 * j4 + e] = __float_as_uint(fmaf(t, a_large ? a_scale : s4[e], b4[e]));
+                        for (int j4 = 0; j4 < 8; ++j4) {
+                            const float4 bv = __ldg(reinterpret_cast<const float4 *>(bias + nn) + j4);
+                            r[4 * j4] = __float_as_uint(__uint_as_float(r[4 * j4]) + bv.x);
+                            r[4 * j4 + 1] = __float_as_uint(__uint_as_float(r[4 * j4 + 1]) + bv.y);
+                            r[4 * j4 + 2] = __float_as_uint(__uint_as_float(r[4 * j4 + 2]) + bv.z);
+                            r[4 * j4 + 3] = __float_as_uint(__uint_as_float(r[4 * j4 + 3]) + bv.w);
                         }
                     }
                     if (layout == kTf32SplitTransposed) {
@@ -395,8 +381,8 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                     const bool split = layout == kTf32SplitRows;
                     for (int t = 0; t < (split ? 4 : 2); ++t) {               // 16 columns each, heads and tails in turn
                         const int hf = split ? t >> 1 : t;
-                        const uint32_t stg = stg0 + (nstore++ & 1) * STG_BYTES;
-                        if (lane == 0) tma_store_wait_read<1>();          // the last but one store has been read
+                        const uint32_t stg = stg0 + nstore++ % T::NSTG * STG_BYTES;
+                        if (lane == 0) tma_store_wait_read<T::NSTG - 1>();          // the store out of this tile has been read
                         __syncwarp();
 #pragma unroll
                         for (int j4 = 0; j4 < 4; ++j4) {
@@ -433,12 +419,10 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
     }
 }
 
-// Weights: a warp per row, up to eight matrices of the same shape a launch (blockIdx.y picks one). dst [rows][2K] fp16 (heads, then
-// tails), then the rows' 2^-s.
+// Weights: a warp per row, up to eight matrices of the same shape a launch (blockIdx.y picks one). dst [rows][3K] bf16.
 struct SplitArgs {
     const float *src[8];
-    __half *dst[8];
-    float *scale[8];
+    __nv_bfloat16 *dst[8];
 };
 template <int K>
 __global__ void __launch_bounds__(256) split_weights_kernel(const SplitArgs args, int64_t src_ld, int rows)
@@ -449,34 +433,25 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const SplitArgs args
     if (row >= rows) return;
     const float4 *src = reinterpret_cast<const float4 *>(args.src[blockIdx.y] + (int64_t)row * src_ld);
     float4 v[K / 128];
-    uint32_t mx = 0;
+#pragma unroll
+    for (int i = 0; i < K / 128; ++i) v[i] = __ldg(src + i * 32 + lane);
+    __nv_bfloat16 *dst = args.dst[blockIdx.y] + (int64_t)row * 3 * K + lane * 4;
 #pragma unroll
     for (int i = 0; i < K / 128; ++i) {
-        v[i] = __ldg(src + i * 32 + lane);
-        mx = max(mx, magnitude_bits(v[i]));
-    }
+        uint2 x[3];
+        split_bf16(v[i].x, v[i].y, x[0].x, x[1].x, x[2].x);
+        split_bf16(v[i].z, v[i].w, x[0].y, x[1].y, x[2].y);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float up, down;
-    scale_of(mx, up, down);
-    __half *dst = args.dst[blockIdx.y] + (int64_t)row * 2 * K;
-#pragma unroll
-    for (int i = 0; i < K / 128; ++i) {
-        uint2 hi, lo;
-        split_f16(v[i].x * up, v[i].y * up, hi.x, lo.x);
-        split_f16(v[i].z * up, v[i].w * up, hi.y, lo.y);
-        *reinterpret_cast<uint2 *>(dst + (i * 32 + lane) * 4) = hi;
-        *reinterpret_cast<uint2 *>(dst + K + (i * 32 + lane) * 4) = lo;
+        for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2 *>(dst + e * K + i * 128) = x[e];
     }
-    if (lane == 0) args.scale[blockIdx.y][row] = down;
 }
 
 template <int KS, int BN>
 void launch_ks(cudaStream_t stream, const RowsMaps &maps, const RowsParams &p, int grid)
 {
-    static const cudaError_t attr = cudaFuncSetAttribute(gemm_f32_rows_kernel<KS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS>::SMEM_BYTES);
+    static const cudaError_t attr = cudaFuncSetAttribute(gemm_f32_rows_kernel<KS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<KS, BN>::SMEM_BYTES);
     KUTACC_CUDA(attr);
-    launch_chained(gemm_f32_rows_kernel<KS, BN>, (unsigned)grid, THREADS, Geo<KS>::SMEM_BYTES, stream, maps, p);
+    launch_chained(gemm_f32_rows_kernel<KS, BN>, (unsigned)grid, THREADS, Geo<KS, BN>::SMEM_BYTES, stream, maps, p);
 }
 
 }  // namespace
@@ -489,8 +464,7 @@ bool split_f32_weights(cudaStream_t stream, int count, const void *const *src, i
         const int j = i < count ? i : 0;
         if ((((uintptr_t)src[j] | (uintptr_t)dst[j]) & 15u) != 0) return false;
         a.src[i] = (const float *)src[j];
-        a.dst[i] = (__half *)dst[j];
-        a.scale[i] = (float *)((char *)dst[j] + (size_t)rows * K * 4);
+        a.dst[i] = (__nv_bfloat16 *)dst[j];
     }
     const dim3 grid((unsigned)((rows + 7) / 8), (unsigned)count);
     KernelTimer timer__("split_weights", stream);
@@ -513,22 +487,22 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
         if ((((uintptr_t)w_split[i] | (uintptr_t)out[i] | (uintptr_t)bias[i]) & 15u) != 0) return false;
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
-    // Few rows: column tiles of half the width where those of four such products run at once; a product is then as long as one
-    // tile's chain: fp32 layer of 8 x 48 rows 34.5 -> 32.6 us, of 8 x 130 rows 45.0 -> 39.0. The rule does not look at nseg, so that a
-    // layer's projections and output run the same code: an output product alone in half tiles cost 40 x 60 rows 44.9 -> 48.9 us.
+    // Few rows: column tiles of half the width while those of four such products are three for each SM. Fewer of them make a CTA wait
+    // on one tile's chain: fp32 layer of 8 heads, 8 x 48 rows 33.8 -> 30.6 us, 20 x 60 38.8 -> 34.9, 24 x 130 57.8 -> 52.2; past the line 12 x 350
+    // rows would be 75.6 -> 77.4, a linear layer of 32768 rows x 1024 channels x 128 columns 77 -> 88 (an instruction of 64 channels takes more than
+    // half the time). The rule does not look at nseg, so that a layer's projections and output run the same code.
     const int sms = std::max(1, sm_count() - runtime().sm_margin);
     const int64_t blocks = (M + BM - 1) / BM;
-    const int BN = blocks * (N / 64) * 4 <= sms ? 64 : 128;
+    const int BN = blocks * (N / 64) * 4 <= 3 * sms ? 64 : 128;
     RowsMaps maps;
     RowsParams p = {};
     if (!make_tensor_map_2d(&maps.a, a, /*elem_bytes=*/4, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 32, BM, 128)) return false;
     for (int i = 0; i < 4; ++i) {
         const int j = i < nseg ? i : 0;
         p.bias[i] = bias[j];
-        p.w_scale[i] = (const float *)((const char *)w_split[j] + (size_t)N * K * 4);
         p.layout[i] = layout ? layout[j] : kTf32Rows;
         p.out_t[i] = (float *)out[j];
-        if (!make_tensor_map_2d(&maps.w[i], w_split[j], 2, (uint64_t)2 * K, (uint64_t)N, (uint64_t)2 * K, 64, BN, 128)) return false;
+        if (!make_tensor_map_2d(&maps.w[i], w_split[j], 2, (uint64_t)3 * K, (uint64_t)N, (uint64_t)3 * K, 64, BN, 128)) return false;
         const uint64_t cols = p.layout[i] == kTf32SplitRows ? 2 * (uint64_t)N : (uint64_t)N;
         if (p.layout[i] == kTf32SplitTransposed)
             maps.out[i] = maps.a;                            // stored directly
@@ -541,19 +515,19 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
     p.S = S > 0 ? S : 1;
     p.vt_pitch = vt_pitch;
     p.err = ew.device;
-    // As in gemm_proj.cu: whole blocks for all full waves, the blocks of the last one in 1 / nsplit of their column tiles each. A
-    // unit costs its column tiles and about two for the way of its rows into shared memory and their split.
-    const int64_t whole = blocks / sms * sms;
+    // Whole blocks for all full waves; the blocks of the last one are dealt out in equal runs of their column tiles. A run costs its
+    // tiles and START tiles for every block it touches, whose rows are loaded and split.
+    constexpr double START = 0.75;
+    p.whole = (int)(blocks / sms * sms);
+    p.rest = (int)(blocks - p.whole) * p.tiles;
     double best = 1e30;
-    for (int ns = 1; ns <= p.tiles; ++ns) {
-        if (p.tiles % ns != 0 || (blocks - whole) * ns + whole > INT32_MAX / 2) continue;
-        const int64_t last = (blocks - whole) * ns;
-        const double cost = (double)((last + sms - 1) / sms) * ((double)p.tiles / ns + 2.0);
+    for (int per = p.tiles; per > 0; per = std::min(per - 1, 4096)) {
+        const int units = (p.rest + per - 1) / per;
+        const double cost = (double)((units + sms - 1) / sms) * (per + START * (p.tiles % per ? 2 : 1));
         if (cost < best * 0.999) {
             best = cost;
-            p.whole = (int)whole;
-            p.nsplit = ns;
-            p.units = (int)(whole + last);
+            p.per = per;
+            p.units = p.whole + units;
         }
     }
     const int grid = std::min(p.units, sms);

@@ -92,7 +92,7 @@ bool tcgen05_gemm_tf32x3(cudaStream_t stream, const void *a_split, const void *c
                          int S = 0, int64_t vt_pitch = 0);
 
 // The same product for K of 128 or 256 (gemm_f32_rows.cu): a [M, K] fp32 with row stride lda, split on the way; the weights split by
-// split_f32_weights into fp16 heads and tails with their rows' scales (each dst rows * K * 4 + rows * 4 bytes).
+// split_f32_weights into three bf16 pieces (each dst rows * K * 6 bytes).
 bool split_f32_weights(cudaStream_t stream, int count, const void *const *src, int64_t src_ld, void *const *dst, int rows, int K);
 bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, const void *const *w_split, const float *const *bias,
                            void *const *out, int64_t ldo, int64_t M, int N, int K, int nseg, const Tf32Layout *layout = nullptr,

@@ -61,7 +61,7 @@ extern "C" void kutacc_af2_linear(kutacc_tensor_h act_h, kutacc_tensor_h weight_
         // fp32 on the tensor memory: up to 256 columns the product splits its activations itself, beyond that both operands are
         // split into tf32 head and tail in the workspace
         const bool rows = k == 128 || k == 256;
-        const size_t as_bytes = rows ? 0 : (size_t)m * 2 * k * 4, ws_bytes = rows ? (size_t)n * (k + 1) * 4 : (size_t)n * 2 * k * 4;
+        const size_t as_bytes = rows ? 0 : (size_t)m * 2 * k * 4, ws_bytes = (size_t)n * k * (rows ? 6 : 8);
         if (rt.reserve_workspace(as_bytes + ws_bytes + 512)) {
             void *a_split = rows ? nullptr : rt.take_workspace(as_bytes), *w_split = rt.take_workspace(ws_bytes);
             const void *wp[1] = {w_split}, *const src[1] = {d_w.dev};

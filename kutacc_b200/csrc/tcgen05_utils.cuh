@@ -25,7 +25,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], bf16 or fp16 inputs, fp32 accumulate, types and shape from idesc
+// D[tmem] (+)= A[smem] * B[smem], bf16 inputs, fp32 accumulate, shape from idesc
 __device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate)
 {
@@ -143,11 +143,6 @@ __host__ __device__ constexpr uint32_t make_instr_desc_bf16(int M, int N)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// the same for fp16 operands
-__host__ __device__ constexpr uint32_t make_instr_desc_f16(int M, int N)
-{
-    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
 // the same for tf32 operands
 __host__ __device__ constexpr uint32_t make_instr_desc_tf32(int M, int N)
 {

@@ -156,3 +156,29 @@ def test_linear_fp32_rows_of_any_magnitude(kutacc_lib, M, N, K):
     ref, terms = ta.double() @ tw.double().T, ta.double().abs() @ tw.double().abs().T
     # operands to 2^-23 each, the product of the tails dropped (2^-24): 3 * 2^-23; up to 2 K / 16 accumulations that truncate at 2^-23
     assert ((tr.double() - ref).abs() <= (3 + K / 8) * 2.0 ** -23 * terms).all()
+
+
+# Elements of a row far apart: column factors up to 2^spread that the other operand takes back, so that every column counts the same; or
+# one column 2^spread above the others whose partners are zero, so that only the small ones count
+@pytest.mark.parametrize("spread", [30, 52, 56])
+@pytest.mark.parametrize("M,N,K,way", [(300, 256, 256, "columns"), (3456, 256, 128, "columns"), (3457, 256, 256, "columns"), (300, 128, 128, "activation"), (19201, 256, 256, "activation"),
+                                       (129, 128, 256, "weight"), (20000, 256, 128, "weight"), (300, 128, 512, "columns")])
+def test_linear_fp32_elements_of_any_magnitude_in_a_row(kutacc_lib, M, N, K, way, spread):
+    g = torch.Generator().manual_seed(M + N + K + spread)
+    a, w = torch.randn(M, K, generator=g).to(DEV), (torch.randn(N, K, generator=g) / K ** 0.5).to(DEV)
+    if way == "columns":
+        col = torch.exp2(torch.randint(-spread, spread + 1, (K,), generator=g).float()).to(DEV)
+        a, w = a * col, w / col
+    else:
+        big, other = (a, w) if way == "activation" else (w, a)
+        at = torch.randint(0, K, (8,), generator=g).to(DEV)
+        big[:, at[0]] *= 2.0 ** spread
+        big[:, at[1]] *= 2.0 ** (2 * spread)
+        other[:, at] = 0
+    tr = torch.full((M, N), 7.0, dtype=torch.float32, device=DEV)
+    api.linear(api.tensor(a), api.tensor(w), None, api.tensor(tr), 0)
+    torch.cuda.synchronize()
+    ref, terms = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # as above: three pieces of 8 bits hold an element whole, products below 2^-22 of the first one are dropped (tf32 pairs: 2^-22 too);
+    # every accumulation of 16 (8) columns truncates at 2^-23
+    assert ((tr.double() - ref).abs() <= (3 + K / 8) * 2.0 ** -23 * terms).all()

@@ -102,6 +102,11 @@ struct Runtime {
 };
 Runtime &runtime();
 bool is_device_pointer(const void *p);
+// two ranges without a common byte
+inline bool apart(const void *a, size_t a_bytes, const void *b, size_t b_bytes)
+{
+    return (uintptr_t)a + a_bytes <= (uintptr_t)b || (uintptr_t)b + b_bytes <= (uintptr_t)a;
+}
 void count_launch(int n = 1);
 
 // Optional per-kernel timing (kutacc_b200_set_profile): a launcher wraps each launch in a

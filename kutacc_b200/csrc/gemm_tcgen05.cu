@@ -530,8 +530,11 @@ bool tcgen05_linear_bias_bf16(cudaStream_t stream, const void *a, const void *w,
     KernelErrorWord &ew = kernel_error_word();
     if (ew.device == nullptr) return false;
     // Few tiles: columns in halves, so that twice as many SMs share the epilogue, which is on the path of a small call. 4 rows x 192
-    // positions x 128 channels, the whole attention call: 20.6 -> 20.3 us. Where halves would need a second wave, tiles of 128.
-    const bool narrow = !relu && (int64_t)B * ((S + BM - 1) / BM) * (N / BNMAX) * 2 <= sm_count();
+    // positions x 128 channels, the whole attention call: 20.6 -> 20.3 us. Where halves would need a second wave, tiles of 128. So also for a result that lies
+    // over its own rows: with 128 channels a tile has read its rows before it writes them, halves would not wait for each other.
+    const int64_t rows = (int64_t)B * S;
+    const bool narrow = !relu && (int64_t)B * ((S + BM - 1) / BM) * (N / BNMAX) * 2 <= sm_count() &&
+                        apart(a, (size_t)((rows - 1) * a_row_stride + K) * 2, out, (size_t)((rows - 1) * out_row_stride + N) * 2);
     GemmMaps maps;
     if (!make_tensor_map_bf16_3d(&maps.a, a, K, S, B, (uint64_t)a_row_stride, (uint64_t)S * a_row_stride, BK, BM, 128))
         return false;

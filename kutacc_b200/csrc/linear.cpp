@@ -58,9 +58,10 @@ extern "C" void kutacc_af2_linear(kutacc_tensor_h act_h, kutacc_tensor_h weight_
     }
     if (dt == kFP32 && beta == 0 && a16 && k % 32 == 0 && n % 128 == 0 && lda % 4 == 0 && ldw % 4 == 0 && k <= INT32_MAX / 2 &&
         n <= INT32_MAX && (((uintptr_t)d_r.dev | (uintptr_t)d_b.dev) & 15u) == 0) {
-        // fp32 on the tensor memory: up to 256 columns the product splits its activations itself, beyond that both operands are
-        // split into tf32 head and tail in the workspace
-        const bool rows = k == 128 || k == 256;
+        // fp32 on the tensor memory: up to 256 columns the product splits its activations itself, beyond that, and where the result
+        // lies over them (several CTAs load the same rows, at different times), both operands are split into tf32 head and tail in the
+        // workspace
+        const bool rows = (k == 128 || k == 256) && apart(d_a.dev, a_bytes, d_r.dev, r_bytes);
         const size_t as_bytes = rows ? 0 : (size_t)m * 2 * k * 4, ws_bytes = (size_t)n * k * (rows ? 6 : 8);
         if (rt.reserve_workspace(as_bytes + ws_bytes + 512)) {
             void *a_split = rows ? nullptr : rt.take_workspace(as_bytes), *w_split = rt.take_workspace(ws_bytes);

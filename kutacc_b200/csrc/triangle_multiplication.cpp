@@ -27,12 +27,6 @@ DeviceArg resolve_out_keeping_gaps(void *p, size_t bytes, bool dense)
     return dense ? resolve_out(p, bytes) : resolve_in(p, bytes);
 }
 
-// two ranges without a common byte
-bool apart(const void *a, size_t a_bytes, const void *b, size_t b_bytes)
-{
-    return (uintptr_t)a + a_bytes <= (uintptr_t)b || (uintptr_t)b + b_bytes <= (uintptr_t)a;
-}
-
 }  // namespace
 }  // namespace kutacc
 

@@ -182,3 +182,36 @@ def test_linear_fp32_elements_of_any_magnitude_in_a_row(kutacc_lib, M, N, K, way
     # as above: three pieces of 8 bits hold an element whole, products below 2^-22 of the first one are dropped (tf32 pairs: 2^-22 too);
     # every accumulation of 16 (8) columns truncates at 2^-23
     assert ((tr.double() - ref).abs() <= (3 + K / 8) * 2.0 ** -23 * terms).all()
+
+
+# M of one block and of blocks whose column tiles go to several CTAs
+@pytest.mark.parametrize("M,K", [(100, 128), (1280, 256), (6000, 128), (30000, 256)])
+def test_linear_fp32_over_its_own_input(kutacc_lib, M, K):
+    g = torch.Generator().manual_seed(M + K)
+    a, w, b = torch.randn(M, K, generator=g).to(DEV), (torch.randn(K, K, generator=g) / K ** 0.5).to(DEV), torch.randn(K, generator=g).to(DEV)
+    ref = a.double() @ w.double().T + b
+    store = torch.cat([a, torch.full((200, K), 7.0, device=DEV)])
+    api.set_profile(True)
+    api.profile_read()
+    api.linear(api.tensor(store[:M]), api.tensor(w), b.data_ptr(), api.tensor(store[:M]), 0)
+    names = [k for k, _ in api.profile_read()]
+    api.set_profile(False)
+    assert "split_weights" not in names and names.count("split_tf32") == 2          # through a copy of the activations
+    assert helpers.rel_err(store[:M].cpu().numpy(), ref.cpu().numpy()) <= 4e-6 and bool((store[M:] == 7.0).all())
+    # and a result that begins in the middle of them
+    store = torch.cat([a, torch.zeros(200, K, device=DEV)])
+    api.linear(api.tensor(store[:M]), api.tensor(w), b.data_ptr(), api.tensor(store[77:M + 77]), 0)
+    assert helpers.rel_err(store[77:M + 77].cpu().numpy(), ref.cpu().numpy()) <= 4e-6 and torch.equal(store[:77], a[:77])
+
+
+@pytest.mark.parametrize("M", [1, 129, 4000, 9472, 20000])
+def test_linear_bf16_over_its_own_input(kutacc_lib, M):
+    # 128 channels: a CTA has read the rows that it writes, whether few row tiles are to be had or many
+    rng = np.random.default_rng(M)
+    a, w = _bf16_cuda(rng.standard_normal((M, 128)).astype(np.float32)), _bf16_cuda(rng.standard_normal((128, 128)).astype(np.float32) / 11)
+    b, out = torch.randn(128, device=DEV), torch.zeros(M, 128, dtype=torch.bfloat16, device=DEV)
+    api.linear(api.tensor(a), api.tensor(w), b.data_ptr(), api.tensor(out), 0)
+    for _ in range(5):
+        x = a.clone()
+        api.linear(api.tensor(x), api.tensor(w), b.data_ptr(), api.tensor(x), 0)
+        assert torch.equal(x, out)

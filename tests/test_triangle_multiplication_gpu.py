@@ -223,3 +223,18 @@ def test_gate_and_out_linear_with_an_output_over_its_input(kutacc_lib, n, c_o, c
     assert torch.equal(gate, gate2) and torch.equal(out, out2)
     want = O.linear_bf16(W.bf16_bits(A["x"]).reshape(-1, c_o), W.bf16_bits(A["gating_w"]), A["gating_b"])
     assert helpers.rel_err(_f32(gate).reshape(-1, c_o), W.as_f32(want)) <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("n", [9, 33, 60])
+def test_gate_linear_over_its_own_input(kutacc_lib, n):
+    """128 channels and layers of two shapes, each in a launch of its own: the gate in the place of the activations that it is made from."""
+    A = _case(970 + n, n, 128, 64)
+    cen, x = _bf(np.random.default_rng(n).standard_normal((n, n, 64)).astype(np.float32)), _bf(A["x"])
+    weights = api.make_tm_linear_weights(128, 64, _bf(A["gating_w"]), torch.from_numpy(A["gating_b"]).to(DEV), _bf(A["out_w"]),
+                                         torch.from_numpy(A["out_b"]).to(DEV))
+    for gate in (torch.zeros_like(x), x):
+        out = torch.zeros((n, n, 128), dtype=torch.bfloat16, device=DEV)
+        api.tm_gate_and_out_linear(api.tensor(gate), api.tensor(out), api.make_tm_acts(n, n, None, x, None), api.tensor(cen), weights)
+        torch.cuda.synchronize()
+        want = want if gate is x else (gate.clone(), out)
+        assert torch.equal(gate, want[0]) and torch.equal(out, want[1])

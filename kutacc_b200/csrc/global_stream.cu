@@ -239,16 +239,17 @@ __global__ void __launch_bounds__(KV_WARPS * 32, 2) global_kv_kernel(const Strea
 // the copies themselves were the bound, 26 us for 61440 records.) Sixteen slices per column whatever the number of columns: a
 // column's sums are split the same way in every batch. More columns than SMs run two CTAs per SM on a shorter ring (250
 // columns x 1500 rows: 41.6 us for the three kernels, with one CTA per SM 44.7); fewer have the longer ring (64 x 5120: 41 us,
-// with the shorter 46). Where those come in two waves and the columns are short, up to 2048 rows, four CTAs per SM of eight
-// warps, each with two slices one after the other: one wave of the chain from the partial sums to the query instead of two
-// (297 x 128: 17.2 -> 15.7 us, 384 x 512: 31.3 -> 29.7, 384 x 2000: 77.4 -> 77.2; but 384 x 5120: 162.9 -> 163.4, 592 x 3000: 150.6 -> 155.5).
+// with the shorter 46). Where those come in two waves and the columns are short, up to 2048 rows, three CTAs per SM (shared memory holds
+// no fourth) of eight warps, each with two slices one after the other: one wave of the chain from the partial sums to the query instead
+// of two (297 x 128: 17.2 -> 15.7 us, 384 x 512: 31.3 -> 29.7, 384 x 2000: 77.4 -> 77.2; but 384 x 5120: 162.9 -> 163.4). From 445
+// columns on (148 SMs) they come in two waves either way and sixteen warps are faster: 445 x 512 32.6 -> 31.7 us, 592 x 512 37.4 -> 35.6, 500 x 1000 61.3 -> 57.2.
 // Half of a long column's time is issue slots (two rows a packed operation and a flushed exponential: 141 instructions a record
 // of 32 rows; 384 x 5120, the three kernels 164.7 -> 162.9 us).
 constexpr int SLICES = 16, Q_BYTES = 2 * REC_BYTES;
 constexpr int core_smem(int warps, int qn) { return warps * qn * (Q_BYTES + 8); }
 
 template <int WARPS, int QN>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 4 : QN == 3 ? 2 : 1) global_softmax_kernel(const StreamArgs a)
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : QN == 3 ? 2 : 1) global_softmax_kernel(const StreamArgs a)
 {
     constexpr int NR = 7;                        // row groups of the pooled sums: a thread for each and channel in sixteen warps
     static_assert(NR * (C + 1) <= SLICES * 32 && SLICES % WARPS == 0, "");
@@ -773,12 +774,15 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
                                  (uint64_t)S * (uint64_t)out_row_stride, C, BM, 128))
         return false;
     static bool configured = false;
+    static int fit16 = 0, fit8 = 0;              // CTAs of the softmax kernel's two forms per SM
     if (!configured) {
         KUTACC_CUDA(cudaFuncSetAttribute(global_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM));
         KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(8, 3)));
         KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(16, 3)));
         KUTACC_CUDA(cudaFuncSetAttribute(global_softmax_kernel<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, core_smem(16, 4)));
         KUTACC_CUDA(cudaFuncSetAttribute(global_stream_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_SMEM));
+        KUTACC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit16, global_softmax_kernel<16, 3>, 16 * 32, core_smem(16, 3)));
+        KUTACC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit8, global_softmax_kernel<8, 3>, 8 * 32, core_smem(8, 3)));
         configured = true;
     }
     const int sms = std::max(1, sm_count() - runtime().sm_margin);
@@ -790,7 +794,7 @@ bool launch_global_stream_bf16(cudaStream_t stream, const void *x, const void *m
     }
     {
         KernelTimer timer__("global_softmax", stream);
-        const int w16 = (B + 2 * sms - 1) / (2 * sms), w8 = (B + 4 * sms - 1) / (4 * sms);       // waves
+        const int at16 = std::max(1, fit16) * sms, at8 = std::max(1, fit8) * sms, w16 = (B + at16 - 1) / at16, w8 = (B + at8 - 1) / at8;       // waves
         if (2 * w8 <= w16 && pl.nrec <= 64)
             launch_chained(global_softmax_kernel<8, 3>, (unsigned)B, 8 * 32, core_smem(8, 3), stream, a);
         else if (B > sms)

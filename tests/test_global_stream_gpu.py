@@ -42,8 +42,8 @@ def test_a_column_does_not_depend_on_the_number_of_columns(kutacc_lib):
     assert np.array_equal(many[:3], runner.out_to_f32(runner.DeviceCase(few).run()))
 
 
-# sixteen warps a column in one wave; eight where two waves become one, up to their longest column; sixteen past it and in three waves
-@pytest.mark.parametrize("B,S", [(200, 700), (297, 31), (297, 2048), (297, 2049), (593, 40)])
+# sixteen warps a column in one wave; eight where two waves become one, up to their longest column and their last wave; sixteen past these
+@pytest.mark.parametrize("B,S", [(200, 700), (297, 31), (297, 2048), (297, 2049), (444, 33), (445, 33), (593, 40)])
 def test_columns_do_not_depend_on_the_warps_they_share(kutacc_lib, B, S):
     w = W.random_global_case(seed=79 + S, B=B, S=S, zero_mask_rows=1)
     many = runner.out_to_f32(runner.DeviceCase(w).run())

@@ -79,8 +79,11 @@ constexpr float kFar = 2147483648.f;          // 2^31: mneg below it is within 6
 // tile from memory (3400), rows of gate and result read and written by the threads they belong to, 32 lines an instruction. 384 x 512
 // rows x 8 heads: 300 -> 267 us; with a pair bias 512 x 512 x 4 338 -> 317 us (the whole call), 1024 residues 2030 -> 1988. Beside the
 // pair bias of heads of 32 there is room for two of its tiles, a ring of their own, and they come one tile after K and V, which a CTA with
-// a single short item feels: 4 x 192 rows 20.5 against 22.2 us, 64 residues 28.7 against 30.7. So there, and for narrow heads, whose
-// rows are short, everything stays in one ring of three.
+// a single short item feels: 4 x 192 rows 20.5 against 22.2 us, 64 residues 28.7 against 30.7. So there, and for narrow heads with a
+// pair bias, everything stays in one ring of three. Narrow heads without one have short rows, of which a TMA tile is slow. Heads of 8:
+// 256 x 64 rows x 8 25.7 us without the tiles and 27.6 with them, 256 x 128 34.5 and 36.5, but 100 x 256 42.5 and 41.3, 256 x 256 79.5 and 75.8,
+// 384 x 512 365 and 336. Heads of 16: 64 x 64 rows x 4 16.0 and 16.5, 256 x 256 x 4 54.0 and 54.6, 300 x 320 x 4 92.8 and 93.9, but with eight items
+// or more a CTA 256 x 384 x 8 174.0 and 170.3, 384 x 512 x 8 388 and 381.
 template <int D, bool STAGED>
 struct Geo {
     static constexpr int ROWS_BYTES = STAGED ? 32 * D * 2 : 0;
@@ -802,8 +805,9 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
     if (!make_tensor_map_bf16_4d(&tq, q, D, Su, H, B, D, Su * D, Su * D * H, T::KD, BM, G, T::ROWB)) return false;
     if (!make_tensor_map_bf16_4d(&tk, k, D, Su, H, B, D, Su * D, Su * D * H, T::KD, BN, G, T::ROWB)) return false;
     if (!make_tensor_map_bf16_4d(&tvt, vt, Su, D, H, B, vp, D * vp, D * vp * H, BN, D, 1, 128)) return false;
-    // with a pair bias where a CTA has several items (see Geo)
-    const bool staged = !nb || (D == 32 && p.n_items > std::max(1, sm_count() - runtime().sm_margin));
+    // where the items are long, or many (see Geo)
+    const int64_t sms = std::max(1, sm_count() - runtime().sm_margin);
+    const bool staged = D == 32 ? !nb || p.n_items > sms : !nb && p.S > 3 * BN && (D == 8 || p.n_items >= 8 * sms);
     RowMaps<true> rows;
     if (staged) {
         const int swizzle = D == 8 ? 0 : D * 2;
@@ -830,6 +834,9 @@ bool launch_d(cudaStream_t stream, const void *q, const void *k, const void *vt,
         return launch_one<D, SPLIT, true, false>(stream, tq, tk, tvt, tnb, RowMaps<false>{}, p);
     }
     tnb = tk;
+    if constexpr (D < 32) {
+        if (!staged) return launch_one<D, SPLIT, false, false>(stream, tq, tk, tvt, tnb, RowMaps<false>{}, p);
+    }
     return launch_one<D, SPLIT, false, true>(stream, tq, tk, tvt, tnb, rows, p);
 }
 

@@ -157,7 +157,8 @@ def test_more_than_2_25_work_items(kutacc_lib):
 # items cut in two or in four; last key tiles of one to four pieces; a batch that does not fill its last item
 @pytest.mark.parametrize("B,S,H,D,nb", [(301, 140, 4, 32, True), (75, 192, 4, 32, True), (161, 257, 4, 32, True), (298, 230, 2, 32, True),
                                         (77, 131, 8, 16, True), (150, 333, 8, 8, True), (160, 49, 4, 32, True), (297, 112, 8, 8, True),
-                                        (600, 17, 2, 32, True), (299, 140, 4, 32, False), (101, 257, 4, 16, False)])
+                                        (600, 17, 2, 32, True), (299, 140, 4, 32, False), (101, 257, 4, 16, False), (85, 192, 8, 8, False), (85, 193, 8, 8, False),
+                                        (193, 385, 8, 16, False), (300, 193, 8, 16, False)])
 def test_rows_do_not_depend_on_the_item_list(kutacc_lib, B, S, H, D, nb):
     w = W.random_gating_case(seed=5 + S, B=B, S=S, H=H, D=D, with_nb=nb, full_mask_rows=1)
     got = runner.out_to_f32(runner.DeviceCase(w).run())

@@ -531,7 +531,7 @@ bool tcgen05_gemm_f32_rows(cudaStream_t stream, const void *a, int64_t lda, cons
         }
     }
     const int grid = std::min(p.units, sms);
-    KernelTimer timer__("gemm_tf32x3_tc", stream);           // the name of the fp32 tensor-memory products, whichever kernel
+    KernelTimer timer__("gemm_f32_rows", stream);
     if (BN == 64)
         K == 128 ? launch_ks<2, 64>(stream, maps, p, grid) : launch_ks<4, 64>(stream, maps, p, grid);
     else

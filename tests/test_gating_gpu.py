@@ -56,11 +56,11 @@ def test_fp32_matches_exact_oracle(kutacc_lib, B, S, H, D, with_nb):
     assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL
 
 
-@pytest.mark.parametrize("B,S,H,D", [(3, 70, 4, 32), (2, 129, 8, 32), (1, 300, 8, 16)])
+@pytest.mark.parametrize("B,S,H,D", [(3, 70, 4, 32), (2, 129, 8, 32), (1, 300, 8, 16), (2, 129, 12, 32), (1, 70, 8, 64)])
 def test_fp32_projections_run_on_the_tensor_memory_gemm(kutacc_lib, B, S, H, D):
-    """fp32 with nchannels a multiple of 128: the projections and the output projection go through the tcgen05 tf32
-    GEMM on operands split into head and tail (three products per multiply), which must stay at fp32 accuracy; the
-    row count B * S is not a multiple of the 128-row tile."""
+    """fp32 with nchannels a multiple of 128: the projections and the output projection go through a tcgen05 GEMM on operands split
+    into three bf16 pieces (128 and 256 channels) or a tf32 head and tail (more), which must stay at fp32 accuracy; the row count
+    B * S is not a multiple of the 128-row tile."""
     w = W.random_gating_case(seed=400 + S, B=B, S=S, H=H, D=D, dtype="fp32", with_nb=True, full_mask_rows=0)
     case = runner.DeviceCase(w)
     api.set_profile(True)
@@ -68,7 +68,8 @@ def test_fp32_projections_run_on_the_tensor_memory_gemm(kutacc_lib, B, S, H, D):
     got = runner.out_to_f32(case.run())
     names = [k for k, _ in api.profile_read()]
     api.set_profile(False)
-    assert names.count("gemm_tf32x3_tc") == 2 and "gemm_tf32x3" not in names
+    kernel, other = ("gemm_f32_rows", "gemm_tf32x3_tc") if H * D <= 256 else ("gemm_tf32x3_tc", "gemm_f32_rows")
+    assert names.count(kernel) == 2 and other not in names and "gemm_tf32x3" not in names
     assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL
     # the host-buffer call takes the same kernels chunk by chunk
     assert np.array_equal(_run(w, device=False), got)

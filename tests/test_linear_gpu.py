@@ -61,8 +61,8 @@ def test_linear_fp32(kutacc_lib):
 
 @pytest.mark.parametrize("M,N,K,bias", [(300, 128, 96, True), (1000, 384, 256, False), (77, 256, 32, True)])
 def test_linear_fp32_on_the_tensor_memory_gemm(kutacc_lib, M, N, K, bias):
-    # fp32 with n % 128 == 0 and k % 32 == 0: tcgen05 kind::tf32 on operands split into head and tail; large values
-    # next to small ones in one row show a dropped tail at once
+    # fp32 with n % 128 == 0 and k % 32 == 0: tcgen05 on operands split into tf32 heads and tails, or for 128 and 256 columns into bf16
+    # pieces; large values next to small ones in one row show a dropped tail at once
     rng = np.random.default_rng(M + N)
     a = (rng.standard_normal((M, K)) * rng.choice([1e-3, 1.0, 300.0], (M, K))).astype(np.float32)
     w = (rng.standard_normal((N, K)) / np.sqrt(K)).astype(np.float32)
@@ -75,7 +75,7 @@ def test_linear_fp32_on_the_tensor_memory_gemm(kutacc_lib, M, N, K, bias):
     api.linear(api.tensor(ta), api.tensor(tw), tb.data_ptr() if bias else None, api.tensor(tr), 0)
     names = [k for k, _ in api.profile_read()]
     api.set_profile(False)
-    assert "gemm_tf32x3_tc" in names
+    assert ("gemm_f32_rows" if K == 256 else "gemm_tf32x3_tc") in names
     ref = O.linear_exact(a, w, b)
     got = tr.cpu().numpy()
     # against the magnitude of the terms of each dot product, not of the (possibly cancelling) result

@@ -158,7 +158,8 @@ attn_f32_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     if (warp == PRODUCER_WARP) {
         // ================= producer =================
         const uint32_t tx = (uint32_t)(2 * G * (K_BYTES + D * 128) + (HAS_NB ? NB_BYTES : 0));
-        auto take = [&](int i) -> int {                                // as in attn_tcgen05.cu
+        static_assert(NST <= 3, "item numbers in the ring: as in attn_tcgen05.cu, item i - 3 has been consumed when that of i + 1 is written");
+        auto take = [&](int i) -> int {
             int w = 0;
             if (lane == 0) {
                 w = atomicAdd(p.counter, 1);

@@ -163,8 +163,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     const int n_mma = min(G, MMA_WARPS);
     // Work items are handed out through an atomic counter in global memory: the producer warp takes the next
     // item number, publishes it to the other roles through a ring of four shared-memory words (one mbarrier each),
-    // and publishes -1 when the list is exhausted. Ring depth: slot i & 3 is written when the products of item i - 2
-    // have all been issued, by which time every role has long read the number of item i - 4.
+    // and publishes -1 when the list is exhausted. Ring depth: the number of item i + 1 is written at the earliest during the loads of
+    // item i, once the stage of a tile of that item is free, that is, NST = 3 tiles before it have been consumed. Even where every item has one
+    // tile, that was item i - 3, whose number, the last in that slot, every role had read to consume it. There is nothing to spare: an
+    // earlier number or a fourth stage needs a longer ring.
+    static_assert(NST <= 3, "item numbers in the ring");
     auto rows_of = [&](int w) { return CUT && w >= p.n_whole ? G / p.parts : G; };
     auto decode = [&](int w, int &q0, int &h, int &b0) {
         int sub = 0;
@@ -295,8 +298,8 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 if (!STAGED) continue;
                 // Q after the item's first tile, whose stage is free earlier than the tile of the Q before it
                 if (kt == 0) ok = load_q(i, q0, h, b0);
-                // The next item's number two tiles before this one's loads end, its Q and first tile on their way to L2. Ring slot
-                // i & 3: every role has read the number of item i - 4, as this tile's stage was free.
+                // The next item's number two tiles before this one's loads end (this tile's stage was free, see above), its Q and first tile on
+                // their way to L2.
                 if (kt == max(nkt - 2, 0)) {
                     next = take(i + 1);
                     if (next >= 0) {

@@ -168,13 +168,14 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
         // ================= producer =================
         if (elect_one()) {
             bool ok = true;
-            int s = 0, round = 0;                                      // next slab's slot, times the ring has gone round
+            int s = 0, round = 0, rows_asked = 0;                      // next slab's slot, times the ring has gone round; row slabs asked for
             for (int n = 0, u = (int)blockIdx.x, at = 0; ok; ++n) {
                 int block, t0, nt;
                 if (!next_part(u, at, block, t0, nt)) break;
                 for (int ks = 0; ks < KS && ok; ++ks) {
                     if (n > 0) ok = mbar_wait(a_empty(ks), (uint32_t)((n - 1) & 1), p.err, 111);
                     if (!ok) break;
+                    ++rows_asked;
                     mbar_arrive_expect_tx(a_full(ks), 2 * SLAB_BYTES);
                     const uint32_t dst = smem + T::OFF_A + ks * 2 * SLAB_BYTES;
                     tma_load_2d(dst, &maps.a, a_full(ks), ks * 64, block * BM);
@@ -197,6 +198,17 @@ gemm_f32_rows_kernel(const __grid_constant__ RowsMaps maps, const __grid_constan
                         if (next_part(u2, at2, next, nt0, nnt))
                             for (int c = 0; c < 2 * KS; ++c) tma_prefetch_2d(&maps.a, c * 32, next * BM);
                     }
+                }
+            }
+            // after a wait that ran out: no copy may still be on its way when the CTA exits
+            if (!ok) {
+                for (int i = 0; i < NW; ++i) {
+                    const int last = i < s ? round : round - 1;
+                    if (last >= 0) mbar_wait(w_full(i), (uint32_t)(last & 1), p.err, 120);
+                }
+                for (int ks = 0; ks < KS; ++ks) {
+                    const int asked = (rows_asked + KS - 1 - ks) / KS;
+                    if (asked > 0) mbar_wait(a_full(ks), (uint32_t)((asked - 1) & 1), p.err, 121);
                 }
             }
         }

@@ -437,7 +437,7 @@ struct SplitArgs {
     __nv_bfloat16 *dst[8];
 };
 template <int K>
-__global__ void __launch_bounds__(256) split_weights_kernel(const SplitArgs args, int64_t src_ld, int rows)
+__global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constant__ SplitArgs args, int64_t src_ld, int rows)
 {
     release_successor();
     wait_for_predecessor();

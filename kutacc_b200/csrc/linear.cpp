@@ -24,7 +24,7 @@ extern "C" void kutacc_af2_linear(kutacc_tensor_h act_h, kutacc_tensor_h weight_
                  weight.sizes().back(), "]");
     if (kutacc_check_err_set) return;
     const int64_t m = act.numel() / k, n = weight.numel() / k;
-    const int64_t lda = act.dim() >= 2 ? act.strides()[(size_t)act.dim() - 2] : k;
+    int64_t lda = act.dim() >= 2 ? act.strides()[(size_t)act.dim() - 2] : k;
     const int64_t ldw = weight.dim() >= 2 ? weight.strides()[(size_t)weight.dim() - 2] : k;
     const DType dt = act.dtype();
     KUTACC_CHECK(dt == kBF16 || dt == kFP32, "addmm dtype invalid, a: [", (int)dt, "]");
@@ -49,19 +49,31 @@ extern "C" void kutacc_af2_linear(kutacc_tensor_h act_h, kutacc_tensor_h weight_
 
     const dev::ElemType et = dt == kFP32 ? dev::kElemF32 : dev::kElemBF16;
     bool ok = false;
-    const bool a16 = (((uintptr_t)d_a.dev | (uintptr_t)d_w.dev) & 15u) == 0;
+    bool a16 = (((uintptr_t)d_a.dev | (uintptr_t)d_w.dev) & 15u) == 0;
+    const bool f32_tc = dt == kFP32 && beta == 0 && a16 && k % 32 == 0 && n % 128 == 0 && lda % 4 == 0 && ldw % 4 == 0 && k <= INT32_MAX / 2 &&
+                        n <= INT32_MAX && (((uintptr_t)d_r.dev | (uintptr_t)d_b.dev) & 15u) == 0;
+    // A result over the activations: several CTAs read the same rows, so it is computed from a copy of them, except where a CTA has read
+    // all of the rows that it writes (bf16, 128 channels in and out, in their very place) and where fp32 operands are split first
+    const bool over = !apart(d_a.dev, a_bytes, d_r.dev, r_bytes);
+    if (over && !f32_tc && !(dt == kBF16 && beta == 0 && a16 && k == 128 && n == 128 && lda == k && ldw == k && d_a.dev == d_r.dev)) {
+        if (!rt.reserve_workspace((size_t)m * k * es + 256)) return;
+        void *copy = rt.take_workspace((size_t)m * k * es);
+        if (kutacc_check_err_set) return;
+        KUTACC_CUDA(cudaMemcpy2DAsync(copy, (size_t)k * es, d_a.dev, (size_t)lda * es, (size_t)k * es, (size_t)m, cudaMemcpyDeviceToDevice, stream));
+        d_a.dev = copy;
+        lda = k;
+        a16 = ((uintptr_t)d_w.dev & 15u) == 0;
+    }
     if (dt == kBF16 && beta == 0 && a16 && k % 64 == 0 && n % 128 == 0 && lda == k && ldw == k && m <= INT32_MAX) {
         // the tcgen05 projection kernel on the [1, m, k] view of the activations
         ok = dev::tcgen05_linear_bias_bf16(stream, d_a.dev, d_w.dev, (const float *)d_b.dev, d_r.dev, n, 1, (int)m, (int)n,
                                            (int)k);
         if (kutacc_check_err_set) return;
     }
-    if (dt == kFP32 && beta == 0 && a16 && k % 32 == 0 && n % 128 == 0 && lda % 4 == 0 && ldw % 4 == 0 && k <= INT32_MAX / 2 &&
-        n <= INT32_MAX && (((uintptr_t)d_r.dev | (uintptr_t)d_b.dev) & 15u) == 0) {
+    if (f32_tc) {
         // fp32 on the tensor memory: up to 256 columns the product splits its activations itself, beyond that, and where the result
-        // lies over them (several CTAs load the same rows, at different times), both operands are split into tf32 head and tail in the
-        // workspace
-        const bool rows = (k == 128 || k == 256) && apart(d_a.dev, a_bytes, d_r.dev, r_bytes);
+        // lies over them, both operands are split into tf32 head and tail in the workspace
+        const bool rows = (k == 128 || k == 256) && !over;
         const size_t as_bytes = rows ? 0 : (size_t)m * 2 * k * 4, ws_bytes = (size_t)n * k * (rows ? 6 : 8);
         if (rt.reserve_workspace(as_bytes + ws_bytes + 512)) {
             void *a_split = rows ? nullptr : rt.take_workspace(as_bytes), *w_split = rt.take_workspace(ws_bytes);

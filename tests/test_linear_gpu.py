@@ -215,3 +215,16 @@ def test_linear_bf16_over_its_own_input(kutacc_lib, M):
         x = a.clone()
         api.linear(api.tensor(x), api.tensor(w), b.data_ptr(), api.tensor(x), 0)
         assert torch.equal(x, out)
+
+
+# more columns than a CTA writes, a result that begins in the middle of the activations, the kernels for other sizes, the old result added
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,K,off,beta", [(5000, 256, 0, 0), (5000, 128, 77, 0), (3000, 192, 0, 0), (700, 20, 3, 0), (700, 128, 0, 1), (900, 4, 0, 0)])
+def test_linear_over_its_own_input(kutacc_lib, M, K, off, beta, dtype):
+    g = torch.Generator().manual_seed(M + K + off)
+    a, w, b = (torch.randn(M, K, generator=g)).to(DEV, dtype), (torch.randn(K, K, generator=g) / K ** 0.5).to(DEV, dtype), torch.randn(K, generator=g).to(DEV)
+    store = torch.cat([a, torch.zeros(off + 1, K, device=DEV, dtype=dtype)])
+    want = (a.double() @ w.double().T + b + beta * store[off:M + off].double()).cpu().numpy()
+    api.linear(api.tensor(store[:M]), api.tensor(w), b.data_ptr(), api.tensor(store[off:M + off]), beta)
+    assert helpers.rel_err(store[off:M + off].double().cpu().numpy(), want) <= (2.0 ** -7 if dtype == torch.bfloat16 else 4e-6)
+    assert torch.equal(store[:off], a[:off])

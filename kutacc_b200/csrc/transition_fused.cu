@@ -136,12 +136,14 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     if (warp == 0) {
         // ================= producer =================
         if (elect_one()) {
-            int s = 0, round = 0;                                  // next unit's slot, times the ring has gone round
+            int unit = 0;                                          // asked for so far (a count and its remainder: with a slot and a
+                                                                   // round 51925 rows of 256 channels take 60.4 us, so 59.6)
             bool ok = true;
             int filled = 0;                                        // slabs of the unit that have been asked for
             auto slab = [&](const CUtensorMap *map, int c0, int c1) {
+                const int s = unit % NUNIT;
                 if (filled == 0) {
-                    if (round > 0 && ok) ok = mbar_wait(w_empty(s), (uint32_t)((round - 1) & 1), p.err, 61);
+                    if (unit >= NUNIT && ok) ok = mbar_wait(w_empty(s), (uint32_t)((unit / NUNIT - 1) & 1), p.err, 61);
                     if (!ok) return;
                     mbar_arrive_expect_tx(w_full(s), SPU * SLAB_BYTES);
                 }
@@ -149,10 +151,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
                 tma_load_3d(smem + OFF_RING + (s * SPU + filled) * SLAB_BYTES, map, w_full(s), c0, c1, 0);
                 if (++filled < SPU) return;
                 filled = 0;
-                if (++s == NUNIT) {
-                    s = 0;
-                    ++round;
-                }
+                ++unit;
             };
             auto load_w1 = [&](int j) {
                 for (int k = 0; k < KX; ++k) slab(&tm_w1, k * BK, j * BH);

@@ -43,6 +43,22 @@ def test_running_max_that_grows_late(kutacc_lib):
     assert helpers.rel_err(got, helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
 
 
+@pytest.mark.parametrize("H,large", [(4, 2.0 ** 45), (8, 1e30), (12, 2.0 ** 60)])
+def test_a_large_channel_without_weights_changes_nothing(kutacc_lib, H, large):
+    # its products are zeros; the elements beside it keep all their bits
+    w = W.random_gating_case(seed=83, B=3, S=70, H=H, D=32, dtype="fp32")
+    for name in ("wq", "wk", "wv", "wg"):
+        w.arrays[name] = w.arrays[name].copy()
+        w.arrays[name][:, 5] = 0
+    out = []
+    for v in (0.0, large):
+        w.arrays["x"] = w.arrays["x"].copy()
+        w.arrays["x"][..., 5] = v
+        out.append(runner.out_to_f32(runner.DeviceCase(w).run()))
+    assert np.array_equal(out[0], out[1])
+    assert helpers.rel_err(out[0], helpers.oracle_exact(w)) <= helpers.FP32_TOL / 4
+
+
 @pytest.mark.parametrize("through_nb", [True, False])
 @pytest.mark.parametrize("value", [-np.inf, LOWEST, -3e9])
 def test_other_mask_values(kutacc_lib, value, through_nb):

@@ -14,7 +14,7 @@
 // work, three products at the full rate, but hold elements below 2^-29 of their row's largest in fewer bits and from 2^-51 on not at all.)
 //
 // The activations stand still, as in gemm_proj.cu: a persistent CTA (one per SM) loads 128 rows, all K columns, as fp32; the
-// epilogue warps split them, the first two pieces into tensor memory, where two thirds of the products read them without a byte of
+// epilogue warps split them, the first two pieces into tensor memory, where five of the six products read them without a byte of
 // shared memory, the third where the fp32 values were; and the weights, split by a kernel of their own (a row of them
 // is used by every CTA), stream past in slabs of 128 channels x 64 columns.
 //   warp 0      producer: rows in slabs of 32 fp32 columns, weight slabs (third, second, first pieces of 64 columns, a ring of five or eight)
@@ -23,7 +23,7 @@
 //   warps 4-11  split the rows, a thread half a row; epilogue, 32 rows x 64 columns each: tcgen05.ld of both accumulators, which frees them,
 //               the split of the next block once the last tile of this one is in registers, bias, staging tile (32 x 16), TMA store
 // What bounds it: the tensor cores and the power they take. 32768 rows x 1024 channels x 256 columns: 68 us, 117000 clocks of a CTA (for
-// its 14 tiles of 6144 clocks of products, and 14000 before the first, whose rows come from HBM), at 1.75 GHz under the power limit; with fp16
+// its 14 tiles of 6144 clocks of products; the first, whose rows come from HBM, is done at 14000), at 1.75 GHz under the power limit; with fp16
 // pairs 65. As a split of the activations and tf32 products 20 + 92. x 128 columns 45 us. Error against 64 bits at K = 128 and 256 (2-norm):
 // 1.3e-7 and 2.4e-7 (tf32 3.4e-7 and 6.4e-7, fp16 pairs 2.0e-7 and 3.5e-7). The fp32 layer of 128 x 256 rows: 290 us with tf32, 234 (fp16 pairs 217).
 //

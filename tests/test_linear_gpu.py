@@ -162,7 +162,9 @@ def test_linear_fp32_rows_of_any_magnitude(kutacc_lib, M, N, K):
 # one column 2^spread above the others whose partners are zero, so that only the small ones count
 @pytest.mark.parametrize("spread", [30, 52, 56])
 @pytest.mark.parametrize("M,N,K,way", [(300, 256, 256, "columns"), (3456, 256, 128, "columns"), (3457, 256, 256, "columns"), (300, 128, 128, "activation"), (19201, 256, 256, "activation"),
-                                       (129, 128, 256, "weight"), (20000, 256, 128, "weight"), (300, 128, 512, "columns")])
+                                       (129, 128, 256, "weight"), (20000, 256, 128, "weight"), (300, 128, 512, "columns"),
+                                       # runs of three of a block's eight column tiles: some begin in one block and end in the next
+                                       (24001, 1024, 256, "columns"), (24001, 1024, 128, "weight")])
 def test_linear_fp32_elements_of_any_magnitude_in_a_row(kutacc_lib, M, N, K, way, spread):
     g = torch.Generator().manual_seed(M + N + K + spread)
     a, w = torch.randn(M, K, generator=g).to(DEV), (torch.randn(N, K, generator=g) / K ** 0.5).to(DEV)
